@@ -43,7 +43,7 @@ InferenceState *inference_state_create_gemma3(llmb200_gemma3_model *model, int m
  * Replaces inference_state_free (src/nn/fast_inference.c:344-370). */
 void inference_state_free(InferenceState *state);
 
-/* One greedy request: token-by-token prefill of the prompt, first output token
+/* One greedy request: prefill of the prompt (in passes over the weights where that is possible), first output token
  * = argmax of the last prompt position, then one forward per further token
  * until max_gen_len tokens, an EOS token or the end of the KV cache. Returns
  * the number of tokens written to output_tokens (>= 1).
@@ -172,8 +172,8 @@ size_t llmb200_state_export_weight(InferenceState *state, int layer, int which, 
  * counterpart in the reference, whose loaders fill the structures that inference_state_create takes. */
 InferenceState *inference_state_create_from_dir(const char *dir, int max_seq_len, int wtype);
 /* Feeds n tokens at the current position and advances it by n; logits of the places want[0..n_want), ascending
- * indexes among the n tokens, are written to logits [n_want][vocab]. Works on every state: model types with a
- * row path run a portion of several tokens in one pass over the weights, the others token by token. Returns 0,
+ * indexes among the n tokens, are written to logits [n_want][vocab]. Works on every state: a portion of several
+ * tokens (Qwen3 / Gemma3: 24 and more) runs in one pass over the weights, otherwise token by token. Returns 0,
  * or a negative code with the position unchanged or, after a device error, undefined. */
 int inference_forward_tokens(InferenceState *state, const uint32_t *tokens, int n, const int *want, int n_want,
                              float *logits);

@@ -560,6 +560,61 @@ int b200_lora_decode(const float *x, const float *A_q, const float *B_q, const f
 int b200_argmax_rows(const float *logits, int n_rows, int vocab, unsigned *next_tokens, unsigned *history,
                      int max_steps, int *ctl, unsigned *done_count, void *stream);
 
+/* ------------------------------------------------------------------------
+ * Rows of activations through the matrices of the per-token path: prompts of Qwen3 / Gemma3 states, and
+ * sequences that advance together. */
+
+/* A product operand: `planes` binary16 planes of rows `ld` halves apart, plane p of row m at
+ * d_x + (p * plane_rows + m) * ld. With d_scale the planes hold the row times a power of two (two planes: 22 bits
+ * of every element) and d_scale[m] is its inverse; one plane without d_scale is the row rounded to binary16. */
+typedef struct {
+    void *d_x; long long ld;
+    int planes, plane_rows;
+    float *d_scale;
+} b200_row_planes;
+
+/* out[m][r] = (x_m . w_r) (+ resid[m][r]) for n rows of x and a packed Q8_0 or F16 matrix (rows x cols), fp32. */
+typedef struct {
+    int wtype;                            /* B200_WT_Q8, B200_WT_F16 */
+    const void *d_w; long long w_stride;  /* packed rows, bytes apart */
+    int rows, cols;                       /* cols: a multiple of 32 (Q8_0) or 8 */
+    const float *d_w_scale;               /* Q8_0: b200_q8_row_scale of the matrix */
+    const void *d_x; long long x_ld;      /* planes as in b200_row_planes */
+    int planes, plane_rows;
+    const float *d_x_scale;               /* [n], or NULL */
+    int n;
+    float *d_out; long long out_ld;
+    const float *d_resid; long long resid_ld;
+    unsigned *d_err;
+    int use_pdl;
+} b200_rows_matmul_args;
+int b200_rows_matmul(const b200_rows_matmul_args *a, void *stream);
+/* Per row of a packed Q8_0 matrix: the power of two that brings the row's largest block scale into [2^7, 2^8). */
+int b200_q8_row_scale(const void *d_w, long long stride, int rows, int cols, float *d_out, void *stream);
+
+/* x [rows][dim] += y (RMS-normed with post_gamma first, if given; y NULL: nothing); out = planes of rms_norm(x) * gamma.
+ * index: out's row m is made from row index[m] of x (y NULL). */
+int b200_rows_norm_planes(float *x, int rows, int dim, const float *y, const float *post_gamma, const float *gamma,
+                          const int *index, float eps, const b200_row_planes *out, void *stream);
+/* out = planes of act(gate) * up for rows of 2 * inter values: (gate, up) pairs, or all gates and then all ups. */
+int b200_rows_glu_planes(const float *gu, int rows, int inter, int pairs, int gelu, const b200_row_planes *out, void *stream);
+int b200_rows_split_planes(const float *x, int rows, int dim, const b200_row_planes *out, void *stream);
+
+/* Attention of n_rows / seq_len sequences' new tokens, positions pos0 .. pos0 + seq_len - 1, over their binary16 caches:
+ * per-head norms, rotation, cache rows, then the sums; fp32 accuracy. */
+typedef struct {
+    int n_q, n_kv, hd, max_seq;           /* hd 64, 128 or 256 */
+    int n_rows, seq_len, pos0;
+    float eps;
+    const float *d_qkv;                   /* [n_rows][n_q + 2 n_kv][hd] */
+    const float *d_q_gamma, *d_k_gamma, *d_inv_freq;
+    void *d_k_cache, *d_v_cache;          /* [n_kv][max_seq][hd] per sequence */
+    long long cache_seq_stride;           /* elements between sequences */
+    void *d_q; float *d_q_scale;          /* scratch: 2 x [n_rows][n_q][hd] halves, [n_rows][n_q] */
+    float *d_out;                         /* [n_rows][n_q][hd] */
+} b200_rows_attn_args;
+int b200_rows_attn(const b200_rows_attn_args *a, void *stream);
+
 /* Number of kernel launches issued through this ABI since the last reset
  * (what bench.py reports as gpu_launches). */
 unsigned long long b200_launch_count(int reset);

@@ -174,6 +174,26 @@ class GqaArgs(C.Structure):
                [("proj_ld", C.c_longlong), ("d_q_rows", C.c_void_p), ("d_out_rows", C.c_void_p), ("out_ld", C.c_longlong)]
 
 
+class RowPlanes(C.Structure):
+    """b200_row_planes (include/llmb200_kernels.h)."""
+    _fields_ = [("d_x", C.c_void_p), ("ld", C.c_longlong), ("planes", C.c_int), ("plane_rows", C.c_int), ("d_scale", C.c_void_p)]
+
+
+class RowsMatmulArgs(C.Structure):
+    """b200_rows_matmul_args (include/llmb200_kernels.h)."""
+    _fields_ = [("wtype", C.c_int), ("d_w", C.c_void_p), ("w_stride", C.c_longlong), ("rows", C.c_int), ("cols", C.c_int),
+                ("d_w_scale", C.c_void_p), ("d_x", C.c_void_p), ("x_ld", C.c_longlong), ("planes", C.c_int), ("plane_rows", C.c_int),
+                ("d_x_scale", C.c_void_p), ("n", C.c_int), ("d_out", C.c_void_p), ("out_ld", C.c_longlong),
+                ("d_resid", C.c_void_p), ("resid_ld", C.c_longlong), ("d_err", C.c_void_p), ("use_pdl", C.c_int)]
+
+
+class RowsAttnArgs(C.Structure):
+    """b200_rows_attn_args (include/llmb200_kernels.h)."""
+    _fields_ = [(n, C.c_int) for n in ("n_q", "n_kv", "hd", "max_seq", "n_rows", "seq_len", "pos0")] + [("eps", C.c_float)] + \
+               [(n, C.c_void_p) for n in ("d_qkv", "d_q_gamma", "d_k_gamma", "d_inv_freq", "d_k_cache", "d_v_cache")] + \
+               [("cache_seq_stride", C.c_longlong), ("d_q", C.c_void_p), ("d_q_scale", C.c_void_p), ("d_out", C.c_void_p)]
+
+
 class GlaArgs(C.Structure):
     """b200_gla_args (include/llmb200_kernels.h)."""
     _fields_ = [(n, C.c_int) for n in ("wtype", "heads", "dim", "vdim", "rank", "n_slots")] + \
@@ -238,7 +258,8 @@ SYMBOLS_MAIN = {
                           "b200_latent_splits", "b200_latent_decode", "b200_latent_rows_prep", "b200_latent_rows_attend", "b200_rows_embed",
                           "b200_rows_postnorm", "b200_rows_norm", "b200_rows_gelu_mul", "b200_rows_softcap",
                           "b200_gqa_splits", "b200_gqa_decode", "b200_gqa_rows_prep", "b200_gqa_rows_attend", "b200_gla_decode", "b200_gla_rows",
-                          "b200_rows_streams", "b200_rows_start", "b200_rows_layer_norm"],
+                          "b200_rows_streams", "b200_rows_start", "b200_rows_layer_norm", "b200_rows_matmul", "b200_q8_row_scale",
+                          "b200_rows_norm_planes", "b200_rows_glu_planes", "b200_rows_split_planes", "b200_rows_attn"],
     "llmb200_inference.h": ["inference_state_create", "inference_state_create_gemma3", "inference_state_free",
                             "inference_generate", "inference_state_model_type", "inference_state_vocab_size",
                             "inference_state_reset", "inference_forward_token", "inference_state_load_eos",
@@ -357,6 +378,11 @@ def lib():
         "b200_rows_embed": (i, [vp, vp, i, i, i, fl, vp, vp, vp]), "b200_rows_postnorm": (i, [C.POINTER(RowsPostnormArgs), vp]),
         "b200_rows_norm": (i, [vp, vp, i, i, i, i, fl, vp, i, vp, vp]), "b200_rows_gelu_mul": (i, [vp, ll, i, i, i, vp, vp]),
         "b200_rows_softcap": (i, [vp, i, i, ll, fl, vp]),
+        "b200_rows_matmul": (i, [C.POINTER(RowsMatmulArgs), vp]), "b200_q8_row_scale": (i, [vp, ll, i, i, vp, vp]),
+        "b200_rows_norm_planes": (i, [vp, i, i, vp, vp, vp, vp, fl, C.POINTER(RowPlanes), vp]),
+        "b200_rows_glu_planes": (i, [vp, i, i, i, i, C.POINTER(RowPlanes), vp]),
+        "b200_rows_split_planes": (i, [vp, i, i, C.POINTER(RowPlanes), vp]),
+        "b200_rows_attn": (i, [C.POINTER(RowsAttnArgs), vp]),
         "b200_gqa_splits": (i, [i, i, i, i, i, i]), "b200_gqa_decode": (i, [C.POINTER(GqaArgs), vp]),
         "b200_gqa_rows_prep": (i, [C.POINTER(GqaArgs), vp]), "b200_gqa_rows_attend": (i, [C.POINTER(GqaArgs), vp]),
         "b200_gla_decode": (i, [C.POINTER(GlaArgs), vp]), "b200_gla_rows": (i, [C.POINTER(GlaArgs), vp]),

@@ -28,6 +28,8 @@
  * of the next.
  */
 #include "engine.h"
+#include "plain_rows.h"
+#include "../../include/llmb200_train_kernels.h"
 
 #include <math.h>
 #include <pthread.h>
@@ -38,7 +40,11 @@
 
 static int enqueue_token(InferenceState *s, int with_lm, int pdl);
 /* Qwen3 and Gemma3: one token at a time, prompts included (as the reference's engine) */
-static const ModelOps per_token_ops = { .enqueue_token = enqueue_token, .whole_token = 1 };
+static int prompt_rows(InferenceState *s, const uint32_t *tokens, int n, const int *want, int n_want, float *logits);
+static int prompt_rows_fit(const InferenceState *s, int n, int least);
+static void prompt_free(InferenceState *s);
+static const ModelOps per_token_ops = { .enqueue_token = enqueue_token, .forward_rows = prompt_rows, .rows_fit = prompt_rows_fit,
+                                        .free_model = prompt_free, .whole_token = 1 };
 
 /* per host thread: the ranks of a single-process group are threads */
 static __thread int g_tp_rank = -1, g_tp_size = -1;
@@ -231,6 +237,7 @@ int llmb200_state_load_layer(InferenceState *s, int li, const LayerWeightRef *r,
         fprintf(stderr, "[FastGen] layer %d: weight shapes do not match the configuration\n", li);
         return B200_E_BADARG;
     }
+    prompt_free(s);                      /* what it keeps about the weights */
     Layer *ly = &s->layers[li];
     const int wt = s->wtype;
     const int ql = s->Hq_l * hd, kl = s->Hkv_l * hd, il = s->IS_l;
@@ -284,6 +291,7 @@ int llmb200_state_finish(InferenceState *s, const float *lm_head, const float *f
     if (!s || !lm_head || !final_norm_gamma || !token_emb) return B200_E_BADARG;
     for (int i = 0; i < s->L; ++i)
         if (!s->layers[i].loaded) { fprintf(stderr, "[FastGen] layer %d was never loaded\n", i); return B200_E_STATE; }
+    prompt_free(s);
     int rc = llmb200_upload_packed(s->wtype, lm_head + (size_t)s->tp_rank * s->V_l * s->D, s->D, s->V_l, 0, s->D,
                                    s->lm.w, s->lm.stride, 0, 1);
     if (rc) return rc;
@@ -1048,6 +1056,133 @@ static const float *forward_token_one(InferenceState *s, int token)
     return s->h_logits;
 }
 
+/* ------------------------------------------------------------ prompts in passes over the weights */
+
+enum { PROMPT_CHUNK = 2048, PROMPT_WANT = 64 };
+
+/* What the row path of a Qwen3 / Gemma3 state keeps (InferenceState.model). */
+typedef struct {
+    PlainRows rows;
+    RowsLayer *layers;
+    RowsMatrix lm;
+    float *scales;               /* Q8_0: the row scales of all matrices, layer after layer, then the LM head's */
+    float *logits;               /* [PROMPT_WANT][V] */
+    int *d_want;
+} Prompt;
+
+static void prompt_free(InferenceState *s)
+{
+    Prompt *m = s->model;
+    if (!m) return;
+    if (g_rt.refs > 0) cudaStreamSynchronize(g_rt.stream);
+    llmb200_plain_rows_free(&m->rows);
+    free(m->layers);
+    cudaFree(m->scales); cudaFree(m->logits); cudaFree(m->d_want);
+    free(m);
+    s->model = NULL;
+}
+
+static int prompt_matrix(const InferenceState *s, const PackedMat *w, float **scale, RowsMatrix *out)
+{
+    out->w = w->w; out->stride = w->stride; out->rows = w->rows; out->cols = w->cols; out->scale = NULL;
+    if (s->wtype != B200_WT_Q8) return 0;
+    out->scale = *scale;
+    K_TRY(b200_q8_row_scale(w->w, w->stride, w->rows, w->cols, *scale, g_rt.stream), return -1);
+    *scale += w->rows;
+    return 0;
+}
+
+/* Row scales and a workspace for passes of at least n rows (at most PROMPT_CHUNK). */
+static int prompt_ready(InferenceState *s, int n)
+{
+    Prompt *m = s->model;
+    if (!m) {
+        m = s->model = calloc(1, sizeof(*m));
+        if (!m) return -1;
+        PlainRows *r = &m->rows;
+        r->D = s->D; r->Hq = s->Hq; r->Hkv = s->Hkv; r->hd = s->hd; r->IS = s->IS;
+        r->gemma = s->mt == MODEL_GEMMA3; r->pairs = 1; r->wtype = s->wtype; r->planes = 2; r->max_seq = s->max_seq;
+        r->d_err = (unsigned *)s->d_err;
+        m->layers = calloc((size_t)s->L, sizeof(RowsLayer));
+        m->logits = llmb200_dev_zero((size_t)PROMPT_WANT * s->V * 4);
+        m->d_want = (int *)llmb200_dev_zero(PROMPT_WANT * 4);
+        size_t rows = (size_t)s->lm.rows;
+        for (int l = 0; l < s->L; ++l) {
+            const Layer *y = &s->layers[l];
+            rows += (size_t)y->qkv.rows + y->o.rows + y->gateup.rows + y->down.rows;
+        }
+        m->scales = s->wtype == B200_WT_Q8 ? llmb200_dev_zero(rows * 4) : NULL;
+        float *scale = m->scales;
+        int rc = !m->layers || !m->logits || !m->d_want || (s->wtype == B200_WT_Q8 && !scale) ? -1 : 0;
+        for (int l = 0; l < s->L && rc == 0; ++l) {
+            const Layer *y = &s->layers[l];
+            RowsLayer *o = &m->layers[l];
+            rc |= prompt_matrix(s, &y->qkv, &scale, &o->qkv);
+            rc |= prompt_matrix(s, &y->o, &scale, &o->o);
+            rc |= prompt_matrix(s, &y->gateup, &scale, &o->gateup);
+            rc |= prompt_matrix(s, &y->down, &scale, &o->down);
+            o->g_input = y->g_input; o->g_post_attn = y->g_post_attn; o->g_pre_ff = y->g_pre_ff; o->g_post_ff = y->g_post_ff;
+            o->g_qn = y->g_qn; o->g_kn = y->g_kn; o->inv_freq = y->inv_freq;
+            o->k_cache = y->k_cache; o->v_cache = y->v_cache;
+        }
+        if (rc == 0) rc = prompt_matrix(s, &s->lm, &scale, &m->lm);
+        if (rc) { prompt_free(s); return -1; }
+    }
+    int cap = 64;                        /* at least the wanted rows of a pass */
+    while (cap < n) cap *= 2;
+    if (cap > m->rows.cap) {
+        CU_TRY(cudaStreamSynchronize(g_rt.stream), return -1);
+        llmb200_plain_rows_free(&m->rows);
+        m->rows.cap = cap;
+        if (llmb200_plain_rows_ready(&m->rows) != 0) { m->rows.cap = 0; return -1; }
+    }
+    return 0;
+}
+
+/* Fewest tokens of a pass, and fewest of a portion of inference_forward_tokens: shorter portions of a Qwen3 / Gemma3 state go through
+ * the per-token path and so keep its very bits (a pass adds in another order). Below four tokens the launches of a pass (ten a
+ * layer, 3 us each) cost more than the tokens. */
+enum { PROMPT_MIN = 4, PORTION_MIN = 24 };
+
+/* An attached adapter and tensor parallelism run on the per-token path. */
+static int prompt_rows_fit(const InferenceState *s, int n, int least)
+{
+    return n >= least && !s->lora && s->tp_size == 1 && s->Hq * s->hd % 8 == 0 && (size_t)s->IS * 4 <= 227 * 1024 && (size_t)s->D * 4 <= 227 * 1024;
+}
+
+static int prompt_rows(InferenceState *s, const uint32_t *tokens, int n, const int *want, int n_want, float *logits)
+{
+    if (prompt_ready(s, n < PROMPT_CHUNK ? n : PROMPT_CHUNK) != 0) return -1;
+    Prompt *m = s->model;
+    PlainRows *r = &m->rows;
+    int w = 0;
+    for (int c0 = 0; c0 < n; c0 += PROMPT_CHUNK) {
+        const int M = n - c0 < PROMPT_CHUNK ? n - c0 : PROMPT_CHUNK, pos0 = s->cur_len + c0;
+        if (llmb200_set_control(s, pos0, s->max_seq + 2, tokens + c0, pos0, M) != 0) return -1;
+        K_TRY(b200_embed_rows(s->emb, (const uint32_t *)(s->d_tokens + pos0), M, s->D, s->V, s->emb_scale, r->x, g_rt.stream), return -1);
+        int last = w;
+        while (last < n_want && want[last] < c0 + M) ++last;
+        if (llmb200_plain_rows_run(r, m->layers, s->L, M, M, pos0, 0, last == w) != 0) return -1;
+        for (int first = 1; w < last; first = 0) {
+            int index[PROMPT_WANT], k = 0;
+            for (; k < PROMPT_WANT && w + k < last; ++k) index[k] = want[w + k] - c0;
+            CU_TRY(cudaMemcpyAsync(m->d_want, index, (size_t)k * 4, cudaMemcpyHostToDevice, g_rt.stream), return -1);
+            if (llmb200_plain_rows_last(r, &m->layers[s->L - 1], s->g_final, m->d_want, k, first ? M : 0) != 0) return -1;
+            if (llmb200_plain_rows_product(r, &m->lm, k, m->logits) != 0) return -1;
+            CU_TRY(cudaMemcpyAsync(logits + (size_t)w * s->V, m->logits, (size_t)k * s->V * 4, cudaMemcpyDeviceToHost, g_rt.stream), return -1);
+            CU_TRY(cudaStreamSynchronize(g_rt.stream), return -1);
+            w += k;
+        }
+    }
+    CU_TRY(cudaStreamSynchronize(g_rt.stream), return -1);
+    return 0;
+}
+
+static int rows_fit(const InferenceState *s, int n, int least)
+{
+    return n > 1 && s->ops->forward_rows && (!s->ops->rows_fit || s->ops->rows_fit(s, n, least));
+}
+
 /* One token through the per-token graph; logits == NULL: none are asked for. */
 static int step_one(InferenceState *s, uint32_t token, float *logits)
 {
@@ -1082,7 +1217,7 @@ int inference_forward_tokens(InferenceState *s, const uint32_t *tokens, int n, c
     }
     follow_sft(s);
     if (ensure_graphs(s) != 0) return -1;
-    if (s->ops->forward_rows && n > 1) {
+    if (rows_fit(s, n, PORTION_MIN)) {
         rc = s->ops->forward_rows(s, tokens, n, want, n_want, logits);
         if (rc == 0) s->cur_len += n;
     } else {
@@ -1119,7 +1254,7 @@ static int generate_one(InferenceState *s, const uint32_t *prompt, int prompt_le
 
     fprintf(stderr, "[FastGen] Prefilling %d tokens...\n", P);
     double t0 = now_ms();
-    if (s->ops->forward_rows && P > 2) {         /* all but the last prompt token in one pass; the last one yields the first id */
+    if (P > 2 && rows_fit(s, P - 1, PROMPT_MIN)) { /* all but the last prompt token in one pass; the last one yields the first id */
         if (s->ops->forward_rows(s, prompt, P - 1, NULL, 0, NULL) != 0) return 0;
         if (llmb200_set_control(s, P - 1, P, prompt, 0, P) != 0) return 0;
     } else {

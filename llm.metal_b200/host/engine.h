@@ -35,6 +35,9 @@ typedef struct {
      * behind them; logits of the tokens want[0..n_want) (ascending places among the n) go to `logits`
      * [n_want][V]. NULL: the model type only has the per-token path. */
     int (*forward_rows)(InferenceState *s, const uint32_t *tokens, int n, const int *want, int n_want, float *logits);
+    /* Whether forward_rows is the way for n tokens, at least `least` where the type has a minimum, in the state's present
+     * configuration (NULL: always). */
+    int (*rows_fit)(const InferenceState *s, int n, int least);
     void (*free_model)(InferenceState *s);
     int whole_token;             /* the whole-token kernel can run this model type */
 } ModelOps;

@@ -1,0 +1,103 @@
+/* Prompts of the Qwen3 / Gemma3 block in passes over the weights (see plain_rows.h).
+ *
+ * Token by token a prompt costs one read of all weights per token; here a pass of up to `cap` tokens reads them once, and the
+ * products run on the tensor cores at the precision of the per-token kernels (b200_rows_matmul). Ten launches a layer:
+ * norm, q/k/v product, heads and cache rows, attention, operand planes, o product, norm, gate/up product, activation, down product. */
+#include "plain_rows.h"
+#include "../../include/llmb200_train_kernels.h"
+
+#include <string.h>
+
+static const float RMS_EPS = 1e-6f;            /* hard-wired in the reference: src/nn/fast_inference.c:383 */
+
+static void *device(size_t bytes)
+{
+    void *p = NULL;
+    CU_TRY(cudaMalloc(&p, bytes), return NULL);
+    return p;
+}
+
+int llmb200_plain_rows_ready(PlainRows *r)
+{
+    const size_t n = (size_t)r->cap, heads = (size_t)r->Hq * r->hd;
+    size_t widest = (size_t)(r->IS > r->D ? r->IS : r->D);
+    if (heads > widest) widest = heads;
+    r->x = device(n * r->D * 4); r->y = device(n * r->D * 4);
+    r->qkv = device(n * (heads + 2 * (size_t)r->Hkv * r->hd) * 4);
+    r->attn = device(n * heads * 4);
+    r->gu = device(n * 2 * r->IS * 4);
+    r->x_scale = device(n * 4); r->q_scale = device(n * r->Hq * 4);
+    r->xh = device(n * widest * 2 * r->planes);
+    r->q = device(n * heads * 2 * 2);
+    if (!r->x || !r->y || !r->qkv || !r->attn || !r->gu || !r->x_scale || !r->q_scale || !r->xh || !r->q) { llmb200_plain_rows_free(r); return -1; }
+    return 0;
+}
+
+void llmb200_plain_rows_free(PlainRows *r)
+{
+    void *b[] = { r->x, r->y, r->qkv, r->attn, r->gu, r->x_scale, r->q_scale, r->xh, r->q };
+    for (size_t i = 0; i < sizeof(b) / sizeof(b[0]); ++i) cudaFree(b[i]);
+    r->x = r->y = r->qkv = r->attn = r->gu = r->x_scale = r->q_scale = NULL;
+    r->xh = r->q = NULL;
+}
+
+static b200_row_planes planes_of(const PlainRows *r, int width)
+{
+    b200_row_planes p = { r->xh, width, r->planes, r->cap, r->planes == 2 ? r->x_scale : NULL };
+    return p;
+}
+
+int llmb200_plain_rows_product(PlainRows *r, const RowsMatrix *m, int n, float *out)
+{
+    b200_rows_matmul_args a;
+    memset(&a, 0, sizeof(a));
+    a.wtype = r->wtype;
+    a.d_w = m->w; a.w_stride = m->stride; a.rows = m->rows; a.cols = m->cols; a.d_w_scale = m->scale;
+    a.d_x = r->xh; a.x_ld = m->cols; a.planes = r->planes; a.plane_rows = r->cap;
+    a.d_x_scale = r->planes == 2 ? r->x_scale : NULL;
+    a.n = n;
+    a.d_out = out; a.out_ld = m->rows;
+    a.d_err = r->d_err;
+    K_TRY(b200_rows_matmul(&a, g_rt.stream), return -1);
+    return 0;
+}
+
+int llmb200_plain_rows_run(PlainRows *r, const RowsLayer *layers, int n_layers, int n_rows, int seq_len, int pos0, long long cache_seq_stride,
+                           int caches_only)
+{
+    void *st = g_rt.stream;
+    const int heads = r->Hq * r->hd;
+    const b200_row_planes p_model = planes_of(r, r->D), p_heads = planes_of(r, heads), p_inter = planes_of(r, r->IS);
+    for (int l = 0; l < n_layers; ++l) {
+        const RowsLayer *y = &layers[l];
+        const float *post = l && r->gemma ? layers[l - 1].g_post_ff : NULL;
+        K_TRY(b200_rows_norm_planes(r->x, n_rows, r->D, l ? r->y : NULL, post, y->g_input, NULL, RMS_EPS, &p_model, st), return -1);
+        if (llmb200_plain_rows_product(r, &y->qkv, n_rows, r->qkv)) return -1;
+        b200_rows_attn_args a;
+        memset(&a, 0, sizeof(a));
+        a.n_q = r->Hq; a.n_kv = r->Hkv; a.hd = r->hd; a.max_seq = r->max_seq;
+        a.n_rows = n_rows; a.seq_len = seq_len; a.pos0 = pos0; a.eps = RMS_EPS;
+        a.d_qkv = r->qkv; a.d_q_gamma = y->g_qn; a.d_k_gamma = y->g_kn; a.d_inv_freq = y->inv_freq;
+        a.d_k_cache = y->k_cache; a.d_v_cache = y->v_cache; a.cache_seq_stride = cache_seq_stride;
+        a.d_q = r->q; a.d_q_scale = r->q_scale; a.d_out = r->attn;
+        K_TRY(b200_rows_attn(&a, st), return -1);
+        if (caches_only && l == n_layers - 1) return 0;          /* nothing reads what the last layer adds */
+        K_TRY(b200_rows_split_planes(r->attn, n_rows, heads, &p_heads, st), return -1);
+        if (llmb200_plain_rows_product(r, &y->o, n_rows, r->y)) return -1;
+        K_TRY(b200_rows_norm_planes(r->x, n_rows, r->D, r->y, r->gemma ? y->g_post_attn : NULL, r->gemma ? y->g_pre_ff : y->g_post_attn,
+                                    NULL, RMS_EPS, &p_model, st), return -1);
+        if (llmb200_plain_rows_product(r, &y->gateup, n_rows, r->gu)) return -1;
+        K_TRY(b200_rows_glu_planes(r->gu, n_rows, r->IS, r->pairs, r->gemma, &p_inter, st), return -1);
+        if (llmb200_plain_rows_product(r, &y->down, n_rows, r->y)) return -1;
+    }
+    return 0;
+}
+
+int llmb200_plain_rows_last(PlainRows *r, const RowsLayer *last_layer, const float *g_final, const int *index, int n, int n_rows)
+{
+    const b200_row_planes p = planes_of(r, r->D);
+    /* first call of a pass: the stream takes the last feed-forward's result in; its planes are not used */
+    if (n_rows > 0) K_TRY(b200_rows_norm_planes(r->x, n_rows, r->D, r->y, r->gemma ? last_layer->g_post_ff : NULL, g_final, NULL, RMS_EPS, &p, g_rt.stream), return -1);
+    K_TRY(b200_rows_norm_planes(r->x, n, r->D, NULL, NULL, g_final, index, RMS_EPS, &p, g_rt.stream), return -1);
+    return 0;
+}

@@ -1,0 +1,36 @@
+/* Prompts of the Qwen3 / Gemma3 block in passes over the weights (internal): shared by the single-sequence states
+ * and the batched engine. */
+#ifndef LLMB200_PLAIN_ROWS_H
+#define LLMB200_PLAIN_ROWS_H
+
+#include "internal.h"
+
+typedef struct { const void *w; long long stride; int rows, cols; const float *scale; } RowsMatrix;   /* scale: Q8_0 only */
+
+typedef struct {
+    RowsMatrix qkv, o, gateup, down;
+    const float *g_input, *g_post_attn, *g_pre_ff, *g_post_ff, *g_qn, *g_kn, *inv_freq;
+    void *k_cache, *v_cache;
+} RowsLayer;
+
+/* Workspace of a pass of up to `cap` rows. planes: 2 where the per-token kernels take fp32 inputs, 1 where they take
+ * binary16 ones. */
+typedef struct {
+    int D, Hq, Hkv, hd, IS, gemma, pairs, wtype, planes, cap, max_seq;
+    unsigned *d_err;
+    float *x, *y, *qkv, *attn, *gu, *x_scale, *q_scale;
+    void *xh, *q;
+} PlainRows;
+
+/* Allocates the workspace; the sizes above d_err must be set. 0, or -1 with everything given back. */
+int llmb200_plain_rows_ready(PlainRows *r);
+void llmb200_plain_rows_free(PlainRows *r);
+/* Runs n_rows / seq_len sequences' tokens (positions pos0 on) through the layers; r->x holds the embedded rows on entry and the
+ * residual stream afterwards, its last feed-forward result still in r->y (last_norm adds it). */
+int llmb200_plain_rows_run(PlainRows *r, const RowsLayer *layers, int n_layers, int n_rows, int seq_len, int pos0, long long cache_seq_stride,
+                           int caches_only);
+/* The products' operand: planes of the final norm of rows index[0..n) (device; ascending) of the stream -> r->xh. */
+int llmb200_plain_rows_last(PlainRows *r, const RowsLayer *last_layer, const float *g_final, const int *index, int n, int n_rows);
+int llmb200_plain_rows_product(PlainRows *r, const RowsMatrix *m, int n, float *out);
+
+#endif
