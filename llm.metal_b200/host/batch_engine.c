@@ -5,13 +5,14 @@
  * Stands in for BatchState / forward_token_batch / qwen3_generate_fast_batch
  * (src/nn/fast_inference.c:696-985). The reference keeps the matvec shape and loops the batch inside
  * the kernel (f16_batch_matvec, shaders/q8_kernels.metal:49-90); with B rows the projections are small
- * matrix products, so here they run on the tensor cores (b200_gemm_f16: binary16 weights, a binary16
- * copy of the B activation rows, fp32 accumulate), the row-wise steps use the training kernels over
- * B rows, and attention is the decode kernel with the batch as a third grid dimension over per-sequence
- * F16 KV caches. The arg-max, the token feedback and the position live on the device: one step is one
+ * matrix products, so here they run on the tensor cores (b200_rows_matmul: the weights as the 128-row side of
+ * the tile, a binary16 copy of the B activation rows as its columns, fp32 accumulate), and attention is the
+ * decode kernel with the batch as a third grid dimension over per-sequence F16 KV caches. Prompts go through
+ * in passes over the weights (plain_rows.h). The arg-max, the token feedback and the position live on the device: one step is one
  * CUDA graph.
  */
 #include "internal.h"
+#include "plain_rows.h"
 #include "../../include/llmb200_inference.h"
 #include "../../include/llmb200_train_kernels.h"
 
@@ -32,7 +33,7 @@ struct llmb200_batch_state {
     BLayer *layers;
     void *lm_head;
     float *g_final, *emb;
-    float *x[2], *ln, *qkv, *att, *gu, *logits, *scratch;
+    float *x, *y, *qkv, *att, *gu, *logits, *scratch;
     void *xh;
     unsigned *tickets, *d_tok, *d_hist, *d_done;
     int *d_ctl;
@@ -45,6 +46,8 @@ struct llmb200_batch_state {
     double last_decode_ms;
     int last_steps;
     int kernels_per_step;
+    PlainRows rows;                       /* prompt passes: allocated with the first prompt, kept */
+    uint32_t *d_prompt;
 };
 typedef struct llmb200_batch_state BState;
 
@@ -79,8 +82,9 @@ void llmb200_batch_free(BState *s)
         void *b[] = { y->qkv, y->o, y->gu, y->down, y->g_in, y->g_post, y->g_q, y->g_k, y->inv_freq, y->k_cache, y->v_cache };
         for (size_t i = 0; i < sizeof(b) / sizeof(b[0]); ++i) cudaFree(b[i]);
     }
-    void *b[] = { s->lm_head, s->g_final, s->emb, s->x[0], s->x[1], s->ln, s->qkv, s->att, s->gu, s->logits, s->scratch,
-                  s->xh, s->tickets, s->d_tok, s->d_hist, s->d_done, s->d_ctl };
+    void *b[] = { s->lm_head, s->g_final, s->emb, s->x, s->y, s->qkv, s->att, s->gu, s->logits, s->scratch,
+                  s->xh, s->tickets, s->d_tok, s->d_hist, s->d_done, s->d_ctl, s->d_prompt };
+    llmb200_plain_rows_free(&s->rows);
     for (size_t i = 0; i < sizeof(b) / sizeof(b[0]); ++i) cudaFree(b[i]);
     if (s->h_tok) cudaFreeHost(s->h_tok);
     if (s->h_ctl) cudaFreeHost(s->h_ctl);
@@ -129,7 +133,7 @@ BState *llmb200_batch_begin(const llmb200_config *c, int batch_size, int max_gen
     }
     s->lm_head = dmalloc(s, (size_t)s->V * D * 2);
     s->g_final = dmalloc(s, D * 4); s->emb = dmalloc(s, (size_t)s->V * D * 4);
-    s->x[0] = dmalloc(s, B * D * 4); s->x[1] = dmalloc(s, B * D * 4); s->ln = dmalloc(s, B * D * 4);
+    s->x = dmalloc(s, B * D * 4); s->y = dmalloc(s, B * D * 4);
     s->qkv = dmalloc(s, B * s->QKV * 4); s->att = dmalloc(s, B * Hq_hd * 4); s->gu = dmalloc(s, B * 2 * s->IS * 4);
     s->logits = dmalloc(s, B * (size_t)s->V * 4);
     size_t widest = (size_t)(2 * s->IS > s->QKV ? 2 * s->IS : s->QKV);
@@ -201,17 +205,24 @@ int llmb200_batch_finish(BState *s, const float *lm_head, const float *final_nor
     return rc;
 }
 
-/* C[B, N] = half(A)[B, K] * Wh[N, K]^T (+ R); A == NULL: the operand is already in xh */
-static void proj(BState *s, const float *A, const void *Wh, int N, int K, float *C, const float *R)
+/* C[B, N] = xh[B, K] * Wh[N, K]^T */
+static void proj(BState *s, const void *Wh, int N, int K, float *C)
 {
-    if (A) B_TRY(s, b200_f32_to_f16(A, (size_t)s->B * K, 1.0f, s->xh, g_rt.stream));
-    b200_gemm_args g;
-    memset(&g, 0, sizeof(g));
-    g.A = (const float *)s->xh; g.a_row = K; g.a_col = 1;
-    g.B = (const float *)Wh; g.b_row = 1; g.b_col = K;
-    g.C = C; g.ldc = N; g.R = R; g.ldr = N;
-    g.M = s->B; g.N = N; g.K = K; g.alpha = 1.0f;
-    B_TRY(s, b200_gemm_f16(&g, g_rt.stream));
+    b200_rows_matmul_args a;
+    memset(&a, 0, sizeof(a));
+    a.wtype = B200_WT_F16;
+    a.d_w = Wh; a.w_stride = (long long)K * 2; a.rows = N; a.cols = K;
+    a.d_x = s->xh; a.x_ld = K; a.planes = 1;
+    a.n = s->B;
+    a.d_out = C; a.out_ld = N;
+    B_TRY(s, b200_rows_matmul(&a, g_rt.stream));
+}
+
+/* the stream takes y in (NULL: nothing); xh = its norm */
+static void norm(BState *s, const float *y, const float *gamma)
+{
+    const b200_row_planes p = { s->xh, s->D, 1, s->B, NULL };
+    B_TRY(s, b200_rows_norm_planes(s->x, s->B, s->D, y, NULL, gamma, NULL, 1e-6f, &p, g_rt.stream));
 }
 
 /* one step for all sequences: tokens from d_tok at position d_ctl[0] */
@@ -219,12 +230,11 @@ static void enqueue_step(BState *s)
 {
     void *st = g_rt.stream;
     const int B = s->B, D = s->D, Hq_hd = s->Hq * s->hd, Hkv_hd = s->Hkv * s->hd;
-    float *x = s->x[0], *x2 = s->x[1];
-    B_TRY(s, b200_embed_rows(s->emb, s->d_tok, B, D, s->V, 1.0f, x, st));
+    B_TRY(s, b200_embed_rows(s->emb, s->d_tok, B, D, s->V, 1.0f, s->x, st));
     for (int l = 0; l < s->L; ++l) {
         BLayer *y = &s->layers[l];
-        B_TRY(s, b200_rms_norm_rows_h(x, y->g_in, s->ln, s->xh, B, D, 1e-6f, st));
-        proj(s, NULL, y->qkv, s->QKV, D, s->qkv, NULL);
+        norm(s, l ? s->y : NULL, y->g_in);
+        proj(s, y->qkv, s->QKV, D, s->qkv);
         b200_attn_args at;
         memset(&at, 0, sizeof(at));
         at.d_qkv = s->qkv; at.d_q_gamma = y->g_q; at.d_k_gamma = y->g_k; at.d_inv_freq = y->inv_freq;
@@ -235,15 +245,63 @@ static void enqueue_step(BState *s)
         at.n_items = B; at.qkv_item_stride = s->QKV; at.out_item_stride = Hq_hd;
         at.cache_item_stride = (long long)Hkv_hd * s->max_seq;
         B_TRY(s, b200_attn_decode(&at, st));
-        proj(s, s->att, y->o, D, Hq_hd, x2, x);                               /* + residual */
-        B_TRY(s, b200_rms_norm_rows_h(x2, y->g_post, s->ln, s->xh, B, D, 1e-6f, st));
-        proj(s, NULL, y->gu, 2 * s->IS, D, s->gu, NULL);
+        B_TRY(s, b200_f32_to_f16(s->att, (size_t)B * Hq_hd, 1.0f, s->xh, st));
+        proj(s, y->o, D, Hq_hd, s->y);
+        norm(s, s->y, y->g_post);
+        proj(s, y->gu, 2 * s->IS, D, s->gu);
         B_TRY(s, b200_silu_mul_rows_h(s->gu, B, s->IS, NULL, s->xh, st));
-        proj(s, NULL, y->down, D, s->IS, x, x2);                              /* + residual */
+        proj(s, y->down, D, s->IS, s->y);
     }
-    B_TRY(s, b200_rms_norm_rows_h(x, s->g_final, s->ln, s->xh, B, D, 1e-6f, st));
-    proj(s, NULL, s->lm_head, s->V, D, s->logits, NULL);
+    norm(s, s->y, s->g_final);
+    proj(s, s->lm_head, s->V, D, s->logits);
     B_TRY(s, b200_argmax_rows(s->logits, B, s->V, s->d_tok, s->d_hist, s->hist_cap, s->d_ctl, s->d_done, st));
+}
+
+/* ------------------------------------------------------------ prompts in passes over the weights */
+
+enum { BATCH_ROWS = 2048 };              /* rows (sequences x positions) of a pass: the products are far from memory-bound there */
+
+static RowsMatrix matrix(const void *w, int rows, int cols)
+{
+    const RowsMatrix m = { w, (long long)cols * 2, rows, cols, NULL };
+    return m;
+}
+
+/* Caches of all sequences' first n tokens; prompts [B][stride]. 0, 1 when the shape is not one of the row path's, -1 on an error. */
+static int prefill_rows(BState *s, const uint32_t *prompts, int stride, int n)
+{
+    const int B = s->B, D = s->D, Hq_hd = s->Hq * s->hd, T0 = BATCH_ROWS / B < n ? BATCH_ROWS / B : n;
+    if ((D | s->IS | Hq_hd) & 7 || (s->hd != 64 && s->hd != 128 && s->hd != 256) || (size_t)s->IS * 4 > 227 * 1024 || (size_t)D * 4 > 227 * 1024) return 1;
+    PlainRows *r = &s->rows;
+    if (r->cap < B * T0) {
+        llmb200_plain_rows_free(r);
+        cudaFree(s->d_prompt); s->d_prompt = NULL;
+        r->D = D; r->Hq = s->Hq; r->Hkv = s->Hkv; r->hd = s->hd; r->IS = s->IS; r->wtype = B200_WT_F16; r->planes = 1; r->max_seq = s->max_seq;
+        r->cap = B * T0;
+        if (llmb200_plain_rows_ready(r) != 0 || cudaMalloc((void **)&s->d_prompt, (size_t)r->cap * 4) != cudaSuccess) { r->cap = 0; return -1; }
+    }
+    RowsLayer *layers = calloc((size_t)s->L, sizeof(RowsLayer));
+    uint32_t *ids = malloc((size_t)B * T0 * 4);
+    int rc = layers && ids ? 0 : -1;
+    for (int l = 0; l < s->L && rc == 0; ++l) {
+        const BLayer *y = &s->layers[l];
+        RowsLayer *o = &layers[l];
+        o->qkv = matrix(y->qkv, s->QKV, D); o->o = matrix(y->o, D, Hq_hd);
+        o->gateup = matrix(y->gu, 2 * s->IS, D); o->down = matrix(y->down, D, s->IS);
+        o->g_input = y->g_in; o->g_post_attn = y->g_post; o->g_qn = y->g_q; o->g_kn = y->g_k; o->inv_freq = y->inv_freq;
+        o->k_cache = y->k_cache; o->v_cache = y->v_cache;
+    }
+    for (int t0 = 0; t0 < n && rc == 0; t0 += T0) {
+        const int T = n - t0 < T0 ? n - t0 : T0;
+        for (int b = 0; b < B; ++b) memcpy(ids + (size_t)b * T, prompts + (size_t)b * stride + t0, (size_t)T * 4);
+        CU_TRY(cudaMemcpyAsync(s->d_prompt, ids, (size_t)B * T * 4, cudaMemcpyHostToDevice, g_rt.stream), rc = -1);
+        if (rc == 0) K_TRY(b200_embed_rows(s->emb, s->d_prompt, B * T, D, s->V, 1.0f, r->x, g_rt.stream), rc = -1);
+        if (rc == 0) rc = llmb200_plain_rows_run(r, layers, s->L, B * T, T, t0, (long long)s->Hkv * s->hd * s->max_seq, 1);
+        if (rc == 0) CU_TRY(cudaStreamSynchronize(g_rt.stream), rc = -1);              /* ids are reused */
+    }
+    free(layers);
+    free(ids);
+    return rc;
 }
 
 static int ensure_graph(BState *s)
@@ -305,10 +363,17 @@ int llmb200_batch_generate(BState *s, const uint32_t *prompts, int prompt_len, u
     struct timespec t0, t1;
     fprintf(stderr, "[BatchGen] Prefilling %d tokens...\n", prompt_len);
     clock_gettime(CLOCK_MONOTONIC, &t0);
-    s->h_ctl[0] = 0; s->h_ctl[1] = 0; s->h_ctl[2] = 0; s->h_ctl[3] = 0;
+    /* all but the last prompt token in passes over the weights; the last one yields the first id */
+    int first = 0;
+    if (prompt_len > 2) {
+        const int rc = prefill_rows(s, prompts, prompt_len, prompt_len - 1);
+        if (rc < 0) return 0;
+        if (rc == 0) first = prompt_len - 1;
+    }
+    s->h_ctl[0] = first; s->h_ctl[1] = 0; s->h_ctl[2] = 0; s->h_ctl[3] = 0;
     CU_TRY(cudaMemcpyAsync(s->d_ctl, s->h_ctl, 16, cudaMemcpyHostToDevice, st), return 0);
     CU_TRY(cudaStreamSynchronize(st), return 0);
-    for (int i = 0; i < prompt_len; ++i) {
+    for (int i = first; i < prompt_len; ++i) {
         for (int b = 0; b < B; ++b) s->h_tok[b] = prompts[(size_t)b * prompt_len + i];
         CU_TRY(cudaMemcpyAsync(s->d_tok, s->h_tok, (size_t)B * 4, cudaMemcpyHostToDevice, st), return 0);
         if (i == prompt_len - 1) {               /* the last prompt position yields the first generated token */
