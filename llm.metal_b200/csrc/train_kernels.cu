@@ -179,163 +179,10 @@ __global__ void qk_norm_rope_bwd_kernel(float *dqkv, const float *qkv, long long
     }
 }
 
-// ---- causal attention, training form: one warp per (sequence, head, query) ---------------------
-// Dynamic shared memory per warp: HD floats (the query or d_out row) + N floats (the score row).
-constexpr int ATT_WARPS = 4;
-
-template <int HD>
-__global__ void __launch_bounds__(ATT_WARPS * 32)
-attn_train_fwd_kernel(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q,
-                      int n_kv, float scale, float *probs, float *out, __half *out_h)
-{
-    extern __shared__ float sh[];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    float *qs = sh + (size_t)w * (HD + N), *sc = qs + HD;
-    const long long unit = (long long)blockIdx.x * ATT_WARPS + w;
-    if (unit >= (long long)n_seq * n_q * N) return;
-    const int i = (int)(unit % N), h = (int)((unit / N) % n_q), s = (int)(unit / ((long long)N * n_q));
-    const int kvh = h / (n_q / n_kv);
-    const size_t row0 = (size_t)s * N;
-    const float *qr = q + ((row0 + i) * n_q + h) * HD;
-    for (int d = l; d < HD; d += 32) qs[d] = qr[d];
-    __syncwarp();
-
-    float mx = -1e30f;
-    for (int j = l; j <= i; j += 32) {
-        const float4 *kr = reinterpret_cast<const float4 *>(k + ((row0 + j) * n_kv + kvh) * HD);
-        float dot = 0.f;
-#pragma unroll 8
-        for (int d4 = 0; d4 < HD / 4; ++d4) {
-            const float4 kk = kr[d4];
-            dot = fmaf(qs[4 * d4], kk.x, dot);
-            dot = fmaf(qs[4 * d4 + 1], kk.y, dot);
-            dot = fmaf(qs[4 * d4 + 2], kk.z, dot);
-            dot = fmaf(qs[4 * d4 + 3], kk.w, dot);
-        }
-        dot *= scale;
-        sc[j] = dot;
-        mx = fmaxf(mx, dot);
-    }
-    mx = warp_max(mx);
-    float sum = 0.f;
-    for (int j = l; j <= i; j += 32) {
-        const float e = expf(sc[j] - mx);
-        sc[j] = e;
-        sum += e;
-    }
-    sum = warp_sum(sum);
-    const float inv = 1.0f / sum;
-    float *pr = probs + (((size_t)s * n_q + h) * N + i) * N;
-    for (int j = l; j < N; j += 32) {
-        const float p = j <= i ? sc[j] * inv : 0.f;
-        if (j <= i) sc[j] = p;
-        pr[j] = p;
-    }
-    __syncwarp();
-    float *o = out + ((row0 + i) * n_q + h) * HD;
-    for (int d = l; d < HD; d += 32) {
-        float acc = 0.f;
-        for (int j = 0; j <= i; ++j) acc = fmaf(sc[j], v[(row0 + j) * v_ld + (size_t)kvh * HD + d], acc);
-        if (out) o[d] = acc;
-        if (out_h) out_h[((row0 + i) * n_q + h) * HD + d] = __float2half_rn(acc);
-    }
-}
-
-template <int HD>
-__global__ void __launch_bounds__(ATT_WARPS * 32)
-attn_bwd_dq_kernel(const float *d_out, const float *probs, const float *k, const float *v, long long v_ld, int n_seq,
-                   int N, int n_q, int n_kv, float scale, float *d_score, float *dqkv, long long ld)
-{
-    extern __shared__ float sh[];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    float *os = sh + (size_t)w * (HD + N), *ds = os + HD;
-    const long long unit = (long long)blockIdx.x * ATT_WARPS + w;
-    if (unit >= (long long)n_seq * n_q * N) return;
-    const int i = (int)(unit % N), h = (int)((unit / N) % n_q), s = (int)(unit / ((long long)N * n_q));
-    const int kvh = h / (n_q / n_kv);
-    const size_t row0 = (size_t)s * N;
-    const float *dor = d_out + ((row0 + i) * n_q + h) * HD;
-    for (int d = l; d < HD; d += 32) os[d] = dor[d];
-    __syncwarp();
-    const float *pr = probs + (((size_t)s * n_q + h) * N + i) * N;
-    float dp = 0.f;
-    for (int j = l; j <= i; j += 32) {
-        const float4 *vr = reinterpret_cast<const float4 *>(v + (row0 + j) * v_ld + (size_t)kvh * HD);
-        float dot = 0.f;
-#pragma unroll 8
-        for (int d4 = 0; d4 < HD / 4; ++d4) {
-            const float4 vv = vr[d4];
-            dot = fmaf(os[4 * d4], vv.x, dot);
-            dot = fmaf(os[4 * d4 + 1], vv.y, dot);
-            dot = fmaf(os[4 * d4 + 2], vv.z, dot);
-            dot = fmaf(os[4 * d4 + 3], vv.w, dot);
-        }
-        ds[j] = dot;
-        dp = fmaf(pr[j], dot, dp);
-    }
-    dp = warp_sum(dp);
-    float *dsr = d_score + (((size_t)s * n_q + h) * N + i) * N;
-    for (int j = l; j < N; j += 32) {
-        const float g = j <= i ? pr[j] * (ds[j] - dp) * scale : 0.f;
-        if (j <= i) ds[j] = g;
-        dsr[j] = g;
-    }
-    __syncwarp();
-    float *dq = dqkv + (row0 + i) * ld + (size_t)h * HD;
-    for (int d = l; d < HD; d += 32) {
-        float acc = 0.f;
-        for (int j = 0; j <= i; ++j) acc = fmaf(ds[j], k[((row0 + j) * n_kv + kvh) * HD + d], acc);
-        dq[d] = acc;
-    }
-}
-
-// One warp per (sequence, kv head, key): dK and dV summed over the later queries of each q head
-// of the group, then over the group in head order (attn_bwd_dkv followed by repeat_kv_bwd).
-template <int HD>
-__global__ void __launch_bounds__(ATT_WARPS * 32)
-attn_bwd_dkv_kernel(const float *d_score, const float *probs, const float *q, const float *d_out, int n_seq, int N,
-                    int n_q, int n_kv, float *dqkv, long long ld)
-{
-    constexpr int PER = HD / 32;
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const long long unit = (long long)blockIdx.x * ATT_WARPS + w;
-    if (unit >= (long long)n_seq * n_kv * N) return;
-    const int j = (int)(unit % N), kvh = (int)((unit / N) % n_kv), s = (int)(unit / ((long long)N * n_kv));
-    const int G = n_q / n_kv;
-    const size_t row0 = (size_t)s * N;
-    float dk[PER], dv[PER];
-#pragma unroll
-    for (int c = 0; c < PER; ++c) dk[c] = dv[c] = 0.f;
-    for (int g = 0; g < G; ++g) {
-        const int h = kvh * G + g;
-        const float *dsc = d_score + ((size_t)s * n_q + h) * N * N;
-        const float *prc = probs + ((size_t)s * n_q + h) * N * N;
-        float hk[PER], hv[PER];
-#pragma unroll
-        for (int c = 0; c < PER; ++c) hk[c] = hv[c] = 0.f;
-        for (int i = j; i < N; ++i) {
-            const float dsv = dsc[(size_t)i * N + j], pv = prc[(size_t)i * N + j];
-            const float *qr = q + ((row0 + i) * n_q + h) * HD;
-            const float *dor = d_out + ((row0 + i) * n_q + h) * HD;
-#pragma unroll
-            for (int c = 0; c < PER; ++c) {
-                hk[c] = fmaf(dsv, qr[l + 32 * c], hk[c]);
-                hv[c] = fmaf(pv, dor[l + 32 * c], hv[c]);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < PER; ++c) { dk[c] += hk[c]; dv[c] += hv[c]; }
-    }
-    float *dkr = dqkv + (row0 + j) * ld + (size_t)(n_q + kvh) * HD;
-    float *dvr = dqkv + (row0 + j) * ld + (size_t)(n_q + n_kv + kvh) * HD;
-#pragma unroll
-    for (int c = 0; c < PER; ++c) { dkr[l + 32 * c] = dk[c]; dvr[l + 32 * c] = dv[c]; }
-}
-
 // ---- causal attention for short sequences (N <= 64): one block per (sequence, head) ----------------
 // The whole 64 x 64 score tile of a head lives in shared memory and every product is a register-tiled
 // shared-memory matmul (256 threads, 4 x 4 or 4 x HD/16 outputs each) instead of one warp walking the keys.
-// Same arithmetic as the per-query kernels above (fp32 FMA, softmax with max subtraction).
+// fp32 FMA, softmax with max subtraction.
 constexpr int AT = 64;            // tile edge: queries and keys
 constexpr int ATP = AT + 4;       // padded row of a transposed operand (keeps float4 reads aligned)
 
@@ -357,14 +204,10 @@ __device__ __forceinline__ void load_rows(float *dst, const float *src, long lon
     }
 }
 
-// acc[a][b] = sum_d At[d][4*ty + a] * Bt[d][4*tx + b]   (both operands transposed, ATP-padded)
+// acc[a][b] += sum_d At[d][4*ty + a] * Bt[d][4*tx + b]   (both operands transposed, ATP-padded)
 template <int HD>
-__device__ __forceinline__ void tile_abt(const float *At, const float *Bt, int ty, int tx, float (&acc)[4][4])
+__device__ __forceinline__ void tile_abt_add(const float *At, const float *Bt, int ty, int tx, float (&acc)[4][4])
 {
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
 #pragma unroll 4
     for (int d = 0; d < HD; ++d) {
         const float4 av = *reinterpret_cast<const float4 *>(At + d * ATP + 4 * ty);
@@ -377,16 +220,22 @@ __device__ __forceinline__ void tile_abt(const float *At, const float *Bt, int t
     }
 }
 
-// out[4*ty + a][CW*tx + c] = sum_j W(j, 4*ty + a) * B[j][CW*tx + c], j < n; W(j, r) = Wm[r*ATP + j] when
-// !WT (the weight matrix is indexed [row][j]) or Wm[j*ATP + r] when WT (indexed [j][row]). B row-major [AT][HD].
-template <int HD, bool WT>
-__device__ __forceinline__ void tile_wb(const float *Wm, const float *B, int n, int ty, int tx, float (&acc)[4][HD / 16])
+template <int HD>
+__device__ __forceinline__ void tile_abt(const float *At, const float *Bt, int ty, int tx, float (&acc)[4][4])
 {
-    constexpr int CW = HD / 16;
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
-        for (int c = 0; c < CW; ++c) acc[a][c] = 0.f;
+        for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
+    tile_abt_add<HD>(At, Bt, ty, tx, acc);
+}
+
+// out[4*ty + a][CW*tx + c] += sum_j W(j, 4*ty + a) * B[j][CW*tx + c], j < n; W(j, r) = Wm[r*ATP + j] when
+// !WT (the weight matrix is indexed [row][j]) or Wm[j*ATP + r] when WT (indexed [j][row]). B row-major [AT][HD].
+template <int HD, bool WT>
+__device__ __forceinline__ void tile_wb_add(const float *Wm, const float *B, int n, int ty, int tx, float (&acc)[4][HD / 16])
+{
+    constexpr int CW = HD / 16;
     for (int j = 0; j < n; ++j) {
         float w[4];
         if (WT) {
@@ -407,6 +256,16 @@ __device__ __forceinline__ void tile_wb(const float *Wm, const float *B, int n, 
 #pragma unroll
             for (int c = 0; c < CW; ++c) acc[a][c] = fmaf(w[a], bv[c], acc[a][c]);
     }
+}
+
+template <int HD, bool WT>
+__device__ __forceinline__ void tile_wb(const float *Wm, const float *B, int n, int ty, int tx, float (&acc)[4][HD / 16])
+{
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < HD / 16; ++c) acc[a][c] = 0.f;
+    tile_wb_add<HD, WT>(Wm, B, n, ty, tx, acc);
 }
 
 template <int HD>
@@ -574,6 +433,234 @@ __global__ void attn_bwd_reduce_kernel(const float *part, int n_seq, int N, int 
         for (int g = 0; g < G; ++g)
             sum += part[((((size_t)s * n_q + kvh * G + g) * N + j) * 2 + which) * hd + d];
         dqkv[row * ld + (size_t)(n_q + (which ? n_kv : 0) + kvh) * hd + d] = sum;
+    }
+}
+
+// ---- causal attention for sequences beyond one tile, and for heads of 256 --------------------------
+// The same register-tiled shared-memory products, one block per (sequence, head, 64 queries) walking the key tiles it can see.
+// One warp per query or key, which walked the rows through L2, spent 2.1 ms a layer on 32 heads x 509 positions of 128
+// (fp32 work: 6.4 GFLOP). The scores go to the probability matrix that is kept anyway and are read back by the thread that wrote
+// them. The longest rows start first. Bound by the fp32 pipes and by shared memory behind them.
+
+// Row statistics are spread over the 16 lanes (tx) that share a row.
+__device__ __forceinline__ float lanes16_sum(float v)
+{
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+template <int HD>
+__global__ void __launch_bounds__(256)
+attn_fwd_long_kernel(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q, int n_kv,
+                     float scale, float *probs, float *out, __half *out_h)
+{
+    extern __shared__ __align__(16) float sh[];
+    float *Qt = sh, *Kt = Qt + HD * ATP, *Vs = Kt, *P = Kt + HD * ATP;
+    const int it = (N + AT - 1) / AT - 1 - (int)blockIdx.x / n_seq, s = blockIdx.x % n_seq, h = blockIdx.y, kvh = h / (n_q / n_kv);
+    const size_t row0 = (size_t)s * N;
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, i0 = it * AT, ni = min(AT, N - i0);
+    load_transposed<HD>(Qt, q + ((row0 + i0) * n_q + h) * HD, (long long)n_q * HD, ni);
+    float *pr = probs + (((size_t)s * n_q + h) * N + i0) * N;
+    float mx[4], l[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) { mx[a] = -1e30f; l[a] = 0.f; }
+    for (int jt = 0; jt <= it; ++jt) {
+        const int j0 = jt * AT;
+        load_transposed<HD>(Kt, k + ((row0 + j0) * n_kv + kvh) * HD, (long long)n_kv * HD, min(AT, N - j0));
+        __syncthreads();
+        float acc[4][4];
+        tile_abt<HD>(Qt, Kt, ty, tx, acc);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const int i = 4 * ty + a;
+            float m = mx[a];
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int j = j0 + 4 * tx + b;
+                acc[a][b] = i < ni && j <= i0 + i ? acc[a][b] * scale : -1e30f;
+                m = fmaxf(m, acc[a][b]);
+                if (i < ni && j <= i0 + i) pr[(size_t)i * N + j] = acc[a][b];
+            }
+            float sum = 0.f;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) if (i < ni && j0 + 4 * tx + b <= i0 + i) sum += expf(acc[a][b] - m);
+            l[a] = l[a] * expf(mx[a] - m) + sum;
+            mx[a] = m;
+        }
+        __syncthreads();
+    }
+    float inv[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        float m = mx[a];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const float sum = lanes16_sum(l[a] * expf(mx[a] - m));
+        mx[a] = m;
+        inv[a] = 4 * ty + a < ni ? 1.0f / sum : 0.f;
+    }
+    float o[4][HD / 16];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < HD / 16; ++c) o[a][c] = 0.f;
+    for (int jt = 0; jt <= it; ++jt) {
+        const int j0 = jt * AT, nj = min(AT, N - j0);
+        load_rows<HD>(Vs, v + (row0 + j0) * v_ld + (size_t)kvh * HD, v_ld, nj);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int i = 4 * ty + a, j = j0 + 4 * tx + b;
+                float p = 0.f;
+                if (i < ni && j < N) {
+                    if (j <= i0 + i) p = expf(pr[(size_t)i * N + j] - mx[a]) * inv[a];
+                    pr[(size_t)i * N + j] = p;
+                }
+                P[i * ATP + 4 * tx + b] = p;
+            }
+        __syncthreads();
+        tile_wb_add<HD, false>(P, Vs, nj, ty, tx, o);
+        __syncthreads();
+    }
+    const int ahead = min((it + 1) * AT, N);                   // columns that no row of the tile sees
+    for (int i = threadIdx.x / 32; i < ni; i += 8)
+        for (int j = ahead + threadIdx.x % 32; j < N; j += 32) pr[(size_t)i * N + j] = 0.f;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int i = 4 * ty + a;
+        if (i >= ni) continue;
+        const size_t base = ((row0 + i0 + i) * n_q + h) * HD + (HD / 16) * tx;
+#pragma unroll
+        for (int c = 0; c < HD / 16; ++c) {
+            if (out) out[base + c] = o[a][c];
+            if (out_h) out_h[base + c] = __float2half_rn(o[a][c]);
+        }
+    }
+}
+
+// d_score = p * (dO . V - sum_j p_j (dO . V_j)) * scale, and dQ = d_score . K, for 64 queries of a head.
+template <int HD>
+__global__ void __launch_bounds__(256)
+attn_bwd_dq_long_kernel(const float *d_out, const float *probs, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q,
+                        int n_kv, float scale, float *d_score, float *dqkv, long long ld)
+{
+    extern __shared__ __align__(16) float sh[];
+    float *Ot = sh, *Vt = Ot + HD * ATP, *Ks = Vt, *G = Vt + HD * ATP;
+    const int it = (N + AT - 1) / AT - 1 - (int)blockIdx.x / n_seq, s = blockIdx.x % n_seq, h = blockIdx.y, kvh = h / (n_q / n_kv);
+    const size_t row0 = (size_t)s * N;
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, i0 = it * AT, ni = min(AT, N - i0);
+    load_transposed<HD>(Ot, d_out + ((row0 + i0) * n_q + h) * HD, (long long)n_q * HD, ni);
+    const size_t tile_rows = (((size_t)s * n_q + h) * N + i0) * N;
+    const float *pr = probs + tile_rows;
+    float *ds = d_score + tile_rows;
+    float dp[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int jt = 0; jt <= it; ++jt) {
+        const int j0 = jt * AT;
+        load_transposed<HD>(Vt, v + (row0 + j0) * v_ld + (size_t)kvh * HD, v_ld, min(AT, N - j0));
+        __syncthreads();
+        float acc[4][4];
+        tile_abt<HD>(Ot, Vt, ty, tx, acc);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int i = 4 * ty + a, j = j0 + 4 * tx + b;
+                if (i < ni && j <= i0 + i) {
+                    ds[(size_t)i * N + j] = acc[a][b];
+                    dp[a] = fmaf(pr[(size_t)i * N + j], acc[a][b], dp[a]);
+                }
+            }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) dp[a] = lanes16_sum(dp[a]);
+    float o[4][HD / 16];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int c = 0; c < HD / 16; ++c) o[a][c] = 0.f;
+    for (int jt = 0; jt <= it; ++jt) {
+        const int j0 = jt * AT, nj = min(AT, N - j0);
+        load_rows<HD>(Ks, k + ((row0 + j0) * n_kv + kvh) * HD, (long long)n_kv * HD, nj);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const int i = 4 * ty + a, j = j0 + 4 * tx + b;
+                float g = 0.f;
+                if (i < ni && j < N) {
+                    if (j <= i0 + i) g = pr[(size_t)i * N + j] * (ds[(size_t)i * N + j] - dp[a]) * scale;
+                    ds[(size_t)i * N + j] = g;
+                }
+                G[i * ATP + 4 * tx + b] = g;
+            }
+        __syncthreads();
+        tile_wb_add<HD, false>(G, Ks, nj, ty, tx, o);
+        __syncthreads();
+    }
+    const int ahead = min((it + 1) * AT, N);
+    for (int i = threadIdx.x / 32; i < ni; i += 8)
+        for (int j = ahead + threadIdx.x % 32; j < N; j += 32) ds[(size_t)i * N + j] = 0.f;
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int i = 4 * ty + a;
+        if (i >= ni) continue;
+        float *dst = dqkv + (row0 + i0 + i) * ld + (size_t)h * HD + (HD / 16) * tx;
+#pragma unroll
+        for (int c = 0; c < HD / 16; ++c) dst[c] = o[a][c];
+    }
+}
+
+// 64 keys x 64 columns of dK (d_score^T . Q) or dV (P^T . dO) of a KV head: summed over the later queries of each query head, then
+// over the heads in order. blockIdx.y = ((kv head * 2 + dK / dV) * (HD / 64) + columns).
+__global__ void __launch_bounds__(256)
+attn_bwd_dkv_long_kernel(const float *d_score, const float *probs, const float *q, const float *d_out, int n_seq, int N, int n_q, int n_kv,
+                         int hd, float *dqkv, long long ld)
+{
+    __shared__ __align__(16) float W[AT * ATP], B[AT * ATP];
+    const int jt = blockIdx.x / n_seq, s = blockIdx.x % n_seq, slices = hd / 64, slice = blockIdx.y % slices;
+    const int which = (blockIdx.y / slices) & 1, kvh = blockIdx.y / (2 * slices), group = n_q / n_kv;
+    const size_t row0 = (size_t)s * N;
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, j0 = jt * AT, nj = min(AT, N - j0);
+    float sum[4][4] = {};
+    for (int g = 0; g < group; ++g) {
+        const int h = kvh * group + g;
+        const float *w = (which ? probs : d_score) + ((size_t)s * n_q + h) * N * N + j0;
+        const float *b = (which ? d_out : q) + (row0 * n_q + h) * hd + slice * 64;
+        float acc[4][4] = {};
+        for (int i0 = j0; i0 < N; i0 += AT) {
+            const int ni = min(AT, N - i0);
+            float wr[AT * AT / 256], br[AT * AT / 256];
+#pragma unroll
+            for (int e = 0; e < AT * AT / 256; ++e) {          // all loads of a tile pair in flight, under the previous product
+                const int i = e * 4 + threadIdx.x / 64, c = threadIdx.x % 64;
+                wr[e] = i < ni && c < nj ? w[(size_t)(i0 + i) * N + c] : 0.f;
+                br[e] = i < ni ? b[(size_t)(i0 + i) * n_q * hd + c] : 0.f;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int e = 0; e < AT * AT / 256; ++e) {
+                const int i = e * 4 + threadIdx.x / 64, c = threadIdx.x % 64;
+                W[i * ATP + c] = wr[e];
+                B[i * ATP + c] = br[e];
+            }
+            __syncthreads();
+            tile_abt_add<AT>(W, B, ty, tx, acc);
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) sum[a][c] += acc[a][c];
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        const int j = 4 * ty + a;
+        if (j >= nj) continue;
+        float *dst = dqkv + (row0 + j0 + j) * ld + (size_t)(n_q + (which ? n_kv : 0) + kvh) * hd + slice * 64 + 4 * tx;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) dst[c] = sum[a][c];
     }
 }
 
@@ -1181,12 +1268,10 @@ static int attn_fwd_launch(const float *q, const float *k, const float *v, long 
         attn_fwd_tile_kernel<HD><<<n_seq * n_q, 256, tsm, st>>>(q, k, v, v_ld, N, n_q, n_kv, scale, probs, out, out_h);
         return done();
     }
-    const size_t smem = (size_t)ATT_WARPS * (HD + N) * sizeof(float);
-    int rc = opt_in_smem(attn_train_fwd_kernel<HD>, smem);
+    const size_t smem = ((size_t)2 * HD * ATP + (size_t)AT * ATP) * sizeof(float);
+    int rc = opt_in_smem(attn_fwd_long_kernel<HD>, smem);
     if (rc) return rc;
-    const long long units = (long long)n_seq * n_q * N;
-    attn_train_fwd_kernel<HD><<<(unsigned)((units + ATT_WARPS - 1) / ATT_WARPS), ATT_WARPS * 32, smem, st>>>(
-        q, k, v, v_ld, n_seq, N, n_q, n_kv, scale, probs, out, out_h);
+    attn_fwd_long_kernel<HD><<<dim3((N + AT - 1) / AT * n_seq, n_q), 256, smem, st>>>(q, k, v, v_ld, n_seq, N, n_q, n_kv, scale, probs, out, out_h);
     return done();
 }
 
@@ -1230,16 +1315,14 @@ static int attn_bwd_launch(const float *d_out, const float *probs, const float *
         attn_bwd_reduce_kernel<<<grid, 256, 0, st>>>(d_score, n_seq, N, n_q, n_kv, HD, dqkv, ld);
         return done();
     }
-    const size_t smem = (size_t)ATT_WARPS * (HD + N) * sizeof(float);
-    int rc = opt_in_smem(attn_bwd_dq_kernel<HD>, smem);
+    const size_t smem = ((size_t)2 * HD * ATP + (size_t)AT * ATP) * sizeof(float);
+    int rc = opt_in_smem(attn_bwd_dq_long_kernel<HD>, smem);
     if (rc) return rc;
-    const long long uq = (long long)n_seq * n_q * N, uk = (long long)n_seq * n_kv * N;
-    attn_bwd_dq_kernel<HD><<<(unsigned)((uq + ATT_WARPS - 1) / ATT_WARPS), ATT_WARPS * 32, smem, st>>>(
-        d_out, probs, k, v, v_ld, n_seq, N, n_q, n_kv, scale, d_score, dqkv, ld);
+    const int tiles = (N + AT - 1) / AT;
+    attn_bwd_dq_long_kernel<HD><<<dim3(tiles * n_seq, n_q), 256, smem, st>>>(d_out, probs, k, v, v_ld, n_seq, N, n_q, n_kv, scale, d_score, dqkv, ld);
     rc = done();
     if (rc) return rc;
-    attn_bwd_dkv_kernel<HD><<<(unsigned)((uk + ATT_WARPS - 1) / ATT_WARPS), ATT_WARPS * 32, 0, st>>>(
-        d_score, probs, q, d_out, n_seq, N, n_q, n_kv, dqkv, ld);
+    attn_bwd_dkv_long_kernel<<<dim3(tiles * n_seq, n_kv * 2 * (HD / 64)), 256, 0, st>>>(d_score, probs, q, d_out, n_seq, N, n_q, n_kv, HD, dqkv, ld);
     return done();
 }
 
