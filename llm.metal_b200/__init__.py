@@ -149,7 +149,7 @@ class GemmArgs(C.Structure):
                 ("C", C.c_void_p), ("ldc", C.c_longlong),
                 ("R", C.c_void_p), ("ldr", C.c_longlong),
                 ("M", C.c_int), ("N", C.c_int), ("K", C.c_int), ("alpha", C.c_float), ("d_err", C.c_void_p),
-                ("Ch", C.c_void_p), ("ldch", C.c_longlong), ("relu2", C.c_int)]
+                ("Ch", C.c_void_p), ("ldch", C.c_longlong), ("relu2", C.c_int), ("round_f16", C.c_int)]
 
 
 class LatentArgs(C.Structure):

@@ -823,7 +823,7 @@ static void loss_device(SFTState *s)
  * into rows 0..rows-1 of the matrix the way wmode says: W <- half(W - lr dW) (f16_sgd_fused,
  * shaders/q8_kernels.metal:1097-1125) or G <- half(G + dW) (f16_grad_accum, :1164-1191). One fp32 sum over
  * the tokens in ascending order per element, one rounding to binary16, as there. The matrices are fp32
- * holders of binary16 values in this mode, so the product adds into them in place and a rounding pass follows. */
+ * holders of binary16 values in this mode, so the product adds into them in place and rounds. */
 static void weight_step(SFTState *s, SftMat *W, float *acc, int rows, const float *dY, long long ldy, const float *X,
                         long long ldx)
 {
@@ -840,8 +840,8 @@ static void weight_step(SFTState *s, SftMat *W, float *acc, int rows, const floa
     g.R = dst; g.ldr = W->cols;                    /* in place: every element is read and written by one thread */
     g.M = rows; g.N = W->cols; g.K = s->M;
     g.alpha = s->wmode == 2 ? 1.0f : -s->sgd_lr;
+    g.round_f16 = 1;
     S_TRY(s, b200_gemm_f32(&g, g_rt.stream));
-    S_TRY(s, b200_round_f16(dst, (size_t)rows * W->cols, g_rt.stream));
     if (s->wmode == 1) s->weights_version++;
 }
 

@@ -1,0 +1,33 @@
+"""The CUDA-core fp32 product in every orientation at the edges of its tiles and splits, against float64 on the same operands.
+
+Bar: K fp32 additions in a random walk, 2^-20 of the sum of the terms' magnitudes."""
+import ctypes as C
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ak", [0, 1])
+@pytest.mark.parametrize("bk", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (64, 64, 32), (65, 63, 33), (64, 1152, 6912), (64, 130, 1000), (7, 16, 2048), (1152, 300, 64)])
+def test_f32_products(lib, pkg, ak, bk, M, N, K):
+    g = torch.Generator().manual_seed(K + 3 * M)
+    A, B, R = (torch.randn(*s, generator=g).cuda() for s in ((M, K), (K, N), (M, N)))
+    a_mem, b_mem = (A.contiguous() if ak else A.T.contiguous()), (B.T.contiguous() if bk else B.contiguous())
+    want, size = A.double() @ B.double(), A.double().abs() @ B.double().abs()
+    outs = []
+    for round_f16 in (0, 0, 1):
+        c = R.clone()
+        a = pkg.GemmArgs()
+        a.A, a.a_row, a.a_col = a_mem.data_ptr(), K if ak else 1, 1 if ak else M
+        a.B, a.b_row, a.b_col = b_mem.data_ptr(), 1 if bk else N, K if bk else 1
+        a.C, a.ldc, a.R, a.ldr = c.data_ptr(), N, c.data_ptr(), N                   # in place
+        a.M, a.N, a.K, a.alpha, a.round_f16 = M, N, K, -0.25, round_f16
+        assert lib.b200_gemm_f32(C.byref(a), None) == 0
+        torch.cuda.synchronize()
+        outs.append(c)
+    assert ((outs[0].double() - (R.double() - 0.25 * want)).abs() <= 2 ** -20 * (size + R.double().abs())).all()
+    assert torch.equal(outs[0], outs[1])                      # the splits add in a fixed order
+    assert torch.equal(outs[2], outs[0].half().float())
