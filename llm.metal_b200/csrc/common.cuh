@@ -14,6 +14,21 @@
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Launch of a kernel that calls pdl_wait() before it touches anything an earlier kernel writes: it may be scheduled while its
+// predecessor drains, if that one says so (pdl_launch_dependents), and otherwise starts after it as usual.
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 // ---- memory ------------------------------------------------------------
 // Streaming 16-byte load that does not allocate in L1 (weights are read once).
 __device__ __forceinline__ uint4 ldg_stream_16(const void *p) {
@@ -61,6 +76,29 @@ __device__ __forceinline__ float block_sum(float v, float *red) {
     }
     __syncthreads();
     return red[32];
+}
+
+// ---- clusters ------------------------------------------------------------
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Sum, in rank order, of the four floats at shared-memory address `addr` (16-byte aligned) of n <= 8 blocks of the cluster: ranks
+// first, first + step, ... All loads are in flight at once: one by one they cost a round trip of 0.25 us each.
+__device__ __forceinline__ float4 sum_ranks4(uint32_t addr, int n, int first, int step) {
+    float4 v[8];
+#pragma unroll
+    for (int z = 0; z < 8; ++z) {
+        if (z < n) {
+            uint32_t at;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(first + z * step));
+            asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[z].x), "=f"(v[z].y), "=f"(v[z].z), "=f"(v[z].w) : "r"(at));
+        }
+    }
+    float4 s = v[0];
+#pragma unroll
+    for (int z = 1; z < 8; ++z)
+        if (z < n) { s.x += v[z].x; s.y += v[z].y; s.z += v[z].z; s.w += v[z].w; }
+    return s;
 }
 
 // Bounded wait for a flag another GPU writes. Returns false when it gave up.

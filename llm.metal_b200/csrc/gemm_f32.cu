@@ -118,22 +118,19 @@ __global__ void __launch_bounds__(THREADS, 3) gemm_f32_kernel(const __grid_const
 #pragma unroll
         for (int i = 0; i < TM; ++i)
             *reinterpret_cast<float4 *>(part + (ty * TM + i) * BN + tx * TN) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
         const uint32_t base = (uint32_t)__cvta_generic_to_shared(part);
         const int rows = BM / gridDim.z, first = blockIdx.z * rows;
-        for (int e = first * BN + tid; e < (first + rows) * BN; e += THREADS) {
+        for (int e = first * BN + 4 * tid; e < (first + rows) * BN; e += 4 * THREADS) {
             const int gm = m0 + e / BN, gn = n0 + e % BN;
-            float v = 0.0f;
-            for (int z = 0; z < (int)gridDim.z; ++z) {
-                uint32_t at;
-                float f;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(base + (uint32_t)e * 4), "r"(z));
-                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(f) : "r"(at) : "memory");
-                v += f;
-            }
-            if (gm < p.M && gn < p.N) p.C[(long long)gm * p.ldc + gn] = finish(p, v, p.R ? p.R + (long long)gm * p.ldr + gn : nullptr);
+            const float4 q = sum_ranks4(base + (uint32_t)e * 4, gridDim.z, 0, 1);
+            const float v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (gm < p.M && gn + j < p.N)
+                    p.C[(long long)gm * p.ldc + gn + j] = finish(p, v[j], p.R ? p.R + (long long)gm * p.ldr + gn + j : nullptr);
         }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
         return;
     }
 #pragma unroll

@@ -24,6 +24,7 @@
 // flight land, frees its tensor memory and returns.
 #include "stream_core.cuh"
 #include "tcgen05.cuh"
+#include "gemm_pair.cuh"
 #include "../../include/llmb200_train_kernels.h"
 
 #include <cuda_bf16.h>
@@ -358,7 +359,7 @@ int launch(const CUtensorMap &ma, const CUtensorMap &mb, EpiArgs e, cudaStream_t
 static int gemm_tc(const b200_gemm_args *a, int f16, void *stream)
 {
     if (!a || !a->A || !a->B || (!a->C && !a->Ch) || a->M <= 0 || a->N <= 0 || a->K <= 0) return B200_E_BADARG;
-    if (a->relu2 && (!a->Ch || a->alpha != 1.0f)) return B200_E_BADARG;
+    if ((a->relu2 && (!a->Ch || a->alpha != 1.0f)) || a->round_f16) return B200_E_BADARG;
     if (a->Ch && (f16 != 2 || a->R || (a->ldch & 7) || (reinterpret_cast<uintptr_t>(a->Ch) & 15))) return B200_E_BADARG;
     if (a->a_col != 1 || a->b_row != 1) return B200_E_UNSUPPORTED;
     const long long lda = a->a_row, ldb = a->b_col;
@@ -368,6 +369,8 @@ static int gemm_tc(const b200_gemm_args *a, int f16, void *stream)
     if (a->N < 64) return B200_E_UNSUPPORTED;                     // the CUDA-core kernel is the better fit
     if ((a->N + 63) / 64 > 65535) return B200_E_UNSUPPORTED;
 
+    PairShape pair;
+    if (f16 && gemm_pair_shape(a->M, a->N, a->K, !a->Ch, &pair)) return gemm_pair_launch(a, f16 - 1, pair, (cudaStream_t)stream);
     CUtensorMap ma, mb;
     EpiArgs e = {a->C, a->ldc, a->R, a->ldr, a->M, a->N, a->K, a->alpha, a->d_err, 128, 0, 0, f16, 1, 1, nullptr,
                  static_cast<__nv_bfloat16 *>(a->Ch), a->ldch, a->relu2};

@@ -51,19 +51,6 @@ struct RowsMat {
     int acc_cols, n_acc;                 // accumulators: columns between them, and how many
 };
 
-__device__ __forceinline__ void cluster_arrive_wait()
-{
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float ld_peer(uint32_t addr, int rank)
-{
-    uint32_t a;
-    float v;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(addr), "r"(rank));
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
-
 __device__ __forceinline__ void cp_async(uint32_t dst, const void *src, int bytes_on)      // 16 bytes, zeros unless on
 {
     asm volatile("cp.async.cg.shared.global.L2::256B [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes_on) : "memory");
@@ -314,20 +301,28 @@ rows_matmul_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     __syncthreads();
     if (p.splits > 1) {
         pdl_wait();                                                     // every thread reads and stores below
-        cluster_arrive_wait();                                          // every block's sums lie in its shared memory
+        cluster_sync();                                                 // every block's sums lie in its shared memory
         const int cols = min(BN, p.n - n0), share = (cols + p.splits - 1) / p.splits;
-        const int c0 = blockIdx.z * share, c1 = min(c0 + share, cols);
+        const int c0 = blockIdx.z * share, c1 = min(c0 + share, cols), row = m0 + 4 * lane;
         const uint32_t part = smem_u32(ring);
-        for (int i = c0 * WM + threadIdx.x; i < c1 * WM && !*abort_flag; i += blockDim.x) {
-            const int c = i / WM, row = m0 + i % WM;
-            float f = 0.0f;
-            for (int z = 0; z < p.splits; ++z) f += ld_peer(part + (uint32_t)i * 4, z);
-            if (row < p.rows) {
-                if (p.resid) f += __ldcg(p.resid + (long long)(n0 + c) * p.resid_ld + row);
-                p.out[(long long)(n0 + c) * p.out_ld + row] = f;
+        const bool vec = row + 4 <= p.rows && (p.out_ld & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+        for (int c = c0 + warp; c < c1 && !*abort_flag; c += blockDim.x / 32) {
+            const float4 q = sum_ranks4(part + (uint32_t)(c * WM + 4 * lane) * 4, p.splits, 0, 1);
+            float v[4] = {q.x, q.y, q.z, q.w};
+            float *o = p.out + (long long)(n0 + c) * p.out_ld + row;
+            if (p.resid) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (row + j < p.rows) v[j] += __ldcg(p.resid + (long long)(n0 + c) * p.resid_ld + row + j);
+            }
+            if (vec) *reinterpret_cast<float4 *>(o) = make_float4(v[0], v[1], v[2], v[3]);
+            else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (row + j < p.rows) o[j] = v[j];
             }
         }
-        cluster_arrive_wait();                                          // nobody leaves while a peer still reads
+        cluster_sync();                                                 // nobody leaves while a peer still reads
     }
     if (*abort_flag) {
         for (int i = 0; i < 200; ++i) __nanosleep(1000);                // copies in flight land before the memory is released
