@@ -17,7 +17,7 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 // Launch of a kernel that calls pdl_wait() before it touches anything an earlier kernel writes: it may be scheduled while its
 // predecessor drains, if that one says so (pdl_launch_dependents), and otherwise starts after it as usual.
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;

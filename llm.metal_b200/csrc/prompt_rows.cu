@@ -4,7 +4,10 @@
 // writes it as one or two binary16 planes of the row times a power of two (2^14 <= largest element < 2^15), so that two planes
 // carry 22 bits of each element whatever the row's size; the factor that takes the power of two out again goes beside
 // it. One plane without a factor is the plain rounding that the batched engine's products take.
-// All of them move each row once: bound by HBM / L2 bytes, a block per row so that a short prompt still spreads over SMs.
+// All of them move each row once: bound by HBM / L2 bytes, a block per row so that a short prompt still spreads over SMs. In short
+// prompts and in decode steps of a batch they and the products are bound by their launches instead, 2 to 4 us each: every kernel lets
+// the next one in at once and waits for the one before it after its set-up, so that a product's weights are on
+// their way into shared memory while the row kernel before it runs.
 #include "stream_core.cuh"
 #include "../../include/llmb200_train_kernels.h"
 
@@ -64,6 +67,8 @@ rows_norm_kernel(float *x, int dim, const float *y, const float *post, const flo
     extern __shared__ __align__(16) float row_sh[];
     __shared__ float red[33];
     const int m = blockIdx.x, n4 = dim >> 2;
+    pdl_launch_dependents();
+    pdl_wait();
     float4 *xr = reinterpret_cast<float4 *>(x + (long long)(index ? index[m] : m) * dim);
     float4 *sh = reinterpret_cast<float4 *>(row_sh);
     const float4 *yr = y ? reinterpret_cast<const float4 *>(y + (long long)m * dim) : nullptr;
@@ -116,27 +121,31 @@ rows_glu_kernel(const float *gu, int inter, int pairs, int gelu, const b200_row_
     extern __shared__ __align__(16) float row_sh[];
     __shared__ float red[33];
     const int m = blockIdx.x, n4 = inter >> 2;
+    pdl_launch_dependents();
+    pdl_wait();
     const float4 *g4 = reinterpret_cast<const float4 *>(gu + (long long)m * 2 * inter);
     float4 *sh = reinterpret_cast<float4 *>(row_sh);
     float mx = 0.0f;
-    for (int i = threadIdx.x; i < n4; i += ROW_THREADS) {
+    // without a factor the row's elements do not depend on one another: several blocks share it
+    for (int i = blockIdx.y * ROW_THREADS + threadIdx.x; i < n4; i += gridDim.y * ROW_THREADS) {
         const float4 a = __ldcs(g4 + (pairs ? 2 * i : i)), b = __ldcs(g4 + (pairs ? 2 * i + 1 : n4 + i));
         const float g[4] = {a.x, pairs ? a.z : a.y, pairs ? b.x : a.z, pairs ? b.z : a.w};
         const float u[4] = {pairs ? a.y : b.x, pairs ? a.w : b.y, pairs ? b.y : b.z, b.w};
         float v[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            v[k] = (gelu ? act_gelu_tanh(g[k]) : act_silu(g[k])) * u[k];
+            v[k] = (gelu ? act_gelu_tanh(g[k]) : g[k] / (1.0f + expf(-g[k]))) * u[k];
             mx = fmaxf(mx, fabsf(v[k]));
         }
-        sh[i] = make_float4(v[0], v[1], v[2], v[3]);
+        if (o.d_scale) sh[i] = make_float4(v[0], v[1], v[2], v[3]);
+        else put4(o, m, i, make_float4(v[0], v[1], v[2], v[3]), 1.0f);
     }
-    float up = 1.0f, down;
     if (o.d_scale) {
-        up = row_up(block_max(mx, red), &down);
+        float down;
+        const float up = row_up(block_max(mx, red), &down);
         if (threadIdx.x == 0) o.d_scale[m] = down;
+        for (int i = threadIdx.x; i < n4; i += ROW_THREADS) put4(o, m, i, sh[i], up);
     }
-    for (int i = threadIdx.x; i < n4; i += ROW_THREADS) put4(o, m, i, sh[i], up);
 }
 
 // Planes of plain rows.
@@ -145,6 +154,8 @@ rows_split_kernel(const float *x, int dim, const b200_row_planes o)
 {
     __shared__ float red[33];
     const int m = blockIdx.x, n4 = dim >> 2;
+    pdl_launch_dependents();
+    pdl_wait();
     const float4 *xr = reinterpret_cast<const float4 *>(x + (long long)m * dim);
     float up = 1.0f, down;
     if (o.d_scale) {
@@ -156,7 +167,7 @@ rows_split_kernel(const float *x, int dim, const b200_row_planes o)
         up = row_up(block_max(mx, red), &down);
         if (threadIdx.x == 0) o.d_scale[m] = down;
     }
-    for (int i = threadIdx.x; i < n4; i += ROW_THREADS) put4(o, m, i, xr[i], up);
+    for (int i = blockIdx.y * ROW_THREADS + threadIdx.x; i < n4; i += gridDim.y * ROW_THREADS) put4(o, m, i, xr[i], up);
 }
 
 // One warp per (row, head): query heads are normed, rotated and stored as two planes with a factor per row and head; key heads
@@ -166,6 +177,8 @@ __global__ void __launch_bounds__(128) rows_qkv_kernel(const b200_rows_attn_args
 {
     constexpr int H2 = HD / 64;                               // pairs (d, d + HD/2) per lane
     const int lane = threadIdx.x & 31, m = blockIdx.x, h = blockIdx.y * 4 + (threadIdx.x >> 5), heads = p.n_q + 2 * p.n_kv;
+    pdl_launch_dependents();
+    pdl_wait();
     if (h >= heads) return;
     const int seq = m / p.seq_len, pos = p.pos0 + m % p.seq_len;
     const float *src = p.d_qkv + (long long)m * heads * HD + (long long)h * HD;
@@ -267,6 +280,8 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
     const long long row0 = (long long)seq * p.seq_len + m0, plane = (long long)p.n_rows * p.n_q * HD;
     const __half *qg = static_cast<const __half *>(p.d_q) + (row0 * p.n_q + h) * HD;
     const int tiles = last / BKEY + 1;
+    pdl_launch_dependents();
+    pdl_wait();
 
     for (int e = tid; e < 2 * BQ * (HD / 8); e += NT) {
         const int c = e % (HD / 8), r = e / (HD / 8) % BQ, u = e / (HD / 8 * BQ);
@@ -419,20 +434,26 @@ int launch_attn(const b200_rows_attn_args &a, cudaStream_t st)
     constexpr size_t smem = (size_t)(2 * NW * 16 * (HD + 8) + 2 * 32 * (HD + 8) + 2 * 32 * (DV + 8)) * 2;
     const int rc = allow_smem(rows_attn_kernel<HD, NW>, smem);
     if (rc) return rc;
-    rows_attn_kernel<HD, NW><<<dim3((a.seq_len + NW * 16 - 1) / (NW * 16), a.n_q * (HD / DV), a.n_rows / a.seq_len), NW * 32, smem, st>>>(a);
     ++g_b200_launches;
-    return (int)cudaGetLastError();
+    return (int)launch_chained(rows_attn_kernel<HD, NW>, dim3((a.seq_len + NW * 16 - 1) / (NW * 16), a.n_q * (HD / DV), a.n_rows / a.seq_len),
+                               dim3(NW * 32), smem, st, a);
 }
 
 template <int HD>
 int rows_attn(const b200_rows_attn_args &a, cudaStream_t st)
 {
-    rows_qkv_kernel<HD><<<dim3(a.n_rows, (a.n_q + 2 * a.n_kv + 3) / 4), 128, 0, st>>>(a);
     ++g_b200_launches;
-    const int rc = (int)cudaGetLastError();
+    const int rc = (int)launch_chained(rows_qkv_kernel<HD>, dim3(a.n_rows, (a.n_q + 2 * a.n_kv + 3) / 4), dim3(128), 0, st, a);
     // 128 query rows a block where that still fills the machine (a tile of keys serves twice the rows), 64 otherwise
     const long long blocks = (long long)((a.seq_len + 127) / 128) * a.n_q * (HD > 128 ? 2 : 1) * (a.n_rows / a.seq_len);
     return rc ? rc : blocks >= 148 ? launch_attn<HD, 8>(a, st) : launch_attn<HD, 4>(a, st);
+}
+
+// Blocks per row where they can share it: about two waves of them, each with an element group for every thread.
+int share_row(int rows, int dim)
+{
+    const int most = (dim / 4 + ROW_THREADS - 1) / ROW_THREADS, want = (148 * 4 + rows - 1) / rows;
+    return want < most ? want : most;
 }
 
 bool planes_ok(const b200_row_planes *o, int rows, int dim)
@@ -449,9 +470,9 @@ extern "C" int b200_rows_norm_planes(float *x, int rows, int dim, const float *y
     if (!x || !gamma || rows <= 0 || dim <= 0 || (dim & 3) || (index && y) || (post_gamma && !y) || !planes_ok(out, rows, dim)) return B200_E_BADARG;
     const int rc = allow_smem(rows_norm_kernel, (size_t)dim * 4);
     if (rc) return rc;
-    rows_norm_kernel<<<rows, ROW_THREADS, (size_t)dim * 4, (cudaStream_t)stream>>>(x, dim, y, post_gamma, gamma, index, eps, *out);
     ++g_b200_launches;
-    return (int)cudaGetLastError();
+    return (int)launch_chained(rows_norm_kernel, dim3(rows), dim3(ROW_THREADS), (size_t)dim * 4, (cudaStream_t)stream, x, dim, y, post_gamma, gamma,
+                               index, eps, *out);
 }
 
 extern "C" int b200_rows_glu_planes(const float *gu, int rows, int inter, int pairs, int gelu, const b200_row_planes *out, void *stream)
@@ -459,17 +480,17 @@ extern "C" int b200_rows_glu_planes(const float *gu, int rows, int inter, int pa
     if (!gu || rows <= 0 || inter <= 0 || (inter & 3) || !planes_ok(out, rows, inter)) return B200_E_BADARG;
     const int rc = allow_smem(rows_glu_kernel, (size_t)inter * 4);
     if (rc) return rc;
-    rows_glu_kernel<<<rows, ROW_THREADS, (size_t)inter * 4, (cudaStream_t)stream>>>(gu, inter, pairs, gelu, *out);
     ++g_b200_launches;
-    return (int)cudaGetLastError();
+    return (int)launch_chained(rows_glu_kernel, dim3(rows, out->d_scale ? 1 : share_row(rows, inter)), dim3(ROW_THREADS),
+                               out->d_scale ? (size_t)inter * 4 : 0, (cudaStream_t)stream, gu, inter, pairs, gelu, *out);
 }
 
 extern "C" int b200_rows_split_planes(const float *x, int rows, int dim, const b200_row_planes *out, void *stream)
 {
     if (!x || rows <= 0 || dim <= 0 || (dim & 3) || !planes_ok(out, rows, dim)) return B200_E_BADARG;
-    rows_split_kernel<<<rows, ROW_THREADS, 0, (cudaStream_t)stream>>>(x, dim, *out);
     ++g_b200_launches;
-    return (int)cudaGetLastError();
+    return (int)launch_chained(rows_split_kernel, dim3(rows, out->d_scale ? 1 : share_row(rows, dim)), dim3(ROW_THREADS), 0, (cudaStream_t)stream,
+                               x, dim, *out);
 }
 
 extern "C" int b200_rows_attn(const b200_rows_attn_args *a, void *stream)

@@ -215,6 +215,7 @@ static void proj(BState *s, const void *Wh, int N, int K, float *C)
     a.d_x = s->xh; a.x_ld = K; a.planes = 1;
     a.n = s->B;
     a.d_out = C; a.out_ld = N;
+    a.use_pdl = 1;
     B_TRY(s, b200_rows_matmul(&a, g_rt.stream));
 }
 
@@ -241,15 +242,16 @@ static void enqueue_step(BState *s)
         at.d_k_cache = y->k_cache; at.d_v_cache = y->v_cache;
         at.d_out = s->att; at.d_scratch = s->scratch; at.d_tickets = s->tickets; at.d_pos = s->d_ctl;
         at.n_q = s->Hq; at.n_kv = s->Hkv; at.hd = s->hd; at.max_seq = s->max_seq; at.n_split = s->n_split;
-        at.eps = 1e-6f; at.use_pdl = 0;
+        at.eps = 1e-6f; at.use_pdl = 1;
         at.n_items = B; at.qkv_item_stride = s->QKV; at.out_item_stride = Hq_hd;
         at.cache_item_stride = (long long)Hkv_hd * s->max_seq;
         B_TRY(s, b200_attn_decode(&at, st));
-        B_TRY(s, b200_f32_to_f16(s->att, (size_t)B * Hq_hd, 1.0f, s->xh, st));
+        const b200_row_planes heads = { s->xh, Hq_hd, 1, B, NULL }, inter = { s->xh, s->IS, 1, B, NULL };
+        B_TRY(s, b200_rows_split_planes(s->att, B, Hq_hd, &heads, st));
         proj(s, y->o, D, Hq_hd, s->y);
         norm(s, s->y, y->g_post);
         proj(s, y->gu, 2 * s->IS, D, s->gu);
-        B_TRY(s, b200_silu_mul_rows_h(s->gu, B, s->IS, NULL, s->xh, st));
+        B_TRY(s, b200_rows_glu_planes(s->gu, B, s->IS, 0, 0, &inter, st));
         proj(s, y->down, D, s->IS, s->y);
     }
     norm(s, s->y, s->g_final);

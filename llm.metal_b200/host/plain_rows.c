@@ -68,6 +68,7 @@ int llmb200_plain_rows_product(PlainRows *r, const RowsMatrix *m, int n, float *
     a.n = n;
     a.d_out = out; a.out_ld = m->rows;
     a.d_err = r->d_err;
+    a.use_pdl = 1;
     K_TRY(b200_rows_matmul(&a, g_rt.stream), return -1);
     return 0;
 }
