@@ -179,488 +179,353 @@ __global__ void qk_norm_rope_bwd_kernel(float *dqkv, const float *qkv, long long
     }
 }
 
-// ---- causal attention for short sequences (N <= 64): one block per (sequence, head) ----------------
-// The whole 64 x 64 score tile of a head lives in shared memory and every product is a register-tiled
-// shared-memory matmul (256 threads, 4 x 4 or 4 x HD/16 outputs each) instead of one warp walking the keys.
-// fp32 FMA, softmax with max subtraction.
-constexpr int AT = 64;            // tile edge: queries and keys
-constexpr int ATP = AT + 4;       // padded row of a transposed operand (keeps float4 reads aligned)
+// ---- causal attention, training form ---------------------------------------------------------------
+// One block per (sequence, head, 64 queries), or 64 keys, walking the tiles it can see; fp32 values throughout, with the products on
+// the tensor cores: an fp32 operand is a TF32 number plus what that leaves (x = hi + lo, 22 bits), a product is hi hi + hi lo + lo hi
+// with fp32 sums (mma.sync m16n8k8: the fragments of both operands are read from plain row-major tiles, in any orientation, with
+// the split on the way; 16-bit planes would need every row's range). Scores and probabilities go to the matrices that are
+// kept anyway and are read back by the thread that wrote them. The next tile's copies run under the current one's products. The
+// longest rows start first.
+// The same tiles as register-tiled fp32 products on the CUDA cores took 649 us a layer forward and backward (32 heads, 509 positions of
+// 128), one warp per query or key 2.1 ms.
+constexpr int AT = 64;                       // tile edge: queries and keys
+constexpr int ATT_THREADS = 256;
 
-// dst[d][i] = src[i][d] for i < n (zero beyond), src rows `ld` floats apart. HD columns.
-template <int HD>
-__device__ __forceinline__ void load_transposed(float *dst, const float *src, long long ld, int n)
+__device__ __forceinline__ void tf32_parts(float x, uint32_t &hi, uint32_t &lo)
 {
-    for (int e = threadIdx.x; e < AT * HD; e += blockDim.x) {
-        const int i = e / HD, d = e % HD;
-        dst[d * ATP + i] = i < n ? src[(size_t)i * ld + d] : 0.f;
-    }
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(x));
+    lo = __float_as_uint(x - __uint_as_float(hi));
 }
-template <int HD>
-__device__ __forceinline__ void load_rows(float *dst, const float *src, long long ld, int n)
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1)
 {
-    for (int e = threadIdx.x; e < AT * HD; e += blockDim.x) {
-        const int i = e / HD, d = e % HD;
-        dst[i * HD + d] = i < n ? src[(size_t)i * ld + d] : 0.f;
-    }
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-// acc[a][b] += sum_d At[d][4*ty + a] * Bt[d][4*tx + b]   (both operands transposed, ATP-padded)
-template <int HD>
-__device__ __forceinline__ void tile_abt_add(const float *At, const float *Bt, int ty, int tx, float (&acc)[4][4])
+// acc += A (16 x K) . B (K x 8 NT) of a warp: a(m, k) at A[m * am + k * ak], b(k, n) at B[k * bk + n * bn]. Lane l holds rows l / 4 and
+// l / 4 + 8, columns 2 (l % 4) and the next of every eight.
+template <int NT>
+__device__ __forceinline__ void mma_add(float (&acc)[NT][4], const float *A, int am, int ak, const float *B, int bk, int bn, int K)
 {
-#pragma unroll 4
-    for (int d = 0; d < HD; ++d) {
-        const float4 av = *reinterpret_cast<const float4 *>(At + d * ATP + 4 * ty);
-        const float4 bv = *reinterpret_cast<const float4 *>(Bt + d * ATP + 4 * tx);
-        const float a4[4] = {av.x, av.y, av.z, av.w}, b4[4] = {bv.x, bv.y, bv.z, bv.w};
+    const int r = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+#pragma unroll 2
+    for (int k = 0; k < K; k += 8) {
+        uint32_t ah[4], al[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int e = 0; e < 4; ++e) tf32_parts(A[(r + 8 * (e & 1)) * am + (k + q + 4 * (e >> 1)) * ak], ah[e], al[e]);
 #pragma unroll
-            for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(a4[a], b4[b], acc[a][b]);
-    }
-}
-
-template <int HD>
-__device__ __forceinline__ void tile_abt(const float *At, const float *Bt, int ty, int tx, float (&acc)[4][4])
-{
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = 0.f;
-    tile_abt_add<HD>(At, Bt, ty, tx, acc);
-}
-
-// out[4*ty + a][CW*tx + c] += sum_j W(j, 4*ty + a) * B[j][CW*tx + c], j < n; W(j, r) = Wm[r*ATP + j] when
-// !WT (the weight matrix is indexed [row][j]) or Wm[j*ATP + r] when WT (indexed [j][row]). B row-major [AT][HD].
-template <int HD, bool WT>
-__device__ __forceinline__ void tile_wb_add(const float *Wm, const float *B, int n, int ty, int tx, float (&acc)[4][HD / 16])
-{
-    constexpr int CW = HD / 16;
-    for (int j = 0; j < n; ++j) {
-        float w[4];
-        if (WT) {
-            const float4 wv = *reinterpret_cast<const float4 *>(Wm + j * ATP + 4 * ty);
-            w[0] = wv.x; w[1] = wv.y; w[2] = wv.z; w[3] = wv.w;
-        } else {
-#pragma unroll
-            for (int a = 0; a < 4; ++a) w[a] = Wm[(4 * ty + a) * ATP + j];
+        for (int n = 0; n < NT; ++n) {
+            uint32_t h0, l0, h1, l1;
+            tf32_parts(B[(k + q) * bk + (n * 8 + r) * bn], h0, l0);
+            tf32_parts(B[(k + q + 4) * bk + (n * 8 + r) * bn], h1, l1);
+            mma_tf32(acc[n], al, h0, h1);
+            mma_tf32(acc[n], ah, l0, l1);
+            mma_tf32(acc[n], ah, h0, h1);
         }
-        float bv[CW];
-#pragma unroll
-        for (int c4 = 0; c4 < CW / 4; ++c4) {
-            const float4 t = *reinterpret_cast<const float4 *>(B + j * HD + CW * tx + 4 * c4);
-            bv[4 * c4] = t.x; bv[4 * c4 + 1] = t.y; bv[4 * c4 + 2] = t.z; bv[4 * c4 + 3] = t.w;
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < CW; ++c) acc[a][c] = fmaf(w[a], bv[c], acc[a][c]);
     }
 }
 
-template <int HD, bool WT>
-__device__ __forceinline__ void tile_wb(const float *Wm, const float *B, int n, int ty, int tx, float (&acc)[4][HD / 16])
+// The same, four columns of eight at a time in sums of their own that join acc in fp32 adds: tensor cores truncate when they
+// accumulate, which over all tiles of a long row would add up (7e-6 of dK at 509 positions, 1e-6 so).
+template <int NT>
+__device__ __forceinline__ void mma_add_apart(float (&acc)[NT][4], const float *A, int am, int ak, const float *B, int bk, int bn, int K)
 {
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int g = 0; g < NT; g += 4) {
+        float t[4][4] = {};
+        mma_add<4>(t, A, am, ak, B + g * 8 * bn, bk, bn, K);
 #pragma unroll
-        for (int c = 0; c < HD / 16; ++c) acc[a][c] = 0.f;
-    tile_wb_add<HD, WT>(Wm, B, n, ty, tx, acc);
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[g + n][e] += t[n][e];
+    }
+}
+
+// Asynchronous copy of n rows (zeros up to 64) of COLS floats, `ld` apart, to rows `pitch` apart; 16 bytes at a time where addresses allow.
+template <int COLS>
+__device__ __forceinline__ void tile_copy(float *dst, int pitch, const float *src, long long ld, int n, int cols = COLS)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    if (((reinterpret_cast<uintptr_t>(src) & 15) | (ld & 3) | (cols & 3)) == 0) {
+        for (int e = threadIdx.x; e < AT * (COLS / 4); e += ATT_THREADS) {
+            const int i = e / (COLS / 4), c = e % (COLS / 4) * 4;
+            const int on = i < n && c < cols ? 16 : 0;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d + (i * pitch + c) * 4), "l"(on ? src + i * ld + c : src), "r"(on) : "memory");
+        }
+    } else {
+        for (int e = threadIdx.x; e < AT * COLS; e += ATT_THREADS) {
+            const int i = e / COLS, c = e % COLS;
+            const int on = i < n && c < cols ? 4 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + (i * pitch + c) * 4), "l"(on ? src + i * ld + c : src), "r"(on) : "memory");
+        }
+    }
+}
+__device__ __forceinline__ void tile_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// Pitches that keep fragment reads off each other's banks: along a row (k contiguous) 4 mod 32, down a column 8 mod 32.
+template <int HD> struct AttnTiles {
+    static constexpr int RP = HD + 4, CP = HD + 8, PP = AT + 4, BUF = AT * CP;
+    static constexpr size_t bytes = ((size_t)AT * RP + 2 * BUF) * sizeof(float);      // one operand, two buffers; the weights replace the operand
+};
+
+// Sums and maxima of a row lie in four lanes of two warps (column halves).
+__device__ __forceinline__ float quad_sum(float v)
+{
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
 template <int HD>
-__global__ void __launch_bounds__(256)
-attn_fwd_tile_kernel(const float *q, const float *k, const float *v, long long v_ld, int N, int n_q, int n_kv,
-                     float scale, float *probs, float *out, __half *out_h)
+__global__ void __launch_bounds__(ATT_THREADS)
+attn_fwd_kernel(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q, int n_kv,
+                float scale, float *probs, float *out, __half *out_h)
 {
+    using L = AttnTiles<HD>;
     extern __shared__ __align__(16) float sh[];
-    // Two operand regions + the score tile: V takes over Q's region once the scores are done, which keeps
-    // the block at ~87 KB (HD 128) so that two blocks share an SM.
-    float *Qt = sh, *Kt = Qt + HD * ATP, *Vs = Qt, *P = Kt + HD * ATP;               // P [AT][ATP]
-    const int h = blockIdx.x % n_q, s = blockIdx.x / n_q, kvh = h / (n_q / n_kv);
-    const size_t row0 = (size_t)s * N;
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    load_transposed<HD>(Qt, q + (row0 * n_q + h) * HD, (long long)n_q * HD, N);
-    load_transposed<HD>(Kt, k + (row0 * n_kv + kvh) * HD, (long long)n_kv * HD, N);
-    __syncthreads();
-    float acc[4][4];
-    tile_abt<HD>(Qt, Kt, ty, tx, acc);
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int i = 4 * ty + a, j = 4 * tx + b;
-            P[i * ATP + j] = (j <= i && i < N) ? acc[a][b] * scale : -1e30f;
-        }
-    __syncthreads();                                          // everybody is done with Q: its region becomes V
-    load_rows<HD>(Vs, v + row0 * v_ld + (size_t)kvh * HD, v_ld, N);
-    {   // softmax: four threads per row, 16 columns each
-        const int i = threadIdx.x / 4, part = threadIdx.x % 4;
-        float *pr = P + i * ATP + 16 * part;
-        float mx = -1e30f;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) mx = fmaxf(mx, pr[c]);
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-        float e[16], sum = 0.f;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            const int j = 16 * part + c;
-            e[c] = (j <= i && i < N) ? expf(pr[c] - mx) : 0.f;
-            sum += e[c];
-        }
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-        const float inv = i < N ? 1.0f / sum : 0.f;
-        float *gp = probs + (((size_t)s * n_q + h) * N + i) * N;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) {
-            const int j = 16 * part + c;
-            const float p = e[c] * inv;
-            pr[c] = p;
-            if (i < N && j < N) gp[j] = p;
-        }
-    }
-    __syncthreads();
-    float o[4][HD / 16];
-    tile_wb<HD, false>(P, Vs, N, ty, tx, o);
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int i = 4 * ty + a;
-        if (i >= N) continue;
-        const size_t base = ((row0 + i) * n_q + h) * HD + (HD / 16) * tx;
-#pragma unroll
-        for (int c = 0; c < HD / 16; ++c) {
-            if (out) out[base + c] = o[a][c];
-            if (out_h) out_h[base + c] = __float2half_rn(o[a][c]);
-        }
-    }
-}
-
-// Backward of one (sequence, head): dq into dqkv, this head's dK and dV into part[s][h][N][2][HD].
-template <int HD>
-__global__ void __launch_bounds__(256)
-attn_bwd_tile_kernel(const float *d_out, const float *probs, const float *q, const float *k, const float *v,
-                     long long v_ld, int N, int n_q, int n_kv, float scale, float *dqkv, long long ld, float *part)
-{
-    extern __shared__ __align__(16) float sh[];
-    // Two operand regions (each holds a transposed [HD][ATP] or a row-major [AT][HD] tile), reloaded as the
-    // four products go by, + the P and dS tiles: ~104 KB for HD 128, so that two blocks share an SM.
-    float *R1 = sh, *R2 = R1 + HD * ATP, *P = R2 + HD * ATP, *dS = P + AT * ATP;
-    float *dOt = R1, *Vt = R2, *Ks = R1, *Qs = R2, *dOs = R1;
-    const int h = blockIdx.x % n_q, s = blockIdx.x / n_q, kvh = h / (n_q / n_kv);
-    const size_t row0 = (size_t)s * N;
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    const float *dop = d_out + (row0 * n_q + h) * HD;
-    load_transposed<HD>(dOt, dop, (long long)n_q * HD, N);
-    load_transposed<HD>(Vt, v + row0 * v_ld + (size_t)kvh * HD, v_ld, N);
-    const float *gp = probs + ((size_t)s * n_q + h) * N * N;
-    for (int e = threadIdx.x; e < AT * AT; e += blockDim.x) {
-        const int i = e / AT, j = e % AT;
-        P[i * ATP + j] = (i < N && j < N) ? gp[(size_t)i * N + j] : 0.f;
-    }
-    __syncthreads();
-    float acc[4][4];
-    tile_abt<HD>(dOt, Vt, ty, tx, acc);                       // d_raw[i][j] = dO_i . V_j
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int i = 4 * ty + a, j = 4 * tx + b;
-            dS[i * ATP + j] = (j <= i && i < N) ? acc[a][b] : 0.f;
-        }
-    __syncthreads();                                          // dO^T and V^T are used up: bring in K and Q
-    load_rows<HD>(Ks, k + (row0 * n_kv + kvh) * HD, (long long)n_kv * HD, N);
-    load_rows<HD>(Qs, q + (row0 * n_q + h) * HD, (long long)n_q * HD, N);
-    {   // d_score = p * (d_raw - sum_k p_k d_raw_k) * scale, four threads per row
-        const int i = threadIdx.x / 4, part4 = threadIdx.x % 4;
-        float *dr = dS + i * ATP + 16 * part4;
-        const float *pr = P + i * ATP + 16 * part4;
-        float dp = 0.f;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) dp = fmaf(pr[c], dr[c], dp);
-        dp += __shfl_xor_sync(0xffffffffu, dp, 1);
-        dp += __shfl_xor_sync(0xffffffffu, dp, 2);
-#pragma unroll
-        for (int c = 0; c < 16; ++c) dr[c] = pr[c] * (dr[c] - dp) * scale;     // p is zero above the diagonal
-    }
-    __syncthreads();
-    float o[4][HD / 16];
-    tile_wb<HD, false>(dS, Ks, N, ty, tx, o);                 // dQ_i = sum_j dS[i][j] K_j
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int i = 4 * ty + a;
-        if (i >= N) continue;
-        float *dst = dqkv + (row0 + i) * ld + (size_t)h * HD + (HD / 16) * tx;
-#pragma unroll
-        for (int c = 0; c < HD / 16; ++c) dst[c] = o[a][c];
-    }
-    float *pk = part + (((size_t)s * n_q + h) * N) * 2 * HD;
-    tile_wb<HD, true>(dS, Qs, N, ty, tx, o);                  // dK_j = sum_i dS[i][j] Q_i
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int j = 4 * ty + a;
-        if (j >= N) continue;
-#pragma unroll
-        for (int c = 0; c < HD / 16; ++c) pk[(size_t)j * 2 * HD + (HD / 16) * tx + c] = o[a][c];
-    }
-    __syncthreads();                                          // K is used up: its region takes dO, row-major
-    load_rows<HD>(dOs, dop, (long long)n_q * HD, N);
-    __syncthreads();
-    tile_wb<HD, true>(P, dOs, N, ty, tx, o);                  // dV_j = sum_i P[i][j] dO_i
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int j = 4 * ty + a;
-        if (j >= N) continue;
-#pragma unroll
-        for (int c = 0; c < HD / 16; ++c) pk[(size_t)j * 2 * HD + HD + (HD / 16) * tx + c] = o[a][c];
-    }
-}
-
-// dK, dV of a KV head = sum over its query heads in head order (repeat_kv_bwd), into the k and v blocks of dqkv.
-__global__ void attn_bwd_reduce_kernel(const float *part, int n_seq, int N, int n_q, int n_kv, int hd, float *dqkv,
-                                       long long ld)
-{
-    const int G = n_q / n_kv;
-    const size_t total = (size_t)n_seq * N * n_kv * 2 * hd;
-    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-        const int d = (int)(e % hd);
-        const int which = (int)((e / hd) % 2);
-        const int kvh = (int)((e / (2 * hd)) % n_kv);
-        const size_t row = e / ((size_t)2 * hd * n_kv);            // s*N + j
-        const int s = (int)(row / N), j = (int)(row % N);
-        float sum = 0.f;
-        for (int g = 0; g < G; ++g)
-            sum += part[((((size_t)s * n_q + kvh * G + g) * N + j) * 2 + which) * hd + d];
-        dqkv[row * ld + (size_t)(n_q + (which ? n_kv : 0) + kvh) * hd + d] = sum;
-    }
-}
-
-// ---- causal attention for sequences beyond one tile, and for heads of 256 --------------------------
-// The same register-tiled shared-memory products, one block per (sequence, head, 64 queries) walking the key tiles it can see.
-// One warp per query or key, which walked the rows through L2, spent 2.1 ms a layer on 32 heads x 509 positions of 128
-// (fp32 work: 6.4 GFLOP). The scores go to the probability matrix that is kept anyway and are read back by the thread that wrote
-// them. The longest rows start first. Bound by the fp32 pipes and by shared memory behind them.
-
-// Row statistics are spread over the 16 lanes (tx) that share a row.
-__device__ __forceinline__ float lanes16_sum(float v)
-{
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-template <int HD>
-__global__ void __launch_bounds__(256)
-attn_fwd_long_kernel(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q, int n_kv,
-                     float scale, float *probs, float *out, __half *out_h)
-{
-    extern __shared__ __align__(16) float sh[];
-    float *Qt = sh, *Kt = Qt + HD * ATP, *Vs = Kt, *P = Kt + HD * ATP;
+    __shared__ float stat[2][2][AT];
+    float *Q = sh, *P = sh, *buf = sh + AT * L::RP;
     const int it = (N + AT - 1) / AT - 1 - (int)blockIdx.x / n_seq, s = blockIdx.x % n_seq, h = blockIdx.y, kvh = h / (n_q / n_kv);
     const size_t row0 = (size_t)s * N;
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, i0 = it * AT, ni = min(AT, N - i0);
-    load_transposed<HD>(Qt, q + ((row0 + i0) * n_q + h) * HD, (long long)n_q * HD, ni);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rw = (warp & 3) * 16, half = warp >> 2;
+    const int i0 = it * AT, ni = min(AT, N - i0), r0 = rw + (lane >> 2), c0 = half * 32 + 2 * (lane & 3);
+    const float *kh = k + (row0 * n_kv + kvh) * HD, *vh = v + row0 * v_ld + (size_t)kvh * HD;
     float *pr = probs + (((size_t)s * n_q + h) * N + i0) * N;
-    float mx[4], l[4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) { mx[a] = -1e30f; l[a] = 0.f; }
+
+    tile_copy<HD>(Q, L::RP, q + ((row0 + i0) * n_q + h) * HD, (long long)n_q * HD, ni);
+    tile_copy<HD>(buf, L::RP, kh, (long long)n_kv * HD, min(AT, N));
+    tile_commit();
+    float mx[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f};
     for (int jt = 0; jt <= it; ++jt) {
         const int j0 = jt * AT;
-        load_transposed<HD>(Kt, k + ((row0 + j0) * n_kv + kvh) * HD, (long long)n_kv * HD, min(AT, N - j0));
+        if (jt < it) {
+            tile_copy<HD>(buf + ((jt + 1) & 1) * L::BUF, L::RP, kh + (size_t)(j0 + AT) * n_kv * HD, (long long)n_kv * HD, min(AT, N - j0 - AT));
+            tile_commit();
+            tile_wait<1>();
+        } else tile_wait<0>();
         __syncthreads();
-        float acc[4][4];
-        tile_abt<HD>(Qt, Kt, ty, tx, acc);
+        float acc[4][4] = {};
+        mma_add<4>(acc, Q + rw * L::RP, L::RP, 1, buf + (jt & 1) * L::BUF + half * 32 * L::RP, 1, L::RP, HD);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int i = 4 * ty + a;
+        for (int a = 0; a < 2; ++a) {
+            const int i = r0 + 8 * a;
             float m = mx[a];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int j = j0 + 4 * tx + b;
-                acc[a][b] = i < ni && j <= i0 + i ? acc[a][b] * scale : -1e30f;
-                m = fmaxf(m, acc[a][b]);
-                if (i < ni && j <= i0 + i) pr[(size_t)i * N + j] = acc[a][b];
-            }
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int j = j0 + c0 + 8 * n + b;
+                    float &x = acc[n][2 * a + b];
+                    x *= scale;
+                    if (i < ni && j <= i0 + i) { m = fmaxf(m, x); pr[(size_t)i * N + j] = x; }
+                }
             float sum = 0.f;
 #pragma unroll
-            for (int b = 0; b < 4; ++b) if (i < ni && j0 + 4 * tx + b <= i0 + i) sum += expf(acc[a][b] - m);
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int b = 0; b < 2; ++b)
+                    if (i < ni && j0 + c0 + 8 * n + b <= i0 + i) sum += expf(acc[n][2 * a + b] - m);
             l[a] = l[a] * expf(mx[a] - m) + sum;
             mx[a] = m;
         }
         __syncthreads();
     }
-    float inv[4];
+    tile_copy<HD>(buf, L::CP, vh, v_ld, min(AT, N));
+    tile_commit();
+    float inv[2];
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        float m = mx[a];
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const float sum = lanes16_sum(l[a] * expf(mx[a] - m));
-        mx[a] = m;
-        inv[a] = 4 * ty + a < ni ? 1.0f / sum : 0.f;
+    for (int a = 0; a < 2; ++a) {
+        float m = fmaxf(mx[a], __shfl_xor_sync(0xffffffffu, mx[a], 1));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+        const float sum = quad_sum(l[a] * expf(mx[a] - m));
+        mx[a] = m; l[a] = sum;
+        if ((lane & 3) == 0) { stat[0][half][r0 + 8 * a] = m; stat[1][half][r0 + 8 * a] = sum; }
     }
-    float o[4][HD / 16];
+    __syncthreads();
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int c = 0; c < HD / 16; ++c) o[a][c] = 0.f;
+    for (int a = 0; a < 2; ++a) {
+        const int i = r0 + 8 * a;
+        const float m0 = stat[0][0][i], m1 = stat[0][1][i], m = fmaxf(m0, m1);
+        mx[a] = m;
+        inv[a] = i < ni ? 1.0f / (stat[1][0][i] * expf(m0 - m) + stat[1][1][i] * expf(m1 - m)) : 0.f;
+    }
+    float o[HD / 16][4] = {};
     for (int jt = 0; jt <= it; ++jt) {
-        const int j0 = jt * AT, nj = min(AT, N - j0);
-        load_rows<HD>(Vs, v + (row0 + j0) * v_ld + (size_t)kvh * HD, v_ld, nj);
+        const int j0 = jt * AT;
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int i = 4 * ty + a, j = j0 + 4 * tx + b;
-                float p = 0.f;
-                if (i < ni && j < N) {
-                    if (j <= i0 + i) p = expf(pr[(size_t)i * N + j] - mx[a]) * inv[a];
-                    pr[(size_t)i * N + j] = p;
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int i = r0 + 8 * a, c = c0 + 8 * n + b, j = j0 + c;
+                    float p = 0.f;
+                    if (i < ni && j < N) {
+                        if (j <= i0 + i) p = expf(pr[(size_t)i * N + j] - mx[a]) * inv[a];
+                        pr[(size_t)i * N + j] = p;
+                    }
+                    P[i * L::PP + c] = p;
                 }
-                P[i * ATP + 4 * tx + b] = p;
-            }
+        if (jt < it) {
+            tile_copy<HD>(buf + ((jt + 1) & 1) * L::BUF, L::CP, vh + (size_t)(j0 + AT) * v_ld, v_ld, min(AT, N - j0 - AT));
+            tile_commit();
+            tile_wait<1>();
+        } else tile_wait<0>();
         __syncthreads();
-        tile_wb_add<HD, false>(P, Vs, nj, ty, tx, o);
+        mma_add_apart<HD / 16>(o, P + rw * L::PP, L::PP, 1, buf + (jt & 1) * L::BUF + half * (HD / 2), L::CP, 1, AT);
         __syncthreads();
     }
     const int ahead = min((it + 1) * AT, N);                   // columns that no row of the tile sees
-    for (int i = threadIdx.x / 32; i < ni; i += 8)
-        for (int j = ahead + threadIdx.x % 32; j < N; j += 32) pr[(size_t)i * N + j] = 0.f;
+    for (int i = warp; i < ni; i += ATT_THREADS / 32)
+        for (int j = ahead + lane; j < N; j += 32) pr[(size_t)i * N + j] = 0.f;
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int i = 4 * ty + a;
+    for (int a = 0; a < 2; ++a) {
+        const int i = r0 + 8 * a;
         if (i >= ni) continue;
-        const size_t base = ((row0 + i0 + i) * n_q + h) * HD + (HD / 16) * tx;
+        const size_t base = ((row0 + i0 + i) * n_q + h) * HD + half * (HD / 2) + 2 * (lane & 3);
 #pragma unroll
-        for (int c = 0; c < HD / 16; ++c) {
-            if (out) out[base + c] = o[a][c];
-            if (out_h) out_h[base + c] = __float2half_rn(o[a][c]);
-        }
+        for (int n = 0; n < HD / 16; ++n)
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                if (out) out[base + 8 * n + b] = o[n][2 * a + b];
+                if (out_h) out_h[base + 8 * n + b] = __float2half_rn(o[n][2 * a + b]);
+            }
     }
 }
 
 // d_score = p * (dO . V - sum_j p_j (dO . V_j)) * scale, and dQ = d_score . K, for 64 queries of a head.
 template <int HD>
-__global__ void __launch_bounds__(256)
-attn_bwd_dq_long_kernel(const float *d_out, const float *probs, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q,
-                        int n_kv, float scale, float *d_score, float *dqkv, long long ld)
+__global__ void __launch_bounds__(ATT_THREADS)
+attn_bwd_dq_kernel(const float *d_out, const float *probs, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q,
+                   int n_kv, float scale, float *d_score, float *dqkv, long long ld)
 {
+    using L = AttnTiles<HD>;
     extern __shared__ __align__(16) float sh[];
-    float *Ot = sh, *Vt = Ot + HD * ATP, *Ks = Vt, *G = Vt + HD * ATP;
+    __shared__ float stat[2][AT];
+    float *O = sh, *G = sh, *buf = sh + AT * L::RP;
     const int it = (N + AT - 1) / AT - 1 - (int)blockIdx.x / n_seq, s = blockIdx.x % n_seq, h = blockIdx.y, kvh = h / (n_q / n_kv);
     const size_t row0 = (size_t)s * N;
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, i0 = it * AT, ni = min(AT, N - i0);
-    load_transposed<HD>(Ot, d_out + ((row0 + i0) * n_q + h) * HD, (long long)n_q * HD, ni);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rw = (warp & 3) * 16, half = warp >> 2;
+    const int i0 = it * AT, ni = min(AT, N - i0), r0 = rw + (lane >> 2), c0 = half * 32 + 2 * (lane & 3);
+    const float *kh = k + (row0 * n_kv + kvh) * HD, *vh = v + row0 * v_ld + (size_t)kvh * HD;
     const size_t tile_rows = (((size_t)s * n_q + h) * N + i0) * N;
     const float *pr = probs + tile_rows;
     float *ds = d_score + tile_rows;
-    float dp[4] = {0.f, 0.f, 0.f, 0.f};
+
+    tile_copy<HD>(O, L::RP, d_out + ((row0 + i0) * n_q + h) * HD, (long long)n_q * HD, ni);
+    tile_copy<HD>(buf, L::RP, vh, v_ld, min(AT, N));
+    tile_commit();
+    float dp[2] = {0.f, 0.f};
     for (int jt = 0; jt <= it; ++jt) {
         const int j0 = jt * AT;
-        load_transposed<HD>(Vt, v + (row0 + j0) * v_ld + (size_t)kvh * HD, v_ld, min(AT, N - j0));
+        if (jt < it) {
+            tile_copy<HD>(buf + ((jt + 1) & 1) * L::BUF, L::RP, vh + (size_t)(j0 + AT) * v_ld, v_ld, min(AT, N - j0 - AT));
+            tile_commit();
+            tile_wait<1>();
+        } else tile_wait<0>();
         __syncthreads();
-        float acc[4][4];
-        tile_abt<HD>(Ot, Vt, ty, tx, acc);
+        float acc[4][4] = {};
+        mma_add<4>(acc, O + rw * L::RP, L::RP, 1, buf + (jt & 1) * L::BUF + half * 32 * L::RP, 1, L::RP, HD);
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int i = 4 * ty + a, j = j0 + 4 * tx + b;
-                if (i < ni && j <= i0 + i) {
-                    ds[(size_t)i * N + j] = acc[a][b];
-                    dp[a] = fmaf(pr[(size_t)i * N + j], acc[a][b], dp[a]);
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int i = r0 + 8 * a, j = j0 + c0 + 8 * n + b;
+                    if (i < ni && j <= i0 + i) {
+                        ds[(size_t)i * N + j] = acc[n][2 * a + b];
+                        dp[a] = fmaf(pr[(size_t)i * N + j], acc[n][2 * a + b], dp[a]);
+                    }
                 }
-            }
         __syncthreads();
     }
+    tile_copy<HD>(buf, L::CP, kh, (long long)n_kv * HD, min(AT, N));
+    tile_commit();
 #pragma unroll
-    for (int a = 0; a < 4; ++a) dp[a] = lanes16_sum(dp[a]);
-    float o[4][HD / 16];
+    for (int a = 0; a < 2; ++a) {
+        dp[a] = quad_sum(dp[a]);
+        if ((lane & 3) == 0) stat[half][r0 + 8 * a] = dp[a];
+    }
+    __syncthreads();
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-        for (int c = 0; c < HD / 16; ++c) o[a][c] = 0.f;
+    for (int a = 0; a < 2; ++a) dp[a] = stat[0][r0 + 8 * a] + stat[1][r0 + 8 * a];
+    float o[HD / 16][4] = {};
     for (int jt = 0; jt <= it; ++jt) {
-        const int j0 = jt * AT, nj = min(AT, N - j0);
-        load_rows<HD>(Ks, k + ((row0 + j0) * n_kv + kvh) * HD, (long long)n_kv * HD, nj);
+        const int j0 = jt * AT;
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int a = 0; a < 2; ++a)
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const int i = 4 * ty + a, j = j0 + 4 * tx + b;
-                float g = 0.f;
-                if (i < ni && j < N) {
-                    if (j <= i0 + i) g = pr[(size_t)i * N + j] * (ds[(size_t)i * N + j] - dp[a]) * scale;
-                    ds[(size_t)i * N + j] = g;
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int i = r0 + 8 * a, c = c0 + 8 * n + b, j = j0 + c;
+                    float g = 0.f;
+                    if (i < ni && j < N) {
+                        if (j <= i0 + i) g = pr[(size_t)i * N + j] * (ds[(size_t)i * N + j] - dp[a]) * scale;
+                        ds[(size_t)i * N + j] = g;
+                    }
+                    G[i * L::PP + c] = g;
                 }
-                G[i * ATP + 4 * tx + b] = g;
-            }
+        if (jt < it) {
+            tile_copy<HD>(buf + ((jt + 1) & 1) * L::BUF, L::CP, kh + (size_t)(j0 + AT) * n_kv * HD, (long long)n_kv * HD, min(AT, N - j0 - AT));
+            tile_commit();
+            tile_wait<1>();
+        } else tile_wait<0>();
         __syncthreads();
-        tile_wb_add<HD, false>(G, Ks, nj, ty, tx, o);
+        mma_add_apart<HD / 16>(o, G + rw * L::PP, L::PP, 1, buf + (jt & 1) * L::BUF + half * (HD / 2), L::CP, 1, AT);
         __syncthreads();
     }
     const int ahead = min((it + 1) * AT, N);
-    for (int i = threadIdx.x / 32; i < ni; i += 8)
-        for (int j = ahead + threadIdx.x % 32; j < N; j += 32) ds[(size_t)i * N + j] = 0.f;
+    for (int i = warp; i < ni; i += ATT_THREADS / 32)
+        for (int j = ahead + lane; j < N; j += 32) ds[(size_t)i * N + j] = 0.f;
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int i = 4 * ty + a;
+    for (int a = 0; a < 2; ++a) {
+        const int i = r0 + 8 * a;
         if (i >= ni) continue;
-        float *dst = dqkv + (row0 + i0 + i) * ld + (size_t)h * HD + (HD / 16) * tx;
+        float *dst = dqkv + (row0 + i0 + i) * ld + (size_t)h * HD + half * (HD / 2) + 2 * (lane & 3);
 #pragma unroll
-        for (int c = 0; c < HD / 16; ++c) dst[c] = o[a][c];
+        for (int n = 0; n < HD / 16; ++n) { dst[8 * n] = o[n][2 * a]; dst[8 * n + 1] = o[n][2 * a + 1]; }
     }
 }
 
 // 64 keys x 64 columns of dK (d_score^T . Q) or dV (P^T . dO) of a KV head: summed over the later queries of each query head, then
 // over the heads in order. blockIdx.y = ((kv head * 2 + dK / dV) * (HD / 64) + columns).
-__global__ void __launch_bounds__(256)
-attn_bwd_dkv_long_kernel(const float *d_score, const float *probs, const float *q, const float *d_out, int n_seq, int N, int n_q, int n_kv,
-                         int hd, float *dqkv, long long ld)
+__global__ void __launch_bounds__(ATT_THREADS)
+attn_bwd_dkv_kernel(const float *d_score, const float *probs, const float *q, const float *d_out, int n_seq, int N, int n_q, int n_kv,
+                    int hd, float *dqkv, long long ld)
 {
-    __shared__ __align__(16) float W[AT * ATP], B[AT * ATP];
+    constexpr int CP = AT + 8, BUF = AT * CP;
+    extern __shared__ __align__(16) float sh[];               // two buffers of (weights, rows)
     const int jt = blockIdx.x / n_seq, s = blockIdx.x % n_seq, slices = hd / 64, slice = blockIdx.y % slices;
     const int which = (blockIdx.y / slices) & 1, kvh = blockIdx.y / (2 * slices), group = n_q / n_kv;
     const size_t row0 = (size_t)s * N;
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, j0 = jt * AT, nj = min(AT, N - j0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rw = (warp & 3) * 16, half = warp >> 2;
+    const int j0 = jt * AT, nj = min(AT, N - j0), tiles = (N - j0 + AT - 1) / AT, steps = group * tiles;
+    auto stage = [&](int t) {
+        const int h = kvh * group + t / tiles, i0 = j0 + t % tiles * AT, ni = min(AT, N - i0);
+        float *w = sh + (t & 1) * 2 * BUF;
+        tile_copy<AT>(w, CP, (which ? probs : d_score) + ((size_t)s * n_q + h) * N * N + (size_t)i0 * N + j0, N, ni, nj);
+        tile_copy<AT>(w + BUF, CP, (which ? d_out : q) + ((row0 + i0) * n_q + h) * hd + slice * 64, (long long)n_q * hd, ni);
+        tile_commit();
+    };
+    stage(0);
     float sum[4][4] = {};
-    for (int g = 0; g < group; ++g) {
-        const int h = kvh * group + g;
-        const float *w = (which ? probs : d_score) + ((size_t)s * n_q + h) * N * N + j0;
-        const float *b = (which ? d_out : q) + (row0 * n_q + h) * hd + slice * 64;
-        float acc[4][4] = {};
-        for (int i0 = j0; i0 < N; i0 += AT) {
-            const int ni = min(AT, N - i0);
-            float wr[AT * AT / 256], br[AT * AT / 256];
-#pragma unroll
-            for (int e = 0; e < AT * AT / 256; ++e) {          // all loads of a tile pair in flight, under the previous product
-                const int i = e * 4 + threadIdx.x / 64, c = threadIdx.x % 64;
-                wr[e] = i < ni && c < nj ? w[(size_t)(i0 + i) * N + c] : 0.f;
-                br[e] = i < ni ? b[(size_t)(i0 + i) * n_q * hd + c] : 0.f;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int e = 0; e < AT * AT / 256; ++e) {
-                const int i = e * 4 + threadIdx.x / 64, c = threadIdx.x % 64;
-                W[i * ATP + c] = wr[e];
-                B[i * ATP + c] = br[e];
-            }
-            __syncthreads();
-            tile_abt_add<AT>(W, B, ty, tx, acc);
-        }
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) sum[a][c] += acc[a][c];
+    for (int t = 0; t < steps; ++t) {
+        if (t + 1 < steps) { stage(t + 1); tile_wait<1>(); }
+        else tile_wait<0>();
+        __syncthreads();
+        const float *w = sh + (t & 1) * 2 * BUF;
+        mma_add_apart<4>(sum, w + rw, 1, CP, w + BUF + half * 32, CP, 1, AT);
+        __syncthreads();
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        const int j = 4 * ty + a;
+    for (int a = 0; a < 2; ++a) {
+        const int j = rw + (lane >> 2) + 8 * a;
         if (j >= nj) continue;
-        float *dst = dqkv + (row0 + j0 + j) * ld + (size_t)(n_q + (which ? n_kv : 0) + kvh) * hd + slice * 64 + 4 * tx;
+        float *dst = dqkv + (row0 + j0 + j) * ld + (size_t)(n_q + (which ? n_kv : 0) + kvh) * hd + slice * 64 + half * 32 + 2 * (lane & 3);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) dst[c] = sum[a][c];
+        for (int n = 0; n < 4; ++n) { dst[8 * n] = sum[n][2 * a]; dst[8 * n + 1] = sum[n][2 * a + 1]; }
     }
 }
 
@@ -1261,17 +1126,10 @@ template <int HD>
 static int attn_fwd_launch(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q,
                            int n_kv, float scale, float *probs, float *out, __half *out_h, cudaStream_t st)
 {
-    if constexpr (HD <= 128) if (N <= AT) {                   // short sequences: one block per (sequence, head)
-        const size_t tsm = ((size_t)2 * HD * ATP + (size_t)AT * ATP) * sizeof(float);
-        int rc = opt_in_smem(attn_fwd_tile_kernel<HD>, tsm);
-        if (rc) return rc;
-        attn_fwd_tile_kernel<HD><<<n_seq * n_q, 256, tsm, st>>>(q, k, v, v_ld, N, n_q, n_kv, scale, probs, out, out_h);
-        return done();
-    }
-    const size_t smem = ((size_t)2 * HD * ATP + (size_t)AT * ATP) * sizeof(float);
-    int rc = opt_in_smem(attn_fwd_long_kernel<HD>, smem);
+    constexpr size_t smem = AttnTiles<HD>::bytes;
+    int rc = opt_in_smem(attn_fwd_kernel<HD>, smem);
     if (rc) return rc;
-    attn_fwd_long_kernel<HD><<<dim3((N + AT - 1) / AT * n_seq, n_q), 256, smem, st>>>(q, k, v, v_ld, n_seq, N, n_q, n_kv, scale, probs, out, out_h);
+    attn_fwd_kernel<HD><<<dim3((N + AT - 1) / AT * n_seq, n_q), ATT_THREADS, smem, st>>>(q, k, v, v_ld, n_seq, N, n_q, n_kv, scale, probs, out, out_h);
     return done();
 }
 
@@ -1301,28 +1159,15 @@ static int attn_bwd_launch(const float *d_out, const float *probs, const float *
                            long long v_ld, int n_seq, int N, int n_q, int n_kv, float scale, float *d_score,
                            float *dqkv, long long ld, cudaStream_t st)
 {
-    if constexpr (HD <= 128) if (N <= AT) {
-        // d_score is used as the per-head dK/dV scratch [S][n_q][N][2][HD] here
-        const size_t tsm = ((size_t)2 * HD * ATP + (size_t)2 * AT * ATP) * sizeof(float);
-        int rc = opt_in_smem(attn_bwd_tile_kernel<HD>, tsm);
-        if (rc) return rc;
-        attn_bwd_tile_kernel<HD><<<n_seq * n_q, 256, tsm, st>>>(d_out, probs, q, k, v, v_ld, N, n_q, n_kv, scale, dqkv, ld,
-                                                                d_score);
-        rc = done();
-        if (rc) return rc;
-        const size_t total = (size_t)n_seq * N * n_kv * 2 * HD;
-        const unsigned grid = (unsigned)((total + 255) / 256 < 148 * 8 ? (total + 255) / 256 : 148 * 8);
-        attn_bwd_reduce_kernel<<<grid, 256, 0, st>>>(d_score, n_seq, N, n_q, n_kv, HD, dqkv, ld);
-        return done();
-    }
-    const size_t smem = ((size_t)2 * HD * ATP + (size_t)AT * ATP) * sizeof(float);
-    int rc = opt_in_smem(attn_bwd_dq_long_kernel<HD>, smem);
+    constexpr size_t smem = AttnTiles<HD>::bytes, smem_kv = 4 * (size_t)AT * (AT + 8) * sizeof(float);
+    int rc = opt_in_smem(attn_bwd_dq_kernel<HD>, smem);
+    if (!rc) rc = opt_in_smem(attn_bwd_dkv_kernel, smem_kv);
     if (rc) return rc;
     const int tiles = (N + AT - 1) / AT;
-    attn_bwd_dq_long_kernel<HD><<<dim3(tiles * n_seq, n_q), 256, smem, st>>>(d_out, probs, k, v, v_ld, n_seq, N, n_q, n_kv, scale, d_score, dqkv, ld);
+    attn_bwd_dq_kernel<HD><<<dim3(tiles * n_seq, n_q), ATT_THREADS, smem, st>>>(d_out, probs, k, v, v_ld, n_seq, N, n_q, n_kv, scale, d_score, dqkv, ld);
     rc = done();
     if (rc) return rc;
-    attn_bwd_dkv_long_kernel<<<dim3(tiles * n_seq, n_kv * 2 * (HD / 64)), 256, 0, st>>>(d_score, probs, q, d_out, n_seq, N, n_q, n_kv, HD, dqkv, ld);
+    attn_bwd_dkv_kernel<<<dim3(tiles * n_seq, n_kv * 2 * (HD / 64)), ATT_THREADS, smem_kv, st>>>(d_score, probs, q, d_out, n_seq, N, n_q, n_kv, HD, dqkv, ld);
     return done();
 }
 

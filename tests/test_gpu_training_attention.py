@@ -1,0 +1,57 @@
+"""Training attention forward and backward over tile edges, against float64.
+
+Bar: operands are split into TF32 pairs (22 bits) and sums of up to hd, 64 or N terms are fp32, truncated per eight terms: max(hd, 64) / 8 x 3 x 2^-24
+of the terms bounds a tile's, fp32 adds join the tiles; 1e-6 measured in 2-norm over a tensor, 5e-6."""
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("S,N,Hq,Hkv,shift", [(1, 1, 2, 1, 0), (2, 63, 4, 2, 0), (3, 64, 2, 2, 0), (1, 65, 4, 1, 1), (2, 200, 4, 2, 0), (1, 509, 8, 2, 0)])
+def test_forward_and_backward(lib, hd, S, N, Hq, Hkv, shift):
+    g = torch.Generator().manual_seed(N + hd)
+    M, G, scale, ld = S * N, Hq // Hkv, hd ** -0.5, (Hq + 2 * Hkv) * hd + 4
+    qkv = torch.randn(M, ld, generator=g).cuda()
+
+    def off(*shape):                                          # `shift` floats off a 16-byte boundary, where that was taken before
+        t = torch.zeros(shape[0] * shape[1] + shift, device="cuda")[shift:].view(*shape)
+        t.copy_(torch.randn(*shape, generator=g))
+        return t
+    q, k, d_out = off(M, Hq * hd), torch.randn(M, Hkv * hd, generator=g).cuda(), off(M, Hq * hd) * 1e-3
+    if shift:
+        d_out = off(M, Hq * hd)
+        d_out *= 1e-3
+    v = qkv[:, (Hq + Hkv) * hd:]
+    probs, out = torch.full((S, Hq, N, N), 7.0, device="cuda"), torch.full((M, Hq * hd), 7.0, device="cuda")
+    half = torch.zeros(M, Hq * hd, dtype=torch.float16, device="cuda")
+    assert lib.b200_attn_train_fwd_h(q.data_ptr(), k.data_ptr(), v.data_ptr(), ld, S, N, Hq, Hkv, hd, scale, probs.data_ptr(), out.data_ptr(),
+                                     half.data_ptr(), None) == 0
+    dqkv = torch.full((M, ld), 7.0, device="cuda")
+    d_score = torch.full((S * Hq * N * max(N, 2 * hd),), float("nan"), device="cuda")
+    assert lib.b200_attn_train_bwd(d_out.data_ptr(), probs.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), ld, S, N, Hq, Hkv, hd, scale,
+                                   d_score.data_ptr(), dqkv.data_ptr(), ld, None) == 0
+    torch.cuda.synchronize()
+
+    def heads(t, n):
+        return t.double().reshape(S, N, n, hd).transpose(1, 2)
+    Q, K, V = (t.detach().clone().requires_grad_() for t in (heads(q, Hq), heads(k, Hkv), heads(v[:, : Hkv * hd], Hkv)))
+    s = Q @ K.repeat_interleave(G, 1).transpose(-1, -2) * scale
+    p = torch.softmax(s.masked_fill(torch.ones(N, N, device="cuda").triu(1).bool(), -torch.inf), -1)
+    o = p @ V.repeat_interleave(G, 1)
+    o.backward(heads(d_out, Hq))
+
+    def rows(t):
+        return t.transpose(1, 2).reshape(M, -1)
+    assert rel(probs, p.detach()) < 5e-6 and (probs.triu(1) == 0).all()
+    assert rel(out, rows(o.detach())) < 5e-6 and torch.equal(half, out.half())
+    got = [dqkv[:, :Hq * hd], dqkv[:, Hq * hd:(Hq + Hkv) * hd], dqkv[:, (Hq + Hkv) * hd:(Hq + 2 * Hkv) * hd]]
+    for name, a, b in zip("qkv", got, (Q.grad, K.grad, V.grad)):
+        size = 1e-3 * (hd * N) ** 0.5                          # one position: dQ and dK are zero up to rounding
+        assert float((a.double() - rows(b)).norm()) <= 5e-6 * float(rows(b).norm()) + 1e-7 * size, name
+    assert (dqkv[:, (Hq + 2 * Hkv) * hd:] == 7.0).all()
