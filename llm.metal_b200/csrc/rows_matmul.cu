@@ -337,7 +337,8 @@ rows_matmul_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 // ---- host side ---------------------------------------------------------------------------------
 
 // Additions to one accumulator: each truncates at 2^-24 of it, so a sum of n is off by about n 2^-25. Rows of 2560 .. 9728 columns:
-// 5e-6 of a result at 600 additions and more, 1e-6 .. 3e-6 within this limit.
+// 5e-6 of a result at 600 additions and more, 1e-6 .. 3e-6 within this limit. (480 let wide Q8_0 tiles run two on an SM, 160 us instead of
+// 223 for 19456 x 2560 x 512, but moved whole prompts from 5.0e-5 to 5.3e-5 off 64 bits.)
 constexpr int MAX_CHAIN = 256;
 constexpr int SMEM_ONE = 220 * 1024, SMEM_TWO = 108 * 1024;      // one block on an SM, or two
 
@@ -371,8 +372,10 @@ bool place_tile(bool q8, int bn, int planes, bool two, Shape *o)
 
 // Tile width, blocks per tile and blocks per SM: the least modelled time. A step of 64 columns takes as long as the slowest of
 // its products (2 clocks a column and product), its operand bytes (an SM takes in about 52 a clock) and,
-// for Q8_0, making the weight tile; a block costs some 3000 clocks beside its steps, and its result goes out
-// at a few clocks a column.
+// for Q8_0, making the weight tile. A block costs some 3000 clocks beside its steps and its result goes out at 8 clocks a column; in
+// several waves of F16 tiles twice that with one block on an SM, and half of it with two, where one's start and end lie under the other's steps
+// (two Q8_0 blocks have tensor memory for narrow tiles only, which gains nothing).
+// Measured, F16, 1531 rows: 19456 x 2560 with one block of 224 columns 332 us, two of 128 291 us; 6144 x 2560 115 and 92 us.
 Shape pick_shape(bool q8, int rows, int cols, int n, int planes, int sms)
 {
     const int mt = (rows + WM - 1) / WM, nkb = (cols + KB - 1) / KB;
@@ -402,7 +405,10 @@ Shape pick_shape(bool q8, int rows, int cols, int n, int planes, int sms)
                 const long long waves = (blocks + place - 1) / place;
                 // two blocks share an SM's time unless the last wave leaves most SMs one block
                 const double share = two ? (waves > 1 || blocks > sms * 3 / 2 ? 2.0 : blocks > sms ? 1.0 + (double)(blocks - sms) / sms : 1.0) : 1.0;
-                const double cost = waves * (share * per * step * (sh.slots < 3 ? 1.1 : 1.0) + 3000.0 + bn * 8.0 + (s > 1 ? 1500.0 + bn * 4.0 : 0.0));
+                const bool under = !q8 && two && s == 1 && waves > 1;
+                const double ends = (under ? 0.5 : !q8 && waves > 1 ? 2.0 : 1.0) * (3000.0 + bn * 8.0) + (s > 1 ? 1500.0 + bn * 4.0 : 0.0);
+                const double each = under && step > 2.0 * bn * products ? step * 52.0 / 56.0 : step;       // they keep the SM's port busier, too
+                const double cost = waves * (share * per * each * (sh.slots < 3 && !under ? 1.1 : 1.0) + ends);
                 if (cost < least) { least = cost; best = sh; best.bn = bn; best.splits = s; best.two = two; }
             }
         }
