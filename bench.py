@@ -5,7 +5,7 @@
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N ... bench.py --gpus N ...
 
 One step = one generate request of the workload (prompt 512, generate 512): a
-token-by-token prefill (untimed, as in the reference's own metric) followed by
+prefill (untimed, as in the reference's own metric) followed by
 511 decode forwards (timed). Weights are seeded random N(0, 0.02) of the named
 architecture, quantised to Q8_0 on the GPU; token ids are uniform random.
 
