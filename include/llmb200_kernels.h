@@ -599,6 +599,8 @@ int b200_rows_norm_planes(float *x, int rows, int dim, const float *y, const flo
 /* out = planes of act(gate) * up for rows of 2 * inter values: (gate, up) pairs, or all gates and then all ups. */
 int b200_rows_glu_planes(const float *gu, int rows, int inter, int pairs, int gelu, const b200_row_planes *out, void *stream);
 int b200_rows_split_planes(const float *x, int rows, int dim, const b200_row_planes *out, void *stream);
+/* out [rows][dim]: row m is row index[m] of x. */
+int b200_rows_gather(const float *x, int rows, int dim, const int *index, float *out, void *stream);
 
 /* Attention of n_rows / seq_len sequences' new tokens, positions pos0 .. pos0 + seq_len - 1, over their binary16 caches:
  * per-head norms, rotation, cache rows, then the sums; fp32 accuracy. */

@@ -259,7 +259,7 @@ SYMBOLS_MAIN = {
                           "b200_rows_postnorm", "b200_rows_norm", "b200_rows_gelu_mul", "b200_rows_softcap",
                           "b200_gqa_splits", "b200_gqa_decode", "b200_gqa_rows_prep", "b200_gqa_rows_attend", "b200_gla_decode", "b200_gla_rows",
                           "b200_rows_streams", "b200_rows_start", "b200_rows_layer_norm", "b200_rows_matmul", "b200_q8_row_scale",
-                          "b200_rows_norm_planes", "b200_rows_glu_planes", "b200_rows_split_planes", "b200_rows_attn"],
+                          "b200_rows_norm_planes", "b200_rows_glu_planes", "b200_rows_split_planes", "b200_rows_gather", "b200_rows_attn"],
     "llmb200_inference.h": ["inference_state_create", "inference_state_create_gemma3", "inference_state_free",
                             "inference_generate", "inference_state_model_type", "inference_state_vocab_size",
                             "inference_state_reset", "inference_forward_token", "inference_state_load_eos",
@@ -382,6 +382,7 @@ def lib():
         "b200_rows_norm_planes": (i, [vp, i, i, vp, vp, vp, vp, fl, C.POINTER(RowPlanes), vp]),
         "b200_rows_glu_planes": (i, [vp, i, i, i, i, C.POINTER(RowPlanes), vp]),
         "b200_rows_split_planes": (i, [vp, i, i, C.POINTER(RowPlanes), vp]),
+        "b200_rows_gather": (i, [vp, i, i, vp, vp, vp]),
         "b200_rows_attn": (i, [C.POINTER(RowsAttnArgs), vp]),
         "b200_gqa_splits": (i, [i, i, i, i, i, i]), "b200_gqa_decode": (i, [C.POINTER(GqaArgs), vp]),
         "b200_gqa_rows_prep": (i, [C.POINTER(GqaArgs), vp]), "b200_gqa_rows_attend": (i, [C.POINTER(GqaArgs), vp]),

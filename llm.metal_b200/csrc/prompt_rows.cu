@@ -170,6 +170,15 @@ rows_split_kernel(const float *x, int dim, const b200_row_planes o)
     for (int i = blockIdx.y * ROW_THREADS + threadIdx.x; i < n4; i += gridDim.y * ROW_THREADS) put4(o, m, i, xr[i], up);
 }
 
+__global__ void __launch_bounds__(ROW_THREADS) rows_gather_kernel(const float *x, int dim, const int *index, float *out)
+{
+    pdl_launch_dependents();
+    pdl_wait();
+    const float4 *src = reinterpret_cast<const float4 *>(x + (long long)index[blockIdx.x] * dim);
+    float4 *dst = reinterpret_cast<float4 *>(out + (long long)blockIdx.x * dim);
+    for (int i = threadIdx.x; i < dim >> 2; i += ROW_THREADS) dst[i] = src[i];
+}
+
 // One warp per (row, head): query heads are normed, rotated and stored as two planes with a factor per row and head; key heads
 // are normed and rotated into the binary16 cache, value heads copied there.
 template <int HD>
@@ -491,6 +500,14 @@ extern "C" int b200_rows_split_planes(const float *x, int rows, int dim, const b
     ++g_b200_launches;
     return (int)launch_chained(rows_split_kernel, dim3(rows, out->d_scale ? 1 : share_row(rows, dim)), dim3(ROW_THREADS), 0, (cudaStream_t)stream,
                                x, dim, *out);
+}
+
+extern "C" int b200_rows_gather(const float *x, int rows, int dim, const int *index, float *out, void *stream)
+{
+    if (!x || !index || !out || rows <= 0 || dim <= 0 || (dim & 3) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15))
+        return B200_E_BADARG;
+    ++g_b200_launches;
+    return (int)launch_chained(rows_gather_kernel, dim3(rows), dim3(ROW_THREADS), 0, (cudaStream_t)stream, x, dim, index, out);
 }
 
 extern "C" int b200_rows_attn(const b200_rows_attn_args *a, void *stream)

@@ -298,7 +298,7 @@ static int prefill_rows(BState *s, const uint32_t *prompts, int stride, int n)
         for (int b = 0; b < B; ++b) memcpy(ids + (size_t)b * T, prompts + (size_t)b * stride + t0, (size_t)T * 4);
         CU_TRY(cudaMemcpyAsync(s->d_prompt, ids, (size_t)B * T * 4, cudaMemcpyHostToDevice, g_rt.stream), rc = -1);
         if (rc == 0) K_TRY(b200_embed_rows(s->emb, s->d_prompt, B * T, D, s->V, 1.0f, r->x, g_rt.stream), rc = -1);
-        if (rc == 0) rc = llmb200_plain_rows_run(r, layers, s->L, B * T, T, t0, (long long)s->Hkv * s->hd * s->max_seq, 1);
+        if (rc == 0) rc = llmb200_plain_rows_run(r, layers, s->L, B * T, T, t0, (long long)s->Hkv * s->hd * s->max_seq, NULL, 0);
         if (rc == 0) CU_TRY(cudaStreamSynchronize(g_rt.stream), rc = -1);              /* ids are reused */
     }
     free(layers);

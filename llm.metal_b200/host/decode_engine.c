@@ -1105,7 +1105,7 @@ static int prompt_ready(InferenceState *s, int n)
         r->d_err = (unsigned *)s->d_err;
         m->layers = calloc((size_t)s->L, sizeof(RowsLayer));
         m->logits = llmb200_dev_zero((size_t)PROMPT_WANT * s->V * 4);
-        m->d_want = (int *)llmb200_dev_zero(PROMPT_WANT * 4);
+        m->d_want = (int *)llmb200_dev_zero(PROMPT_CHUNK * 4);
         size_t rows = (size_t)s->lm.rows;
         for (int l = 0; l < s->L; ++l) {
             const Layer *y = &s->layers[l];
@@ -1162,17 +1162,19 @@ static int prompt_rows(InferenceState *s, const uint32_t *tokens, int n, const i
         K_TRY(b200_embed_rows(s->emb, (const uint32_t *)(s->d_tokens + pos0), M, s->D, s->V, s->emb_scale, r->x, g_rt.stream), return -1);
         int last = w;
         while (last < n_want && want[last] < c0 + M) ++last;
-        if (llmb200_plain_rows_run(r, m->layers, s->L, M, M, pos0, 0, last == w) != 0) return -1;
-        for (int first = 1; w < last; first = 0) {
-            int index[PROMPT_WANT], k = 0;
-            for (; k < PROMPT_WANT && w + k < last; ++k) index[k] = want[w + k] - c0;
-            CU_TRY(cudaMemcpyAsync(m->d_want, index, (size_t)k * 4, cudaMemcpyHostToDevice, g_rt.stream), return -1);
-            if (llmb200_plain_rows_last(r, &m->layers[s->L - 1], s->g_final, m->d_want, k, first ? M : 0) != 0) return -1;
+        int index[PROMPT_CHUNK];
+        const int n_last = last - w;
+        for (int k = 0; k < n_last; ++k) index[k] = want[w + k] - c0;
+        if (n_last) CU_TRY(cudaMemcpyAsync(m->d_want, index, (size_t)n_last * 4, cudaMemcpyHostToDevice, g_rt.stream), return -1);
+        if (llmb200_plain_rows_run(r, m->layers, s->L, M, M, pos0, 0, m->d_want, n_last) != 0) return -1;
+        for (int first = 0; first < n_last; first += PROMPT_WANT) {
+            const int k = n_last - first < PROMPT_WANT ? n_last - first : PROMPT_WANT;
+            if (llmb200_plain_rows_last(r, &m->layers[s->L - 1], s->g_final, first, k) != 0) return -1;
             if (llmb200_plain_rows_product(r, &m->lm, k, m->logits) != 0) return -1;
-            CU_TRY(cudaMemcpyAsync(logits + (size_t)w * s->V, m->logits, (size_t)k * s->V * 4, cudaMemcpyDeviceToHost, g_rt.stream), return -1);
-            CU_TRY(cudaStreamSynchronize(g_rt.stream), return -1);
-            w += k;
+            CU_TRY(cudaMemcpyAsync(logits + (size_t)(w + first) * s->V, m->logits, (size_t)k * s->V * 4, cudaMemcpyDeviceToHost, g_rt.stream), return -1);
         }
+        CU_TRY(cudaStreamSynchronize(g_rt.stream), return -1);        /* index and d_want are reused */
+        w = last;
     }
     CU_TRY(cudaStreamSynchronize(g_rt.stream), return -1);
     return 0;

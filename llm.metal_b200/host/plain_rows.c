@@ -22,22 +22,22 @@ int llmb200_plain_rows_ready(PlainRows *r)
     const size_t n = (size_t)r->cap, heads = (size_t)r->Hq * r->hd;
     size_t widest = (size_t)(r->IS > r->D ? r->IS : r->D);
     if (heads > widest) widest = heads;
-    r->x = device(n * r->D * 4); r->y = device(n * r->D * 4);
+    r->x = device(n * r->D * 4); r->y = device(n * r->D * 4); r->last = device(n * r->D * 4);
     r->qkv = device(n * (heads + 2 * (size_t)r->Hkv * r->hd) * 4);
     r->attn = device(n * heads * 4);
     r->gu = device(n * 2 * r->IS * 4);
     r->x_scale = device(n * 4); r->q_scale = device(n * r->Hq * 4);
     r->xh = device(n * widest * 2 * r->planes);
     r->q = device(n * heads * 2 * 2);
-    if (!r->x || !r->y || !r->qkv || !r->attn || !r->gu || !r->x_scale || !r->q_scale || !r->xh || !r->q) { llmb200_plain_rows_free(r); return -1; }
+    if (!r->x || !r->y || !r->last || !r->qkv || !r->attn || !r->gu || !r->x_scale || !r->q_scale || !r->xh || !r->q) { llmb200_plain_rows_free(r); return -1; }
     return 0;
 }
 
 void llmb200_plain_rows_free(PlainRows *r)
 {
-    void *b[] = { r->x, r->y, r->qkv, r->attn, r->gu, r->x_scale, r->q_scale, r->xh, r->q };
+    void *b[] = { r->x, r->y, r->last, r->qkv, r->attn, r->gu, r->x_scale, r->q_scale, r->xh, r->q };
     for (size_t i = 0; i < sizeof(b) / sizeof(b[0]); ++i) cudaFree(b[i]);
-    r->x = r->y = r->qkv = r->attn = r->gu = r->x_scale = r->q_scale = NULL;
+    r->x = r->y = r->last = r->qkv = r->attn = r->gu = r->x_scale = r->q_scale = NULL;
     r->xh = r->q = NULL;
 }
 
@@ -74,7 +74,7 @@ int llmb200_plain_rows_product(PlainRows *r, const RowsMatrix *m, int n, float *
 }
 
 int llmb200_plain_rows_run(PlainRows *r, const RowsLayer *layers, int n_layers, int n_rows, int seq_len, int pos0, long long cache_seq_stride,
-                           int caches_only)
+                           const int *index, int n_last)
 {
     void *st = g_rt.stream;
     const int heads = r->Hq * r->hd;
@@ -92,10 +92,18 @@ int llmb200_plain_rows_run(PlainRows *r, const RowsLayer *layers, int n_layers, 
         a.d_k_cache = y->k_cache; a.d_v_cache = y->v_cache; a.cache_seq_stride = cache_seq_stride;
         a.d_q = r->q; a.d_q_scale = r->q_scale; a.d_out = r->attn;
         K_TRY(b200_rows_attn(&a, st), return -1);
-        if (caches_only && l == n_layers - 1) return 0;          /* nothing reads what the last layer adds */
-        K_TRY(b200_rows_split_planes(r->attn, n_rows, heads, &p_heads, st), return -1);
+        float *x = r->x, *attn = r->attn;
+        if (l == n_layers - 1) {
+            if (n_last == 0) return 0;
+            /* attention rows go where the query planes were: as many bytes */
+            K_TRY(b200_rows_gather(r->x, n_last, r->D, index, r->last, st), return -1);
+            K_TRY(b200_rows_gather(r->attn, n_last, heads, index, r->q, st), return -1);
+            x = r->last; attn = r->q;
+            n_rows = n_last;
+        }
+        K_TRY(b200_rows_split_planes(attn, n_rows, heads, &p_heads, st), return -1);
         if (llmb200_plain_rows_product(r, &y->o, n_rows, r->y)) return -1;
-        K_TRY(b200_rows_norm_planes(r->x, n_rows, r->D, r->y, r->gemma ? y->g_post_attn : NULL, r->gemma ? y->g_pre_ff : y->g_post_attn,
+        K_TRY(b200_rows_norm_planes(x, n_rows, r->D, r->y, r->gemma ? y->g_post_attn : NULL, r->gemma ? y->g_pre_ff : y->g_post_attn,
                                     NULL, RMS_EPS, &p_model, st), return -1);
         if (llmb200_plain_rows_product(r, &y->gateup, n_rows, r->gu)) return -1;
         K_TRY(b200_rows_glu_planes(r->gu, n_rows, r->IS, r->pairs, r->gemma, &p_inter, st), return -1);
@@ -104,11 +112,10 @@ int llmb200_plain_rows_run(PlainRows *r, const RowsLayer *layers, int n_layers, 
     return 0;
 }
 
-int llmb200_plain_rows_last(PlainRows *r, const RowsLayer *last_layer, const float *g_final, const int *index, int n, int n_rows)
+int llmb200_plain_rows_last(PlainRows *r, const RowsLayer *last_layer, const float *g_final, int first, int n)
 {
     const b200_row_planes p = planes_of(r, r->D);
-    /* first call of a pass: the stream takes the last feed-forward's result in; its planes are not used */
-    if (n_rows > 0) K_TRY(b200_rows_norm_planes(r->x, n_rows, r->D, r->y, r->gemma ? last_layer->g_post_ff : NULL, g_final, NULL, RMS_EPS, &p, g_rt.stream), return -1);
-    K_TRY(b200_rows_norm_planes(r->x, n, r->D, NULL, NULL, g_final, index, RMS_EPS, &p, g_rt.stream), return -1);
+    const size_t at = (size_t)first * r->D;
+    K_TRY(b200_rows_norm_planes(r->last + at, n, r->D, r->y + at, r->gemma ? last_layer->g_post_ff : NULL, g_final, NULL, RMS_EPS, &p, g_rt.stream), return -1);
     return 0;
 }

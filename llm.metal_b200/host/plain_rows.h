@@ -18,19 +18,19 @@ typedef struct {
 typedef struct {
     int D, Hq, Hkv, hd, IS, gemma, pairs, wtype, planes, cap, max_seq;
     unsigned *d_err;
-    float *x, *y, *qkv, *attn, *gu, *x_scale, *q_scale;
+    float *x, *y, *last, *qkv, *attn, *gu, *x_scale, *q_scale;
     void *xh, *q;
 } PlainRows;
 
 /* Allocates the workspace; the sizes above d_err must be set. 0, or -1 with everything given back. */
 int llmb200_plain_rows_ready(PlainRows *r);
 void llmb200_plain_rows_free(PlainRows *r);
-/* Runs n_rows / seq_len sequences' tokens (positions pos0 on) through the layers; r->x holds the embedded rows on entry and the
- * residual stream afterwards, its last feed-forward result still in r->y (last_norm adds it). */
+/* Runs n_rows / seq_len sequences' tokens (positions pos0 on) through the layers; r->x holds the embedded rows on entry. What follows the
+ * last layer's attention is formed for rows index[0..n_last) (device memory) only: nobody reads it of the others. */
 int llmb200_plain_rows_run(PlainRows *r, const RowsLayer *layers, int n_layers, int n_rows, int seq_len, int pos0, long long cache_seq_stride,
-                           int caches_only);
-/* The products' operand: planes of the final norm of rows index[0..n) (device; ascending) of the stream -> r->xh. */
-int llmb200_plain_rows_last(PlainRows *r, const RowsLayer *last_layer, const float *g_final, const int *index, int n, int n_rows);
+                           const int *index, int n_last);
+/* The LM head's operand: planes of the final norm of the index-th rows first .. first + n - 1 of the last run -> r->xh. */
+int llmb200_plain_rows_last(PlainRows *r, const RowsLayer *last_layer, const float *g_final, int first, int n);
 int llmb200_plain_rows_product(PlainRows *r, const RowsMatrix *m, int n, float *out);
 
 #endif
