@@ -205,5 +205,14 @@ def test_prompt_equals_its_tokens(lib, pkg, synth, family, fp16):
     spread = np.abs(one).max()
     for parts in ([150], [24, 5, 1, 64, 25, 31], [149, 1]):
         assert np.abs(feed(parts) - one).max() <= 1e-3 * spread, parts
+    few = np.array([0, 77, 149], dtype=np.int32)                # the last layer is formed for these rows only; then the cache goes on
+    lg = np.zeros((3, V), np.float32)
+    lib.inference_state_reset(s)
+    assert lib.inference_forward_tokens(s, toks.ctypes.data_as(pkg.c_u32_p), 150, few.ctypes.data_as(pkg.c_int_p), 3, lg.ctypes.data_as(pkg.c_float_p)) == 0
+    assert np.abs(lg - one[few]).max() <= 1e-3 * spread
+    lib.inference_state_reset(s)
+    assert lib.inference_forward_tokens(s, toks.ctypes.data_as(pkg.c_u32_p), 149, None, 0, None) == 0
+    after = np.ctypeslib.as_array(lib.inference_forward_token(s, int(toks[149])), (V,))
+    assert np.abs(after - one[149]).max() <= 1e-3 * spread
     lib.inference_state_free(s)
     (synth.llmb200_synth_free_gemma3 if gemma else synth.llmb200_synth_free_qwen3)(model)
