@@ -205,7 +205,7 @@ rows_matmul_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     const int on = kb < nkb && m < p.rows && b + (c >> 1) < nblk;
                     cp_async(dst + r * 64 + ((c ^ (r >> 1)) & 3) * 16, on ? p.w + (long long)m * p.w_stride + (size_t)b * 32 + c * 16 : p.w, on ? 16 : 0);
                 }
-                // the scales of both blocks: one aligned word, the second half inside the row's padding where there is no second block
+                // the scales of both blocks: one aligned word; where there is no second block its half is padding that nobody writes
                 const int on = kb < nkb && row < p.rows;
                 cp_async4(dst + 2048 + lane * 4, on ? p.w + (long long)row * p.w_stride + p.cols + b * 2 : p.w, on ? 4 : 0);
                 asm volatile("cp.async.commit_group;" ::: "memory");
@@ -220,7 +220,7 @@ rows_matmul_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 uint4 q[4];
 #pragma unroll
                 for (int c = 0; c < 4; ++c) q[c] = lds_128(src + lane * 64 + ((c ^ (lane >> 1)) & 3) * 16);
-                const uint32_t sc[2] = {lds_u16(src + 2048 + lane * 4), lds_u16(src + 2048 + lane * 4 + 2)};
+                const uint32_t sc[2] = {lds_u16(src + 2048 + lane * 4), (kb0 + kb) * 2 + 1 < nblk ? lds_u16(src + 2048 + lane * 4 + 2) : 0u};
                 __syncwarp();
                 fetch(kb + 2 * DEPTH, slot);
                 ok = wait_or_abort(&empty_bar[s], ((kb / slots) & 1) ^ 1, abort_flag);

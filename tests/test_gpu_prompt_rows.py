@@ -216,3 +216,46 @@ def test_prompt_equals_its_tokens(lib, pkg, synth, family, fp16):
     assert np.abs(after - one[149]).max() <= 1e-3 * spread
     lib.inference_state_free(s)
     (synth.llmb200_synth_free_gemma3 if gemma else synth.llmb200_synth_free_qwen3)(model)
+
+
+@pytest.mark.parametrize("cols", [32, 96, 2592])
+@pytest.mark.parametrize("planes,n", [(1, 5), (2, 5), (2, 300)])
+def test_an_odd_number_of_blocks_reads_no_padding(lib, pkg, synth, cols, planes, n):
+    """The word that holds a row's last scale ends in padding that the packing kernels do not write: NaN there must not matter."""
+    rows = 136
+    stride = lib.b200_packed_row_stride(pkg.B200_WT_Q8, cols)
+    d_w = torch.full((rows * stride,), 0xFF, dtype=torch.uint8, device="cuda")
+    d_src = dev(weights(synth, rows, cols, 5))
+    assert lib.b200_q8_pack(d_src.data_ptr(), cols, rows, cols, d_w.data_ptr(), stride, 0, 1, None) == 0
+    exact_w = q8_values(lib, d_w, stride, rows, cols)
+    x = torch.randn(n, cols, generator=torch.Generator().manual_seed(cols)).cuda()
+    px, scale, args = planes_buffer(pkg, n, n, cols, planes, planes == 2)
+    assert lib.b200_rows_split_planes(x.data_ptr(), n, cols, C.byref(args), None) == 0
+    ws = torch.zeros(rows, dtype=torch.float32, device="cuda")
+    assert lib.b200_q8_row_scale(d_w.data_ptr(), stride, rows, cols, ws.data_ptr(), None) == 0
+    out = torch.zeros(n, rows, device="cuda")
+    a = pkg.RowsMatmulArgs(pkg.B200_WT_Q8, d_w.data_ptr(), stride, rows, cols, ws.data_ptr(), px.data_ptr(), cols, planes, n,
+                           scale.data_ptr() if scale is not None else None, n, out.data_ptr(), rows, None, rows, None, 0)
+    assert lib.b200_rows_matmul(C.byref(a), None) == 0
+    assert rel(out, x.double() @ exact_w.T) < (1e-5 if planes == 2 else 6e-4)
+
+
+def test_q8_models_of_odd_block_counts(lib, pkg, synth):
+    """Widths of 17 and 49 blocks; the memory that the state allocates holds what its last owner left there."""
+    dirt = torch.full((1 << 28,), 0xFF, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    del dirt
+    torch.cuda.empty_cache()
+    sp = pkg.spec("tiny-qwen3", n_layers=2, d_model=544, intermediate_size=1568, gamma_jitter=0.1)
+    model = synth.llmb200_synth_qwen3(C.byref(sp), 4)
+    s = lib.inference_state_create(model, 64, 0)
+    assert s
+    toks = np.random.default_rng(5).integers(0, sp.vocab_size, 40).astype(np.uint32)
+    one = np.stack([np.ctypeslib.as_array(lib.inference_forward_token(s, int(t)), (sp.vocab_size,)).copy() for t in toks])
+    lib.inference_state_reset(s)
+    lg = np.zeros_like(one)
+    assert lib.inference_forward_tokens(s, toks.ctypes.data_as(pkg.c_u32_p), 40, np.arange(40, dtype=np.int32).ctypes.data_as(pkg.c_int_p), 40,
+                                        lg.ctypes.data_as(pkg.c_float_p)) == 0
+    assert np.abs(lg - one).max() <= 1e-3 * np.abs(one).max()
+    lib.inference_state_free(s)
+    synth.llmb200_synth_free_qwen3(model)
