@@ -18,6 +18,7 @@ extern unsigned long long g_b200_launches;
 namespace {
 
 constexpr int ROW_THREADS = 256;
+constexpr size_t ROW_HELD = 227 * 1024 - 256;    // bytes of a row that shared memory holds beside a kernel's own
 
 __device__ __forceinline__ float block_max(float v, float *red)
 {
@@ -61,6 +62,8 @@ __device__ __forceinline__ void put4(const b200_row_planes &o, long long row, in
 }
 
 // x += (post ? post-normed y : y); planes of the RMS-normed x. index: row m of the output is row index[m] of x (no update then).
+// HELD: the row stays in shared memory between the walks over it; wider rows are read again from where they lie.
+template <bool HELD>
 __global__ void __launch_bounds__(ROW_THREADS)
 rows_norm_kernel(float *x, int dim, const float *y, const float *post, const float *gamma, const int *index, float eps, const b200_row_planes o)
 {
@@ -77,7 +80,7 @@ rows_norm_kernel(float *x, int dim, const float *y, const float *post, const flo
         float ss = 0.0f;
         for (int i = threadIdx.x; i < n4; i += ROW_THREADS) {
             const float4 v = yr[i];
-            sh[i] = v;
+            if (HELD) sh[i] = v;
             ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
         }
         yinv = 1.0f / sqrtf(block_sum(ss, red) / (float)dim + eps);
@@ -86,7 +89,7 @@ rows_norm_kernel(float *x, int dim, const float *y, const float *post, const flo
     for (int i = threadIdx.x; i < n4; i += ROW_THREADS) {
         float4 v = xr[i];
         if (yr) {
-            float4 a = post ? sh[i] : yr[i];
+            float4 a = HELD && post ? sh[i] : yr[i];
             if (post) {
                 const float4 g = reinterpret_cast<const float4 *>(post)[i];
                 a.x *= yinv * g.x; a.y *= yinv * g.y; a.z *= yinv * g.z; a.w *= yinv * g.w;
@@ -94,16 +97,20 @@ rows_norm_kernel(float *x, int dim, const float *y, const float *post, const flo
             v.x += a.x; v.y += a.y; v.z += a.z; v.w += a.w;
             xr[i] = v;
         }
-        sh[i] = v;
+        if (HELD) sh[i] = v;
         ss = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, ss))));
     }
     const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)dim + eps);
+    auto normed = [&](int i) {
+        const float4 g = reinterpret_cast<const float4 *>(gamma)[i];
+        float4 v = HELD ? sh[i] : xr[i];
+        v.x *= inv * g.x; v.y *= inv * g.y; v.z *= inv * g.z; v.w *= inv * g.w;
+        return v;
+    };
     float mx = 0.0f;
     for (int i = threadIdx.x; i < n4; i += ROW_THREADS) {
-        const float4 g = reinterpret_cast<const float4 *>(gamma)[i];
-        float4 v = sh[i];
-        v.x *= inv * g.x; v.y *= inv * g.y; v.z *= inv * g.z; v.w *= inv * g.w;
-        sh[i] = v;
+        const float4 v = normed(i);
+        if (HELD) sh[i] = v;
         mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }
     float up = 1.0f, down;
@@ -111,10 +118,12 @@ rows_norm_kernel(float *x, int dim, const float *y, const float *post, const flo
         up = row_up(block_max(mx, red), &down);
         if (threadIdx.x == 0) o.d_scale[m] = down;
     }
-    for (int i = threadIdx.x; i < n4; i += ROW_THREADS) put4(o, m, i, sh[i], up);
+    for (int i = threadIdx.x; i < n4; i += ROW_THREADS) put4(o, m, i, HELD ? sh[i] : normed(i), up);
 }
 
-// Planes of act(gate) * up. Rows of 2 * inter: (gate, up) side by side in pairs, or all gates and then all ups.
+// Planes of act(gate) * up. Rows of 2 * inter: (gate, up) side by side in pairs, or all gates and then all ups. HELD as above; it matters
+// with a factor only.
+template <bool HELD>
 __global__ void __launch_bounds__(ROW_THREADS)
 rows_glu_kernel(const float *gu, int inter, int pairs, int gelu, const b200_row_planes o)
 {
@@ -125,27 +134,28 @@ rows_glu_kernel(const float *gu, int inter, int pairs, int gelu, const b200_row_
     pdl_wait();
     const float4 *g4 = reinterpret_cast<const float4 *>(gu + (long long)m * 2 * inter);
     float4 *sh = reinterpret_cast<float4 *>(row_sh);
-    float mx = 0.0f;
-    // without a factor the row's elements do not depend on one another: several blocks share it
-    for (int i = blockIdx.y * ROW_THREADS + threadIdx.x; i < n4; i += gridDim.y * ROW_THREADS) {
+    auto value = [&](int i) {
         const float4 a = __ldcs(g4 + (pairs ? 2 * i : i)), b = __ldcs(g4 + (pairs ? 2 * i + 1 : n4 + i));
         const float g[4] = {a.x, pairs ? a.z : a.y, pairs ? b.x : a.z, pairs ? b.z : a.w};
         const float u[4] = {pairs ? a.y : b.x, pairs ? a.w : b.y, pairs ? b.y : b.z, b.w};
         float v[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            v[k] = (gelu ? act_gelu_tanh(g[k]) : g[k] / (1.0f + expf(-g[k]))) * u[k];
-            mx = fmaxf(mx, fabsf(v[k]));
-        }
-        if (o.d_scale) sh[i] = make_float4(v[0], v[1], v[2], v[3]);
-        else put4(o, m, i, make_float4(v[0], v[1], v[2], v[3]), 1.0f);
+        for (int k = 0; k < 4; ++k) v[k] = (gelu ? act_gelu_tanh(g[k]) : g[k] / (1.0f + expf(-g[k]))) * u[k];
+        return make_float4(v[0], v[1], v[2], v[3]);
+    };
+    if (!o.d_scale) {                        // the row's elements do not depend on one another: several blocks share it
+        for (int i = blockIdx.y * ROW_THREADS + threadIdx.x; i < n4; i += gridDim.y * ROW_THREADS) put4(o, m, i, value(i), 1.0f);
+        return;
     }
-    if (o.d_scale) {
-        float down;
-        const float up = row_up(block_max(mx, red), &down);
-        if (threadIdx.x == 0) o.d_scale[m] = down;
-        for (int i = threadIdx.x; i < n4; i += ROW_THREADS) put4(o, m, i, sh[i], up);
+    float mx = 0.0f, down;
+    for (int i = threadIdx.x; i < n4; i += ROW_THREADS) {
+        const float4 v = value(i);
+        if (HELD) sh[i] = v;
+        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
     }
+    const float up = row_up(block_max(mx, red), &down);
+    if (threadIdx.x == 0) o.d_scale[m] = down;
+    for (int i = threadIdx.x; i < n4; i += ROW_THREADS) put4(o, m, i, HELD ? sh[i] : value(i), up);
 }
 
 // Planes of plain rows.
@@ -430,10 +440,10 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
 }
 
 template <typename K>
-int allow_smem(K kern, size_t smem)
+int allow_smem(K kern, size_t smem)          // beside less than 1 KB of a kernel's own
 {
     if (smem > 227 * 1024) return B200_E_TOOLARGE;
-    return smem > 48 * 1024 ? (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : 0;
+    return smem > 47 * 1024 ? (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) : 0;
 }
 
 template <int HD, int NW>
@@ -477,21 +487,24 @@ extern "C" int b200_rows_norm_planes(float *x, int rows, int dim, const float *y
                                      const int *index, float eps, const b200_row_planes *out, void *stream)
 {
     if (!x || !gamma || rows <= 0 || dim <= 0 || (dim & 3) || (index && y) || (post_gamma && !y) || !planes_ok(out, rows, dim)) return B200_E_BADARG;
-    const int rc = allow_smem(rows_norm_kernel, (size_t)dim * 4);
+    const size_t smem = (size_t)dim * 4 <= ROW_HELD ? (size_t)dim * 4 : 0;
+    const auto kern = smem ? rows_norm_kernel<true> : rows_norm_kernel<false>;
+    const int rc = allow_smem(kern, smem);
     if (rc) return rc;
     ++g_b200_launches;
-    return (int)launch_chained(rows_norm_kernel, dim3(rows), dim3(ROW_THREADS), (size_t)dim * 4, (cudaStream_t)stream, x, dim, y, post_gamma, gamma,
-                               index, eps, *out);
+    return (int)launch_chained(kern, dim3(rows), dim3(ROW_THREADS), smem, (cudaStream_t)stream, x, dim, y, post_gamma, gamma, index, eps, *out);
 }
 
 extern "C" int b200_rows_glu_planes(const float *gu, int rows, int inter, int pairs, int gelu, const b200_row_planes *out, void *stream)
 {
     if (!gu || rows <= 0 || inter <= 0 || (inter & 3) || !planes_ok(out, rows, inter)) return B200_E_BADARG;
-    const int rc = allow_smem(rows_glu_kernel, (size_t)inter * 4);
+    const size_t smem = out->d_scale && (size_t)inter * 4 <= ROW_HELD ? (size_t)inter * 4 : 0;
+    const auto kern = smem ? rows_glu_kernel<true> : rows_glu_kernel<false>;
+    const int rc = allow_smem(kern, smem);
     if (rc) return rc;
     ++g_b200_launches;
-    return (int)launch_chained(rows_glu_kernel, dim3(rows, out->d_scale ? 1 : share_row(rows, inter)), dim3(ROW_THREADS),
-                               out->d_scale ? (size_t)inter * 4 : 0, (cudaStream_t)stream, gu, inter, pairs, gelu, *out);
+    return (int)launch_chained(kern, dim3(rows, out->d_scale ? 1 : share_row(rows, inter)), dim3(ROW_THREADS), smem, (cudaStream_t)stream, gu, inter,
+                               pairs, gelu, *out);
 }
 
 extern "C" int b200_rows_split_planes(const float *x, int rows, int dim, const b200_row_planes *out, void *stream)

@@ -273,7 +273,7 @@ static RowsMatrix matrix(const void *w, int rows, int cols)
 static int prefill_rows(BState *s, const uint32_t *prompts, int stride, int n)
 {
     const int B = s->B, D = s->D, Hq_hd = s->Hq * s->hd, T0 = BATCH_ROWS / B < n ? BATCH_ROWS / B : n;
-    if ((D | s->IS | Hq_hd) & 7 || (s->hd != 64 && s->hd != 128 && s->hd != 256) || (size_t)s->IS * 4 > 227 * 1024 || (size_t)D * 4 > 227 * 1024) return 1;
+    if ((D | s->IS | Hq_hd) & 7 || (s->hd != 64 && s->hd != 128 && s->hd != 256)) return 1;
     PlainRows *r = &s->rows;
     if (r->cap < B * T0) {
         llmb200_plain_rows_free(r);

@@ -1147,7 +1147,7 @@ enum { PROMPT_MIN = 4, PORTION_MIN = 24 };
 /* An attached adapter and tensor parallelism run on the per-token path. */
 static int prompt_rows_fit(const InferenceState *s, int n, int least)
 {
-    return n >= least && !s->lora && s->tp_size == 1 && s->Hq * s->hd % 8 == 0 && (size_t)s->IS * 4 <= 227 * 1024 && (size_t)s->D * 4 <= 227 * 1024;
+    return n >= least && !s->lora && s->tp_size == 1 && s->Hq * s->hd % 8 == 0;
 }
 
 static int prompt_rows(InferenceState *s, const uint32_t *tokens, int n, const int *want, int n_want, float *logits)

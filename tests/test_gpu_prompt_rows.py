@@ -259,3 +259,31 @@ def test_q8_models_of_odd_block_counts(lib, pkg, synth):
     assert np.abs(lg - one).max() <= 1e-3 * np.abs(one).max()
     lib.inference_state_free(s)
     synth.llmb200_synth_free_qwen3(model)
+
+
+@pytest.mark.parametrize("planes", [1, 2])
+@pytest.mark.parametrize("dim", [12288, 58016, 58112, 60000])
+def test_rows_wider_than_shared_memory(lib, pkg, planes, dim):
+    """Rows that just fill the 48 KB a kernel has without asking, and either side of the 58 048 values that it can be given beside its own."""
+    g = torch.Generator().manual_seed(dim)
+    gu, x, y = (torch.randn(2, n * dim, generator=g).cuda() for n in (2, 1, 1))
+    gamma, post = torch.randn(dim, generator=g).cuda(), torch.randn(dim, generator=g).cuda()
+    buf, scale, args = planes_buffer(pkg, 2, 2, dim, planes, planes == 2)
+
+    def value():
+        torch.cuda.synchronize()
+        return buf.double().view(planes, 2, dim).sum(0) * (scale[:, None].double() if planes == 2 else 1.0)
+
+    def norm(t, w):
+        return t * torch.rsqrt(t.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+    bar = 2e-6 if planes == 2 else 4e-4
+    for pairs in (0, 1):
+        gate, up = (gu[:, 0::2], gu[:, 1::2]) if pairs else (gu[:, :dim], gu[:, dim:])
+        assert lib.b200_rows_glu_planes(gu.data_ptr(), 2, dim, pairs, 0, C.byref(args), None) == 0
+        assert rel(value(), torch.nn.functional.silu(gate.double()) * up.double()) < bar
+    for with_post in (False, True):
+        xs = x.clone()
+        assert lib.b200_rows_norm_planes(xs.data_ptr(), 2, dim, y.data_ptr(), post.data_ptr() if with_post else None, gamma.data_ptr(), None, 1e-6,
+                                         C.byref(args), None) == 0
+        want = x.double() + (norm(y.double(), post) if with_post else y.double())
+        assert rel(xs, want) < 1e-6 and rel(value(), norm(want, gamma)) < bar
