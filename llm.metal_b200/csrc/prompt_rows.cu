@@ -32,12 +32,20 @@ __device__ __forceinline__ float block_max(float v, float *red)
     return v;
 }
 
-// The power of two that brings a row's largest magnitude into [2^14, 2^15): up, and its inverse for the results. Rows of
-// zeros, infinities or NaN stay as they are.
+// What an element counts for in its row's largest magnitude: infinities and NaN nothing, they stay what they are under any factor.
+__device__ __forceinline__ float magnitude(float v)
+{
+    const float a = fabsf(v);
+    return a < INFINITY ? a : 0.0f;
+}
+__device__ __forceinline__ float magnitude4(float4 v) { return fmaxf(fmaxf(magnitude(v.x), magnitude(v.y)), fmaxf(magnitude(v.z), magnitude(v.w))); }
+
+// The power of two that brings a row's largest finite magnitude into [2^14, 2^15): up, and its inverse for the results. Rows of
+// zeros stay as they are.
 __device__ __forceinline__ float row_up(float mx, float *down)
 {
     int e = 0;
-    if (mx > 0.0f && mx < INFINITY) { e = 14 - ilogbf(mx); e = e > 120 ? 120 : e; }
+    if (mx > 0.0f) { e = 14 - ilogbf(mx); e = e > 120 ? 120 : e; }
     *down = ldexpf(1.0f, -e);
     return ldexpf(1.0f, e);
 }
@@ -51,6 +59,14 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t &hi, uint3
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
 
+// The second plane of an element whose first is an infinity or NaN holds nothing: infinity minus infinity would make it NaN.
+__device__ __forceinline__ uint32_t finite_low(uint32_t hi, uint32_t lo)
+{
+    if ((hi & 0x7c00u) == 0x7c00u) lo &= 0xffff0000u;
+    if ((hi & 0x7c000000u) == 0x7c000000u) lo &= 0x0000ffffu;
+    return lo;
+}
+
 __device__ __forceinline__ void put4(const b200_row_planes &o, long long row, int i4, float4 v, float up)
 {
     uint2 hi, lo;
@@ -58,7 +74,7 @@ __device__ __forceinline__ void put4(const b200_row_planes &o, long long row, in
     split_pair(v.z * up, v.w * up, hi.y, lo.y);
     __half *d = static_cast<__half *>(o.d_x) + row * o.ld + 4 * i4;
     *reinterpret_cast<uint2 *>(d) = hi;
-    if (o.planes == 2) *reinterpret_cast<uint2 *>(d + (long long)o.plane_rows * o.ld) = lo;
+    if (o.planes == 2) *reinterpret_cast<uint2 *>(d + (long long)o.plane_rows * o.ld) = make_uint2(finite_low(hi.x, lo.x), finite_low(hi.y, lo.y));
 }
 
 // x += (post ? post-normed y : y); planes of the RMS-normed x. index: row m of the output is row index[m] of x (no update then).
@@ -111,7 +127,7 @@ rows_norm_kernel(float *x, int dim, const float *y, const float *post, const flo
     for (int i = threadIdx.x; i < n4; i += ROW_THREADS) {
         const float4 v = normed(i);
         if (HELD) sh[i] = v;
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        mx = fmaxf(mx, magnitude4(v));
     }
     float up = 1.0f, down;
     if (o.d_scale) {
@@ -151,7 +167,7 @@ rows_glu_kernel(const float *gu, int inter, int pairs, int gelu, const b200_row_
     for (int i = threadIdx.x; i < n4; i += ROW_THREADS) {
         const float4 v = value(i);
         if (HELD) sh[i] = v;
-        mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+        mx = fmaxf(mx, magnitude4(v));
     }
     const float up = row_up(block_max(mx, red), &down);
     if (threadIdx.x == 0) o.d_scale[m] = down;
@@ -172,7 +188,7 @@ rows_split_kernel(const float *x, int dim, const b200_row_planes o)
         float mx = 0.0f;
         for (int i = threadIdx.x; i < n4; i += ROW_THREADS) {
             const float4 v = xr[i];
-            mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+            mx = fmaxf(mx, magnitude4(v));
         }
         up = row_up(block_max(mx, red), &down);
         if (threadIdx.x == 0) o.d_scale[m] = down;
@@ -225,7 +241,7 @@ __global__ void __launch_bounds__(128) rows_qkv_kernel(const b200_rows_attn_args
     if (h < p.n_q) {
         float mx = 0.0f, down;
 #pragma unroll
-        for (int j = 0; j < H2; ++j) mx = fmaxf(mx, fmaxf(fabsf(a[j]), fabsf(b[j])));
+        for (int j = 0; j < H2; ++j) mx = fmaxf(mx, fmaxf(magnitude(a[j]), magnitude(b[j])));
         const float up = row_up(warp_max(mx), &down);
         const long long at = ((long long)m * p.n_q + h) * HD, plane = (long long)p.n_rows * p.n_q * HD;
         __half *q = static_cast<__half *>(p.d_q);
@@ -237,7 +253,8 @@ __global__ void __launch_bounds__(128) rows_qkv_kernel(const b200_rows_attn_args
                 const __half hi = __float2half_rn(f);
                 const long long i = at + lane + 32 * j + k * (HD / 2);
                 q[i] = hi;
-                q[plane + i] = __float2half_rn(f - __half2float(hi));
+                const float rest = f - __half2float(hi);
+                q[plane + i] = __float2half_rn(fabsf(rest) < INFINITY ? rest : 0.0f);          // as finite_low
             }
         }
         if (lane == 0) p.d_q_scale[(long long)m * p.n_q + h] = down;

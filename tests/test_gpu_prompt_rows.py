@@ -287,3 +287,20 @@ def test_rows_wider_than_shared_memory(lib, pkg, planes, dim):
                                          C.byref(args), None) == 0
         want = x.double() + (norm(y.double(), post) if with_post else y.double())
         assert rel(xs, want) < 1e-6 and rel(value(), norm(want, gamma)) < bar
+
+
+def test_planes_of_rows_with_infinities(lib, pkg):
+    """An infinity is one plane's infinity and nothing in the other; it takes neither the range nor the bits of the row's other elements."""
+    rows, dim = 3, 256
+    x = torch.randn(rows, dim, generator=torch.Generator().manual_seed(1)) * 1e5
+    x[0, 7], x[1, 9], x[2, 11] = torch.inf, -torch.inf, torch.nan
+    finite = torch.isfinite(x)
+    buf, scale, args = planes_buffer(pkg, rows, rows, dim, 2)
+    d = x.cuda()
+    assert lib.b200_rows_split_planes(d.data_ptr(), rows, dim, C.byref(args), None) == 0
+    torch.cuda.synchronize()
+    hi, lo = (p.double().cpu() for p in buf.view(2, rows, dim))
+    value = (hi + lo) * scale.cpu()[:, None].double()
+    assert ((value - x.double()).abs()[finite] <= 2 ** -22 * x.double().abs()[finite] + 2 ** -38 * 4e5).all()
+    assert float(value[0, 7]) == float("inf") and float(value[1, 9]) == -float("inf") and torch.isnan(value[2, 11])
+    assert float(lo[0, 7]) == 0 and float(lo[1, 9]) == 0
