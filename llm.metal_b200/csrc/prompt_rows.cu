@@ -287,6 +287,11 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ bool not_finite8(uint4 v)          // whether one of eight binary16 values is an infinity or NaN
+{
+    const auto top = [](uint32_t w) { return (w & 0x7c007c00u) + 0x04000400u; };
+    return (top(v.x) | top(v.y) | top(v.z) | top(v.w)) & 0x80008000u;
+}
 __device__ __forceinline__ float ex2(float x)                // 2^x, 2 ulp, 0 for -inf
 {
     float y;
@@ -297,7 +302,8 @@ __device__ __forceinline__ float ex2(float x)                // 2^x, 2 ulp, 0 fo
 // warp, 32 keys a step with the next step's copies in flight. Keys and values are binary16 as they lie; queries and weights are
 // fp32 numbers as two binary16 planes, one product each, so a step costs twice the products of a 16-bit attention and loses
 // nothing. Weights are formed times 2^14, which keeps the small ones' second plane away from binary16's lowest numbers; the
-// factor cancels in the division by their sum. mma.sync and not tcgen05: the products are a small share of a prompt
+// factor cancels in the division by their sum. Tiles that hold an infinity or NaN (values beyond binary16) are summed in plain multiply-adds
+// over the keys that a row sees: a later key's weight of zero would not keep them out, nor a second plane of zero. mma.sync and not tcgen05: the products are a small share of a prompt
 // (prompts of 1500 tokens: a tenth of the time of the matrix products), and the split of the weights stays in registers.
 template <int HD, int NW>
 __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn_args p)
@@ -354,7 +360,13 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
         const int slot = tile & 1;
         if (tile + 1 < tiles) { stage(tile + 1, slot ^ 1); cp_wait<1>(); }
         else cp_wait<0>();
-        __syncthreads();
+        // every thread looks through what it copied itself: the barrier that follows tells all of them
+        bool odd = false;
+        for (int e = tid; e < BKEY * (HD / 8); e += NT)
+            odd |= not_finite8(lds_128(smem_u32(ksm + (slot * BKEY + e / (HD / 8)) * KS + e % (HD / 8) * 8)));
+        for (int e = tid; e < BKEY * (DV / 8); e += NT)
+            odd |= not_finite8(lds_128(smem_u32(vsm + (slot * BKEY + e / (DV / 8)) * VS + e % (DV / 8) * 8)));
+        const bool plainly = __syncthreads_or(odd);
         const int k0 = tile * BKEY, w_first = first + warp * 16;
         if (k0 <= w_first + 15) {                            // else all of it is ahead of the warp's rows
             float s[BKEY / 8][4];
@@ -362,20 +374,33 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
             for (int i = 0; i < BKEY / 8; ++i)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) s[i][k] = 0.0f;
-            const uint32_t kaddr = smem_u32(ksm + slot * BKEY * KS + ((lane & 7) + ((lane >> 4) << 3)) * KS + ((lane >> 3) & 1) * 8);
-#pragma unroll 4
-            for (int kk = 0; kk < HD; kk += 16) {
-                uint32_t a[4], a2[4];
-                ldsm4(qaddr + kk * 2, a);
-                ldsm4(qaddr + (BQ * KS + kk) * 2, a2);
+            if (plainly) {
+                for (int d = 0; d < HD; ++d) {
+                    float f[2];
 #pragma unroll
-                for (int n = 0; n < BKEY / 16; ++n) {
-                    uint32_t b[4];
-                    ldsm4(kaddr + (uint32_t)(n * 16 * KS + kk) * 2, b);
-                    mma_f16(s[2 * n], a, b[0], b[1]);
-                    mma_f16(s[2 * n + 1], a, b[2], b[3]);
-                    mma_f16(s[2 * n], a2, b[0], b[1]);
-                    mma_f16(s[2 * n + 1], a2, b[2], b[3]);
+                    for (int r = 0; r < 2; ++r) f[r] = __half2float(qsm[(r0 + 8 * r) * KS + d]) + __half2float(qsm[(BQ + r0 + 8 * r) * KS + d]);
+#pragma unroll
+                    for (int n = 0; n < BKEY / 8; ++n)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k)
+                            s[n][k] = fmaf(f[k >> 1], __half2float(ksm[(slot * BKEY + n * 8 + (lane & 3) * 2 + (k & 1)) * KS + d]), s[n][k]);
+                }
+            } else {
+                const uint32_t kaddr = smem_u32(ksm + slot * BKEY * KS + ((lane & 7) + ((lane >> 4) << 3)) * KS + ((lane >> 3) & 1) * 8);
+#pragma unroll 4
+                for (int kk = 0; kk < HD; kk += 16) {
+                    uint32_t a[4], a2[4];
+                    ldsm4(qaddr + kk * 2, a);
+                    ldsm4(qaddr + (BQ * KS + kk) * 2, a2);
+#pragma unroll
+                    for (int n = 0; n < BKEY / 16; ++n) {
+                        uint32_t b[4];
+                        ldsm4(kaddr + (uint32_t)(n * 16 * KS + kk) * 2, b);
+                        mma_f16(s[2 * n], a, b[0], b[1]);
+                        mma_f16(s[2 * n + 1], a, b[2], b[3]);
+                        mma_f16(s[2 * n], a2, b[0], b[1]);
+                        mma_f16(s[2 * n + 1], a2, b[2], b[3]);
+                    }
                 }
             }
             if (k0 + BKEY - 1 > w_first) {
@@ -397,8 +422,9 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
                 mt[r] = fmaxf(mt[r], __shfl_xor_sync(0xffffffffu, mt[r], 1));
                 mt[r] = fmaxf(mt[r], __shfl_xor_sync(0xffffffffu, mt[r], 2));
             }
-            // differences first: the score at the maximum weighs exactly one (times 2^14), whatever its size
-            const float corr[2] = {ex2((mx[0] - mt[0]) * sc[0]), ex2((mx[1] - mt[1]) * sc[1])};
+            // differences first: the score at the maximum weighs exactly one (times 2^14), whatever its size; no difference of infinities
+            const float top[2] = {mt[0] == -INFINITY ? 0.0f : mt[0], mt[1] == -INFINITY ? 0.0f : mt[1]};
+            const float corr[2] = {ex2((mx[0] - top[0]) * sc[0]), ex2((mx[1] - top[1]) * sc[1])};
             const bool moved = mt[0] != mx[0] || mt[1] != mx[1];
             mx[0] = mt[0]; mx[1] = mt[1];
             float ls[2] = {0.0f, 0.0f};
@@ -406,7 +432,7 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
             for (int n = 0; n < BKEY / 8; ++n)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    s[n][k] = ex2(fmaf(s[n][k] - mt[k >> 1], sc[k >> 1], 14.0f));
+                    s[n][k] = ex2(fmaf(s[n][k] - top[k >> 1], sc[k >> 1], 14.0f));
                     ls[k >> 1] += s[n][k];
                 }
             l[0] = fmaf(l[0], corr[0], ls[0]);
@@ -415,31 +441,51 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
 #pragma unroll
                 for (int i = 0; i < DV / 8; ++i) { o[i][0] *= corr[0]; o[i][1] *= corr[0]; o[i][2] *= corr[1]; o[i][3] *= corr[1]; }
             }
-            const uint32_t vaddr = smem_u32(vsm + slot * BKEY * VS + (lane & 15) * VS + (lane >> 4) * 8);
-            uint32_t a[BKEY / 16][4], a2[BKEY / 16][4];
+            if (plainly) {
+                const int d0 = first + r0 - k0;              // the last key that row r0 sees, from the tile's first
 #pragma unroll
-            for (int kk = 0; kk < BKEY / 16; ++kk) {
-                split_pair(s[2 * kk][0], s[2 * kk][1], a[kk][0], a2[kk][0]);
-                split_pair(s[2 * kk][2], s[2 * kk][3], a[kk][1], a2[kk][1]);
-                split_pair(s[2 * kk + 1][0], s[2 * kk + 1][1], a[kk][2], a2[kk][2]);
-                split_pair(s[2 * kk + 1][2], s[2 * kk + 1][3], a[kk][3], a2[kk][3]);
-            }
-            // the step's sums start from zero and join the rows' in fp32 adds: tensor cores truncate when they accumulate, which
-            // over a long prompt would add up (5e-6 of a row at 700 keys otherwise)
+                for (int n = 0; n < BKEY / 8; ++n)
 #pragma unroll
-            for (int n = 0; n < DV / 16; ++n) {
-                float t[2][4] = {};
+                    for (int j = 0; j < 2; ++j)
+                        for (int from = 0; from < 4; ++from) {
+                            const int key = n * 8 + from * 2 + j;
+                            const float p0 = __shfl_sync(0xffffffffu, s[n][j], (lane & ~3) | from);
+                            const float p1 = __shfl_sync(0xffffffffu, s[n][2 + j], (lane & ~3) | from);
+                            const __half *v = vsm + (slot * BKEY + key) * VS + (lane & 3) * 2;
+#pragma unroll
+                            for (int i = 0; i < DV / 8; ++i) {
+                                const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(v + i * 8));
+                                if (key <= d0) { o[i][0] = fmaf(p0, f.x, o[i][0]); o[i][1] = fmaf(p0, f.y, o[i][1]); }
+                                if (key <= d0 + 8) { o[i][2] = fmaf(p1, f.x, o[i][2]); o[i][3] = fmaf(p1, f.y, o[i][3]); }
+                            }
+                        }
+            } else {
+                const uint32_t vaddr = smem_u32(vsm + slot * BKEY * VS + (lane & 15) * VS + (lane >> 4) * 8);
+                uint32_t a[BKEY / 16][4], a2[BKEY / 16][4];
 #pragma unroll
                 for (int kk = 0; kk < BKEY / 16; ++kk) {
-                    uint32_t b[4];
-                    ldsm4_t(vaddr + (uint32_t)(kk * 16 * VS + n * 16) * 2, b);
-                    mma_f16(t[0], a2[kk], b[0], b[1]);
-                    mma_f16(t[1], a2[kk], b[2], b[3]);
-                    mma_f16(t[0], a[kk], b[0], b[1]);
-                    mma_f16(t[1], a[kk], b[2], b[3]);
+                    split_pair(s[2 * kk][0], s[2 * kk][1], a[kk][0], a2[kk][0]);
+                    split_pair(s[2 * kk][2], s[2 * kk][3], a[kk][1], a2[kk][1]);
+                    split_pair(s[2 * kk + 1][0], s[2 * kk + 1][1], a[kk][2], a2[kk][2]);
+                    split_pair(s[2 * kk + 1][2], s[2 * kk + 1][3], a[kk][3], a2[kk][3]);
                 }
+                // the step's sums start from zero and join the rows' in fp32 adds: tensor cores truncate when they accumulate, which
+                // over a long prompt would add up (5e-6 of a row at 700 keys otherwise)
 #pragma unroll
-                for (int k = 0; k < 4; ++k) { o[2 * n][k] += t[0][k]; o[2 * n + 1][k] += t[1][k]; }
+                for (int n = 0; n < DV / 16; ++n) {
+                    float t[2][4] = {};
+#pragma unroll
+                    for (int kk = 0; kk < BKEY / 16; ++kk) {
+                        uint32_t b[4];
+                        ldsm4_t(vaddr + (uint32_t)(kk * 16 * VS + n * 16) * 2, b);
+                        mma_f16(t[0], a2[kk], b[0], b[1]);
+                        mma_f16(t[1], a2[kk], b[2], b[3]);
+                        mma_f16(t[0], a[kk], b[0], b[1]);
+                        mma_f16(t[1], a[kk], b[2], b[3]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) { o[2 * n][k] += t[0][k]; o[2 * n + 1][k] += t[1][k]; }
+                }
             }
         }
         __syncthreads();                                     // the slot is overwritten by the next round's copies

@@ -304,3 +304,54 @@ def test_planes_of_rows_with_infinities(lib, pkg):
     assert ((value - x.double()).abs()[finite] <= 2 ** -22 * x.double().abs()[finite] + 2 ** -38 * 4e5).all()
     assert float(value[0, 7]) == float("inf") and float(value[1, 9]) == -float("inf") and torch.isnan(value[2, 11])
     assert float(lo[0, 7]) == 0 and float(lo[1, 9]) == 0
+
+
+@pytest.mark.parametrize("hd,n_q,n_kv", [(64, 8, 2), (128, 4, 2), (256, 2, 1)])
+@pytest.mark.parametrize("poison", [1e30, float("nan")])
+def test_attention_leaves_later_values_out(lib, pkg, hd, n_q, n_kv, poison):
+    """What one position's value or key holds reaches the rows that see it, as in the sums of the per-token path, and no other."""
+    N, at, heads = 150, 75, n_q + 2 * n_kv
+    g = torch.Generator().manual_seed(hd)
+    qkv = torch.randn(N, heads, hd, generator=g).cuda()
+    freq = torch.tensor([1.0 / 1e4 ** (2 * d / hd) for d in range(hd // 2)], dtype=torch.float32).cuda()
+
+    def run(x, kc=None):
+        kc = torch.zeros(n_kv, N, hd, dtype=torch.float16, device="cuda") if kc is None else kc
+        vc = torch.zeros_like(kc)
+        q = torch.zeros(2 * N * n_q * hd, dtype=torch.float16, device="cuda")
+        qs, out = torch.zeros(N * n_q, device="cuda"), torch.zeros(N, n_q, hd, device="cuda")
+        a = pkg.RowsAttnArgs(n_q, n_kv, hd, N, N, N, 0, 1e-6, x.data_ptr(), None, None, freq.data_ptr(), kc.data_ptr(), vc.data_ptr(), 0,
+                             q.data_ptr(), qs.data_ptr(), out.data_ptr())
+        assert lib.b200_rows_attn(C.byref(a), None) == 0
+        torch.cuda.synchronize()
+        return out
+    plain = run(qkv)
+
+    def same(out, rows):                                      # a tile with an infinity is summed in another order
+        a, b = out[rows].double(), plain[rows].double()
+        assert torch.isfinite(a).all() and float(((a - b).norm(dim=-1) / b.norm(dim=-1)).max()) < 2e-6
+    bad = qkv.clone()
+    bad[at, n_q + n_kv:, 3] = poison                          # one element of every value head
+    out = run(bad)
+    same(out, slice(0, at))
+    assert rel(out[at:, :, 4:], plain[at:, :, 4:].double()) < 1e-6
+    assert (torch.isnan(out[at:, :, 3]) if poison != poison else torch.isposinf(out[at:, :, 3])).all()
+    bad = qkv.clone()
+    bad[at, n_q:n_q + n_kv, :] = poison                       # a key: its scores are infinite or NaN
+    same(run(bad), slice(0, at))
+    bad = qkv.clone()
+    bad[at, n_q:n_q + n_kv, 5] = poison                       # rows whose score with it is minus infinity give it no weight
+    kc = torch.zeros(n_kv, N, hd, dtype=torch.float16, device="cuda")
+    out = run(bad, kc)
+    k = kc.double().repeat_interleave(n_q // n_kv, 0)
+    x = bad[:, :n_q].double()
+    ang = (torch.arange(N, device="cuda", dtype=torch.float32)[:, None] * freq).double()[:, None]
+    x = torch.cat([x[..., : hd // 2] * ang.cos() - x[..., hd // 2:] * ang.sin(), x[..., : hd // 2] * ang.sin() + x[..., hd // 2:] * ang.cos()], -1)
+    s = (x.transpose(0, 1)[:, :, None] * k[:, None]).sum(-1) / hd ** 0.5
+    s = s.masked_fill(torch.ones(N, N, device="cuda").triu(1).bool(), -torch.inf)
+    hit = torch.isfinite(torch.softmax(s, -1)).all(-1).transpose(0, 1)
+    assert torch.equal(torch.isfinite(out).all(-1), hit) and (poison != poison or 0 < int(hit[at:].sum()) < hit[at:].numel())
+    bad = qkv.clone()
+    bad[at, :n_q, 5] = poison                                 # a query is its own row's only
+    out = run(bad)
+    assert torch.equal(out[:at], plain[:at]) and torch.equal(out[at + 1:], plain[at + 1:])
