@@ -387,21 +387,34 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
                 }
             } else {
                 const uint32_t kaddr = smem_u32(ksm + slot * BKEY * KS + ((lane & 7) + ((lane >> 4) << 3)) * KS + ((lane >> 3) & 1) * 8);
-#pragma unroll 4
-                for (int kk = 0; kk < HD; kk += 16) {
-                    uint32_t a[4], a2[4];
-                    ldsm4(qaddr + kk * 2, a);
-                    ldsm4(qaddr + (BQ * KS + kk) * 2, a2);
+                float low[BKEY / 8][4] = {};
+#pragma unroll 1
+                for (int d0 = 0; d0 < HD; d0 += 32) {
+                    float t[BKEY / 8][4] = {};
 #pragma unroll
-                    for (int n = 0; n < BKEY / 16; ++n) {
-                        uint32_t b[4];
-                        ldsm4(kaddr + (uint32_t)(n * 16 * KS + kk) * 2, b);
-                        mma_f16(s[2 * n], a, b[0], b[1]);
-                        mma_f16(s[2 * n + 1], a, b[2], b[3]);
-                        mma_f16(s[2 * n], a2, b[0], b[1]);
-                        mma_f16(s[2 * n + 1], a2, b[2], b[3]);
+                    for (int kk = d0; kk < d0 + 32; kk += 16) {
+                        uint32_t a[4], a2[4];
+                        ldsm4(qaddr + kk * 2, a);
+                        ldsm4(qaddr + (BQ * KS + kk) * 2, a2);
+#pragma unroll
+                        for (int n = 0; n < BKEY / 16; ++n) {
+                            uint32_t b[4];
+                            ldsm4(kaddr + (uint32_t)(n * 16 * KS + kk) * 2, b);
+                            mma_f16(t[2 * n], a, b[0], b[1]);
+                            mma_f16(t[2 * n + 1], a, b[2], b[3]);
+                            mma_f16(low[2 * n], a2, b[0], b[1]);
+                            mma_f16(low[2 * n + 1], a2, b[2], b[3]);
+                        }
                     }
+#pragma unroll
+                    for (int n = 0; n < BKEY / 8; ++n)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) s[n][k] += t[n][k];
                 }
+#pragma unroll
+                for (int n = 0; n < BKEY / 8; ++n)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) s[n][k] += low[n][k];
             }
             if (k0 + BKEY - 1 > w_first) {
                 const int d0 = first + r0 - k0 - (lane & 3) * 2;
@@ -432,7 +445,7 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
             for (int n = 0; n < BKEY / 8; ++n)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    s[n][k] = ex2(fmaf(s[n][k] - top[k >> 1], sc[k >> 1], 14.0f));
+                    s[n][k] = ex2((s[n][k] - top[k >> 1]) * sc[k >> 1]) * 16384.0f;      // the factor in the exponent would cost its bits
                     ls[k >> 1] += s[n][k];
                 }
             l[0] = fmaf(l[0], corr[0], ls[0]);
@@ -469,20 +482,18 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
                     split_pair(s[2 * kk + 1][0], s[2 * kk + 1][1], a[kk][2], a2[kk][2]);
                     split_pair(s[2 * kk + 1][2], s[2 * kk + 1][3], a[kk][3], a2[kk][3]);
                 }
-                // the step's sums start from zero and join the rows' in fp32 adds: tensor cores truncate when they accumulate, which
-                // over a long prompt would add up (5e-6 of a row at 700 keys otherwise)
+                // the step's sums start from zero, corrections first, and join the rows' in fp32 adds: tensor cores truncate when they
+                // accumulate, which over a long prompt would add up (5e-6 of a row at 700 keys otherwise)
 #pragma unroll
                 for (int n = 0; n < DV / 16; ++n) {
                     float t[2][4] = {};
+                    uint32_t b[BKEY / 16][4];
 #pragma unroll
-                    for (int kk = 0; kk < BKEY / 16; ++kk) {
-                        uint32_t b[4];
-                        ldsm4_t(vaddr + (uint32_t)(kk * 16 * VS + n * 16) * 2, b);
-                        mma_f16(t[0], a2[kk], b[0], b[1]);
-                        mma_f16(t[1], a2[kk], b[2], b[3]);
-                        mma_f16(t[0], a[kk], b[0], b[1]);
-                        mma_f16(t[1], a[kk], b[2], b[3]);
-                    }
+                    for (int kk = 0; kk < BKEY / 16; ++kk) ldsm4_t(vaddr + (uint32_t)(kk * 16 * VS + n * 16) * 2, b[kk]);
+#pragma unroll
+                    for (int kk = 0; kk < BKEY / 16; ++kk) { mma_f16(t[0], a2[kk], b[kk][0], b[kk][1]); mma_f16(t[1], a2[kk], b[kk][2], b[kk][3]); }
+#pragma unroll
+                    for (int kk = 0; kk < BKEY / 16; ++kk) { mma_f16(t[0], a[kk], b[kk][0], b[kk][1]); mma_f16(t[1], a[kk], b[kk][2], b[kk][3]); }
 #pragma unroll
                     for (int k = 0; k < 4; ++k) { o[2 * n][k] += t[0][k]; o[2 * n + 1][k] += t[1][k]; }
                 }

@@ -355,3 +355,39 @@ def test_attention_leaves_later_values_out(lib, pkg, hd, n_q, n_kv, poison):
     bad[at, :n_q, 5] = poison                                 # a query is its own row's only
     out = run(bad)
     assert torch.equal(out[:at], plain[:at]) and torch.equal(out[at + 1:], plain[at + 1:])
+
+
+@pytest.mark.parametrize("n_q,n_kv,hd,N", [(8, 2, 64, 200), (8, 2, 128, 500), (4, 1, 256, 200)])
+def test_attention_is_as_exact_as_the_per_token_kernel(lib, pkg, n_q, n_kv, hd, N):
+    """Both against float64 over the keys and values that each left in its cache. Bar: the per-token kernel's error and a half of it again."""
+    g, heads = torch.Generator().manual_seed(hd), n_q + 2 * n_kv
+    qkv = torch.randn(N, heads, hd, generator=g).cuda()
+    qg, kg = (1 + 0.3 * torch.randn(hd, generator=g)).cuda(), (1 + 0.3 * torch.randn(hd, generator=g)).cuda()
+    freq = torch.tensor([1.0 / 1e4 ** (2 * d / hd) for d in range(hd // 2)], dtype=torch.float32).cuda()
+    ang = (torch.arange(N, device="cuda", dtype=torch.float32)[:, None] * freq).double()[:, None]
+    x = qkv[:, :n_q].double()
+    x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * qg.double()
+    u, w = x[..., : hd // 2], x[..., hd // 2:]
+    x = torch.cat([u * ang.cos() - w * ang.sin(), u * ang.sin() + w * ang.cos()], -1)
+    errors = []
+    for rows in (0, 1):
+        kc, vc = (torch.zeros(n_kv, N, hd, dtype=torch.float16, device="cuda") for _ in range(2))
+        out = torch.zeros(N, n_q, hd, device="cuda")
+        if rows:
+            q, qs = torch.zeros(2 * N * n_q * hd, dtype=torch.float16, device="cuda"), torch.zeros(N * n_q, device="cuda")
+            a = pkg.RowsAttnArgs(n_q, n_kv, hd, N, N, N, 0, 1e-6, qkv.data_ptr(), qg.data_ptr(), kg.data_ptr(), freq.data_ptr(), kc.data_ptr(),
+                                 vc.data_ptr(), 0, q.data_ptr(), qs.data_ptr(), out.data_ptr())
+            assert lib.b200_rows_attn(C.byref(a), None) == 0
+        else:
+            scratch, tickets = torch.zeros(lib.b200_attn_scratch_floats(n_q, hd, 4), device="cuda"), torch.zeros(n_kv, dtype=torch.int32, device="cuda")
+            pos = torch.arange(N, dtype=torch.int32, device="cuda")
+            for i in range(N):
+                a = pkg.AttnArgs(qkv[i].data_ptr(), qg.data_ptr(), kg.data_ptr(), freq.data_ptr(), kc.data_ptr(), vc.data_ptr(), out[i].data_ptr(),
+                                 scratch.data_ptr(), tickets.data_ptr(), pos[i:].data_ptr(), n_q, n_kv, hd, N, 4, 1e-6, 0)
+                assert lib.b200_attn_decode(C.byref(a), None) == 0
+        torch.cuda.synchronize()
+        k, v = (t.double().repeat_interleave(n_q // n_kv, 0) for t in (kc, vc))
+        s = torch.einsum("ihd,hjd->hij", x, k) / hd ** 0.5
+        s = s.masked_fill(torch.ones(N, N, device="cuda").triu(1).bool(), -torch.inf)
+        errors.append(rel(out, torch.einsum("hij,hjd->ihd", torch.softmax(s, -1), v)))
+    assert errors[1] <= 1.5 * errors[0], errors
