@@ -28,6 +28,8 @@ typedef struct {
     int loaded;
 } BLayer;
 
+enum { BATCH_ROWS = 2048 };              /* rows (sequences x positions) of a prompt pass: the products are far from memory-bound there */
+
 struct llmb200_batch_state {
     int D, Hq, Hkv, hd, IS, V, L, B, max_seq, QKV, n_split;
     BLayer *layers;
@@ -47,7 +49,7 @@ struct llmb200_batch_state {
     int last_steps;
     int kernels_per_step;
     PlainRows rows;                       /* prompt passes: allocated with the first prompt, kept */
-    uint32_t *d_prompt;
+    uint32_t *d_prompt;                   /* [BATCH_ROWS] */
 };
 typedef struct llmb200_batch_state BState;
 
@@ -143,6 +145,7 @@ BState *llmb200_batch_begin(const llmb200_config *c, int batch_size, int max_gen
     s->tickets = dmalloc(s, B * s->Hkv * 4);
     s->d_tok = dmalloc(s, B * 4); s->d_hist = dmalloc(s, (size_t)s->hist_cap * B * 4);
     s->d_done = dmalloc(s, 4); s->d_ctl = dmalloc(s, 16);
+    s->d_prompt = dmalloc(s, BATCH_ROWS * 4);
     if (!s->err) {
         cudaMemsetAsync(s->tickets, 0, B * s->Hkv * 4, g_rt.stream);
         cudaMemsetAsync(s->d_done, 0, 4, g_rt.stream);
@@ -261,27 +264,24 @@ static void enqueue_step(BState *s)
 
 /* ------------------------------------------------------------ prompts in passes over the weights */
 
-enum { BATCH_ROWS = 2048 };              /* rows (sequences x positions) of a pass: the products are far from memory-bound there */
-
 static RowsMatrix matrix(const void *w, int rows, int cols)
 {
     const RowsMatrix m = { w, (long long)cols * 2, rows, cols, NULL };
     return m;
 }
 
-/* Caches of all sequences' first n tokens; prompts [B][stride]. 0, 1 when the shape is not one of the row path's, -1 on an error. */
+/* Caches of all sequences' first n tokens; prompts [B][stride]. 0, 1 when the shape is not one of the row path's or memory has no room for
+ * a pass, -1 on an error. */
 static int prefill_rows(BState *s, const uint32_t *prompts, int stride, int n)
 {
-    const int B = s->B, D = s->D, Hq_hd = s->Hq * s->hd, T0 = BATCH_ROWS / B < n ? BATCH_ROWS / B : n;
+    const int B = s->B, D = s->D, Hq_hd = s->Hq * s->hd;
+    int T0 = BATCH_ROWS / B < n ? BATCH_ROWS / B : n;
     if ((D | s->IS | Hq_hd) & 7 || (s->hd != 64 && s->hd != 128 && s->hd != 256)) return 1;
     PlainRows *r = &s->rows;
-    if (r->cap < B * T0) {
-        llmb200_plain_rows_free(r);
-        cudaFree(s->d_prompt); s->d_prompt = NULL;
-        r->D = D; r->Hq = s->Hq; r->Hkv = s->Hkv; r->hd = s->hd; r->IS = s->IS; r->wtype = B200_WT_F16; r->planes = 1; r->max_seq = s->max_seq;
-        r->cap = B * T0;
-        if (llmb200_plain_rows_ready(r) != 0 || cudaMalloc((void **)&s->d_prompt, (size_t)r->cap * 4) != cudaSuccess) { r->cap = 0; return -1; }
-    }
+    r->D = D; r->Hq = s->Hq; r->Hkv = s->Hkv; r->hd = s->hd; r->IS = s->IS; r->wtype = B200_WT_F16; r->planes = 1; r->max_seq = s->max_seq;
+    const int fit = llmb200_plain_rows_fit(r, B * T0, B * (T0 < 8 ? T0 : 8));
+    if (fit != 0) return fit;
+    if (T0 > r->cap / B) T0 = r->cap / B;
     RowsLayer *layers = calloc((size_t)s->L, sizeof(RowsLayer));
     uint32_t *ids = malloc((size_t)B * T0 * 4);
     int rc = layers && ids ? 0 : -1;

@@ -1092,13 +1092,14 @@ static int prompt_matrix(const InferenceState *s, const PackedMat *w, float **sc
     return 0;
 }
 
-/* Row scales and a workspace for passes of at least n rows (at most PROMPT_CHUNK). */
+/* Row scales and a workspace for passes of n rows (at most PROMPT_CHUNK), or of fewer where device memory has no more.
+ * 0, 1 when there is no room for any, or -1 after a device error. */
 static int prompt_ready(InferenceState *s, int n)
 {
     Prompt *m = s->model;
     if (!m) {
         m = s->model = calloc(1, sizeof(*m));
-        if (!m) return -1;
+        if (!m) return 1;
         PlainRows *r = &m->rows;
         r->D = s->D; r->Hq = s->Hq; r->Hkv = s->Hkv; r->hd = s->hd; r->IS = s->IS;
         r->gemma = s->mt == MODEL_GEMMA3; r->pairs = 1; r->wtype = s->wtype; r->planes = 2; r->max_seq = s->max_seq;
@@ -1113,7 +1114,12 @@ static int prompt_ready(InferenceState *s, int n)
         }
         m->scales = s->wtype == B200_WT_Q8 ? llmb200_dev_zero(rows * 4) : NULL;
         float *scale = m->scales;
-        int rc = !m->layers || !m->logits || !m->d_want || (s->wtype == B200_WT_Q8 && !scale) ? -1 : 0;
+        if (!m->layers || !m->logits || !m->d_want || (s->wtype == B200_WT_Q8 && !scale)) {
+            cudaGetLastError();              /* the caller goes on without: no launch is to report this */
+            prompt_free(s);
+            return 1;
+        }
+        int rc = 0;
         for (int l = 0; l < s->L && rc == 0; ++l) {
             const Layer *y = &s->layers[l];
             RowsLayer *o = &m->layers[l];
@@ -1130,13 +1136,7 @@ static int prompt_ready(InferenceState *s, int n)
     }
     int cap = 64;                        /* at least the wanted rows of a pass */
     while (cap < n) cap *= 2;
-    if (cap > m->rows.cap) {
-        CU_TRY(cudaStreamSynchronize(g_rt.stream), return -1);
-        llmb200_plain_rows_free(&m->rows);
-        m->rows.cap = cap;
-        if (llmb200_plain_rows_ready(&m->rows) != 0) { m->rows.cap = 0; return -1; }
-    }
-    return 0;
+    return llmb200_plain_rows_fit(&m->rows, cap, 64);
 }
 
 /* Fewest tokens of a pass, and fewest of a portion of inference_forward_tokens: shorter portions of a Qwen3 / Gemma3 state go through
@@ -1152,12 +1152,14 @@ static int prompt_rows_fit(const InferenceState *s, int n, int least)
 
 static int prompt_rows(InferenceState *s, const uint32_t *tokens, int n, const int *want, int n_want, float *logits)
 {
-    if (prompt_ready(s, n < PROMPT_CHUNK ? n : PROMPT_CHUNK) != 0) return -1;
+    const int ready = prompt_ready(s, n < PROMPT_CHUNK ? n : PROMPT_CHUNK);
+    if (ready != 0) return ready;
     Prompt *m = s->model;
     PlainRows *r = &m->rows;
+    const int chunk = r->cap < PROMPT_CHUNK ? r->cap : PROMPT_CHUNK;
     int w = 0;
-    for (int c0 = 0; c0 < n; c0 += PROMPT_CHUNK) {
-        const int M = n - c0 < PROMPT_CHUNK ? n - c0 : PROMPT_CHUNK, pos0 = s->cur_len + c0;
+    for (int c0 = 0; c0 < n; c0 += chunk) {
+        const int M = n - c0 < chunk ? n - c0 : chunk, pos0 = s->cur_len + c0;
         if (llmb200_set_control(s, pos0, s->max_seq + 2, tokens + c0, pos0, M) != 0) return -1;
         K_TRY(b200_embed_rows(s->emb, (const uint32_t *)(s->d_tokens + pos0), M, s->D, s->V, s->emb_scale, r->x, g_rt.stream), return -1);
         int last = w;
@@ -1219,10 +1221,10 @@ int inference_forward_tokens(InferenceState *s, const uint32_t *tokens, int n, c
     }
     follow_sft(s);
     if (ensure_graphs(s) != 0) return -1;
-    if (rows_fit(s, n, PORTION_MIN)) {
-        rc = s->ops->forward_rows(s, tokens, n, want, n_want, logits);
-        if (rc == 0) s->cur_len += n;
-    } else {
+    rc = rows_fit(s, n, PORTION_MIN) ? s->ops->forward_rows(s, tokens, n, want, n_want, logits) : 1;
+    if (rc == 0) s->cur_len += n;
+    if (rc > 0) {                            /* not a portion for a pass, or no memory for one */
+        rc = 0;
         for (int i = 0; i < n && rc == 0; ++i) {
             const int wanted = w < n_want && want[w] == i;
             rc = step_one(s, tokens[i], wanted ? logits + (size_t)w * s->V : NULL);
@@ -1256,8 +1258,10 @@ static int generate_one(InferenceState *s, const uint32_t *prompt, int prompt_le
 
     fprintf(stderr, "[FastGen] Prefilling %d tokens...\n", P);
     double t0 = now_ms();
-    if (P > 2 && rows_fit(s, P - 1, PROMPT_MIN)) { /* all but the last prompt token in one pass; the last one yields the first id */
-        if (s->ops->forward_rows(s, prompt, P - 1, NULL, 0, NULL) != 0) return 0;
+    /* all but the last prompt token in passes, where they fit; the last one yields the first id */
+    const int rows = P > 2 && rows_fit(s, P - 1, PROMPT_MIN) ? s->ops->forward_rows(s, prompt, P - 1, NULL, 0, NULL) : 1;
+    if (rows < 0) return 0;
+    if (rows == 0) {
         if (llmb200_set_control(s, P - 1, P, prompt, 0, P) != 0) return 0;
     } else {
         for (int i = 0; i < P - 1; ++i) CU_TRY(cudaGraphLaunch(s->g_nolm, g_rt.stream), return 0);

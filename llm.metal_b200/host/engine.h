@@ -33,7 +33,8 @@ typedef struct {
     int (*enqueue_token)(InferenceState *s, int with_lm, int pdl);
     /* Run n tokens (already checked) from position s->cur_len on in one pass over the weights and leave the cache
      * behind them; logits of the tokens want[0..n_want) (ascending places among the n) go to `logits`
-     * [n_want][V]. NULL: the model type only has the per-token path. */
+     * [n_want][V]. 0, a negative code, or 1 before anything was launched: no memory for a pass, the per-token path is to
+     * take the tokens. NULL: the model type only has that path. */
     int (*forward_rows)(InferenceState *s, const uint32_t *tokens, int n, const int *want, int n_want, float *logits);
     /* Whether forward_rows is the way for n tokens, at least `least` where the type has a minimum, in the state's present
      * configuration (NULL: always). */

@@ -10,35 +10,48 @@
 
 static const float RMS_EPS = 1e-6f;            /* hard-wired in the reference: src/nn/fast_inference.c:383 */
 
-static void *device(size_t bytes)
-{
-    void *p = NULL;
-    CU_TRY(cudaMalloc(&p, bytes), return NULL);
-    return p;
-}
-
-int llmb200_plain_rows_ready(PlainRows *r)
+/* One allocation: the buffers lie in it one after the other, on 256-byte boundaries. 0, 1 when memory has no room, or -1. */
+static int allocate(PlainRows *r)
 {
     const size_t n = (size_t)r->cap, heads = (size_t)r->Hq * r->hd;
-    size_t widest = (size_t)(r->IS > r->D ? r->IS : r->D);
+    size_t widest = (size_t)(r->IS > r->D ? r->IS : r->D), total = 0;
     if (heads > widest) widest = heads;
-    r->x = device(n * r->D * 4); r->y = device(n * r->D * 4); r->last = device(n * r->D * 4);
-    r->qkv = device(n * (heads + 2 * (size_t)r->Hkv * r->hd) * 4);
-    r->attn = device(n * heads * 4);
-    r->gu = device(n * 2 * r->IS * 4);
-    r->x_scale = device(n * 4); r->q_scale = device(n * r->Hq * 4);
-    r->xh = device(n * widest * 2 * r->planes);
-    r->q = device(n * heads * 2 * 2);
-    if (!r->x || !r->y || !r->last || !r->qkv || !r->attn || !r->gu || !r->x_scale || !r->q_scale || !r->xh || !r->q) { llmb200_plain_rows_free(r); return -1; }
+    const struct { void **at; size_t bytes; } part[] = {
+        { (void **)&r->x, n * r->D * 4 }, { (void **)&r->y, n * r->D * 4 }, { (void **)&r->last, n * r->D * 4 },
+        { (void **)&r->qkv, n * (heads + 2 * (size_t)r->Hkv * r->hd) * 4 }, { (void **)&r->attn, n * heads * 4 },
+        { (void **)&r->gu, n * 2 * r->IS * 4 }, { (void **)&r->x_scale, n * 4 }, { (void **)&r->q_scale, n * r->Hq * 4 },
+        { &r->xh, n * widest * 2 * r->planes }, { &r->q, n * heads * 2 * 2 } };
+    for (size_t i = 0; i < sizeof(part) / sizeof(part[0]); ++i) total += (part[i].bytes + 255) / 256 * 256;
+    const cudaError_t e = cudaMalloc(&r->block, total);
+    if (e != cudaSuccess) {
+        cudaGetLastError();                          /* the caller may go on without: no launch is to report this */
+        r->block = NULL;
+        return e == cudaErrorMemoryAllocation ? 1 : -1;
+    }
+    char *at = r->block;
+    for (size_t i = 0; i < sizeof(part) / sizeof(part[0]); ++i) { *part[i].at = at; at += (part[i].bytes + 255) / 256 * 256; }
     return 0;
+}
+
+int llmb200_plain_rows_fit(PlainRows *r, int want, int least)
+{
+    if (r->cap >= want) return 0;
+    CU_TRY(cudaStreamSynchronize(g_rt.stream), return -1);
+    llmb200_plain_rows_free(r);
+    for (int cap = want;; cap = cap / 2 > least ? cap / 2 : least) {
+        r->cap = cap;
+        const int rc = allocate(r);
+        if (rc == 0) return 0;
+        r->cap = 0;
+        if (rc < 0 || cap <= least) return rc;
+    }
 }
 
 void llmb200_plain_rows_free(PlainRows *r)
 {
-    void *b[] = { r->x, r->y, r->last, r->qkv, r->attn, r->gu, r->x_scale, r->q_scale, r->xh, r->q };
-    for (size_t i = 0; i < sizeof(b) / sizeof(b[0]); ++i) cudaFree(b[i]);
-    r->x = r->y = r->last = r->qkv = r->attn = r->gu = r->x_scale = r->q_scale = NULL;
-    r->xh = r->q = NULL;
+    cudaFree(r->block);
+    r->block = NULL;
+    r->cap = 0;
 }
 
 static b200_row_planes planes_of(const PlainRows *r, int width)

@@ -16,14 +16,17 @@ typedef struct {
 /* Workspace of a pass of up to `cap` rows. planes: 2 where the per-token kernels take fp32 inputs, 1 where they take
  * binary16 ones. */
 typedef struct {
-    int D, Hq, Hkv, hd, IS, gemma, pairs, wtype, planes, cap, max_seq;
+    int D, Hq, Hkv, hd, IS, gemma, pairs, wtype, planes, max_seq;
     unsigned *d_err;
+    int cap;
     float *x, *y, *last, *qkv, *attn, *gu, *x_scale, *q_scale;
     void *xh, *q;
+    void *block;                         /* all of them */
 } PlainRows;
 
-/* Allocates the workspace; the sizes above d_err must be set. 0, or -1 with everything given back. */
-int llmb200_plain_rows_ready(PlainRows *r);
+/* A workspace for passes of `want` rows (the sizes above cap must be set), or of fewer, down to `least`, where device memory has no more:
+ * r->cap says. 0, 1 when not even that could be had, -1 after a device error. What there was before is given back first. */
+int llmb200_plain_rows_fit(PlainRows *r, int want, int least);
 void llmb200_plain_rows_free(PlainRows *r);
 /* Runs n_rows / seq_len sequences' tokens (positions pos0 on) through the layers; r->x holds the embedded rows on entry. What follows the
  * last layer's attention is formed for rows index[0..n_last) (device memory) only: nobody reads it of the others. */
