@@ -196,6 +196,10 @@ double llmb200_batch_last_decode_ms(llmb200_batch_state *state, int *n_steps);
 int llmb200_batch_graph_kernels(llmb200_batch_state *state);
 /* The logits [batch][vocab] of the last step, copied to dst (cap floats); NULL if it does not fit. */
 const float *llmb200_batch_logits(llmb200_batch_state *state, float *dst, size_t cap);
+/* 0, or the word that a kernel of this state left when one of its waits ran out (-1: it could not be read). It stays set, and
+ * llmb200_batch_generate returns 0 from then on. llmb200_batch_error_word: where it lies in device memory (16 bytes). */
+int llmb200_batch_error(llmb200_batch_state *state);
+void *llmb200_batch_error_word(llmb200_batch_state *state);
 void llmb200_batch_free(llmb200_batch_state *state);
 
 #ifdef __cplusplus

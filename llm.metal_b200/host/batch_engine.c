@@ -38,6 +38,7 @@ struct llmb200_batch_state {
     float *x, *y, *qkv, *att, *gu, *logits, *scratch;
     void *xh;
     unsigned *tickets, *d_tok, *d_hist, *d_done;
+    unsigned *d_err;                      /* 16 bytes; the first word is set by a kernel whose wait ran out, and stays set */
     int *d_ctl;
     unsigned *h_tok;                      /* pinned [max(B, max_hist)] */
     int *h_ctl;
@@ -85,7 +86,7 @@ void llmb200_batch_free(BState *s)
         for (size_t i = 0; i < sizeof(b) / sizeof(b[0]); ++i) cudaFree(b[i]);
     }
     void *b[] = { s->lm_head, s->g_final, s->emb, s->x, s->y, s->qkv, s->att, s->gu, s->logits, s->scratch,
-                  s->xh, s->tickets, s->d_tok, s->d_hist, s->d_done, s->d_ctl, s->d_prompt };
+                  s->xh, s->tickets, s->d_tok, s->d_hist, s->d_done, s->d_ctl, s->d_prompt, s->d_err };
     llmb200_plain_rows_free(&s->rows);
     for (size_t i = 0; i < sizeof(b) / sizeof(b[0]); ++i) cudaFree(b[i]);
     if (s->h_tok) cudaFreeHost(s->h_tok);
@@ -145,11 +146,12 @@ BState *llmb200_batch_begin(const llmb200_config *c, int batch_size, int max_gen
     s->tickets = dmalloc(s, B * s->Hkv * 4);
     s->d_tok = dmalloc(s, B * 4); s->d_hist = dmalloc(s, (size_t)s->hist_cap * B * 4);
     s->d_done = dmalloc(s, 4); s->d_ctl = dmalloc(s, 16);
-    s->d_prompt = dmalloc(s, BATCH_ROWS * 4);
+    s->d_prompt = dmalloc(s, BATCH_ROWS * 4); s->d_err = dmalloc(s, 16);
     if (!s->err) {
         cudaMemsetAsync(s->tickets, 0, B * s->Hkv * 4, g_rt.stream);
         cudaMemsetAsync(s->d_done, 0, 4, g_rt.stream);
         cudaMemsetAsync(s->d_ctl, 0, 16, g_rt.stream);
+        cudaMemsetAsync(s->d_err, 0, 16, g_rt.stream);
         size_t ht = (size_t)s->hist_cap * B;
         if (cudaMallocHost((void **)&s->h_tok, (ht > B ? ht : B) * 4) != cudaSuccess ||
             cudaMallocHost((void **)&s->h_ctl, 16) != cudaSuccess)
@@ -218,6 +220,7 @@ static void proj(BState *s, const void *Wh, int N, int K, float *C)
     a.d_x = s->xh; a.x_ld = K; a.planes = 1;
     a.n = s->B;
     a.d_out = C; a.out_ld = N;
+    a.d_err = s->d_err;
     a.use_pdl = 1;
     B_TRY(s, b200_rows_matmul(&a, g_rt.stream));
 }
@@ -279,6 +282,7 @@ static int prefill_rows(BState *s, const uint32_t *prompts, int stride, int n)
     if ((D | s->IS | Hq_hd) & 7 || (s->hd != 64 && s->hd != 128 && s->hd != 256)) return 1;
     PlainRows *r = &s->rows;
     r->D = D; r->Hq = s->Hq; r->Hkv = s->Hkv; r->hd = s->hd; r->IS = s->IS; r->wtype = B200_WT_F16; r->planes = 1; r->max_seq = s->max_seq;
+    r->d_err = s->d_err;
     const int fit = llmb200_plain_rows_fit(r, B * T0, B * (T0 < 8 ? T0 : 8));
     if (fit != 0) return fit;
     if (T0 > r->cap / B) T0 = r->cap / B;
@@ -348,6 +352,15 @@ void llmb200_batch_set_eos(BState *s, const int *eos, int n)
     s->n_eos = n < 0 ? 0 : n > 4 ? 4 : n;
     for (int i = 0; i < s->n_eos; ++i) s->eos[i] = eos[i];
 }
+
+int llmb200_batch_error(BState *s)
+{
+    unsigned err = 0;
+    if (!s || cudaStreamSynchronize(g_rt.stream) != cudaSuccess || cudaMemcpy(&err, s->d_err, 4, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
+    return (int)err;
+}
+
+void *llmb200_batch_error_word(BState *s) { return s ? s->d_err : NULL; }
 
 /* prompts [B][prompt_len] (every sequence its own prompt of the same length), output [B][max_gen_len].
  * Returns the number of steps generated (every sequence gets that many tokens), 0 on error. */
@@ -421,7 +434,9 @@ int llmb200_batch_generate(BState *s, const uint32_t *prompts, int prompt_len, u
     }
     for (int b = 0; b < B; ++b)
         for (int g = 0; g < n_gen; ++g) output_tokens[(size_t)b * max_gen_len + g] = s->h_tok[(size_t)g * B + b];
-    return s->err ? 0 : n_gen;
+    const int timed_out = llmb200_batch_error(s);
+    if (timed_out) fprintf(stderr, "[BatchGen] a device-side wait ran out (0x%x): the results are invalid\n", (unsigned)timed_out);
+    return s->err || timed_out ? 0 : n_gen;
 }
 
 double llmb200_batch_last_decode_ms(BState *s, int *n_steps)

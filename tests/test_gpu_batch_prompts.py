@@ -148,3 +148,18 @@ def test_prompts_without_memory_for_a_pass(pkg, lib, room):
     assert generate(pkg, lib, b, prompts, G)[0] == G
     lib.llmb200_batch_free(b)
     lib.inference_state_free(s)
+
+
+def test_a_raised_error_word_fails_the_call(pkg, lib):
+    """What a kernel whose wait ran out leaves behind: the answer of such a call is not an answer."""
+    cfg, B, G, P = dict(sc.SMALL), 2, 3, 20
+    b, _ = states(pkg, lib, cfg, B, G, 64, single=False)
+    prompts = np.random.default_rng(P).integers(0, 512, (B, P)).astype(np.uint32)
+    assert generate(pkg, lib, b, prompts, G)[0] == G and lib.llmb200_batch_error(b) == 0
+    word, row = torch.full((4,), 0x7203, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    assert lib.b200_rows_gather(word.data_ptr(), 1, 4, row.data_ptr(), lib.llmb200_batch_error_word(b), None) == 0      # a copy of 16 bytes
+    torch.cuda.synchronize()
+    assert lib.llmb200_batch_error(b) == 0x7203 and generate(pkg, lib, b, prompts, G)[0] == 0
+    assert generate(pkg, lib, b, np.ascontiguousarray(prompts[:, :2]), G)[0] == 0
+    lib.llmb200_batch_free(b)
