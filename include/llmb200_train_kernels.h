@@ -105,13 +105,12 @@ int b200_qk_norm_rope_bwd(float *dqkv, const float *qkv, long long ld, long long
 /* Causal attention over each sequence (attn_train_fwd :769-851 with repeat_kv
  * :476-492 folded into the indexing). q [rows, n_q*hd], k [rows, n_kv*hd],
  * v = columns v_off.. of a matrix with row stride v_ld. probs [S, n_q, N, N]
- * keeps the softmax (zeros above the diagonal); out [rows, n_q*hd]. */
+ * keeps the softmax (zeros above the diagonal); out [rows, n_q*hd]. fp32 multiply-adds on the CUDA cores. */
 int b200_attn_train_fwd(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int seq_len,
                         int n_q, int n_kv, int hd, float scale, float *probs, float *out, void *stream);
 /* attn_bwd_dq (:857-925), attn_bwd_dkv (:931-968) and repeat_kv_bwd (:973-992):
  * d_out [rows, n_q*hd] -> dq, dk, dv written into the q, k, v column blocks of
- * dqkv [rows, ld]. d_score is scratch of S*n_q*N*max(N, 2*hd) floats (the
- * score gradients, or per-head dK/dV partial sums for short sequences). */
+ * dqkv [rows, ld]. d_score is scratch of S*n_q*N*N floats (the score gradients). */
 int b200_attn_train_bwd(const float *d_out, const float *probs, const float *q, const float *k, const float *v,
                         long long v_ld, int n_seq, int seq_len, int n_q, int n_kv, int hd, float scale,
                         float *d_score, float *dqkv, long long ld, void *stream);
@@ -196,6 +195,12 @@ int b200_rms_norm_bwd_rows_h(const float *x, const float *dy, long long dy_ld, c
 /* out may be NULL when out_h is given */
 int b200_attn_train_fwd_h(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int seq_len,
                           int n_q, int n_kv, int hd, float scale, float *probs, float *out, void *out_h, void *stream);
+/* The same two on the tensor cores, every fp32 operand as the sum of two TF32 numbers. */
+int b200_attn_train_fwd_tc(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int seq_len,
+                           int n_q, int n_kv, int hd, float scale, float *probs, float *out, void *out_h, void *stream);
+int b200_attn_train_bwd_tc(const float *d_out, const float *probs, const float *q, const float *k, const float *v,
+                           long long v_ld, int n_seq, int seq_len, int n_q, int n_kv, int hd, float scale,
+                           float *d_score, float *dqkv, long long ld, void *stream);
 /* act may be NULL when act_h is given; likewise d_gu / d_gu_h */
 int b200_silu_mul_rows_h(const float *gu, int rows, int inter, float *act, void *act_h, void *stream);
 int b200_silu_mul_bwd_rows_h(const float *d_act, const float *gu, int rows, int inter, float *d_gu, void *d_gu_h,

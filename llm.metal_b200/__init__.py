@@ -278,7 +278,7 @@ SYMBOLS_MAIN = {
                                 "b200_qk_norm_rope", "b200_qk_norm_rope_bwd", "b200_attn_train_fwd",
                                 "b200_attn_train_bwd", "b200_silu_mul_rows", "b200_silu_mul_bwd_rows", "b200_lora_add", "b200_lora_pack", "b200_xty_skinny",
                                 "b200_softmax_ce_rows", "b200_sumsq_partials", "b200_clip_adamw",
-                                "b200_rms_norm_rows_h", "b200_rms_norm_bwd_rows_h", "b200_attn_train_fwd_h",
+                                "b200_rms_norm_rows_h", "b200_rms_norm_bwd_rows_h", "b200_attn_train_fwd_h", "b200_attn_train_fwd_tc", "b200_attn_train_bwd_tc",
                                 "b200_silu_mul_rows_h", "b200_silu_mul_bwd_rows_h", "b200_softmax_ce_rows_h",
                                 "b200_grpo_policy_grad", "b200_scale", "b200_sgd_apply_f16", "b200_gelu_mul_rows", "b200_gelu_mul_bwd_rows", "b200_add"],
     "llmb200_sft.h": ["sft_state_create", "sft_state_free", "sft_train_step", "forward_to_logits", "sft_backward",
@@ -414,6 +414,8 @@ def lib():
         "b200_rms_norm_rows_h": (i, [vp, vp, vp, vp, i, i, fl, vp]),
         "b200_rms_norm_bwd_rows_h": (i, [vp, vp, ll, vp, vp, i, i, fl, i, fl, vp, fl, vp]),
         "b200_attn_train_fwd_h": (i, [vp, vp, vp, ll, i, i, i, i, i, fl, vp, vp, vp, vp]),
+        "b200_attn_train_fwd_tc": (i, [vp, vp, vp, ll, i, i, i, i, i, fl, vp, vp, vp, vp]),
+        "b200_attn_train_bwd_tc": (i, [vp, vp, vp, vp, vp, ll, i, i, i, i, i, fl, vp, vp, ll, vp]),
         "b200_silu_mul_rows_h": (i, [vp, i, i, vp, vp, vp]),
         "b200_silu_mul_bwd_rows_h": (i, [vp, vp, i, i, vp, vp, fl, vp]),
         "b200_softmax_ce_rows_h": (i, [vp, vp, i, i, fl, vp, vp, vp, fl, vp]),

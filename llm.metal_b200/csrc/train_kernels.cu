@@ -226,15 +226,62 @@ __device__ __forceinline__ void mma_add(float (&acc)[NT][4], const float *A, int
     }
 }
 
-// The same, four columns of eight at a time in sums of their own that join acc in fp32 adds: tensor cores truncate when they
-// accumulate, which over all tiles of a long row would add up (7e-6 of dK at 509 positions, 1e-6 so).
+// The same sums as fp32 multiply-adds in order of k, for operands whose k are contiguous (b(k, n) at B[n * bn + k]).
 template <int NT>
-__device__ __forceinline__ void mma_add_apart(float (&acc)[NT][4], const float *A, int am, int ak, const float *B, int bk, int bn, int K)
+__device__ __forceinline__ void fma_add(float (&acc)[NT][4], const float *A, int am, const float *B, int bn, int K)
 {
+    const int r = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+#pragma unroll 2
+    for (int k = 0; k < K; k += 4) {
+        const float4 a0 = *reinterpret_cast<const float4 *>(A + r * am + k), a1 = *reinterpret_cast<const float4 *>(A + (r + 8) * am + k);
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const float4 b = *reinterpret_cast<const float4 *>(B + (n * 8 + 2 * q + e) * bn + k);
+                acc[n][e] = fmaf(a0.w, b.w, fmaf(a0.z, b.z, fmaf(a0.y, b.y, fmaf(a0.x, b.x, acc[n][e]))));
+                acc[n][2 + e] = fmaf(a1.w, b.w, fmaf(a1.z, b.z, fmaf(a1.y, b.y, fmaf(a1.x, b.x, acc[n][2 + e]))));
+            }
+    }
+}
+
+// Scores of 16 x 8 NT: rows of A times rows of B, K long. TC: tensor cores.
+template <bool TC, int NT>
+__device__ __forceinline__ void score_tile(float (&acc)[NT][4], const float *A, int am, const float *B, int bn, int K)
+{
+    if (TC) {
+        mma_add<NT>(acc, A, am, 1, B, 1, bn, K);
+    } else {
+        fma_add<NT>(acc, A, am, B, bn, K);
+    }
+}
+
+// acc += weights (16 x 64) . rows (64 x 8 NT), row r + 8 a of the fragment over k in [from[a], to[a]), beyond which its weights are zero.
+// Four columns of eight at a time in sums of their own that join acc in fp32 adds: tensor cores truncate when they
+// accumulate, which over all tiles of a long row would add up (7e-6 of dK at 509 positions, 1e-6 so). fp32 sums leave the other k out.
+template <bool TC, int NT>
+__device__ __forceinline__ void weighted_rows(float (&acc)[NT][4], const float *A, int am, int ak, const float *B, int bk, const int (&from)[2],
+                                              const int (&to)[2])
+{
+    const int r = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
 #pragma unroll
     for (int g = 0; g < NT; g += 4) {
         float t[4][4] = {};
-        mma_add<4>(t, A, am, ak, B + g * 8 * bn, bk, bn, K);
+        if (TC) {
+            mma_add<4>(t, A, am, ak, B + g * 8, bk, 1, AT);
+        } else {
+#pragma unroll 4
+            for (int k = min(from[0], from[1]); k < max(to[0], to[1]); ++k) {
+                const float w0 = A[r * am + k * ak], w1 = A[(r + 8) * am + k * ak];
+                const bool on0 = k >= from[0] && k < to[0], on1 = k >= from[1] && k < to[1];
+#pragma unroll
+                for (int n = 0; n < 4; ++n) {
+                    const float2 b = *reinterpret_cast<const float2 *>(B + k * bk + (g + n) * 8 + 2 * q);
+                    if (on0) { t[n][0] = fmaf(w0, b.x, t[n][0]); t[n][1] = fmaf(w0, b.y, t[n][1]); }
+                    if (on1) { t[n][2] = fmaf(w1, b.x, t[n][2]); t[n][3] = fmaf(w1, b.y, t[n][3]); }
+                }
+            }
+        }
 #pragma unroll
         for (int n = 0; n < 4; ++n)
 #pragma unroll
@@ -277,7 +324,7 @@ __device__ __forceinline__ float quad_sum(float v)
     return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-template <int HD>
+template <int HD, bool TC>
 __global__ void __launch_bounds__(ATT_THREADS)
 attn_fwd_kernel(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q, int n_kv,
                 float scale, float *probs, float *out, __half *out_h)
@@ -306,7 +353,7 @@ attn_fwd_kernel(const float *q, const float *k, const float *v, long long v_ld, 
         } else tile_wait<0>();
         __syncthreads();
         float acc[4][4] = {};
-        mma_add<4>(acc, Q + rw * L::RP, L::RP, 1, buf + (jt & 1) * L::BUF + half * 32 * L::RP, 1, L::RP, HD);
+        score_tile<TC>(acc, Q + rw * L::RP, L::RP, buf + (jt & 1) * L::BUF + half * 32 * L::RP, L::RP, HD);
 #pragma unroll
         for (int a = 0; a < 2; ++a) {
             const int i = r0 + 8 * a;
@@ -373,7 +420,8 @@ attn_fwd_kernel(const float *q, const float *k, const float *v, long long v_ld, 
             tile_wait<1>();
         } else tile_wait<0>();
         __syncthreads();
-        mma_add_apart<HD / 16>(o, P + rw * L::PP, L::PP, 1, buf + (jt & 1) * L::BUF + half * (HD / 2), L::CP, 1, AT);
+        const int from[2] = {0, 0}, to[2] = {r0 < ni ? min(AT, i0 + r0 - j0 + 1) : 0, r0 + 8 < ni ? min(AT, i0 + r0 + 8 - j0 + 1) : 0};
+        weighted_rows<TC>(o, P + rw * L::PP, L::PP, 1, buf + (jt & 1) * L::BUF + half * (HD / 2), L::CP, from, to);
         __syncthreads();
     }
     const int ahead = min((it + 1) * AT, N);                   // columns that no row of the tile sees
@@ -395,7 +443,7 @@ attn_fwd_kernel(const float *q, const float *k, const float *v, long long v_ld, 
 }
 
 // d_score = p * (dO . V - sum_j p_j (dO . V_j)) * scale, and dQ = d_score . K, for 64 queries of a head.
-template <int HD>
+template <int HD, bool TC>
 __global__ void __launch_bounds__(ATT_THREADS)
 attn_bwd_dq_kernel(const float *d_out, const float *probs, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q,
                    int n_kv, float scale, float *d_score, float *dqkv, long long ld)
@@ -426,7 +474,7 @@ attn_bwd_dq_kernel(const float *d_out, const float *probs, const float *k, const
         } else tile_wait<0>();
         __syncthreads();
         float acc[4][4] = {};
-        mma_add<4>(acc, O + rw * L::RP, L::RP, 1, buf + (jt & 1) * L::BUF + half * 32 * L::RP, 1, L::RP, HD);
+        score_tile<TC>(acc, O + rw * L::RP, L::RP, buf + (jt & 1) * L::BUF + half * 32 * L::RP, L::RP, HD);
 #pragma unroll
         for (int a = 0; a < 2; ++a)
 #pragma unroll
@@ -474,7 +522,8 @@ attn_bwd_dq_kernel(const float *d_out, const float *probs, const float *k, const
             tile_wait<1>();
         } else tile_wait<0>();
         __syncthreads();
-        mma_add_apart<HD / 16>(o, G + rw * L::PP, L::PP, 1, buf + (jt & 1) * L::BUF + half * (HD / 2), L::CP, 1, AT);
+        const int from[2] = {0, 0}, to[2] = {r0 < ni ? min(AT, i0 + r0 - j0 + 1) : 0, r0 + 8 < ni ? min(AT, i0 + r0 + 8 - j0 + 1) : 0};
+        weighted_rows<TC>(o, G + rw * L::PP, L::PP, 1, buf + (jt & 1) * L::BUF + half * (HD / 2), L::CP, from, to);
         __syncthreads();
     }
     const int ahead = min((it + 1) * AT, N);
@@ -492,6 +541,7 @@ attn_bwd_dq_kernel(const float *d_out, const float *probs, const float *k, const
 
 // 64 keys x 64 columns of dK (d_score^T . Q) or dV (P^T . dO) of a KV head: summed over the later queries of each query head, then
 // over the heads in order. blockIdx.y = ((kv head * 2 + dK / dV) * (HD / 64) + columns).
+template <bool TC>
 __global__ void __launch_bounds__(ATT_THREADS)
 attn_bwd_dkv_kernel(const float *d_score, const float *probs, const float *q, const float *d_out, int n_seq, int N, int n_q, int n_kv,
                     int hd, float *dqkv, long long ld)
@@ -517,7 +567,9 @@ attn_bwd_dkv_kernel(const float *d_score, const float *probs, const float *q, co
         else tile_wait<0>();
         __syncthreads();
         const float *w = sh + (t & 1) * 2 * BUF;
-        mma_add_apart<4>(sum, w + rw, 1, CP, w + BUF + half * 32, CP, 1, AT);
+        const int i0 = j0 + t % tiles * AT, ni = min(AT, N - i0), first = j0 + rw + (lane >> 2) - i0;
+        const int from[2] = {max(0, first), max(0, first + 8)}, to[2] = {ni, ni};
+        weighted_rows<TC>(sum, w + rw, 1, CP, w + BUF + half * 32, CP, from, to);
         __syncthreads();
     }
 #pragma unroll
@@ -1123,28 +1175,42 @@ static bool attn_shape_ok(int n_seq, int seq_len, int n_q, int n_kv, int hd)
     return n_seq > 0 && seq_len > 0 && n_q > 0 && n_kv > 0 && n_q % n_kv == 0 && (hd == 64 || hd == 128 || hd == 256);
 }
 
-template <int HD>
+template <int HD, bool TC>
 static int attn_fwd_launch(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q,
                            int n_kv, float scale, float *probs, float *out, __half *out_h, cudaStream_t st)
 {
     constexpr size_t smem = AttnTiles<HD>::bytes;
-    int rc = opt_in_smem(attn_fwd_kernel<HD>, smem);
+    int rc = opt_in_smem(attn_fwd_kernel<HD, TC>, smem);
     if (rc) return rc;
-    attn_fwd_kernel<HD><<<dim3((N + AT - 1) / AT * n_seq, n_q), ATT_THREADS, smem, st>>>(q, k, v, v_ld, n_seq, N, n_q, n_kv, scale, probs, out, out_h);
+    attn_fwd_kernel<HD, TC><<<dim3((N + AT - 1) / AT * n_seq, n_q), ATT_THREADS, smem, st>>>(q, k, v, v_ld, n_seq, N, n_q, n_kv, scale, probs, out, out_h);
     return done();
+}
+
+template <bool TC>
+static int attn_fwd(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int seq_len, int n_q, int n_kv, int hd, float scale,
+                    float *probs, float *out, void *out_h, void *stream)
+{
+    if (!q || !k || !v || !probs || (!out && !out_h) || !attn_shape_ok(n_seq, seq_len, n_q, n_kv, hd)) return B200_E_BADARG;
+    if ((v_ld & 3) || ((uintptr_t)v & 15) || ((uintptr_t)k & 15)) return B200_E_BADARG;     // 16-byte row loads
+    cudaStream_t st = (cudaStream_t)stream;
+    __half *oh = static_cast<__half *>(out_h);
+    if (hd == 64) return attn_fwd_launch<64, TC>(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, probs, out, oh, st);
+    if (hd == 128) return attn_fwd_launch<128, TC>(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, probs, out, oh, st);
+    return attn_fwd_launch<256, TC>(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, probs, out, oh, st);
 }
 
 extern "C" int b200_attn_train_fwd_h(const float *q, const float *k, const float *v, long long v_ld, int n_seq,
                                      int seq_len, int n_q, int n_kv, int hd, float scale, float *probs, float *out,
                                      void *out_h, void *stream)
 {
-    if (!q || !k || !v || !probs || (!out && !out_h) || !attn_shape_ok(n_seq, seq_len, n_q, n_kv, hd)) return B200_E_BADARG;
-    if ((v_ld & 3) || ((uintptr_t)v & 15) || ((uintptr_t)k & 15)) return B200_E_BADARG;     // 16-byte row loads
-    cudaStream_t st = (cudaStream_t)stream;
-    __half *oh = static_cast<__half *>(out_h);
-    if (hd == 64) return attn_fwd_launch<64>(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, probs, out, oh, st);
-    if (hd == 128) return attn_fwd_launch<128>(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, probs, out, oh, st);
-    return attn_fwd_launch<256>(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, probs, out, oh, st);
+    return attn_fwd<false>(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, hd, scale, probs, out, out_h, stream);
+}
+
+extern "C" int b200_attn_train_fwd_tc(const float *q, const float *k, const float *v, long long v_ld, int n_seq,
+                                      int seq_len, int n_q, int n_kv, int hd, float scale, float *probs, float *out,
+                                      void *out_h, void *stream)
+{
+    return attn_fwd<true>(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, hd, scale, probs, out, out_h, stream);
 }
 
 extern "C" int b200_attn_train_fwd(const float *q, const float *k, const float *v, long long v_ld, int n_seq,
@@ -1155,34 +1221,48 @@ extern "C" int b200_attn_train_fwd(const float *q, const float *k, const float *
     return b200_attn_train_fwd_h(q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, hd, scale, probs, out, nullptr, stream);
 }
 
-template <int HD>
+template <int HD, bool TC>
 static int attn_bwd_launch(const float *d_out, const float *probs, const float *q, const float *k, const float *v,
                            long long v_ld, int n_seq, int N, int n_q, int n_kv, float scale, float *d_score,
                            float *dqkv, long long ld, cudaStream_t st)
 {
     constexpr size_t smem = AttnTiles<HD>::bytes, smem_kv = 4 * (size_t)AT * (AT + 8) * sizeof(float);
-    int rc = opt_in_smem(attn_bwd_dq_kernel<HD>, smem);
-    if (!rc) rc = opt_in_smem(attn_bwd_dkv_kernel, smem_kv);
+    int rc = opt_in_smem(attn_bwd_dq_kernel<HD, TC>, smem);
+    if (!rc) rc = opt_in_smem(attn_bwd_dkv_kernel<TC>, smem_kv);
     if (rc) return rc;
     const int tiles = (N + AT - 1) / AT;
-    attn_bwd_dq_kernel<HD><<<dim3(tiles * n_seq, n_q), ATT_THREADS, smem, st>>>(d_out, probs, k, v, v_ld, n_seq, N, n_q, n_kv, scale, d_score, dqkv, ld);
+    attn_bwd_dq_kernel<HD, TC><<<dim3(tiles * n_seq, n_q), ATT_THREADS, smem, st>>>(d_out, probs, k, v, v_ld, n_seq, N, n_q, n_kv, scale, d_score, dqkv, ld);
     rc = done();
     if (rc) return rc;
-    attn_bwd_dkv_kernel<<<dim3(tiles * n_seq, n_kv * 2 * (HD / 64)), ATT_THREADS, smem_kv, st>>>(d_score, probs, q, d_out, n_seq, N, n_q, n_kv, HD, dqkv, ld);
+    attn_bwd_dkv_kernel<TC><<<dim3(tiles * n_seq, n_kv * 2 * (HD / 64)), ATT_THREADS, smem_kv, st>>>(d_score, probs, q, d_out, n_seq, N, n_q, n_kv, HD, dqkv, ld);
     return done();
+}
+
+template <bool TC>
+static int attn_bwd(const float *d_out, const float *probs, const float *q, const float *k, const float *v, long long v_ld, int n_seq, int seq_len,
+                    int n_q, int n_kv, int hd, float scale, float *d_score, float *dqkv, long long ld, void *stream)
+{
+    if (!d_out || !probs || !q || !k || !v || !d_score || !dqkv || !attn_shape_ok(n_seq, seq_len, n_q, n_kv, hd))
+        return B200_E_BADARG;
+    if ((v_ld & 3) || ((uintptr_t)v & 15)) return B200_E_BADARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    if (hd == 64) return attn_bwd_launch<64, TC>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, d_score, dqkv, ld, st);
+    if (hd == 128) return attn_bwd_launch<128, TC>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, d_score, dqkv, ld, st);
+    return attn_bwd_launch<256, TC>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, d_score, dqkv, ld, st);
 }
 
 extern "C" int b200_attn_train_bwd(const float *d_out, const float *probs, const float *q, const float *k,
                                    const float *v, long long v_ld, int n_seq, int seq_len, int n_q, int n_kv, int hd,
                                    float scale, float *d_score, float *dqkv, long long ld, void *stream)
 {
-    if (!d_out || !probs || !q || !k || !v || !d_score || !dqkv || !attn_shape_ok(n_seq, seq_len, n_q, n_kv, hd))
-        return B200_E_BADARG;
-    if ((v_ld & 3) || ((uintptr_t)v & 15)) return B200_E_BADARG;
-    cudaStream_t st = (cudaStream_t)stream;
-    if (hd == 64) return attn_bwd_launch<64>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, d_score, dqkv, ld, st);
-    if (hd == 128) return attn_bwd_launch<128>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, d_score, dqkv, ld, st);
-    return attn_bwd_launch<256>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, scale, d_score, dqkv, ld, st);
+    return attn_bwd<false>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, hd, scale, d_score, dqkv, ld, stream);
+}
+
+extern "C" int b200_attn_train_bwd_tc(const float *d_out, const float *probs, const float *q, const float *k,
+                                      const float *v, long long v_ld, int n_seq, int seq_len, int n_q, int n_kv, int hd,
+                                      float scale, float *d_score, float *dqkv, long long ld, void *stream)
+{
+    return attn_bwd<true>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, hd, scale, d_score, dqkv, ld, stream);
 }
 
 extern "C" int b200_silu_mul_rows_h(const float *gu, int rows, int inter, float *act, void *act_h, void *stream)

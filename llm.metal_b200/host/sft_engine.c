@@ -382,7 +382,7 @@ static SFTState *sft_begin(const llmb200_config *cfg, int seq_len, int n_seq, in
     s->d_lnx = dalloc(s, (size_t)M * (s->D + s->XR));
     s->d_act = dalloc(s, (size_t)M * s->IS); s->d_gu = dalloc(s, (size_t)M * 2 * s->IS);
     s->d_att = dalloc(s, (size_t)M * s->Hq_hd); s->dqkv = dalloc(s, (size_t)M * s->QKV);
-    s->d_score = dalloc(s, (size_t)s->S * s->Hq * s->N * (s->N > 2 * s->hd ? s->N : 2 * s->hd));
+    s->d_score = dalloc(s, (size_t)s->S * s->Hq * s->N * s->N);
     if (s->use_tc) {
         size_t widest = (size_t)s->V;
         if ((size_t)2 * s->IS > widest) widest = (size_t)2 * s->IS;
@@ -781,8 +781,9 @@ static void forward_device(SFTState *s)
                                    s->eps, l->q_f, l->k_f, st));
         /* with tensor cores on, the operand of the next product is written as binary16 straight into xh and
          * the fp32 copy of a tensor nothing else reads (attention output, activation) is not written at all */
-        S_TRY(s, b200_attn_train_fwd_h(l->q_f, l->k_f, l->qkv_out + s->Hq_hd + s->Hkv_hd, s->QKVX, s->S, s->N, s->Hq,
-                                       s->Hkv, s->hd, attn_scale, l->probs, s->use_tc ? NULL : s->att, s->xh, st));
+        S_TRY(s, (s->use_tc ? b200_attn_train_fwd_tc : b200_attn_train_fwd_h)(
+                     l->q_f, l->k_f, l->qkv_out + s->Hq_hd + s->Hkv_hd, s->QKVX, s->S, s->N, s->Hq, s->Hkv, s->hd, attn_scale,
+                     l->probs, s->use_tc ? NULL : s->att, s->xh, st));
         if (s->gemma) {
             /* Gemma3 (:697-704, :725-738): o -> post-attention norm -> + residual -> pre-FFN norm -> GeGLU FFN ->
              * post-FFN norm -> + residual; the raw projection outputs are saved for the backward pass. dx is free here. */
@@ -904,8 +905,9 @@ static void backward_device(SFTState *s)
         }
         /* dqkv is about to be rewritten: the LoRA-gradient products of the layer above must have read it */
         if (s->side_pending) { S_TRY(s, (int)cudaStreamWaitEvent(st, s->ev_join, 0)); s->side_pending = 0; }
-        S_TRY(s, b200_attn_train_bwd(s->d_att, l->probs, l->q_f, l->k_f, v, s->QKVX, s->S, s->N, s->Hq, s->Hkv, s->hd,
-                                     attn_scale, s->d_score, s->dqkv, QKV, st));
+        S_TRY(s, (s->use_tc ? b200_attn_train_bwd_tc : b200_attn_train_bwd)(
+                     s->d_att, l->probs, l->q_f, l->k_f, v, s->QKVX, s->S, s->N, s->Hq, s->Hkv, s->hd, attn_scale, s->d_score, s->dqkv,
+                     QKV, st));
         S_TRY(s, b200_qk_norm_rope_bwd(s->dqkv, l->qkv_out, s->QKVX, QKV, l->g_q, l->g_k, l->inv_freq, M, s->N, s->Hq,
                                        s->Hkv, s->hd, s->eps, st));
         const float *dq = s->dqkv, *dv = s->dqkv + s->Hq_hd + s->Hkv_hd;

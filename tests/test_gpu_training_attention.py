@@ -55,3 +55,63 @@ def test_forward_and_backward(lib, hd, S, N, Hq, Hkv, shift):
         size = 1e-3 * (hd * N) ** 0.5                          # one position: dQ and dK are zero up to rounding
         assert float((a.double() - rows(b)).norm()) <= 5e-6 * float(rows(b).norm()) + 1e-7 * size, name
     assert (dqkv[:, (Hq + 2 * Hkv) * hd:] == 7.0).all()
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("poison", [float("inf"), float("nan")])
+@pytest.mark.parametrize("tc", [0])
+def test_other_rows_stay_out(lib, hd, poison, tc):
+    """An infinity or NaN at one position reaches the sums that contain it and no other: later keys and values are left out, not weighted zero."""
+    S, N, Hq, Hkv, at = 2, 200, 2, 1, 70
+    g = torch.Generator().manual_seed(hd)
+    M, ld = S * N, (Hq + 2 * Hkv) * hd
+    qkv = torch.randn(M, ld, generator=g).cuda()
+    tensors = dict(q=torch.randn(M, Hq * hd, generator=g).cuda(), k=torch.randn(M, Hkv * hd, generator=g).cuda(),
+                   v=qkv, d=torch.randn(M, Hq * hd, generator=g).cuda())
+
+    def run(t):
+        v = t["v"][:, (Hq + Hkv) * hd:]
+        probs, out = torch.zeros(S, Hq, N, N, device="cuda"), torch.zeros(M, Hq * hd, device="cuda")
+        d_score, dqkv = torch.zeros(S * Hq * N * N, device="cuda"), torch.zeros(M, ld, device="cuda")
+        fwd, bwd = (lib.b200_attn_train_fwd_tc, lib.b200_attn_train_bwd_tc) if tc else (lib.b200_attn_train_fwd_h, lib.b200_attn_train_bwd)
+        assert fwd(t["q"].data_ptr(), t["k"].data_ptr(), v.data_ptr(), ld, S, N, Hq, Hkv, hd, hd ** -0.5, probs.data_ptr(), out.data_ptr(), None,
+                   None) == 0
+        assert bwd(t["d"].data_ptr(), probs.data_ptr(), t["q"].data_ptr(), t["k"].data_ptr(), v.data_ptr(), ld, S, N, Hq, Hkv, hd,
+                   hd ** -0.5, d_score.data_ptr(), dqkv.data_ptr(), ld, None) == 0
+        torch.cuda.synchronize()
+        return out, dqkv[:, : Hq * hd], dqkv[:, Hq * hd:]
+    plain = run(tensors)
+    rows = torch.arange(M, device="cuda")
+    others, before, after = rows != at, (rows < at) | (rows >= N), (rows > at)
+    # which rows of (out, dQ, dK and dV) do not contain position `at` of the poisoned tensor
+    free = dict(q=(others, others, after), k=(before, before, rows >= N), v=(before, before, rows >= N), d=(others, others, after))
+    for name, keep in free.items():
+        t = dict(tensors)
+        t[name] = tensors[name].clone()
+        t[name][at, -hd // 2:] = poison                       # of v's rows the last columns are the values
+        for part, a, b, k in zip(("out", "dq", "dkv"), run(t), plain, keep):
+            if tc:                                            # a fragment with an infinity is summed in fp32 instead
+                assert torch.isfinite(a[k]).all() and rel(a[k], b[k].double()) < 2e-6, (name, part)
+            else:
+                assert torch.equal(a[k], b[k]), (name, part)
+
+
+@pytest.mark.parametrize("tensor_cores", [False, True])
+def test_the_engine_takes_the_form_it_was_asked_for(lib, pkg, tensor_cores):
+    """With tensor cores off every product is fp32 on the CUDA cores, the attention's too: its probabilities are that form's to the bit."""
+    import _sft_common as sc
+    cfg, N, S = sc.SMALL, 40, 2
+    Hq, Hkv, hd = cfg["n_q_heads"], cfg["n_kv_heads"], cfg["head_dim"]
+    eng = sc.Engine(pkg, cfg, sc.make_weights(pkg, cfg), sc.make_lora(pkg, cfg, 4, b_std=0.02), N, S, 4, 8.0, tensor_cores=tensor_cores)
+    ids = sc.tokens(pkg, N * S, 3, cfg["vocab_size"]).reshape(S, N)
+    eng.forward_backward(ids, ids)
+    q, k = (torch.from_numpy(eng.export(what, 1, N * S * h * hd)).cuda() for what, h in ((sc.Q_FINAL, Hq), (sc.K_FINAL, Hkv)))
+    got = torch.from_numpy(eng.export(sc.PROBS, 1, S * Hq * N * N)).cuda()
+    v, out, same = torch.zeros(N * S, Hkv * hd, device="cuda"), torch.zeros(N * S, Hq * hd, device="cuda"), []
+    for fwd in (lib.b200_attn_train_fwd_h, lib.b200_attn_train_fwd_tc):
+        probs = torch.zeros_like(got)
+        assert fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), Hkv * hd, S, N, Hq, Hkv, hd, hd ** -0.5, probs.data_ptr(), out.data_ptr(), None, None) == 0
+        torch.cuda.synchronize()
+        same.append(torch.equal(probs, got))
+    assert same == [not tensor_cores, tensor_cores]
+    eng.close()
