@@ -245,20 +245,38 @@ __device__ __forceinline__ void fma_add(float (&acc)[NT][4], const float *A, int
     }
 }
 
-// Scores of 16 x 8 NT: rows of A times rows of B, K long. TC: tensor cores.
+// Whether any lane holds an infinity or NaN.
+template <int NT>
+__device__ __forceinline__ bool any_not_finite(const float (&t)[NT][4])
+{
+    float z = 0.f;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) z = fmaf(t[n][e], 0.f, z);
+    return __any_sync(0xffffffffu, z != z);
+}
+
+// Scores of 16 x 8 NT: rows of A times rows of B, HD long. TC: tensor cores; sums that come out infinite or NaN are formed again as
+// fp32 sums, because the parts of an infinity are an infinity and a NaN.
 template <bool TC, int NT>
 __device__ __forceinline__ void score_tile(float (&acc)[NT][4], const float *A, int am, const float *B, int bn, int K)
 {
     if (TC) {
         mma_add<NT>(acc, A, am, 1, B, 1, bn, K);
-    } else {
-        fma_add<NT>(acc, A, am, B, bn, K);
+        if (!any_not_finite(acc)) return;
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
     }
+    fma_add<NT>(acc, A, am, B, bn, K);
 }
 
 // acc += weights (16 x 64) . rows (64 x 8 NT), row r + 8 a of the fragment over k in [from[a], to[a]), beyond which its weights are zero.
 // Four columns of eight at a time in sums of their own that join acc in fp32 adds: tensor cores truncate when they
-// accumulate, which over all tiles of a long row would add up (7e-6 of dK at 509 positions, 1e-6 so). fp32 sums leave the other k out.
+// accumulate, which over all tiles of a long row would add up (7e-6 of dK at 509 positions, 1e-6 so). fp32 sums leave the other k
+// out, and so do those of the tensor cores when they come out infinite or NaN: zero times a later row's infinity is NaN.
 template <bool TC, int NT>
 __device__ __forceinline__ void weighted_rows(float (&acc)[NT][4], const float *A, int am, int ak, const float *B, int bk, const int (&from)[2],
                                               const int (&to)[2])
@@ -267,9 +285,14 @@ __device__ __forceinline__ void weighted_rows(float (&acc)[NT][4], const float *
 #pragma unroll
     for (int g = 0; g < NT; g += 4) {
         float t[4][4] = {};
-        if (TC) {
-            mma_add<4>(t, A, am, ak, B + g * 8, bk, 1, AT);
-        } else {
+        if (TC) mma_add<4>(t, A, am, ak, B + g * 8, bk, 1, AT);
+        if (!TC || any_not_finite(t)) {
+            if (TC) {
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) t[n][e] = 0.f;
+            }
 #pragma unroll 4
             for (int k = min(from[0], from[1]); k < max(to[0], to[1]); ++k) {
                 const float w0 = A[r * am + k * ak], w1 = A[(r + 8) * am + k * ak];

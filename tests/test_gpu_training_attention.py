@@ -59,7 +59,7 @@ def test_forward_and_backward(lib, hd, S, N, Hq, Hkv, shift):
 
 @pytest.mark.parametrize("hd", [64, 128, 256])
 @pytest.mark.parametrize("poison", [float("inf"), float("nan")])
-@pytest.mark.parametrize("tc", [0])
+@pytest.mark.parametrize("tc", [0, 1])
 def test_other_rows_stay_out(lib, hd, poison, tc):
     """An infinity or NaN at one position reaches the sums that contain it and no other: later keys and values are left out, not weighted zero."""
     S, N, Hq, Hkv, at = 2, 200, 2, 1, 70
