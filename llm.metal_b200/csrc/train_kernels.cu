@@ -204,26 +204,41 @@ __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], 
 }
 
 // acc += A (16 x K) . B (K x 8 NT) of a warp: a(m, k) at A[m * am + k * ak], b(k, n) at B[k * bk + n * bn]. Lane l holds rows l / 4 and
-// l / 4 + 8, columns 2 (l % 4) and the next of every eight.
+// l / 4 + 8, columns 2 (l % 4) and the next of every eight. K: a multiple of 32.
+// Tensor cores truncate what they add to an accumulator, 1.4e-8 of it a time: the corrections have one of their own, and the sums of 32 of k
+// start from zero and join acc in fp32 adds.
 template <int NT>
 __device__ __forceinline__ void mma_add(float (&acc)[NT][4], const float *A, int am, int ak, const float *B, int bk, int bn, int K)
 {
     const int r = (threadIdx.x & 31) >> 2, q = threadIdx.x & 3;
+    float low[NT][4] = {};
+#pragma unroll 1
+    for (int k0 = 0; k0 < K; k0 += 32) {
+        float t[NT][4] = {};
 #pragma unroll 2
-    for (int k = 0; k < K; k += 8) {
-        uint32_t ah[4], al[4];
+        for (int k = k0; k < k0 + 32; k += 8) {
+            uint32_t ah[4], al[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) tf32_parts(A[(r + 8 * (e & 1)) * am + (k + q + 4 * (e >> 1)) * ak], ah[e], al[e]);
+            for (int e = 0; e < 4; ++e) tf32_parts(A[(r + 8 * (e & 1)) * am + (k + q + 4 * (e >> 1)) * ak], ah[e], al[e]);
 #pragma unroll
-        for (int n = 0; n < NT; ++n) {
-            uint32_t h0, l0, h1, l1;
-            tf32_parts(B[(k + q) * bk + (n * 8 + r) * bn], h0, l0);
-            tf32_parts(B[(k + q + 4) * bk + (n * 8 + r) * bn], h1, l1);
-            mma_tf32(acc[n], al, h0, h1);
-            mma_tf32(acc[n], ah, l0, l1);
-            mma_tf32(acc[n], ah, h0, h1);
+            for (int n = 0; n < NT; ++n) {
+                uint32_t h0, l0, h1, l1;
+                tf32_parts(B[(k + q) * bk + (n * 8 + r) * bn], h0, l0);
+                tf32_parts(B[(k + q + 4) * bk + (n * 8 + r) * bn], h1, l1);
+                mma_tf32(low[n], al, h0, h1);
+                mma_tf32(low[n], ah, l0, l1);
+                mma_tf32(t[n], ah, h0, h1);
+            }
         }
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[n][e] += t[n][e];
     }
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[n][e] += low[n][e];
 }
 
 // The same sums as fp32 multiply-adds in order of k, for operands whose k are contiguous (b(k, n) at B[n * bn + k]).

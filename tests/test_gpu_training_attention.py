@@ -115,3 +115,35 @@ def test_the_engine_takes_the_form_it_was_asked_for(lib, pkg, tensor_cores):
         same.append(torch.equal(probs, got))
     assert same == [not tensor_cores, tensor_cores]
     eng.close()
+
+
+@pytest.mark.parametrize("S,N,Hq,Hkv,hd", [(2, 64, 8, 2, 128), (1, 509, 8, 2, 128), (1, 64, 4, 1, 256), (1, 200, 8, 2, 64)])
+def test_tensor_cores_lose_nothing(lib, S, N, Hq, Hkv, hd):
+    """Both forms against float64 on the same inputs. Bar of the fp32 form: some hundred fp32 roundings of 2^-25 in a random walk, 1e-6. Of the
+    tensor-core form: the fp32 form's own error and a half of it again."""
+    g = torch.Generator().manual_seed(N + hd)
+    M, G, ld = S * N, Hq // Hkv, (Hq + 2 * Hkv) * hd
+    qkv = torch.randn(M, ld, generator=g).cuda()
+    q, k, d_out = (torch.randn(M, h * hd, generator=g).cuda() for h in (Hq, Hkv, Hq))
+    v = qkv[:, (Hq + Hkv) * hd:]
+
+    def heads(t, n):
+        return t.double().reshape(S, N, n, hd).transpose(1, 2)
+    Q, K, V = (t.detach().clone().requires_grad_() for t in (heads(q, Hq), heads(k, Hkv), heads(v[:, : Hkv * hd], Hkv)))
+    s = Q @ K.repeat_interleave(G, 1).transpose(-1, -2) * hd ** -0.5
+    p = torch.softmax(s.masked_fill(torch.ones(N, N, device="cuda").triu(1).bool(), -torch.inf), -1)
+    o = p @ V.repeat_interleave(G, 1)
+    o.backward(heads(d_out, Hq))
+    rows = [t.transpose(1, 2).reshape(M, -1) for t in (o.detach(), Q.grad, K.grad, V.grad)]
+    errors = []
+    for fwd, bwd in ((lib.b200_attn_train_fwd_h, lib.b200_attn_train_bwd), (lib.b200_attn_train_fwd_tc, lib.b200_attn_train_bwd_tc)):
+        probs, out = torch.zeros(S, Hq, N, N, device="cuda"), torch.zeros(M, Hq * hd, device="cuda")
+        d_score, dqkv = torch.zeros(S * Hq * N * N, device="cuda"), torch.zeros(M, ld, device="cuda")
+        assert fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), ld, S, N, Hq, Hkv, hd, hd ** -0.5, probs.data_ptr(), out.data_ptr(), None, None) == 0
+        assert bwd(d_out.data_ptr(), probs.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), ld, S, N, Hq, Hkv, hd, hd ** -0.5,
+                   d_score.data_ptr(), dqkv.data_ptr(), ld, None) == 0
+        torch.cuda.synchronize()
+        got = [out, dqkv[:, : Hq * hd], dqkv[:, Hq * hd:(Hq + Hkv) * hd], dqkv[:, (Hq + Hkv) * hd:]]
+        errors.append([rel(probs, p.detach())] + [rel(a, b) for a, b in zip(got, rows)])
+    assert max(errors[0]) < 1e-6, errors
+    assert all(b <= 1.5 * a for a, b in zip(*errors)), errors
