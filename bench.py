@@ -1086,7 +1086,7 @@ def sft_main(args, rank, local_rank, world):
         except Exception:
             peak, peak_kind = 1590.0, "fallback"
         ach = 2.0 * M * 2 * IS * D / sec / 1e12
-        roofline = {"bound": "tensor", "kernel": f"gemm_tf32_kernel, binary16 operands: gate/up forward (M {M}, N {2 * IS}, K {D})",
+        roofline = {"bound": "tensor", "kernel": f"gemm_pair_kernel, binary16 operands: gate/up forward (M {M}, N {2 * IS}, K {D})",
                     "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak, "peak_source": peak_kind,
                     "traffic": None, "us_per_launch": sec * 1e6}
     step_flops = sft_flops_per_token(sp) * M

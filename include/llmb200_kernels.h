@@ -565,8 +565,10 @@ int b200_argmax_rows(const float *logits, int n_rows, int vocab, unsigned *next_
  * sequences that advance together. */
 
 /* A product operand: `planes` binary16 planes of rows `ld` halves apart, plane p of row m at
- * d_x + (p * plane_rows + m) * ld. With d_scale the planes hold the row times a power of two (two planes: 22 bits
- * of every element) and d_scale[m] is its inverse; one plane without d_scale is the row rounded to binary16. */
+ * d_x + (p * plane_rows + m) * ld. With d_scale the planes hold the row times a power of two that brings its largest finite
+ * element into [2^14, 2^15), and d_scale[m] is its inverse. Two planes hold 22 bits of every element down to 2^-16 of the largest; below, the
+ * second plane is subnormal and an element is off by up to 2^-39 of the largest. Infinities and NaN lie in the first plane. One plane without
+ * d_scale is the row rounded to binary16. */
 typedef struct {
     void *d_x; long long ld;
     int planes, plane_rows;
@@ -586,7 +588,9 @@ typedef struct {
     float *d_out; long long out_ld;
     const float *d_resid; long long resid_ld;
     unsigned *d_err;
-    int use_pdl;
+    int use_pdl;                          /* programmatic dependent launch: the weights and d_w_scale are read ahead of the wait for the preceding
+                                             launch on the stream, so they must be complete before that one starts; d_x, d_x_scale and
+                                             d_resid may come from it */
 } b200_rows_matmul_args;
 int b200_rows_matmul(const b200_rows_matmul_args *a, void *stream);
 /* Per row of a packed Q8_0 matrix: the power of two that brings the row's largest block scale into [2^7, 2^8). */

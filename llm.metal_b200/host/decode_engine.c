@@ -39,7 +39,7 @@
 #include <time.h>
 
 static int enqueue_token(InferenceState *s, int with_lm, int pdl);
-/* Qwen3 and Gemma3: one token at a time, prompts included (as the reference's engine) */
+/* Qwen3 and Gemma3: tokens one at a time (as the reference's engine), prompts and longer portions in passes over the weights */
 static int prompt_rows(InferenceState *s, const uint32_t *tokens, int n, const int *want, int n_want, float *logits);
 static int prompt_rows_fit(const InferenceState *s, int n, int least);
 static void prompt_free(InferenceState *s);
@@ -1139,9 +1139,10 @@ static int prompt_ready(InferenceState *s, int n)
     return llmb200_plain_rows_fit(&m->rows, cap, 64);
 }
 
-/* Fewest tokens of a pass, and fewest of a portion of inference_forward_tokens: shorter portions of a Qwen3 / Gemma3 state go through
- * the per-token path and so keep its very bits (a pass adds in another order). Below four tokens the launches of a pass (ten a
- * layer, 3 us each) cost more than the tokens. */
+/* Fewest tokens of a prompt's pass: below four tokens the launches of a pass (ten a layer, 3 us each) cost more than the tokens.
+ * Fewest of a portion of inference_forward_tokens: a promise and not a matter of time. Portions of a Qwen3 / Gemma3 state that are shorter give
+ * the per-token path's very bits, as all of them did before there were passes (a pass adds in another order); programs that
+ * step through short portions and compare may hold on to that. */
 enum { PROMPT_MIN = 4, PORTION_MIN = 24 };
 
 /* An attached adapter and tensor parallelism run on the per-token path. */

@@ -341,7 +341,7 @@ def test_command_line(pkg, tmp_path):
 
 
 def test_other_model_types_take_portions_too(pkg, lib, synth):
-    """inference_forward_tokens on a Qwen3 state: token by token behind the same call."""
+    """inference_forward_tokens on a Qwen3 state: a portion too short for a pass gives the bits of its tokens one by one."""
     sp = pkg.spec("tiny-qwen3", n_layers=2)
     model = synth.llmb200_synth_qwen3(C.byref(sp), 4)
     st = lib.inference_state_create(model, 64, 0)
