@@ -391,3 +391,42 @@ def test_attention_is_as_exact_as_the_per_token_kernel(lib, pkg, n_q, n_kv, hd, 
         s = s.masked_fill(torch.ones(N, N, device="cuda").triu(1).bool(), -torch.inf)
         errors.append(rel(out, torch.einsum("hij,hjd->ihd", torch.softmax(s, -1), v)))
     assert errors[1] <= 1.5 * errors[0], errors
+
+
+def per_token(lib, pkg, d_w, stride, rows, cols, wt, x):
+    out = torch.zeros(len(x), rows, device="cuda")
+    for i in range(len(x)):
+        a = pkg.MatvecArgs()
+        a.d_w, a.row_stride, a.rows, a.cols, a.wtype = d_w.data_ptr(), stride, rows, cols, wt
+        a.in_mode, a.d_in_vec = pkg.B200_IN_VEC, x[i].data_ptr()
+        a.out_mode, a.n_out, a.eps = pkg.B200_OUT_STORE, 1, 1e-6
+        a.d_out[0] = out[i].data_ptr()
+        assert lib.b200_matvec(C.byref(a), None) == 0
+    torch.cuda.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("wtype", ["q8", "f16"])
+@pytest.mark.parametrize("rows,cols,n", [(512, 1536, 15), (2560, 2560, 4), (6144, 2560, 130), (2560, 9728, 48), (2560, 9728, 512), (2560, 4096, 1531)])
+def test_products_stay_near_fp32_sums(lib, pkg, synth, wtype, rows, cols, n):
+    """Against float64. Four truncated additions a step, half a unit each: up to 1.4e-7 of the result; the planes' last bits, 22 in either
+    operand: 0.7e-7; up to 152 rounded additions in a random walk: 1.5e-7. Bar: their sum in squares and a third, 3e-7. The per-token kernel's fp32
+    sums on the same operands are 1e-7 off and must not be more than three times as exact."""
+    wt = pkg.B200_WT_Q8 if wtype == "q8" else pkg.B200_WT_F16
+    d_w, stride = pack(lib, pkg, weights(synth, rows, cols, 3), wt)
+    exact_w = q8_values(lib, d_w, stride, rows, cols) if wtype == "q8" else d_w.view(torch.float16).view(rows, stride // 2)[:, :cols].double()
+    x = torch.randn(n, cols, generator=torch.Generator().manual_seed(n)).cuda()
+    px, scale, args = planes_buffer(pkg, n, n, cols, 2)
+    assert lib.b200_rows_split_planes(x.data_ptr(), n, cols, C.byref(args), None) == 0
+    ws, err = torch.zeros(rows, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    if wtype == "q8":
+        assert lib.b200_q8_row_scale(d_w.data_ptr(), stride, rows, cols, ws.data_ptr(), None) == 0
+    out = torch.zeros(n, rows, device="cuda")
+    a = pkg.RowsMatmulArgs(wt, d_w.data_ptr(), stride, rows, cols, ws.data_ptr(), px.data_ptr(), cols, 2, n, scale.data_ptr(), n, out.data_ptr(),
+                           rows, None, rows, err.data_ptr(), 0)
+    assert lib.b200_rows_matmul(C.byref(a), None) == 0
+    torch.cuda.synchronize()
+    want = x.double() @ exact_w.T
+    few = min(n, 8)
+    ours, theirs = rel(out, want), rel(per_token(lib, pkg, d_w, stride, rows, cols, wt, x[:few]), want[:few])
+    assert int(err) == 0 and ours <= min(3e-7, 3 * theirs), (ours, theirs)
