@@ -261,51 +261,6 @@ def test_q8_models_of_odd_block_counts(lib, pkg, synth):
     synth.llmb200_synth_free_qwen3(model)
 
 
-@pytest.mark.parametrize("planes", [1, 2])
-@pytest.mark.parametrize("dim", [12288, 58016, 58112, 60000])
-def test_rows_wider_than_shared_memory(lib, pkg, planes, dim):
-    """Rows that just fill the 48 KB a kernel has without asking, and either side of the 58 048 values that it can be given beside its own."""
-    g = torch.Generator().manual_seed(dim)
-    gu, x, y = (torch.randn(2, n * dim, generator=g).cuda() for n in (2, 1, 1))
-    gamma, post = torch.randn(dim, generator=g).cuda(), torch.randn(dim, generator=g).cuda()
-    buf, scale, args = planes_buffer(pkg, 2, 2, dim, planes, planes == 2)
-
-    def value():
-        torch.cuda.synchronize()
-        return buf.double().view(planes, 2, dim).sum(0) * (scale[:, None].double() if planes == 2 else 1.0)
-
-    def norm(t, w):
-        return t * torch.rsqrt(t.square().mean(-1, keepdim=True) + 1e-6) * w.double()
-    bar = 2e-6 if planes == 2 else 4e-4
-    for pairs in (0, 1):
-        gate, up = (gu[:, 0::2], gu[:, 1::2]) if pairs else (gu[:, :dim], gu[:, dim:])
-        assert lib.b200_rows_glu_planes(gu.data_ptr(), 2, dim, pairs, 0, C.byref(args), None) == 0
-        assert rel(value(), torch.nn.functional.silu(gate.double()) * up.double()) < bar
-    for with_post in (False, True):
-        xs = x.clone()
-        assert lib.b200_rows_norm_planes(xs.data_ptr(), 2, dim, y.data_ptr(), post.data_ptr() if with_post else None, gamma.data_ptr(), None, 1e-6,
-                                         C.byref(args), None) == 0
-        want = x.double() + (norm(y.double(), post) if with_post else y.double())
-        assert rel(xs, want) < 1e-6 and rel(value(), norm(want, gamma)) < bar
-
-
-def test_planes_of_rows_with_infinities(lib, pkg):
-    """An infinity is one plane's infinity and nothing in the other; it takes neither the range nor the bits of the row's other elements."""
-    rows, dim = 3, 256
-    x = torch.randn(rows, dim, generator=torch.Generator().manual_seed(1)) * 1e5
-    x[0, 7], x[1, 9], x[2, 11] = torch.inf, -torch.inf, torch.nan
-    finite = torch.isfinite(x)
-    buf, scale, args = planes_buffer(pkg, rows, rows, dim, 2)
-    d = x.cuda()
-    assert lib.b200_rows_split_planes(d.data_ptr(), rows, dim, C.byref(args), None) == 0
-    torch.cuda.synchronize()
-    hi, lo = (p.double().cpu() for p in buf.view(2, rows, dim))
-    value = (hi + lo) * scale.cpu()[:, None].double()
-    assert ((value - x.double()).abs()[finite] <= 2 ** -22 * x.double().abs()[finite] + 2 ** -38 * 4e5).all()
-    assert float(value[0, 7]) == float("inf") and float(value[1, 9]) == -float("inf") and torch.isnan(value[2, 11])
-    assert float(lo[0, 7]) == 0 and float(lo[1, 9]) == 0
-
-
 @pytest.mark.parametrize("hd,n_q,n_kv", [(64, 8, 2), (128, 4, 2), (256, 2, 1)])
 @pytest.mark.parametrize("poison", [1e30, float("nan")])
 def test_attention_leaves_later_values_out(lib, pkg, hd, n_q, n_kv, poison):
@@ -357,40 +312,49 @@ def test_attention_leaves_later_values_out(lib, pkg, hd, n_q, n_kv, poison):
     assert torch.equal(out[:at], plain[:at]) and torch.equal(out[at + 1:], plain[at + 1:])
 
 
-@pytest.mark.parametrize("n_q,n_kv,hd,N", [(8, 2, 64, 200), (8, 2, 128, 500), (4, 1, 256, 200)])
-def test_attention_is_as_exact_as_the_per_token_kernel(lib, pkg, n_q, n_kv, hd, N):
-    """Both against float64 over the keys and values that each left in its cache. Bar: the per-token kernel's error and a half of it again."""
-    g, heads = torch.Generator().manual_seed(hd), n_q + 2 * n_kv
-    qkv = torch.randn(N, heads, hd, generator=g).cuda()
-    qg, kg = (1 + 0.3 * torch.randn(hd, generator=g)).cuda(), (1 + 0.3 * torch.randn(hd, generator=g)).cuda()
-    freq = torch.tensor([1.0 / 1e4 ** (2 * d / hd) for d in range(hd // 2)], dtype=torch.float32).cuda()
-    ang = (torch.arange(N, device="cuda", dtype=torch.float32)[:, None] * freq).double()[:, None]
-    x = qkv[:, :n_q].double()
-    x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * qg.double()
-    u, w = x[..., : hd // 2], x[..., hd // 2:]
-    x = torch.cat([u * ang.cos() - w * ang.sin(), u * ang.sin() + w * ang.cos()], -1)
-    errors = []
-    for rows in (0, 1):
-        kc, vc = (torch.zeros(n_kv, N, hd, dtype=torch.float16, device="cuda") for _ in range(2))
-        out = torch.zeros(N, n_q, hd, device="cuda")
-        if rows:
-            q, qs = torch.zeros(2 * N * n_q * hd, dtype=torch.float16, device="cuda"), torch.zeros(N * n_q, device="cuda")
-            a = pkg.RowsAttnArgs(n_q, n_kv, hd, N, N, N, 0, 1e-6, qkv.data_ptr(), qg.data_ptr(), kg.data_ptr(), freq.data_ptr(), kc.data_ptr(),
-                                 vc.data_ptr(), 0, q.data_ptr(), qs.data_ptr(), out.data_ptr())
-            assert lib.b200_rows_attn(C.byref(a), None) == 0
-        else:
-            scratch, tickets = torch.zeros(lib.b200_attn_scratch_floats(n_q, hd, 4), device="cuda"), torch.zeros(n_kv, dtype=torch.int32, device="cuda")
-            pos = torch.arange(N, dtype=torch.int32, device="cuda")
-            for i in range(N):
-                a = pkg.AttnArgs(qkv[i].data_ptr(), qg.data_ptr(), kg.data_ptr(), freq.data_ptr(), kc.data_ptr(), vc.data_ptr(), out[i].data_ptr(),
-                                 scratch.data_ptr(), tickets.data_ptr(), pos[i:].data_ptr(), n_q, n_kv, hd, N, 4, 1e-6, 0)
-                assert lib.b200_attn_decode(C.byref(a), None) == 0
+def test_planes_of_rows_with_infinities(lib, pkg):
+    """An infinity is one plane's infinity and nothing in the other; it takes neither the range nor the bits of the row's other elements."""
+    rows, dim = 3, 256
+    x = torch.randn(rows, dim, generator=torch.Generator().manual_seed(1)) * 1e5
+    x[0, 7], x[1, 9], x[2, 11] = torch.inf, -torch.inf, torch.nan
+    finite = torch.isfinite(x)
+    buf, scale, args = planes_buffer(pkg, rows, rows, dim, 2)
+    d = x.cuda()
+    assert lib.b200_rows_split_planes(d.data_ptr(), rows, dim, C.byref(args), None) == 0
+    torch.cuda.synchronize()
+    hi, lo = (p.double().cpu() for p in buf.view(2, rows, dim))
+    value = (hi + lo) * scale.cpu()[:, None].double()
+    assert ((value - x.double()).abs()[finite] <= 2 ** -22 * x.double().abs()[finite] + 2 ** -38 * 4e5).all()
+    assert float(value[0, 7]) == float("inf") and float(value[1, 9]) == -float("inf") and torch.isnan(value[2, 11])
+    assert float(lo[0, 7]) == 0 and float(lo[1, 9]) == 0
+
+
+@pytest.mark.parametrize("planes", [1, 2])
+@pytest.mark.parametrize("dim", [12288, 58016, 58112, 60000])
+def test_rows_wider_than_shared_memory(lib, pkg, planes, dim):
+    """Rows that just fill the 48 KB a kernel has without asking, and either side of the 58 048 values that it can be given beside its own."""
+    g = torch.Generator().manual_seed(dim)
+    gu, x, y = (torch.randn(2, n * dim, generator=g).cuda() for n in (2, 1, 1))
+    gamma, post = torch.randn(dim, generator=g).cuda(), torch.randn(dim, generator=g).cuda()
+    buf, scale, args = planes_buffer(pkg, 2, 2, dim, planes, planes == 2)
+
+    def value():
         torch.cuda.synchronize()
-        k, v = (t.double().repeat_interleave(n_q // n_kv, 0) for t in (kc, vc))
-        s = torch.einsum("ihd,hjd->hij", x, k) / hd ** 0.5
-        s = s.masked_fill(torch.ones(N, N, device="cuda").triu(1).bool(), -torch.inf)
-        errors.append(rel(out, torch.einsum("hij,hjd->ihd", torch.softmax(s, -1), v)))
-    assert errors[1] <= 1.5 * errors[0], errors
+        return buf.double().view(planes, 2, dim).sum(0) * (scale[:, None].double() if planes == 2 else 1.0)
+
+    def norm(t, w):
+        return t * torch.rsqrt(t.square().mean(-1, keepdim=True) + 1e-6) * w.double()
+    bar = 2e-6 if planes == 2 else 4e-4
+    for pairs in (0, 1):
+        gate, up = (gu[:, 0::2], gu[:, 1::2]) if pairs else (gu[:, :dim], gu[:, dim:])
+        assert lib.b200_rows_glu_planes(gu.data_ptr(), 2, dim, pairs, 0, C.byref(args), None) == 0
+        assert rel(value(), torch.nn.functional.silu(gate.double()) * up.double()) < bar
+    for with_post in (False, True):
+        xs = x.clone()
+        assert lib.b200_rows_norm_planes(xs.data_ptr(), 2, dim, y.data_ptr(), post.data_ptr() if with_post else None, gamma.data_ptr(), None, 1e-6,
+                                         C.byref(args), None) == 0
+        want = x.double() + (norm(y.double(), post) if with_post else y.double())
+        assert rel(xs, want) < 1e-6 and rel(value(), norm(want, gamma)) < bar
 
 
 def per_token(lib, pkg, d_w, stride, rows, cols, wt, x):
@@ -430,3 +394,98 @@ def test_products_stay_near_fp32_sums(lib, pkg, synth, wtype, rows, cols, n):
     few = min(n, 8)
     ours, theirs = rel(out, want), rel(per_token(lib, pkg, d_w, stride, rows, cols, wt, x[:few]), want[:few])
     assert int(err) == 0 and ours <= min(3e-7, 3 * theirs), (ours, theirs)
+
+
+@pytest.mark.parametrize("n_q,n_kv,hd,N", [(8, 2, 64, 200), (8, 2, 128, 500), (4, 1, 256, 200)])
+def test_attention_is_as_exact_as_the_per_token_kernel(lib, pkg, n_q, n_kv, hd, N):
+    """Both against float64 over the keys and values that each left in its cache. Bar: the per-token kernel's error and a half of it again."""
+    g, heads = torch.Generator().manual_seed(hd), n_q + 2 * n_kv
+    qkv = torch.randn(N, heads, hd, generator=g).cuda()
+    qg, kg = (1 + 0.3 * torch.randn(hd, generator=g)).cuda(), (1 + 0.3 * torch.randn(hd, generator=g)).cuda()
+    freq = torch.tensor([1.0 / 1e4 ** (2 * d / hd) for d in range(hd // 2)], dtype=torch.float32).cuda()
+    ang = (torch.arange(N, device="cuda", dtype=torch.float32)[:, None] * freq).double()[:, None]
+    x = qkv[:, :n_q].double()
+    x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + 1e-6) * qg.double()
+    u, w = x[..., : hd // 2], x[..., hd // 2:]
+    x = torch.cat([u * ang.cos() - w * ang.sin(), u * ang.sin() + w * ang.cos()], -1)
+    errors = []
+    for rows in (0, 1):
+        kc, vc = (torch.zeros(n_kv, N, hd, dtype=torch.float16, device="cuda") for _ in range(2))
+        out = torch.zeros(N, n_q, hd, device="cuda")
+        if rows:
+            q, qs = torch.zeros(2 * N * n_q * hd, dtype=torch.float16, device="cuda"), torch.zeros(N * n_q, device="cuda")
+            a = pkg.RowsAttnArgs(n_q, n_kv, hd, N, N, N, 0, 1e-6, qkv.data_ptr(), qg.data_ptr(), kg.data_ptr(), freq.data_ptr(), kc.data_ptr(),
+                                 vc.data_ptr(), 0, q.data_ptr(), qs.data_ptr(), out.data_ptr())
+            assert lib.b200_rows_attn(C.byref(a), None) == 0
+        else:
+            scratch, tickets = torch.zeros(lib.b200_attn_scratch_floats(n_q, hd, 4), device="cuda"), torch.zeros(n_kv, dtype=torch.int32, device="cuda")
+            pos = torch.arange(N, dtype=torch.int32, device="cuda")
+            for i in range(N):
+                a = pkg.AttnArgs(qkv[i].data_ptr(), qg.data_ptr(), kg.data_ptr(), freq.data_ptr(), kc.data_ptr(), vc.data_ptr(), out[i].data_ptr(),
+                                 scratch.data_ptr(), tickets.data_ptr(), pos[i:].data_ptr(), n_q, n_kv, hd, N, 4, 1e-6, 0)
+                assert lib.b200_attn_decode(C.byref(a), None) == 0
+        torch.cuda.synchronize()
+        k, v = (t.double().repeat_interleave(n_q // n_kv, 0) for t in (kc, vc))
+        s = torch.einsum("ihd,hjd->hij", x, k) / hd ** 0.5
+        s = s.masked_fill(torch.ones(N, N, device="cuda").triu(1).bool(), -torch.inf)
+        errors.append(rel(out, torch.einsum("hij,hjd->ihd", torch.softmax(s, -1), v)))
+    assert errors[1] <= 1.5 * errors[0], errors
+
+
+@pytest.mark.parametrize("wtype", ["q8", "f16"])
+def test_chained_products(lib, pkg, synth, wtype):
+    """use_pdl: a product that starts while the kernel that makes its operand is still at it, over and over with other operands."""
+    wt, rows, cols, n = pkg.B200_WT_Q8 if wtype == "q8" else pkg.B200_WT_F16, 1024, 2560, 40
+    d_w, stride = pack(lib, pkg, weights(synth, rows, cols, 3), wt)
+    ws = torch.zeros(rows, device="cuda")
+    if wtype == "q8":
+        assert lib.b200_q8_row_scale(d_w.data_ptr(), stride, rows, cols, ws.data_ptr(), None) == 0
+    px, scale, args = planes_buffer(pkg, n, n, cols, 2)
+    x = torch.randn(12, n, cols, generator=torch.Generator().manual_seed(1)).cuda()
+
+    def run(pdl):
+        out = torch.zeros(12, n, rows, device="cuda")
+        torch.cuda.synchronize()
+        for i in range(12):
+            assert lib.b200_rows_split_planes(x[i].data_ptr(), n, cols, C.byref(args), None) == 0
+            a = pkg.RowsMatmulArgs(wt, d_w.data_ptr(), stride, rows, cols, ws.data_ptr(), px.data_ptr(), cols, 2, n, scale.data_ptr(), n,
+                                   out[i].data_ptr(), rows, None, rows, None, pdl)
+            assert lib.b200_rows_matmul(C.byref(a), None) == 0
+            if not pdl:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return out
+    assert torch.equal(run(1), run(0))
+
+
+def test_prompts_beyond_one_pass(lib, pkg, synth):
+    """2500 tokens: a second pass over 452, wanted rows in both and at their edges, in a workspace that a short prompt made first."""
+    sp = pkg.spec("tiny-qwen3", n_layers=2, gamma_jitter=0.1)
+    model = synth.llmb200_synth_qwen3(C.byref(sp), 4)
+    s = lib.inference_state_create(model, 4096, 1)
+    assert s
+    V = sp.vocab_size
+    toks = np.random.default_rng(9).integers(0, V, 2500).astype(np.uint32)
+    want = [0, 1000, 2047, 2048, 2300, 2499]
+    one = []
+    for i, t in enumerate(toks):
+        lg = np.ctypeslib.as_array(lib.inference_forward_token(s, int(t)), (V,))
+        if i in want:
+            one.append(lg.copy())
+    one = np.stack(one)
+
+    def passes(n, want):
+        lg = np.zeros((len(want), V), dtype=np.float32)
+        lib.inference_state_reset(s)
+        assert lib.inference_forward_tokens(s, toks.ctypes.data_as(pkg.c_u32_p), n, (C.c_int * len(want))(*want), len(want),
+                                            lg.ctypes.data_as(pkg.c_float_p)) == 0
+        return lg
+    first = passes(40, [0])
+    lg = passes(2500, want)
+    assert np.abs(lg - one).max() <= 1e-3 * np.abs(one).max()
+    assert np.abs(first[0] - one[0]).max() <= 1e-3 * np.abs(one).max()
+    assert np.abs(passes(2500, [2499])[0] - one[-1]).max() <= 1e-3 * np.abs(one).max()
+    many = passes(2500, list(range(1990, 2120)))               # more wanted rows than the head takes at once, in both passes
+    assert np.abs(many[2047 - 1990] - one[2]).max() <= 1e-3 * np.abs(one).max() and np.abs(many[2048 - 1990] - one[3]).max() <= 1e-3 * np.abs(one).max()
+    lib.inference_state_free(s)
+    synth.llmb200_synth_free_qwen3(model)
