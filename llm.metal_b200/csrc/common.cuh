@@ -51,6 +51,16 @@ __device__ __forceinline__ void st_release_sys(unsigned *p, unsigned v) {
     asm volatile("st.release.sys.global.u32 [%0], %1;" :: "l"(p), "r"(v) : "memory");
 }
 
+// ---- pairs of fp32 values in one instruction ------------------------------
+__device__ __forceinline__ void add_pair(float &a, float &b, float x, float y) {
+    asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tadd.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}"
+        : "+f"(a), "+f"(b) : "f"(x), "f"(y));
+}
+__device__ __forceinline__ void mul_pair(float &a, float &b, float x, float y) {
+    asm("{\n\t.reg .b64 p, q;\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\tmul.rn.f32x2 p, p, q;\n\tmov.b64 {%0, %1}, p;\n\t}"
+        : "+f"(a), "+f"(b) : "f"(x), "f"(y));
+}
+
 // ---- reductions --------------------------------------------------------
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

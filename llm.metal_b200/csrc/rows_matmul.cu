@@ -16,8 +16,8 @@
 // 2.6e-7 of a result at 512 .. 9728 columns, where the per-token kernels' fp32 sums are 0.8e-7 .. 1.2e-7 off and up to three accumulators of
 // 256 additions each, without drains, were 0.3e-6 .. 5e-6. Every second step would be 3e-7 .. 4e-7. One plane: a single chain, 1e-6 .. 1e-5 beside
 // the 2e-4 of its rounded operand.
-// Measured, two planes, drained every step and before (three accumulators): Q8_0 19456 x 2560, 48 / 512 / 1531 rows 54 / 213 / 533 us and
-// 51 / 224 / 569; F16 43 / 142 / 325 and 38 / 122 / 291: bound by operand staging (48 KB a step of a 128-column tile at 52 bytes a clock) and the
+// Measured, two planes, drained every step and before (three accumulators): Q8_0 19456 x 2560, 48 / 512 / 1531 rows 53 / 209 / 518 us and
+// 51 / 224 / 569; F16 42 / 133 / 302 and 38 / 122 / 291: bound by operand staging (48 KB a step of a 128-column tile at 52 bytes a clock) and the
 // wait of two blocks on an SM with two accumulators each for their drains.
 //
 // Block: warp 0 fills the ring with TMA (activation planes; F16 weight tiles), one lane of warp 1 issues tcgen05.mma, the last four
@@ -311,7 +311,7 @@ rows_matmul_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     if constexpr (LOAD == 32) tmem_ld32(at + c, u);
                     else tmem_ld16(at + c, u);
 #pragma unroll
-                    for (int j = 0; j < LOAD; ++j) sum[c + j] += __uint_as_float(u[j]);
+                    for (int j = 0; j < LOAD; j += 2) add_pair(sum[c + j], sum[c + j + 1], __uint_as_float(u[j]), __uint_as_float(u[j + 1]));
                 }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
