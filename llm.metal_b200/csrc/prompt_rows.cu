@@ -2,8 +2,8 @@
 //
 // The matrix products between them are b200_rows_matmul; here is what feeds it. Every kernel that makes a product's operand
 // writes it as one or two binary16 planes of the row times a power of two (2^14 <= largest element < 2^15), so that two planes
-// carry 22 bits of each element whatever the row's size; the factor that takes the power of two out again goes beside
-// it. One plane without a factor is the plain rounding that the batched engine's products take.
+// carry 22 bits of each element down to 2^-16 of the row's largest, and 2^-39 of the largest below; the factor that takes the power
+// of two out again goes beside it. One plane without a factor is the plain rounding that the batched engine's products take.
 // All of them move each row once: bound by HBM / L2 bytes, a block per row so that a short prompt still spreads over SMs. In short
 // prompts and in decode steps of a batch they and the products are bound by their launches instead, 2 to 4 us each: every kernel lets
 // the next one in at once and waits for the one before it after its set-up, so that a product's weights are on
@@ -287,10 +287,14 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ bool not_finite8(uint4 v)          // whether one of eight binary16 values is an infinity or NaN
+// z takes zero times eight binary16 values: it is NaN from the first infinity or NaN among them on.
+__device__ __forceinline__ void zero_times8(__half2 &z, uint4 v)
 {
-    const auto top = [](uint32_t w) { return (w & 0x7c007c00u) + 0x04000400u; };
-    return (top(v.x) | top(v.y) | top(v.z) | top(v.w)) & 0x80008000u;
+    const __half2 zero = __floats2half2_rn(0.0f, 0.0f);
+    z = __hfma2(*reinterpret_cast<const __half2 *>(&v.x), zero, z);
+    z = __hfma2(*reinterpret_cast<const __half2 *>(&v.y), zero, z);
+    z = __hfma2(*reinterpret_cast<const __half2 *>(&v.z), zero, z);
+    z = __hfma2(*reinterpret_cast<const __half2 *>(&v.w), zero, z);
 }
 __device__ __forceinline__ float ex2(float x)                // 2^x, 2 ulp, 0 for -inf
 {
@@ -298,6 +302,35 @@ __device__ __forceinline__ float ex2(float x)                // 2^x, 2 ulp, 0 fo
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
+// A tile's scores and weighted sums in plain multiply-adds, laid out over the lanes as the tensor cores' fragments are; arrays through
+// memory and out of line, so that the tiles that never need them keep their registers.
+template <int HD, int BKEY>
+__device__ __noinline__ void plain_scores(const __half *q, int plane, const __half *k, float *s)      // q: this lane's first row; the other 8 below
+{
+    constexpr int KS = HD + 8;
+    for (int e = 0; e < BKEY / 2; ++e) {
+        const __half *x = q + (e >> 1 & 1) * 8 * KS, *y = k + (e / 4 * 8 + (threadIdx.x & 3) * 2 + (e & 1)) * KS;
+        float t = 0.0f;
+        for (int d = 0; d < HD; ++d) t = fmaf(__half2float(x[d]) + __half2float(x[plane + d]), __half2float(y[d]), t);
+        s[e] = t;
+    }
+}
+template <int DV, int BKEY>
+__device__ __noinline__ void plain_sums(const __half *v, int last, const float *w, float *o)           // last: the last key that the first row sees
+{
+    constexpr int VS = DV + 8;
+    const int lane = threadIdx.x & 31;
+    for (int key = 0; key < BKEY; ++key) {
+        const int e = key / 8 * 4 + (key & 1), from = (lane & ~3) | (key % 8 / 2);
+        const float p0 = __shfl_sync(0xffffffffu, w[e], from), p1 = __shfl_sync(0xffffffffu, w[e + 2], from);
+        for (int i = 0; i < DV / 8; ++i) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(v + key * VS + i * 8 + (lane & 3) * 2));
+            if (key <= last) { o[4 * i] = fmaf(p0, f.x, o[4 * i]); o[4 * i + 1] = fmaf(p0, f.y, o[4 * i + 1]); }
+            if (key <= last + 8) { o[4 * i + 2] = fmaf(p1, f.x, o[4 * i + 2]); o[4 * i + 3] = fmaf(p1, f.y, o[4 * i + 3]); }
+        }
+    }
+}
+
 // Causal attention of the new rows over the binary16 cache at fp32 accuracy: online softmax on mma.sync tiles, 16 query rows a
 // warp, 32 keys a step with the next step's copies in flight. Keys and values are binary16 as they lie; queries and weights are
 // fp32 numbers as two binary16 planes, one product each, so a step costs twice the products of a 16-bit attention and loses
@@ -306,9 +339,10 @@ __device__ __forceinline__ float ex2(float x)                // 2^x, 2 ulp, 0 fo
 // over the keys that a row sees: a later key's weight of zero would not keep them out, nor a second plane of zero. mma.sync and not tcgen05: the products are a small share of a prompt
 // (prompts of 1500 tokens: a tenth of the time of the matrix products), and the split of the weights stays in registers.
 template <int HD, int NW>
-__global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn_args p)
+__global__ void __launch_bounds__(NW * 32, HD == 256 ? 1 : HD == 128 && NW == 4 ? 3 : 16 / NW) rows_attn_kernel(const b200_rows_attn_args p)
 {
     constexpr int DV = HD < 128 ? HD : 128, KS = HD + 8, VS = DV + 8, BQ = NW * 16, NT = NW * 32, BKEY = 32;
+    static_assert(BKEY * (HD / 8) % NT == 0 && BKEY * (DV / 8) % NT == 0, "every thread copies as many chunks");
     extern __shared__ __align__(16) unsigned char smem[];
     __half *qsm = reinterpret_cast<__half *>(smem);          // [2 planes][BQ][KS]
     __half *ksm = qsm + 2 * BQ * KS;                         // [2][BKEY][KS]
@@ -361,12 +395,14 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
         if (tile + 1 < tiles) { stage(tile + 1, slot ^ 1); cp_wait<1>(); }
         else cp_wait<0>();
         // every thread looks through what it copied itself: the barrier that follows tells all of them
-        bool odd = false;
-        for (int e = tid; e < BKEY * (HD / 8); e += NT)
-            odd |= not_finite8(lds_128(smem_u32(ksm + (slot * BKEY + e / (HD / 8)) * KS + e % (HD / 8) * 8)));
-        for (int e = tid; e < BKEY * (DV / 8); e += NT)
-            odd |= not_finite8(lds_128(smem_u32(vsm + (slot * BKEY + e / (DV / 8)) * VS + e % (DV / 8) * 8)));
-        const bool plainly = __syncthreads_or(odd);
+        __half2 z = __floats2half2_rn(0.0f, 0.0f);
+#pragma unroll
+        for (int e = 0; e < BKEY * (HD / 8); e += NT)
+            zero_times8(z, lds_128(smem_u32(ksm + (slot * BKEY + (tid + e) / (HD / 8)) * KS + (tid + e) % (HD / 8) * 8)));
+#pragma unroll
+        for (int e = 0; e < BKEY * (DV / 8); e += NT)
+            zero_times8(z, lds_128(smem_u32(vsm + (slot * BKEY + (tid + e) / (DV / 8)) * VS + (tid + e) % (DV / 8) * 8)));
+        const bool plainly = __syncthreads_or(!__hbeq2(z, z));
         const int k0 = tile * BKEY, w_first = first + warp * 16;
         if (k0 <= w_first + 15) {                            // else all of it is ahead of the warp's rows
             float s[BKEY / 8][4];
@@ -375,16 +411,10 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
 #pragma unroll
                 for (int k = 0; k < 4; ++k) s[i][k] = 0.0f;
             if (plainly) {
-                for (int d = 0; d < HD; ++d) {
-                    float f[2];
+                float t[BKEY / 8 * 4];
+                plain_scores<HD, BKEY>(qsm + r0 * KS, BQ * KS, ksm + slot * BKEY * KS, t);
 #pragma unroll
-                    for (int r = 0; r < 2; ++r) f[r] = __half2float(qsm[(r0 + 8 * r) * KS + d]) + __half2float(qsm[(BQ + r0 + 8 * r) * KS + d]);
-#pragma unroll
-                    for (int n = 0; n < BKEY / 8; ++n)
-#pragma unroll
-                        for (int k = 0; k < 4; ++k)
-                            s[n][k] = fmaf(f[k >> 1], __half2float(ksm[(slot * BKEY + n * 8 + (lane & 3) * 2 + (k & 1)) * KS + d]), s[n][k]);
-                }
+                for (int i = 0; i < BKEY / 2; ++i) s[i / 4][i % 4] = t[i];
             } else {
                 const uint32_t kaddr = smem_u32(ksm + slot * BKEY * KS + ((lane & 7) + ((lane >> 4) << 3)) * KS + ((lane >> 3) & 1) * 8);
                 float low[BKEY / 8][4] = {};
@@ -409,12 +439,12 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
 #pragma unroll
                     for (int n = 0; n < BKEY / 8; ++n)
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) s[n][k] += t[n][k];
+                        for (int k = 0; k < 4; k += 2) add_pair(s[n][k], s[n][k + 1], t[n][k], t[n][k + 1]);
                 }
 #pragma unroll
                 for (int n = 0; n < BKEY / 8; ++n)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) s[n][k] += low[n][k];
+                    for (int k = 0; k < 4; k += 2) add_pair(s[n][k], s[n][k + 1], low[n][k], low[n][k + 1]);
             }
             if (k0 + BKEY - 1 > w_first) {
                 const int d0 = first + r0 - k0 - (lane & 3) * 2;
@@ -452,26 +482,17 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
             l[1] = fmaf(l[1], corr[1], ls[1]);
             if (__any_sync(0xffffffffu, moved)) {
 #pragma unroll
-                for (int i = 0; i < DV / 8; ++i) { o[i][0] *= corr[0]; o[i][1] *= corr[0]; o[i][2] *= corr[1]; o[i][3] *= corr[1]; }
+                for (int i = 0; i < DV / 8; ++i) { mul_pair(o[i][0], o[i][1], corr[0], corr[0]); mul_pair(o[i][2], o[i][3], corr[1], corr[1]); }
             }
             if (plainly) {
-                const int d0 = first + r0 - k0;              // the last key that row r0 sees, from the tile's first
+                float w[BKEY / 8 * 4], t[DV / 8 * 4];
 #pragma unroll
-                for (int n = 0; n < BKEY / 8; ++n)
+                for (int i = 0; i < BKEY / 2; ++i) w[i] = s[i / 4][i % 4];
 #pragma unroll
-                    for (int j = 0; j < 2; ++j)
-                        for (int from = 0; from < 4; ++from) {
-                            const int key = n * 8 + from * 2 + j;
-                            const float p0 = __shfl_sync(0xffffffffu, s[n][j], (lane & ~3) | from);
-                            const float p1 = __shfl_sync(0xffffffffu, s[n][2 + j], (lane & ~3) | from);
-                            const __half *v = vsm + (slot * BKEY + key) * VS + (lane & 3) * 2;
+                for (int i = 0; i < DV / 2; ++i) t[i] = o[i / 4][i % 4];
+                plain_sums<DV, BKEY>(vsm + slot * BKEY * VS, first + r0 - k0, w, t);
 #pragma unroll
-                            for (int i = 0; i < DV / 8; ++i) {
-                                const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(v + i * 8));
-                                if (key <= d0) { o[i][0] = fmaf(p0, f.x, o[i][0]); o[i][1] = fmaf(p0, f.y, o[i][1]); }
-                                if (key <= d0 + 8) { o[i][2] = fmaf(p1, f.x, o[i][2]); o[i][3] = fmaf(p1, f.y, o[i][3]); }
-                            }
-                        }
+                for (int i = 0; i < DV / 2; ++i) o[i / 4][i % 4] = t[i];
             } else {
                 const uint32_t vaddr = smem_u32(vsm + slot * BKEY * VS + (lane & 15) * VS + (lane >> 4) * 8);
                 uint32_t a[BKEY / 16][4], a2[BKEY / 16][4];
@@ -495,7 +516,7 @@ __global__ void __launch_bounds__(NW * 32) rows_attn_kernel(const b200_rows_attn
 #pragma unroll
                     for (int kk = 0; kk < BKEY / 16; ++kk) { mma_f16(t[0], a[kk], b[kk][0], b[kk][1]); mma_f16(t[1], a[kk], b[kk][2], b[kk][3]); }
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) { o[2 * n][k] += t[0][k]; o[2 * n + 1][k] += t[1][k]; }
+                    for (int k = 0; k < 4; k += 2) { add_pair(o[2 * n][k], o[2 * n][k + 1], t[0][k], t[0][k + 1]); add_pair(o[2 * n + 1][k], o[2 * n + 1][k + 1], t[1][k], t[1][k + 1]); }
                 }
             }
         }
