@@ -369,8 +369,10 @@ static int gemm_tc(const b200_gemm_args *a, int f16, void *stream)
     if (a->N < 64) return B200_E_UNSUPPORTED;                     // the CUDA-core kernel is the better fit
     if ((a->N + 63) / 64 > 65535) return B200_E_UNSUPPORTED;
 
+    // the experiments' variables are about this kernel: with one of them set, every product comes here
+    static const bool experiment = getenv("LLMB200_GEMM_BN") || getenv("LLMB200_GEMM_KSUB") || getenv("LLMB200_GEMM_SPLIT_NKB");
     PairShape pair;
-    if (f16 && gemm_pair_shape(a->M, a->N, a->K, !a->Ch, &pair)) return gemm_pair_launch(a, f16 - 1, pair, (cudaStream_t)stream);
+    if (f16 && !experiment && gemm_pair_shape(a->M, a->N, a->K, !a->Ch, &pair)) return gemm_pair_launch(a, f16 - 1, pair, (cudaStream_t)stream);
     CUtensorMap ma, mb;
     EpiArgs e = {a->C, a->ldc, a->R, a->ldr, a->M, a->N, a->K, a->alpha, a->d_err, 128, 0, 0, f16, 1, 1, nullptr,
                  static_cast<__nv_bfloat16 *>(a->Ch), a->ldch, a->relu2};
