@@ -1,5 +1,5 @@
 // The large products of 16-bit operands on pairs of SMs (sm_100a): C[M,N] = alpha * A[M,K] * B[N,K]^T (+ R), as gemm_tf32.cu
-// defines it, for more than 128 rows. b200_gemm_f16 / _bf16 come here when a product is large enough.
+// defines it, for more than 128 rows. b200_gemm_f16 / _bf16 come here when that is modelled faster.
 //
 // What bounds these products is operand staging: an SM takes in about 58 bytes a clock, and a 128 x 176 tile by itself wants 110
 // to keep its tensor core busy. Here two SMs work on a 256 x bn tile (tcgen05 cta_group::2): each loads its own 128 rows of A and
@@ -276,12 +276,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // at 58 a clock, whichever is more; the last epilogue is not hidden (some 20 clocks a column), and sums of splits go
 // through shared memory. The width is a multiple of 16 up to 256. CLUSTERS: how many clusters of 2, 4, 6, 8 blocks are resident
 // on 148 SMs (the occupancy calculator's figures).
-bool gemm_pair_shape(int M, int N, int K, bool may_split, PairShape *out)
+// What comes back is held against the form of one SM per tile: clocks of the shape taken, fitted to 200 products (M 129 .. 2048, N 256 .. 19456,
+// K 256 .. 16384, chains of 20 launches), 8 % rms.
+double gemm_pair_shape(int M, int N, int K, bool may_split, PairShape *out)
 {
-    if (M <= SM_ROWS || N < 256) return false;
+    if (M <= SM_ROWS || N < 256) return 1e30;
     const int pairs = tc_sm_count() / 2, mt = (M + 2 * SM_ROWS - 1) / (2 * SM_ROWS), nkb = (K + KB - 1) / KB;
     constexpr int CLUSTERS[5] = {0, 74, 33, 22, 15};
-    double least = 1e30;
+    double least = 1e30, clocks = 1e30;
     for (int bn = 64; bn <= 256; bn += 16) {
         const long long tiles = (long long)mt * ((N + bn - 1) / bn);
         double step = 2.0 * bn;
@@ -290,11 +292,14 @@ bool gemm_pair_shape(int M, int N, int K, bool may_split, PairShape *out)
             if (s > 1 && (!may_split || nkb / s < 8)) break;
             const long long place = (long long)CLUSTERS[s] * pairs / 74, waves = (tiles + place - 1) / place;
             if (s > 1 && waves > 1) break;
-            const double cost = waves * ((nkb + s - 1) / s) * step + 1500.0 + bn * 20.0 + (s > 1 ? 1500.0 + bn * 15.0 : 0.0);
-            if (cost < least) { least = cost; out->bn = bn; out->splits = s; }
+            const double steps = waves * ((nkb + s - 1) / s) * step, cost = steps + 1500.0 + bn * 20.0 + (s > 1 ? 1500.0 + bn * 15.0 : 0.0);
+            if (cost < least) {
+                least = cost; out->bn = bn; out->splits = s;
+                clocks = 1.32 * steps + 3450.0 * waves + 3250.0 + bn * 74.0 + (s > 1 ? 3450.0 + bn * 43.0 : 0.0);
+            }
         }
     }
-    return true;
+    return clocks;
 }
 
 int gemm_pair_launch(const b200_gemm_args *a, int fmt, const PairShape &sh, cudaStream_t st)

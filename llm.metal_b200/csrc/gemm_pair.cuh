@@ -5,7 +5,7 @@
 #include <cuda_runtime.h>
 
 struct PairShape { int bn, splits; };
-// Whether a product is one for pairs, and how.
-bool gemm_pair_shape(int M, int N, int K, bool may_split, PairShape *out);
+// How pairs would take a product, and the modelled clocks (1e30: not at all, 128 rows or fewer, or fewer than 256 columns).
+double gemm_pair_shape(int M, int N, int K, bool may_split, PairShape *out);
 // Operands checked by the caller; fmt 0: binary16, 1: bfloat16.
 int gemm_pair_launch(const b200_gemm_args *a, int fmt, const PairShape &sh, cudaStream_t st);

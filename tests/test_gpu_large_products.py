@@ -49,3 +49,24 @@ def test_pair_products(lib, pkg, dtype, M, N, K):
             w = want.clamp(min=0).square() if relu2 else want
             bar = 2 ** -8 * w.abs() + (2 * want.abs() if relu2 else 1) * 1e-5 * size + 1e-6      # one bfloat16 rounding
             assert ((h.double() - w).abs() <= bar).all() and int(err) == 0
+
+
+# as pairs: one wave of tiles, split in three, less than a step; as tiles of one SM: a ragged end, several widths, many rows
+@pytest.mark.parametrize("M,N,K", [(512, 19456, 2560), (300, 768, 3000), (130, 264, 136), (257, 300, 1000), (384, 3072, 512), (384, 4096, 512),
+                                    (2048, 1024, 256)])
+def test_products_on_either_side_of_the_cost_model(lib, pkg, M, N, K):
+    """Two forms share these products by modelled time; both are held against float64 on shapes that the model gives them."""
+    g = torch.Generator().manual_seed(M + N)
+    A, B, R = torch.randn(M, K, generator=g).half().cuda(), torch.randn(N, K, generator=g).half().cuda(), torch.randn(M, N, generator=g).cuda()
+    err, outs = torch.zeros(1, dtype=torch.int32, device="cuda"), []
+    for _ in range(2):
+        c = R.clone()
+        a = pkg.GemmArgs()
+        a.A, a.a_row, a.a_col, a.B, a.b_row, a.b_col = A.data_ptr(), K, 1, B.data_ptr(), 1, K
+        a.C, a.ldc, a.R, a.ldr, a.M, a.N, a.K, a.alpha, a.d_err = c.data_ptr(), N, c.data_ptr(), N, M, N, K, 0.5, err.data_ptr()      # in place
+        assert lib.b200_gemm_f16(C.byref(a), None) == 0
+        torch.cuda.synchronize()
+        outs.append(c)
+    size = A.double().abs() @ B.double().abs().T
+    assert int(err) == 0 and torch.equal(outs[0], outs[1])
+    assert ((outs[0].double() - (0.5 * (A.double() @ B.double().T) + R.double())).abs() <= 1e-5 * size + 1e-6).all()
