@@ -14,7 +14,8 @@
 // transposing stores are spread over the banks by xor-ing k into the low bits of the position.
 // A training step has 64 rows, so a product is few tiles with a long k (64 x 1152 x 6912: 18): up to eight blocks of a cluster
 // share a tile along k, and each adds up an eighth of it from the others' shared memory, in rank order.
-// Two full-parameter steps of 64 tokens (two layers of 1152 x 6912, vocabulary 8192): 14.9 ms with one block a tile and no prefetch, 4.1 ms.
+// Two full-parameter steps of 64 tokens (two layers of 1152 x 6912, vocabulary 8192): 14.9 ms with one block a tile and no prefetch, 4.1 ms with
+// this kernel (3.5 with the tiled attention since).
 // Bound by the latency of a step's operands where an SM has one block (64 x 1152 x 13824: 93 us), by the fp32 pipes elsewhere.
 #include "common.cuh"
 #include "../../include/llmb200_train_kernels.h"

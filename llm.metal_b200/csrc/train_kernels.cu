@@ -180,15 +180,15 @@ __global__ void qk_norm_rope_bwd_kernel(float *dqkv, const float *qkv, long long
 }
 
 // ---- causal attention, training form ---------------------------------------------------------------
-// One block per (sequence, head, 64 queries), or 64 keys, walking the tiles it can see; fp32 values throughout, with the products on
-// the tensor cores: an fp32 operand is a TF32 number plus what that leaves (x = hi + lo, 22 bits), a product is hi hi + hi lo + lo hi
-// with fp32 sums (mma.sync m16n8k8: the fragments of both operands are read from plain row-major tiles, in any orientation, with
-// the split on the way; 16-bit planes would need every row's range). Scores and probabilities go to the matrices that are
-// kept anyway and are read back by the thread that wrote them. The next tile's copies run under the current one's products. The
-// longest rows start first.
-// A layer forward and backward, 32 heads, 509 positions of 128: 500 us; the same tiles as register-tiled fp32 products on the CUDA cores
-// 649 us, one warp per query or key 2.1 ms. Bound by instructions (the split of every operand element) and by the
-// single-word accesses to the score matrix.
+// One block per (sequence, head, 64 queries), or 64 keys, walking the tiles it can see; fp32 values throughout. The products have two forms with
+// the same layout over the lanes: fp32 multiply-adds on the CUDA cores, and the tensor cores (mma.sync m16n8k8), where an fp32
+// operand is a TF32 number plus what that leaves (x = hi + lo, 22 bits) and a product is hi hi + hi lo + lo hi. The fragments of both
+// operands are read from plain row-major tiles, in any orientation, with the split on the way; 16-bit planes would need every
+// row's range. Scores and probabilities go to the matrices that are kept anyway and are read back by the thread that wrote them.
+// The next tile's copies run under the current one's products. The longest rows start first.
+// A layer forward and backward, 32 heads, 509 positions of 128: 515 us on the tensor cores, 718 us on the CUDA cores, one warp per query
+// or key 2.2 ms. Bound by instructions (the split of every operand element; shared-memory reads of the fp32 form) and by the single-word
+// accesses to the score matrix. Off float64 2e-7 .. 4e-7 as fp32 and no more on the tensor cores.
 constexpr int AT = 64;                       // tile edge: queries and keys
 constexpr int ATT_THREADS = 256;
 
