@@ -98,7 +98,7 @@ extern "C" int b200_matvec(const b200_matvec_args *ap, void *stream)
     // Up to two slices per thread: keeps a group at <= 320 threads for rows of up to 640 slices, so that
     // two blocks (this kernel's and the next one's) fit on an SM; 960 consumers + the producer warp at most.
     // Measured on the 2560 x 9728 down projection: two slices per thread 12.3 us, one slice 16.3 us.
-    const int spt = nsl <= 320 ? 1 : a.wtype == B200_WT_F32 && nsl > 1920 ? 4 : 2;
+    const int spt = nsl <= 320 ? 1 : a.wtype == B200_WT_F32 && nsl > 960 ? 4 : 2;
     if ((nsl + spt - 1) / spt > 960) return B200_E_TOOLARGE;
     Geometry geo;
     geo.T = (((nsl + spt - 1) / spt) + 31) / 32 * 32;
@@ -116,17 +116,20 @@ extern "C" int b200_matvec(const b200_matvec_args *ap, void *stream)
     // Ring slots: a multiple of the group count, so that a slot is always consumed by the same group.
     // A group works through its stages in order, hence never waits on a slot whose previous phase is
     // still open -- mbarrier parity waits cannot tell phase k from phase k-2.
-    const int ring_budget = knobs().ring_kb * 1024;
+    geo.xs = a.in_mode != B200_IN_VEC || a.d_norm_gamma ? (a.cols + 3) / 4 * 4 : 0;
+    geo.win = 0; geo.part = 0;                       // by the number of rows, in launch()
+    int ring_budget = knobs().ring_kb * 1024;
+    const int room = 224 * 1024 - (int)beside_ring(geo.xs, 2 * 2048);
+    if (ring_budget > room) ring_budget = room;
     while (geo.NG > 1 && (long long)geo.NG * geo.slot_bytes > ring_budget) --geo.NG;
     int per_group = ring_budget / (int)(geo.NG * geo.slot_bytes);
     if (per_group < 1) per_group = 1;
     while (per_group > 1 && per_group * geo.NG > 12) --per_group;
     geo.nstage = per_group * geo.NG;
-    geo.share_x = geo.NG > 1 && (a.in_mode != B200_IN_VEC || a.d_norm_gamma) && (size_t)spt * geo.T * E * 4 <= 16384;
-
     int grid = a.grid;
     if (grid <= 0) grid = sm_count();                // one block per SM
     if (grid > units) grid = units;
+    geo.base = units / grid; geo.rem = units % grid;
     cudaStream_t st = (cudaStream_t)stream;
     if (a.wtype == B200_WT_Q8)
         return spt == 1 ? launch_by_rows<B200_WT_Q8, 1>(a, geo, rb, grid, st) : launch_by_rows<B200_WT_Q8, 2>(a, geo, rb, grid, st);

@@ -7,9 +7,14 @@
 // and the ring keeps ~100 KB per block in flight without holding registers.
 // Consumer threads own fixed 16-byte column slices (16 int8 quants or 8
 // halves) of every row, so their slice of the input vector stays in registers
-// for the whole kernel; consumer groups take stages round-robin, finish the RB
-// rows of a stage with one transposing shuffle reduction per warp plus a
-// fixed-order sum over the group's warps (reproducible run to run).
+// for the whole kernel; consumer groups take stages round-robin. Warps run free of each other: a warp folds the RB rows of a stage across
+// its lanes with one transposing shuffle reduction and leaves its sums in shared memory; one barrier per window of some 2000 sums (all
+// rows of a block but for an LM head), then a thread per row adds the warps' sums in fixed order (reproducible run to run) and
+// stores the result.
+// Bound by instructions and their latencies with 4 to 5 warps on a scheduler, not by HBM: the input vector is assembled by all consumers, a barrier
+// per sum, and nothing divides. A barrier and a one-warp epilogue per stage, 64-bit divisions, norms by one group: 0.28 ms a token of 41 such
+// launches (2048 wide, bfloat16), 0.25 now; fp32 210 us and 182. Two blocks of half the ring on an SM, so that the next launch's
+// weights arrive early: no gain (0.28), blocks of one launch then share SMs.
 //
 // Launched with programmatic dependent launch, a block of the NEXT kernel in
 // the stream starts as soon as an SM has room for it (with the default 192 KB
@@ -38,71 +43,117 @@ struct Geometry {
     int NG;             // consumer groups
     int nstage;         // ring slots
     unsigned slot_bytes;  // bytes per slot (RB rows, rounded up to 128)
-    int share_x;        // 1: group 0 assembles the input vector and hands it to the other groups through shared memory
+    int base, rem;      // row units of a block, and the blocks that have one more
+    int per_warp;       // 65536 / (warps of a group), rounded up: which group a warp belongs to without a division
+    int win, part;      // stages per window of rows (a multiple of NG), floats of its warp sums; two windows take turns
+    int xs;             // floats of the input vector in shared memory; 0: it is read as it is
 };
 
-// blockDim.x = NG*T consumers + 32 producer threads.
-// RMS norm of the vector a group of T threads holds, `groups` equal consecutive parts of its first `dim` elements
-// each by its own mean square. In place; one part after the other, so the sums are in a fixed order.
-template <int SPT, int E>
-__device__ __forceinline__ void norm_parts(float (&x)[SPT][E], const int (&col)[SPT], const float (&gamma)[SPT][E], int dim,
-                                           int groups, float eps, float *gred, int bar_id, int T, int t)
+// Sums of K values over the nC consumer threads; every thread gets them. One barrier: calls take the halves of `red` (2 x 4 x 32 floats,
+// zeros where there is no warp) in turn, and between a call and the next but one lies the barrier of the one between.
+template <int K>
+__device__ __forceinline__ void block_sums(float (&v)[K], float *red, int &turn, int nC, int tid)
 {
-    const int len = dim / groups;
-    for (int k = 0; k < groups; ++k) {
-        const int lo = k * len, hi = lo + len;
-        float ss = 0.0f;
+    float *r = red + 128 * turn;
+    turn ^= 1;
 #pragma unroll
-        for (int s = 0; s < SPT; ++s)
+    for (int k = 0; k < K; ++k) {
+        v[k] = warp_sum(v[k]);
+        if ((tid & 31) == 0) r[k * 32 + (tid >> 5)] = v[k];
+    }
+    named_barrier(1, nC);
 #pragma unroll
-            for (int e = 0; e < E; ++e)
-                if (col[s] + e >= lo && col[s] + e < hi) ss = fmaf(x[s][e], x[s][e], ss);
-        ss = group_sum(ss, gred, bar_id, T, t);
-        const float inv = 1.0f / sqrtf(ss / (float)len + eps);
-#pragma unroll
-        for (int s = 0; s < SPT; ++s)
-#pragma unroll
-            for (int e = 0; e < E; ++e)
-                if (col[s] + e >= lo && col[s] + e < hi) x[s][e] = gamma[s][e] * (x[s][e] * inv);
+    for (int k = 0; k < K; ++k) {
+        float tot = 0.0f;
+        for (int i = 0; i < nC >> 5; i += 4) {
+            const float4 q = *reinterpret_cast<const float4 *>(r + k * 32 + i);
+            tot += q.x; tot += q.y; tot += q.z; tot += q.w;
+        }
+        v[k] = tot;
     }
 }
 
-// Layer norm (mean taken off, variance of the deviations, weight and bias) of the first `dim` elements, in place; the
-// columns past them hold zeros before and after (their weight and bias are zero).
-template <int SPT, int E>
-__device__ __forceinline__ void layer_norm(float (&x)[SPT][E], const int (&col)[SPT], const float (&gamma)[SPT][E],
-                                           const float (&beta)[SPT][E], int dim, float eps, float *gred, int bar_id, int T, int t)
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<float4 *>(p) = v; }
+__device__ __forceinline__ float squares(float4 v, float s) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, s)))); }
+
+// Weights of a norm for this thread's items (four elements each, nC items apart): those of the first one are fetched before the wait for the
+// previous kernel, they are constants.
+struct NormWeights {
+    const float *at;
+    float4 first;
+    __device__ __forceinline__ void fetch(const float *p, int tid, int cols)
+    {
+        at = p;
+        first = p && 4 * tid < cols ? ld4(p + 4 * tid) : make_float4(0, 0, 0, 0);
+    }
+    __device__ __forceinline__ float4 get(int it, int e) const { return it == 0 ? first : ld4(at + e); }
+};
+
+// A thread's items of the vector in shared memory.
+#define B200_ITEMS(it, e) for (int it = 0, e = 4 * tid; e < cols; ++it, e += 4 * nC)
+
+// RMS norm of the vector, `groups` equal consecutive parts of its first `dim` elements each by its own mean square; what follows them stays.
+__device__ __forceinline__ void norm_parts(float *xs, const NormWeights &gamma, int cols, int dim, int groups, float eps, float *red, int &turn,
+                                           int nC, int tid)
 {
-    float sum = 0.0f;
+    const int len = dim / groups;
+    for (int k0 = 0; k0 < groups; k0 += 4) {                             // four parts a barrier
+        float ss[4] = {};
+        B200_ITEMS(it, e) {
+            const float4 q = ld4(xs + e);
+            const float f[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int s = 0; s < SPT; ++s)
+            for (int k = 0; k < 4; ++k) {
+                const int lo = (k0 + k) * len, hi = k0 + k < groups ? lo + len : lo;
 #pragma unroll
-        for (int e = 0; e < E; ++e) sum += x[s][e];
-    const float mean = group_sum(sum, gred, bar_id, T, t) / (float)dim;
-    float ss = 0.0f;
+                for (int j = 0; j < 4; ++j)
+                    if (e + j >= lo && e + j < hi) ss[k] = fmaf(f[j], f[j], ss[k]);
+            }
+        }
+        block_sums<4>(ss, red, turn, nC, tid);
 #pragma unroll
-    for (int s = 0; s < SPT; ++s)
+        for (int k = 0; k < 4; ++k) ss[k] = 1.0f / sqrtf(ss[k] / (float)len + eps);
+        B200_ITEMS(it, e) {
+            const float4 q = ld4(xs + e), g = gamma.get(it, e);
+            float f[4] = {q.x, q.y, q.z, q.w};
+            const float w[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
-        for (int e = 0; e < E; ++e)
-            if (col[s] + e < dim) { x[s][e] -= mean; ss = fmaf(x[s][e], x[s][e], ss); }
-    ss = group_sum(ss, gred, bar_id, T, t);
-    const float inv = 1.0f / sqrtf(ss / (float)dim + eps);
+            for (int k = 0; k < 4; ++k) {
+                const int lo = (k0 + k) * len, hi = k0 + k < groups ? lo + len : lo;
 #pragma unroll
-    for (int s = 0; s < SPT; ++s)
-#pragma unroll
-        for (int e = 0; e < E; ++e) x[s][e] = fmaf(gamma[s][e], x[s][e] * inv, beta[s][e]);
+                for (int j = 0; j < 4; ++j)
+                    if (e + j >= lo && e + j < hi) f[j] = w[j] * (f[j] * ss[k]);
+            }
+            st4(xs + e, make_float4(f[0], f[1], f[2], f[3]));
+        }
+    }
 }
 
-template <int SPT, int E>
-__device__ __forceinline__ void load_slices(float (&v)[SPT][E], const float *src, const int (&col)[SPT], const bool (&on)[SPT])
+// Layer norm (mean taken off, variance of the deviations, weight and bias) of the first `dim` elements; the
+// columns past them hold zeros before and after (their weight and bias are zero).
+__device__ __forceinline__ void layer_norm(float *xs, const NormWeights &gamma, const NormWeights &beta, int cols, int dim, float eps, float *red,
+                                           int &turn, int nC, int tid)
 {
-#pragma unroll
-    for (int s = 0; s < SPT; ++s)
-#pragma unroll
-        for (int e = 0; e < E; e += 4) {
-            const float4 v4 = on[s] ? *reinterpret_cast<const float4 *>(src + col[s] + e) : make_float4(0, 0, 0, 0);
-            v[s][e] = v4.x; v[s][e + 1] = v4.y; v[s][e + 2] = v4.z; v[s][e + 3] = v4.w;
-        }
+    float sum[1] = {0.0f}, ss[1] = {0.0f};
+    B200_ITEMS(it, e) { const float4 q = ld4(xs + e); sum[0] += (q.x + q.y) + (q.z + q.w); }
+    block_sums<1>(sum, red, turn, nC, tid);
+    const float mean = sum[0] / (float)dim;
+    B200_ITEMS(it, e) {
+        float4 q = ld4(xs + e);
+        if (e < dim) q.x -= mean;
+        if (e + 1 < dim) q.y -= mean;
+        if (e + 2 < dim) q.z -= mean;
+        if (e + 3 < dim) q.w -= mean;
+        st4(xs + e, q);
+        ss[0] = squares(q, ss[0]);
+    }
+    block_sums<1>(ss, red, turn, nC, tid);
+    const float inv = 1.0f / sqrtf(ss[0] / (float)dim + eps);
+    B200_ITEMS(it, e) {
+        const float4 q = ld4(xs + e), g = gamma.get(it, e), b = beta.get(it, e);
+        st4(xs + e, make_float4(fmaf(g.x, q.x * inv, b.x), fmaf(g.y, q.y * inv, b.y), fmaf(g.z, q.z * inv, b.z), fmaf(g.w, q.w * inv, b.w)));
+    }
 }
 
 // Which of the optional parts an instantiation holds (registers decide how well the row loop runs): FAM_PLAIN the parts
@@ -117,27 +168,26 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
     constexpr int E = (WT == B200_WT_Q8) ? 16 : (WT == B200_WT_F32) ? 4 : 8;       // elements per 16-byte slice
     constexpr bool EXT = FAM == FAM_POST, STR = FAM == FAM_STREAMS;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int T = geo.T, NG = geo.NG, nstage = geo.nstage, nwg = T >> 5, nC = NG * T;
+    const int T = geo.T, NG = geo.NG, nstage = geo.nstage, nwg = T >> 5, nwgp = nwg | 1, nC = NG * T;
     unsigned char *ring = smem_raw;
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + (size_t)nstage * geo.slot_bytes);
     uint64_t *empty = full + nstage;
-    float *wpart = reinterpret_cast<float *>(empty + nstage);   // [NG][2][nwg][RB]
-    float *red = wpart + (size_t)NG * 2 * nwg * RB;             // [NG][32]
-    float *am_v = red + NG * 32;                                // [NG*RB]
-    int *am_i = reinterpret_cast<int *>(am_v + NG * RB);        // [NG*RB]
-    float *xs = reinterpret_cast<float *>(am_i + NG * RB);      // [SPT*T*E] when geo.share_x
+    float *red = reinterpret_cast<float *>(ring + (size_t)nstage * geo.slot_bytes + 256);   // [2][4][32]
+    float *am_v = red + 256;                                    // [32], a value per warp
+    int *am_i = reinterpret_cast<int *>(am_v + 32);             // [32]
+    float *xs = reinterpret_cast<float *>(am_i + 32);           // [geo.xs], the assembled input
+    float *wpart = xs + geo.xs;                                 // one or two windows of [rows][nwgp] warp sums
     __shared__ int s_last;
     __shared__ float s_conn[STR ? B200_MAX_STREAMS * (B200_MAX_STREAMS + 2) : 1];     // mix, out, next read of the streams
 
     const int tid = threadIdx.x;
+    for (int i = tid; i < 256; i += blockDim.x) red[i] = 0.0f;
     const int ralign = (p.out_mode == B200_OUT_GLU) ? 2 : 1;
-    const long long units = p.rows / ralign;
-    const int r0 = (int)(units * blockIdx.x / gridDim.x) * ralign;
-    const int r1 = (int)(units * (blockIdx.x + 1) / gridDim.x) * ralign;
+    const int bid = blockIdx.x, r0 = (bid * geo.base + min(bid, geo.rem)) * ralign, r1 = r0 + (geo.base + (bid < geo.rem)) * ralign;
     const int nst = (r1 - r0 + RB - 1) / RB;
 
-    if (tid == 0) {
-        for (int i = 0; i < nstage; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], T); }
+    if (tid < nstage) {
+        mbar_init(&full[tid], 1); mbar_init(&empty[tid], nwg);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -178,47 +228,19 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
     }
 
     // ---------------- consumers ----------------
-    const int g = tid / T, t = tid - g * T, lane = t & 31, wg = t >> 5;
-    float *gred = red + g * 32;
-    int col[SPT];
-    bool on[SPT];
-#pragma unroll
-    for (int s = 0; s < SPT; ++s) { col[s] = (s * T + t) * E; on[s] = col[s] < p.cols; }
+    const int g = ((tid >> 5) * geo.per_warp) >> 16, t = tid - g * T, lane = t & 31, wg = t >> 5, cols = p.cols;
+    const bool assemble = geo.xs > 0;            // otherwise the input is a vector that each thread reads its slices of
+    int turn = 0;                                // which half of red the next sum takes
 
     // The norm weights are constants: their round trip is taken before the wait for the previous
     // kernel, not after it.
-    float gm[SPT][E];
-    const bool pre_gamma = p.d_norm_gamma && (!geo.share_x || g == 0);
-    if (pre_gamma) {
-#pragma unroll
-        for (int s = 0; s < SPT; ++s)
-#pragma unroll
-            for (int e = 0; e < E; e += 4) {
-                float4 v4 = on[s] ? *reinterpret_cast<const float4 *>(p.d_norm_gamma + col[s] + e) : make_float4(0, 0, 0, 0);
-                gm[s][e] = v4.x; gm[s][e + 1] = v4.y; gm[s][e + 2] = v4.z; gm[s][e + 3] = v4.w;
-            }
-    }
-
-    float gp[EXT ? SPT : 1][E];                  // the same for the norm of a post-norm input
-    if constexpr (EXT) {
-        if (p.in_mode == B200_IN_POSTNORM && (!geo.share_x || g == 0)) {
-#pragma unroll
-            for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                for (int e = 0; e < E; e += 4) {
-                    const float4 v4 = on[s] ? *reinterpret_cast<const float4 *>(p.d_slot_norm_gamma + col[s] + e) : make_float4(0, 0, 0, 0);
-                    gp[s][e] = v4.x; gp[s][e + 1] = v4.y; gp[s][e + 2] = v4.z; gp[s][e + 3] = v4.w;
-                }
-        }
-    }
-
-    float gb[STR ? SPT : 1][E];                  // bias of a layer norm
+    NormWeights gm, gp, gb;
+    gm.fetch(p.d_norm_gamma, tid, cols);
+    gp.fetch(p.d_slot_norm_gamma, tid, cols);                        // of a post-norm input, of normalised slot sums, or of embeddings
     if constexpr (STR) {
-        if (pre_gamma && p.d_norm_beta) load_slices<SPT, E>(gb, p.d_norm_beta, col, on);
-        if (p.out_mode == B200_OUT_STREAMS && wg == 0) {         // the epilogue warp of every group, same values
-            for (int i = lane; i < p.n_streams * (p.n_streams + 2); i += 32) s_conn[i] = p.d_connect[i];
-            __syncwarp();
-        }
+        gb.fetch(p.d_norm_beta, tid, cols);
+        if (p.out_mode == B200_OUT_STREAMS)                      // read after the barrier that ends the first window
+            for (int i = tid; i < p.n_streams * (p.n_streams + 2); i += nC) s_conn[i] = p.d_connect[i];
     }
 
     pdl_wait();
@@ -235,290 +257,221 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
     }
 
     // ---------------- input assembly ----------------
-    // Every SM needs the whole input vector. When it has to be assembled (slot sums, norms), one group
-    // per block does it and passes it on through shared memory: the few KB involved are read by all
-    // SMs at once, and every extra reader of the same L2 lines queues behind the others.
-    float x[SPT][E];
-    if (!geo.share_x || g == 0) {
-    if (p.in_mode == B200_IN_VEC || (EXT && p.in_mode == B200_IN_POSTNORM)) {
-#pragma unroll
-        for (int s = 0; s < SPT; ++s)
-#pragma unroll
-            for (int e = 0; e < E; e += 4) {
-                float4 v4 = on[s] ? *reinterpret_cast<const float4 *>(p.d_in_vec + col[s] + e) : make_float4(0, 0, 0, 0);
-                x[s][e] = v4.x; x[s][e + 1] = v4.y; x[s][e + 2] = v4.z; x[s][e + 3] = v4.w;
-            }
-        if constexpr (EXT) {
-            if (p.in_mode == B200_IN_POSTNORM) {
-                float mix[SPT][E];                       // fetched before the norm's reductions
-#pragma unroll
-                for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                    for (int e = 0; e < E; e += 4) {
-                        const float4 v4 = on[s] && p.d_mix_in ? *reinterpret_cast<const float4 *>(p.d_mix_in + col[s] + e) : make_float4(0, 0, 0, 0);
-                        mix[s][e] = v4.x; mix[s][e + 1] = v4.y; mix[s][e + 2] = v4.z; mix[s][e + 3] = v4.w;
-                    }
-                const float coef = p.d_mix_in ? *p.d_mix_coef : 1.0f;
-                norm_parts<SPT, E>(x, col, gp, p.norm_dim > 0 ? p.norm_dim : p.cols, p.norm_groups > 1 ? p.norm_groups : 1, p.eps,
-                                   gred, 2 + g, T, t);
-                const bool store = blockIdx.x == 0 && g == 0;
-#pragma unroll
-                for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                    for (int e = 0; e < E; e += 4) {
-                        if (store && on[s] && p.d_post_copy)
-                            *reinterpret_cast<float4 *>(p.d_post_copy + col[s] + e) = make_float4(x[s][e], x[s][e + 1], x[s][e + 2], x[s][e + 3]);
+    // Every SM needs the whole input vector. Where it has to be assembled (slot sums, norms) all consumers of a block do it together, four
+    // elements a thread, in shared memory: one read of the vector a block (all SMs read the same few KB of L2 at once, and every
+    // extra reader queues behind the others), a barrier per sum.
+    if (assemble) {
+        const bool store = blockIdx.x == 0;
+        if (p.in_mode == B200_IN_VEC || (EXT && p.in_mode == B200_IN_POSTNORM)) {
+            B200_ITEMS(it, e) st4(xs + e, ld4(p.d_in_vec + e));
+            if constexpr (EXT) {
+                if (p.in_mode == B200_IN_POSTNORM) {
+                    float4 mix0 = make_float4(0, 0, 0, 0);               // fetched before the norm's sums
+                    if (p.d_mix_in && 4 * tid < cols) mix0 = ld4(p.d_mix_in + 4 * tid);
+                    const float coef = p.d_mix_in ? *p.d_mix_coef : 1.0f;
+                    norm_parts(xs, gp, cols, p.norm_dim > 0 ? p.norm_dim : cols, p.norm_groups > 1 ? p.norm_groups : 1, p.eps, red, turn, nC, tid);
+                    B200_ITEMS(it, e) {
+                        float4 q = ld4(xs + e);
+                        if (store && p.d_post_copy) st4(p.d_post_copy + e, q);
                         if (p.d_mix_in) {
-#pragma unroll
-                            for (int k = 0; k < 4; ++k) x[s][e + k] = fmaf(coef, x[s][e + k], mix[s][e + k]);
+                            const float4 m = it == 0 ? mix0 : ld4(p.d_mix_in + e);
+                            q = make_float4(fmaf(coef, q.x, m.x), fmaf(coef, q.y, m.y), fmaf(coef, q.z, m.z), fmaf(coef, q.w, m.w));
+                            st4(xs + e, q);
                         }
-                        if (store && on[s] && p.d_resid_out)
-                            *reinterpret_cast<float4 *>(p.d_resid_out + col[s] + e) = make_float4(x[s][e], x[s][e + 1], x[s][e + 2], x[s][e + 3]);
+                        if (store && p.d_resid_out) st4(p.d_resid_out + e, q);
                     }
-            }
-        }
-    } else {
-        if (p.in_mode == B200_IN_EMBED) {
-            long long tok = p.d_tokens[*p.d_pos];
-            if (tok < 0 || tok >= p.emb_rows) tok = 0;      // never index outside the table
-            const float *er = p.d_emb + tok * (long long)p.cols;
-#pragma unroll
-            for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                for (int e = 0; e < E; e += 4) {
-                    float4 v4 = on[s] ? *reinterpret_cast<const float4 *>(er + col[s] + e) : make_float4(0, 0, 0, 0);
-                    x[s][e] = v4.x * p.emb_scale; x[s][e + 1] = v4.y * p.emb_scale;
-                    x[s][e + 2] = v4.z * p.emb_scale; x[s][e + 3] = v4.w * p.emb_scale;
-                }
-            if constexpr (STR) {
-                if (p.d_emb_pos) {
-                    float row[SPT][E];
-                    load_slices<SPT, E>(row, p.d_emb_pos + (long long)min(*p.d_pos, p.emb_pos_rows - 1) * p.cols, col, on);
-#pragma unroll
-                    for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                        for (int e = 0; e < E; ++e) x[s][e] += row[s][e];
-                }
-                if (p.d_slot_norm_beta) {
-                    float w[SPT][E], b[SPT][E];
-                    load_slices<SPT, E>(w, p.d_slot_norm_gamma, col, on);
-                    load_slices<SPT, E>(b, p.d_slot_norm_beta, col, on);
-                    layer_norm<SPT, E>(x, col, w, b, p.norm_dim > 0 ? p.norm_dim : p.cols, p.eps, gred, 2 + g, T, t);
                 }
             }
         } else {
-            float sacc[SPT][E];
-#pragma unroll
-            for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                for (int e = 0; e < E; ++e) sacc[s][e] = 0.0f;
-            for (int k = 0; k < p.n_slots; ++k) {
-                const float *sl = p.d_slots + (long long)k * p.slot_stride;
-#pragma unroll
-                for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                    for (int e = 0; e < E; e += 4) {
-                        if (on[s]) {
-                            // slots may be written by other GPUs: read them from L2, the point of coherence, never from L1
-                            float4 v4 = __ldcg(reinterpret_cast<const float4 *>(sl + col[s] + e));
-                            sacc[s][e] += v4.x; sacc[s][e + 1] += v4.y; sacc[s][e + 2] += v4.z; sacc[s][e + 3] += v4.w;
-                        }
+            if (p.in_mode == B200_IN_EMBED) {
+                long long tok = p.d_tokens[*p.d_pos];
+                if (tok < 0 || tok >= p.emb_rows) tok = 0;      // never index outside the table
+                const float *er = p.d_emb + tok * (long long)cols;
+                const float *row = STR && p.d_emb_pos ? p.d_emb_pos + (long long)min(*p.d_pos, p.emb_pos_rows - 1) * cols : nullptr;
+                B200_ITEMS(it, e) {
+                    float4 q = ld4(er + e);
+                    q.x *= p.emb_scale; q.y *= p.emb_scale; q.z *= p.emb_scale; q.w *= p.emb_scale;
+                    if (row) { const float4 r = ld4(row + e); q.x += r.x; q.y += r.y; q.z += r.z; q.w += r.w; }
+                    st4(xs + e, q);
+                }
+                if constexpr (STR) {
+                    if (p.d_slot_norm_beta) {
+                        NormWeights b;
+                        b.fetch(p.d_slot_norm_beta, tid, cols);
+                        layer_norm(xs, gp, b, cols, p.norm_dim > 0 ? p.norm_dim : cols, p.eps, red, turn, nC, tid);
                     }
-            }
-            if (p.d_slot_norm_gamma) {
-                float ss = 0.0f;
-#pragma unroll
-                for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                    for (int e = 0; e < E; ++e) ss = fmaf(sacc[s][e], sacc[s][e], ss);
-                ss = group_sum(ss, gred, 2 + g, T, t);
-                const float inv = 1.0f / sqrtf(ss / (float)p.cols + p.eps);
-#pragma unroll
-                for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                    for (int e = 0; e < E; ++e)
-                        if (on[s]) sacc[s][e] = p.d_slot_norm_gamma[col[s] + e] * sacc[s][e] * inv;
-            }
-#pragma unroll
-            for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                for (int e = 0; e < E; e += 4) {
-                    float4 v4 = on[s] ? *reinterpret_cast<const float4 *>(p.d_resid_in + col[s] + e) : make_float4(0, 0, 0, 0);
-                    x[s][e] = v4.x + sacc[s][e]; x[s][e + 1] = v4.y + sacc[s][e + 1];
-                    x[s][e + 2] = v4.z + sacc[s][e + 2]; x[s][e + 3] = v4.w + sacc[s][e + 3];
                 }
-        }
-        if (blockIdx.x == 0 && g == 0 && p.d_resid_out) {
-#pragma unroll
-            for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                for (int e = 0; e < E; e += 4)
-                    if (on[s])
-                        *reinterpret_cast<float4 *>(p.d_resid_out + col[s] + e) =
-                            make_float4(x[s][e], x[s][e + 1], x[s][e + 2], x[s][e + 3]);
-        }
-        if constexpr (STR) {
-            if (p.in_mode == B200_IN_EMBED && p.d_mix_coef) {    // what the first reader takes of the streams, all equal here
-                const float c = *p.d_mix_coef;
-#pragma unroll
-                for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                    for (int e = 0; e < E; ++e) x[s][e] *= c;
+            } else {
+                float ss[1] = {0.0f};
+                B200_ITEMS(it, e) {
+                    float4 a = make_float4(0, 0, 0, 0);
+                    for (int k = 0; k < p.n_slots; ++k) {
+                        // slots may be written by other GPUs: read them from L2, the point of coherence, never from L1
+                        const float4 q = __ldcg(reinterpret_cast<const float4 *>(p.d_slots + (long long)k * p.slot_stride + e));
+                        a.x += q.x; a.y += q.y; a.z += q.z; a.w += q.w;
+                    }
+                    if (p.d_slot_norm_gamma) ss[0] = squares(a, ss[0]);
+                    else { const float4 r = ld4(p.d_resid_in + e); a.x += r.x; a.y += r.y; a.z += r.z; a.w += r.w; }
+                    st4(xs + e, a);
+                }
+                if (p.d_slot_norm_gamma) {
+                    block_sums<1>(ss, red, turn, nC, tid);
+                    const float inv = 1.0f / sqrtf(ss[0] / (float)cols + p.eps);
+                    B200_ITEMS(it, e) {
+                        const float4 a = ld4(xs + e), w = gp.get(it, e), r = ld4(p.d_resid_in + e);
+                        st4(xs + e, make_float4(r.x + w.x * a.x * inv, r.y + w.y * a.y * inv, r.z + w.z * a.z * inv, r.w + w.w * a.w * inv));
+                    }
+                }
+            }
+            if (store && p.d_resid_out) B200_ITEMS(it, e) st4(p.d_resid_out + e, ld4(xs + e));
+            if constexpr (STR) {
+                if (p.in_mode == B200_IN_EMBED && p.d_mix_coef) {    // what the first reader takes of the streams, all equal here
+                    const float c = *p.d_mix_coef;
+                    B200_ITEMS(it, e) { const float4 q = ld4(xs + e); st4(xs + e, make_float4(c * q.x, c * q.y, c * q.z, c * q.w)); }
+                }
             }
         }
-    }
-    if ((EXT || STR) && p.d_norm_gamma) {
-        if constexpr (STR) layer_norm<SPT, E>(x, col, gm, gb, p.norm_dim > 0 ? p.norm_dim : p.cols, p.eps, gred, 2 + g, T, t);
-        if constexpr (EXT)
-            norm_parts<SPT, E>(x, col, gm, p.norm_dim > 0 ? p.norm_dim : p.cols, p.norm_groups > 1 ? p.norm_groups : 1, p.eps, gred, 2 + g, T, t);
-    } else if (p.d_norm_gamma) {
-        float ss = 0.0f;
-#pragma unroll
-        for (int s = 0; s < SPT; ++s)
-#pragma unroll
-            for (int e = 0; e < E; ++e) ss = fmaf(x[s][e], x[s][e], ss);
-        ss = group_sum(ss, gred, 2 + g, T, t);
-        const float inv = 1.0f / sqrtf(ss / (float)p.cols + p.eps);
-#pragma unroll
-        for (int s = 0; s < SPT; ++s)
-#pragma unroll
-            for (int e = 0; e < E; ++e) x[s][e] = gm[s][e] * x[s][e] * inv;
-    }
-    }
-    if (p.d_in_copy && blockIdx.x == 0 && g == 0) {
-#pragma unroll
-        for (int s = 0; s < SPT; ++s)
-#pragma unroll
-            for (int e = 0; e < E; e += 4)
-                if (on[s])
-                    *reinterpret_cast<float4 *>(p.d_in_copy + col[s] + e) = make_float4(x[s][e], x[s][e + 1], x[s][e + 2], x[s][e + 3]);
-    }
-    if (geo.share_x) {
-        if (g == 0) {
-#pragma unroll
-            for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                for (int e = 0; e < E; e += 4)
-                    *reinterpret_cast<float4 *>(xs + (size_t)(s * T + t) * E + e) = make_float4(x[s][e], x[s][e + 1], x[s][e + 2], x[s][e + 3]);
+        if (p.d_norm_gamma) {
+            if constexpr (STR) layer_norm(xs, gm, gb, cols, p.norm_dim > 0 ? p.norm_dim : cols, p.eps, red, turn, nC, tid);
+            else if constexpr (EXT)
+                norm_parts(xs, gm, cols, p.norm_dim > 0 ? p.norm_dim : cols, p.norm_groups > 1 ? p.norm_groups : 1, p.eps, red, turn, nC, tid);
+            else {
+                float ss[1] = {0.0f};
+                B200_ITEMS(it, e) ss[0] = squares(ld4(xs + e), ss[0]);
+                block_sums<1>(ss, red, turn, nC, tid);
+                const float inv = 1.0f / sqrtf(ss[0] / (float)cols + p.eps);
+                B200_ITEMS(it, e) {
+                    const float4 q = ld4(xs + e), w = gm.get(it, e);
+                    st4(xs + e, make_float4(w.x * q.x * inv, w.y * q.y * inv, w.z * q.z * inv, w.w * q.w * inv));
+                }
+            }
         }
+        if (p.d_in_copy && store) B200_ITEMS(it, e) st4(p.d_in_copy + e, ld4(xs + e));
         named_barrier(1, nC);
-        if (g != 0) {
-#pragma unroll
-            for (int s = 0; s < SPT; ++s)
-#pragma unroll
-                for (int e = 0; e < E; e += 4) {
-                    const float4 v4 = *reinterpret_cast<const float4 *>(xs + (size_t)(s * T + t) * E + e);
-                    x[s][e] = v4.x; x[s][e + 1] = v4.y; x[s][e + 2] = v4.z; x[s][e + 3] = v4.w;
-                }
-        }
     }
-
-    // ---------------- consume the ring: group g takes stages g, g+NG, ... ----------------
-    float best_v = -INFINITY;
-    int best_i = 0x7fffffff;
+    float x[SPT][E];
     // Byte offsets of this thread's slices inside a row. Threads past the end of the row read slice 0
     // (valid memory) against a zero input slice and drop the result.
     uint32_t qoff[SPT], soff[SPT];
 #pragma unroll
     for (int s = 0; s < SPT; ++s) {
-        const int c = on[s] ? col[s] : 0;
+        const int col = (s * T + t) * E;
+        const bool on = col < cols;
+#pragma unroll
+        for (int e = 0; e < E; e += 4) {
+            const float4 q = !on ? make_float4(0, 0, 0, 0) : ld4((assemble ? xs : p.d_in_vec) + col + e);
+            x[s][e] = q.x; x[s][e + 1] = q.y; x[s][e + 2] = q.z; x[s][e + 3] = q.w;
+        }
+        const int c = on ? col : 0;
         qoff[s] = (uint32_t)(WT == B200_WT_Q8 ? c : WT == B200_WT_F32 ? 4 * c : 2 * c);
-        soff[s] = (uint32_t)p.cols + (uint32_t)(c >> 5) * 2u;   // Q8: scales follow the quants of a row
+        soff[s] = (uint32_t)cols + (uint32_t)(c >> 5) * 2u;      // Q8: scales follow the quants of a row
     }
-    const uint32_t ring_s = smem_u32(ring), stride = (uint32_t)p.row_stride;
-    for (int i = g, it = 0; i < nst; i += NG, ++it) {
-        const int slot = i % nstage;
-        const int row0 = r0 + i * RB;
-        const int nr = min(RB, r1 - row0);
-        float o_resid = 0.0f, o_gate = 0.0f;            // what the gated output adds to and scales by
-        if constexpr (EXT) {
-            if (p.out_mode == B200_OUT_GATED && wg == 0 && lane < nr) {
-                o_resid = p.d_out_resid[row0 + lane];
-                o_gate = p.d_out_gate[row0 + lane] + p.d_out_gate_bias[row0 + lane];
-            }
-        }
-        // Streams: lane = row + RB * j holds streams j, j + 32/RB, ... of its row.
-        constexpr int LPR = 32 / RB, XS = (B200_MAX_STREAMS + LPR - 1) / LPR;
-        float old[STR ? XS : 1];
-        if constexpr (STR) {
-            if (p.out_mode == B200_OUT_STREAMS && wg == 0) {
-#pragma unroll
-                for (int k = 0; k < XS; ++k) {
-                    const int s = lane / RB + k * LPR, r = lane % RB;
-                    old[k] = s < p.n_streams && r < nr ? p.d_streams_in[s * p.streams_in_stride + row0 + r] : 0.0f;
-                }
-            }
-        }
-        if (!mbar_wait(&full[slot], (i / nstage) & 1) && p.d_err) *p.d_err = 3;
-        const uint32_t sb = ring_s + (uint32_t)slot * geo.slot_bytes;
-        // Rows past nr hold stale bytes; they are computed like the others (no predicates in the
-        // hot loop), stay in their own reduction lane and are never emitted.
-        uint4 wq[RB][SPT];
-        uint32_t ws[RB][SPT];
-#pragma unroll
-        for (int j = 0; j < RB; ++j)
-#pragma unroll
-            for (int s = 0; s < SPT; ++s) {
-                wq[j][s] = lds_128(sb + (uint32_t)j * stride + qoff[s]);
-                if (WT == B200_WT_Q8) ws[j][s] = lds_u16(sb + (uint32_t)j * stride + soff[s]);
-            }
-        float v[RB];
-#pragma unroll
-        for (int j = 0; j < RB; ++j) {
-            float acc = 0.0f;
-#pragma unroll
-            for (int s = 0; s < SPT; ++s) {
-                float d;
-                if (WT == B200_WT_Q8) d = __half2float(__ushort_as_half((unsigned short)ws[j][s])) * dot16_q8(wq[j][s], x[s]);
-                else if (WT == B200_WT_BF16) d = dot8_bf16(wq[j][s], x[s]);
-                else if (WT == B200_WT_F32) d = dot4_f32(wq[j][s], x[s]);
-                else d = dot8_f16(wq[j][s], x[s]);
-                acc += d;                      // threads past the end of the row hold a zero input slice
-            }
-            v[j] = acc;
-        }
-        mbar_arrive(&empty[slot]);             // this thread no longer reads the slot
+    if (p.d_in_copy && !assemble && blockIdx.x == 0) B200_ITEMS(it, e) st4(p.d_in_copy + e, ld4(p.d_in_vec + e));
 
-        const float tot = reduce_rows<RB>(v, lane);
-        float *wp = wpart + (size_t)((g * 2 + (it & 1)) * nwg) * RB;
-        if (lane < RB) wp[wg * RB + lane] = tot;
-        named_barrier(2 + g, T);
-        if (wg == 0) {
-            float y = 0.0f;
-            if (lane < RB)
-                for (int w = 0; w < nwg; ++w) y += wp[w * RB + lane];
-            const int row = row0 + lane;
-            if (p.out_mode == B200_OUT_GLU) {
-                const float u = __shfl_down_sync(0xffffffffu, y, 1);
-                if (EXT && p.glu_rows > 0 && row >= p.glu_rows) {
-                    if (lane < nr) p.d_out2[row - p.glu_rows] = y;
-                } else if (lane < nr && !(lane & 1)) {
-                    const float a = p.act == 0 ? act_silu(y) : act_gelu_tanh(y);
-                    p.d_out[0][p.out_offset + (row >> 1)] = a * u;
+    // ---------------- consume the ring: group g takes stages g, g+NG, ... ----------------
+    float best_v = -INFINITY;
+    int best_i = 0x7fffffff;
+    const uint32_t ring_s = smem_u32(ring), stride = (uint32_t)p.row_stride;
+    int slot = g;
+    unsigned phase = 0;
+    for (int s0 = 0, buf = 0; s0 < nst; s0 += geo.win, buf ^= 1) {
+        const int s1 = min(s0 + geo.win, nst), w0 = r0 + s0 * RB, n = min(r1 - w0, (s1 - s0) * RB);
+        float *part = wpart + buf * geo.part;
+        // what a gated output adds to and scales by, or the streams of the row, for the row that this thread emits first: on their way
+        // while the rows are multiplied
+        float o_resid = 0.0f, o_gate = 0.0f, old[STR ? B200_MAX_STREAMS : 1];
+        if constexpr (EXT) {
+            if (p.out_mode == B200_OUT_GATED && tid < n) {
+                o_resid = p.d_out_resid[w0 + tid];
+                o_gate = p.d_out_gate[w0 + tid] + p.d_out_gate_bias[w0 + tid];
+            }
+        }
+        if constexpr (STR) {
+            if (p.out_mode == B200_OUT_STREAMS) {
+#pragma unroll
+                for (int k = 0; k < B200_MAX_STREAMS; ++k)
+                    old[k] = k < p.n_streams && tid < n ? p.d_streams_in[k * p.streams_in_stride + w0 + tid] : 0.0f;
+            }
+        }
+        for (int i = s0 + g; i < s1; i += NG) {
+            if (!mbar_wait(&full[slot], phase) && p.d_err) *p.d_err = 3;
+            const uint32_t sb = ring_s + (uint32_t)slot * geo.slot_bytes;
+            // Rows past the end hold stale bytes; they are computed like the others (no predicates in the
+            // hot loop), stay in their own reduction lane and are never emitted.
+            uint4 wq[RB][SPT];
+            uint32_t ws[RB][SPT];
+#pragma unroll
+            for (int j = 0; j < RB; ++j)
+#pragma unroll
+                for (int s = 0; s < SPT; ++s) {
+                    wq[j][s] = lds_128(sb + (uint32_t)j * stride + qoff[s]);
+                    if (WT == B200_WT_Q8) ws[j][s] = lds_u16(sb + (uint32_t)j * stride + soff[s]);
                 }
-            } else if (EXT && p.out_mode == B200_OUT_GATED) {
-                if (lane < nr) p.d_out[0][p.out_offset + row] = fmaf(p.resid_alpha, o_resid, sigmoid_f32(o_gate) * y);
+            float v[RB];
+#pragma unroll
+            for (int j = 0; j < RB; ++j) {
+                float acc = 0.0f;
+#pragma unroll
+                for (int s = 0; s < SPT; ++s) {
+                    float d;
+                    if (WT == B200_WT_Q8) d = __half2float(__ushort_as_half((unsigned short)ws[j][s])) * dot16_q8(wq[j][s], x[s]);
+                    else if (WT == B200_WT_BF16) d = dot8_bf16(wq[j][s], x[s]);
+                    else if (WT == B200_WT_F32) d = dot4_f32(wq[j][s], x[s]);
+                    else d = dot8_f16(wq[j][s], x[s]);
+                    acc += d;                      // threads past the end of the row hold a zero input slice
+                }
+                v[j] = acc;
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[slot]);              // this warp no longer reads the slot
+            slot += NG;
+            if (slot >= nstage) { slot -= nstage; phase ^= 1; }
+            const float tot = reduce_rows<RB>(v, lane);
+            if (lane < RB) part[((i - s0) * RB + lane) * nwgp + wg] = tot;
+        }
+        named_barrier(1, nC);
+
+        // ---------------- a thread per row: the warps' sums in order, and the epilogue ----------------
+        // (the next window's sums go to the other buffer, and nobody comes back to this one before the next barrier)
+        auto row_sum = [&](int i) {
+            float y = 0.0f;
+            for (int w = 0; w < nwg; ++w) y += part[i * nwgp + w];
+            return y;
+        };
+        if (p.out_mode == B200_OUT_GLU) {
+            for (int i = 2 * tid; i < n; i += 2 * nC) {
+                const float y = row_sum(i), u = row_sum(i + 1);
+                const int row = w0 + i;
+                if (EXT && p.glu_rows > 0 && row >= p.glu_rows) { p.d_out2[row - p.glu_rows] = y; p.d_out2[row + 1 - p.glu_rows] = u; }
+                else p.d_out[0][p.out_offset + (row >> 1)] = (p.act == 0 ? act_silu(y) : act_gelu_tanh(y)) * u;
+            }
+            continue;
+        }
+        for (int i = tid; i < n; i += nC) {
+            float y = row_sum(i);
+            const int row = w0 + i;
+            if (EXT && p.out_mode == B200_OUT_GATED) {
+                if (i != tid) { o_resid = p.d_out_resid[row]; o_gate = p.d_out_gate[row] + p.d_out_gate_bias[row]; }
+                p.d_out[0][p.out_offset + row] = fmaf(p.resid_alpha, o_resid, sigmoid_f32(o_gate) * y);
             } else if (STR && p.out_mode == B200_OUT_STREAMS) {
                 if constexpr (STR) {
-                    const int n = p.n_streams, r = lane % RB;
-                    const float yr = __shfl_sync(0xffffffffu, y, r);
-                    float next = 0.0f;
-                    for (int to = 0; to < n; ++to) {
-                        float a = 0.0f;
+                    const int ns = p.n_streams;
+                    if (i != tid) {
 #pragma unroll
-                        for (int k = 0; k < XS; ++k) {
-                            const int s = lane / RB + k * LPR;
-                            if (s < n) a = fmaf(s_conn[s * n + to], old[k], a);
-                        }
-#pragma unroll
-                        for (int o = RB; o < 32; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-                        a = fmaf(s_conn[n * n + to], yr, a);
-                        if (r < nr && lane / RB == to % LPR) p.d_streams_out[to * p.streams_out_stride + row0 + r] = a;
-                        next = fmaf(s_conn[n * n + n + to], a, next);
+                        for (int k = 0; k < B200_MAX_STREAMS; ++k) old[k] = k < ns ? p.d_streams_in[k * p.streams_in_stride + row] : 0.0f;
                     }
-                    if (lane < nr) p.d_out[0][p.out_offset + row] = next;
+                    float next = 0.0f;
+                    for (int to = 0; to < ns; ++to) {
+                        float a = s_conn[ns * ns + to] * y;
+#pragma unroll
+                        for (int k = 0; k < B200_MAX_STREAMS; ++k)
+                            if (k < ns) a = fmaf(s_conn[k * ns + to], old[k], a);
+                        p.d_streams_out[to * p.streams_out_stride + row] = a;
+                        next = fmaf(s_conn[ns * ns + ns + to], a, next);
+                    }
+                    p.d_out[0][p.out_offset + row] = next;
                 }
-            } else if (lane < nr) {
+            } else {
                 if (EXT && p.softcap > 0.0f) y = p.softcap * tanhf(y / p.softcap);
                 if (STR && p.act == B200_ACT_RELU2) y = act_relu2(y);
                 for (int q = 0; q < p.n_out; ++q) p.d_out[q][p.out_offset + row] = y;
@@ -530,7 +483,15 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
     if (!p.d_ticket) return;
 
     // ---------------- last-block bookkeeping ----------------
-    if (p.d_argmax_scratch && wg == 0 && lane < RB) { am_v[g * RB + lane] = best_v; am_i[g * RB + lane] = best_i; }
+    if (p.d_argmax_scratch) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, best_v, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
+            if (better(ov, oi, best_v, best_i)) { best_v = ov; best_i = oi; }
+        }
+        if (lane == 0) { am_v[tid >> 5] = best_v; am_i[tid >> 5] = best_i; }
+    }
     // The barrier orders every thread's stores (peers' slots included) before thread 0; its system-wide
     // fence is cumulative, so one fence per block publishes them all before the ticket is taken.
     named_barrier(1, nC);
@@ -538,7 +499,7 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
         __threadfence_system();
         if (p.d_argmax_scratch) {
             float bv = am_v[0]; int bi = am_i[0];
-            for (int k = 1; k < NG * RB; ++k) if (better(am_v[k], am_i[k], bv, bi)) { bv = am_v[k]; bi = am_i[k]; }
+            for (int k = 1; k < nC / 32; ++k) if (better(am_v[k], am_i[k], bv, bi)) { bv = am_v[k]; bi = am_i[k]; }
             p.d_argmax_scratch[2 * blockIdx.x] = bv;
             reinterpret_cast<int *>(p.d_argmax_scratch)[2 * blockIdx.x + 1] = bi;
             __threadfence();
@@ -583,15 +544,23 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
     }
 }
 
+// Bytes of shared memory beside the ring: barriers, sums of norms, arg-max, the input vector, the warps' sums of `part` floats.
+inline size_t beside_ring(int xs, int part) { return 256 + (256 + 64 + (size_t)xs + part) * sizeof(float); }
+
 template <int WT, int SPT, int RB, int MAXT, int FAM>
-int launch(const b200_matvec_args &a, const Geometry &geo, int grid, cudaStream_t st)
+int launch(const b200_matvec_args &a, Geometry geo, int grid, cudaStream_t st)
 {
-    const int nwg = geo.T / 32;
-    const size_t smem = (size_t)geo.nstage * geo.slot_bytes + (size_t)geo.nstage * 16 +
-                        ((size_t)geo.NG * 2 * nwg * RB + (size_t)geo.NG * 32 + (size_t)geo.NG * RB * 2) * sizeof(float) +
-                        (geo.share_x ? (size_t)SPT * geo.T * (WT == B200_WT_Q8 ? 16 : WT == B200_WT_F32 ? 4 : 8) * sizeof(float) : 0);
+    const int ralign = a.out_mode == B200_OUT_GLU ? 2 : 1;
+    const int nst = ((geo.base + (geo.rem > 0)) * ralign + RB - 1) / RB;                  // of the block with the most rows
+    // windows of about 2048 warp sums
+    const int nwgp = (geo.T / 32) | 1, round = geo.NG * RB * nwgp;
+    geo.per_warp = (65536 + geo.T / 32 - 1) / (geo.T / 32);
+    geo.win = (2048 / round < 1 ? 1 : 2048 / round) * geo.NG;
+    if (geo.win > nst) geo.win = (nst + geo.NG - 1) / geo.NG * geo.NG;
+    geo.part = geo.win * RB * nwgp;
+    const size_t smem = (size_t)geo.nstage * geo.slot_bytes + beside_ring(geo.xs, geo.part * (nst > geo.win ? 2 : 1));
     auto kern = matvec_kernel<WT, SPT, RB, MAXT, FAM>;
-    if (smem > 220 * 1024) return B200_E_TOOLARGE;
+    if (smem > 224 * 1024) return B200_E_TOOLARGE;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;

@@ -144,19 +144,6 @@ __device__ __forceinline__ bool better(float v, int i, float bv, int bi)
     return v > bv || (v == bv && i < bi);
 }
 
-// Sum of v over the T threads of one consumer group; every thread gets it.
-__device__ __forceinline__ float group_sum(float v, float *red, int bar_id, int T, int t)
-{
-    const int lane = t & 31, w = t >> 5, nw = T >> 5;
-    v = warp_sum(v);
-    named_barrier(bar_id, T);              // protect `red` from a previous use
-    if (lane == 0) red[w] = v;
-    named_barrier(bar_id, T);
-    float tot = 0.0f;
-    for (int i = 0; i < nw; ++i) tot += red[i];
-    return tot;
-}
-
 // v[j] holds this lane's partial of row j. Returns, in every lane, the warp
 // total of row (lane & (RB-1)): RB-1 exchanges fold the rows across lane bits,
 // the remaining log2(32/RB) butterflies add the lane groups.
