@@ -823,7 +823,7 @@ static void loss_device(SFTState *s)
 /* Full-parameter mode: the weight gradient dW = dY^T X over the M token rows (dY [M, ldy], X [M, ldx]) goes
  * into rows 0..rows-1 of the matrix the way wmode says: W <- half(W - lr dW) (f16_sgd_fused,
  * shaders/q8_kernels.metal:1097-1125) or G <- half(G + dW) (f16_grad_accum, :1164-1191). One fp32 sum over
- * the tokens per element, in ascending order below 256 tokens and in up to eight stretches that join in a fixed order beyond (b200_gemm_f32),
+ * the tokens per element, in ascending order below 256 tokens and in stretches that join in a fixed order beyond (b200_gemm_f32),
  * and one rounding to binary16, as there. The matrices are fp32
  * holders of binary16 values in this mode, so the product adds into them in place and rounds. */
 static void weight_step(SFTState *s, SftMat *W, float *acc, int rows, const float *dY, long long ldy, const float *X,

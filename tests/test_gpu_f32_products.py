@@ -31,3 +31,31 @@ def test_f32_products(lib, pkg, ak, bk, M, N, K):
     assert ((outs[0].double() - (R.double() - 0.25 * want)).abs() <= 2 ** -20 * (size + R.double().abs())).all()
     assert torch.equal(outs[0], outs[1])                      # the splits add in a fixed order
     assert torch.equal(outs[2], outs[0].half().float())
+
+
+@pytest.mark.parametrize("ak", [0, 1])
+@pytest.mark.parametrize("bk", [0, 1])
+@pytest.mark.parametrize("M,N,K,pad", [(64, 1152, 769, 0), (33, 200, 257, 1), (64, 64, 1030, 3), (130, 70, 96, 1), (1, 700, 4100, 2)])
+def test_f32_products_off_boundaries(lib, pkg, ak, bk, M, N, K, pad):
+    """Operands, results and residuals that start `pad` floats behind a 16-byte boundary, in wider lines; every count of blocks per tile. Bar as above."""
+    g = torch.Generator().manual_seed(K + M)
+
+    def placed(t):
+        rows, cols = t.shape
+        whole = torch.full((rows * (cols + pad) + 4,), float("nan"), device="cuda")
+        view = whole[pad:pad + rows * (cols + pad)].view(rows, cols + pad)[:, :cols]
+        view.copy_(t)
+        return whole, view
+
+    A, B, R = (torch.randn(*s, generator=g).cuda() for s in ((M, K), (K, N), (M, N)))
+    (_a, am), (_b, bm), (_r, rm), (_c, cm) = placed(A if ak else A.T), placed(B.T if bk else B), placed(R), placed(torch.zeros_like(R))
+    a = pkg.GemmArgs()
+    a.A, a.a_row, a.a_col = am.data_ptr(), am.stride(0) if ak else 1, 1 if ak else am.stride(0)
+    a.B, a.b_row, a.b_col = bm.data_ptr(), 1 if bk else bm.stride(0), bm.stride(0) if bk else 1
+    a.C, a.ldc, a.R, a.ldr = cm.data_ptr(), cm.stride(0), rm.data_ptr(), rm.stride(0)
+    a.M, a.N, a.K, a.alpha = M, N, K, 1.0
+    assert lib.b200_gemm_f32(C.byref(a), None) == 0
+    torch.cuda.synchronize()
+    want, size = A.double() @ B.double() + R.double(), A.double().abs() @ B.double().abs() + R.double().abs()
+    assert ((cm.double() - want).abs() <= 2 ** -20 * size).all()
+    assert torch.isnan(_c).sum() == _c.numel() - M * N        # nothing outside the result is written
