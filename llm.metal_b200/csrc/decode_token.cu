@@ -121,7 +121,7 @@ struct Smem {
     unsigned char *ring;
     uint64_t *full, *empty, *att_bar;
     float *part, *red, *resid, *scratch;
-    volatile int *flags;                             // [0] abort, [1] always 0
+    volatile int *flags;                             // [0] abort, [1] always 0, [2] epoch, [3] position, [4] token id, [5] phase of att_bar before this token, [6] tokens left
     const b200_token_layer *layers;
 };
 
@@ -359,7 +359,7 @@ __device__ __forceinline__ float stage_residual(const b200_token_args &p, int ki
     float *gam = sm.scratch + D;
     float ss = 0.0f;
     if (kind == B200_ST_QKV && l == 0) {
-        long long tok = p.d_tokens[*p.d_pos];
+        long long tok = sm.flags[4];
         if (tok < 0 || tok >= p.emb_rows) tok = 0;   // never index outside the table
         const float *er = p.d_emb + tok * (long long)D;
 #pragma unroll 1
@@ -569,7 +569,7 @@ __device__ __forceinline__ float fused_residual_q8(const b200_token_args &p, int
     uint32_t *rec = reinterpret_cast<uint32_t *>(sm.scratch);
     const float *er = nullptr;
     if (from_emb) {
-        long long tok = p.d_tokens[*p.d_pos];
+        long long tok = sm.flags[4];
         if (tok < 0 || tok >= p.emb_rows) tok = 0;   // never index outside the table
         er = p.d_emb + tok * (long long)D;
     } else {
@@ -913,6 +913,7 @@ __device__ __forceinline__ unsigned run_matvec(const b200_token_args &p, int kin
 #pragma unroll 1
             for (int ww = 1; ww < TK_NWARP; ++ww) if (better(am_v[ww], am_i[ww], best_v, best_i)) { best_v = am_v[ww]; best_i = am_i[ww]; }
             if (p.n_ranks > 1) __threadfence_system();   // this block's logits are visible before its pair is
+            else if (p.n_tokens > 1) __threadfence();    // and so are its cache rows, which other blocks read for the launch's next token
             fl_store<false>(p.d_am + 2 * blockIdx.x, best_v, flag);
             fl_store<false>(p.d_am + 2 * blockIdx.x + 1, __int_as_float(best_i), flag);
         }
@@ -1090,7 +1091,7 @@ __device__ __forceinline__ void attention_stage(const b200_token_args &p, int l,
                 }
                 named_barrier(2, ATT_T);
             }
-            if (!mbar_wait_abort(sm.att_bar, (unsigned)(l * nsub + sub) & 1u, sm.flags, spin) && !sm.flags[0]) raise(sm.flags, p.d_err, 6);
+            if (!mbar_wait_abort(sm.att_bar, (unsigned)(sm.flags[5] + l * nsub + sub) & 1u, sm.flags, spin) && !sm.flags[0]) raise(sm.flags, p.d_err, 6);
             if (TRACE && trace && tid == 0 && sub == 0) trace[8] = global_ns();
             // same trip count for every key lane of the block, so that the warp-wide shuffles stay convergent
             const int rounds = (c1 - c0 + KL - 1) / KL;
@@ -1289,6 +1290,70 @@ __device__ __noinline__ unsigned produce_stage(const b200_token_args &p, int kin
     return sm.flags[0] ? (seq | 0x80000000u) : seq;
 }
 
+// The best row of all blocks (and all ranks), by one warp. Block 0 keeps it; where the launch goes on every block calls this and gets ready for the
+// next token.
+template <bool MULTI>
+__device__ __forceinline__ void next_token(const b200_token_args &p, bool more)
+{
+    const Smem sm = smem_of(p);
+    const int lane = threadIdx.x, pos = sm.flags[3];
+    const unsigned flag_lm = (unsigned)sm.flags[2] * (unsigned)(p.n_layers + 1) + (unsigned)p.n_layers + 1u;
+    float bv = -INFINITY; int bi = 0x7fffffff;
+#pragma unroll 1
+    for (int b0 = lane; b0 < (int)gridDim.x; b0 += 32 * 4) {
+        float v[4], fi[4];
+        const int cnt = ((int)gridDim.x - b0 + 31) / 32;
+        fl_poll<4, 64, false>(p.d_am + 2 * b0, cnt, flag_lm, v, fi, sm.flags, p.d_err, spin_of(p));
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (u < cnt && better(v[u], __float_as_int(fi[u]), bv, bi)) { bv = v[u]; bi = __float_as_int(fi[u]); }
+    }
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+        if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
+    }
+    if (bi == 0x7fffffff) bi = 0;            // nothing compared greater (all NaN): index 0, as the reference's loop
+    bi += (int)p.logits_offset;              // global row of a sharded LM head
+    if (p.n_ranks > 1) {
+        // (value, row) to every rank, then the best of all ranks, lowest row on ties
+        __threadfence_system();
+        if (lane < p.n_ranks) {
+            fl_store<true>(p.d_peer_am[lane], bv, flag_lm);
+            fl_store<true>(p.d_peer_am[lane] + 1, __int_as_float(bi), flag_lm);
+        }
+        float gv[1], gf[1];
+        fl_poll<1, 2, true>(p.d_am_rank + 2 * (lane < p.n_ranks ? lane : 0), lane < p.n_ranks ? 1 : 0, flag_lm, gv, gf, sm.flags, p.d_err, spin_of(p));
+        float xv = lane < p.n_ranks ? gv[0] : -INFINITY;
+        int xi = lane < p.n_ranks ? __float_as_int(gf[0]) : 0x7fffffff;
+#pragma unroll 1
+        for (int o = 16; o > 0; o >>= 1) {
+            const float ov = __shfl_xor_sync(0xffffffffu, xv, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, xi, o);
+            if (better(ov, oi, xv, xi)) { xv = ov; xi = oi; }
+        }
+        if (xi == 0x7fffffff) xi = 0;
+        bi = xi;
+        __threadfence_system();
+    }
+    if (lane == 0) {
+        const bool own = pos + 1 >= *p.d_prompt_len;
+        if (blockIdx.x == 0 && own) p.d_tokens[pos + 1] = bi;
+        if (more) {
+            // the next token of this launch; the cache rows of this one, written by other blocks, are read by bulk copies from now on
+            const int n = pos + 1, chunk = (n + p.n_split - 1) / p.n_split;
+            sm.flags[5] = (sm.flags[5] + p.n_layers * ((chunk + p.att_keys - 1) / p.att_keys)) & 1;
+            sm.flags[4] = own ? bi : p.d_tokens[pos + 1];
+            sm.flags[3] = pos + 1;
+            sm.flags[2] = sm.flags[2] + 1;
+            sm.flags[6] = sm.flags[6] - 1;
+            __threadfence();
+            asm volatile("fence.proxy.async;" ::: "memory");
+        }
+    }
+}
+
 template <int WT, bool TRACE, bool MULTI>
 __global__ void __launch_bounds__(TK_THREADS, 1)
 decode_token_kernel(const __grid_constant__ b200_token_args p)
@@ -1296,14 +1361,16 @@ decode_token_kernel(const __grid_constant__ b200_token_args p)
     const Smem sm = smem_of(p);
     const int tid = threadIdx.x;
     const int spin = spin_of(p);
-    const int L = p.n_layers;
+    const int L = p.n_layers, n_tok = !MULTI && p.n_tokens > 1 ? p.n_tokens : 1;
 
     if (tid == 0) {
         for (int i = 0; i < TK_SLOTS; ++i) { mbar_init(&sm.full[i], 1); mbar_init(&sm.empty[i], TK_NWARP); }
         mbar_init(sm.att_bar, 1);
         sm.flags[0] = 0; sm.flags[1] = 0;
         sm.flags[2] = (int)*p.d_epoch;               // read back from shared memory wherever it is needed: one
-        sm.flags[3] = *p.d_pos;                      // register less to carry through every stage
+        const int pos = *p.d_pos;                    // register less to carry through every stage
+        sm.flags[3] = pos; sm.flags[4] = p.d_tokens[pos]; sm.flags[5] = 0;
+        sm.flags[6] = n_tok;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -1320,6 +1387,8 @@ decode_token_kernel(const __grid_constant__ b200_token_args p)
     if (tid >= TK_NC) {
         if (tid == TK_NC) {
             unsigned seq = 0;
+#pragma unroll 1
+            for (int tk = 0; tk < n_tok && !(seq >> 31); ++tk) {
 #pragma unroll 1
             for (int l = 0; l < L && !(seq >> 31); ++l) {
 #pragma unroll 1
@@ -1340,6 +1409,7 @@ decode_token_kernel(const __grid_constant__ b200_token_args p)
                 }
             }
             if (!(seq >> 31) && p.with_lm) seq = produce_stage(p, B200_ST_LM, p.w_lm, seq, tr ? tr + (size_t)(6 * L) * TK_TRACE_WORDS : nullptr);
+            }
             seq &= 0x7fffffffu;
             // copies still in flight must land before the block may leave: wait for the last fill of every slot
             const unsigned nfill = seq < TK_SLOTS ? seq : TK_SLOTS;
@@ -1358,8 +1428,7 @@ decode_token_kernel(const __grid_constant__ b200_token_args p)
     unsigned state = 0;                              // chunk number | parity of the window number << 31
     const bool tail = p.with_lm || p.n_ranks > 1;    // the LM head, or the residual update that ends a prompt position
 #pragma unroll 1
-    for (int l = 0; l <= L; ++l) {
-        if (l == L && !tail) break;
+    for (int l = 0; l < L || tail; ++l) {
 #pragma unroll 1
         for (int k = 0; k < 5; ++k) {
             if (l == L && k > 0) break;
@@ -1374,60 +1443,17 @@ decode_token_kernel(const __grid_constant__ b200_token_args p)
                 state = run_matvec<WT, TRACE, MULTI>(p, kind, l, (unsigned)sm.flags[2], state, t);
             }
         }
+        if (l < L) continue;
+        if (MULTI || sm.flags[6] <= 1) break;                            // no token left
+        named_barrier(1, TK_NC);                                         // everybody has read that
+        if (tid < 32) next_token<MULTI>(p, true);
+        named_barrier(1, TK_NC);
+        l = -1;
     }
-
-    const unsigned ep = (unsigned)sm.flags[2];
-    const int pos = sm.flags[3];
-    const unsigned flag_lm = ep * (unsigned)(L + 1) + (unsigned)L + 1u;
-    if (p.with_lm) {
-        // --- block 0 folds the best rows of all blocks (and all ranks) ---
-        if (blockIdx.x == 0 && tid < 32) {
-            const int lane = tid;
-            float bv = -INFINITY; int bi = 0x7fffffff;
-#pragma unroll 1
-            for (int b0 = lane; b0 < (int)gridDim.x; b0 += 32 * 4) {
-                float v[4], fi[4];
-                const int cnt = ((int)gridDim.x - b0 + 31) / 32;
-                fl_poll<4, 64, false>(p.d_am + 2 * b0, cnt, flag_lm, v, fi, sm.flags, p.d_err, spin);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (u < cnt && better(v[u], __float_as_int(fi[u]), bv, bi)) { bv = v[u]; bi = __float_as_int(fi[u]); }
-            }
-#pragma unroll 1
-            for (int o = 16; o > 0; o >>= 1) {
-                const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-            }
-            if (bi == 0x7fffffff) bi = 0;            // nothing compared greater (all NaN): index 0, as the reference's loop
-            bi += (int)p.logits_offset;              // global row of a sharded LM head
-            if (p.n_ranks > 1) {
-                // (value, row) to every rank, then the best of all ranks, lowest row on ties
-                __threadfence_system();
-                if (lane < p.n_ranks) {
-                    fl_store<true>(p.d_peer_am[lane], bv, flag_lm);
-                    fl_store<true>(p.d_peer_am[lane] + 1, __int_as_float(bi), flag_lm);
-                }
-                float gv[1], gf[1];
-                fl_poll<1, 2, true>(p.d_am_rank + 2 * (lane < p.n_ranks ? lane : 0), lane < p.n_ranks ? 1 : 0, flag_lm, gv, gf, sm.flags, p.d_err, spin);
-                float xv = lane < p.n_ranks ? gv[0] : -INFINITY;
-                int xi = lane < p.n_ranks ? __float_as_int(gf[0]) : 0x7fffffff;
-#pragma unroll 1
-                for (int o = 16; o > 0; o >>= 1) {
-                    const float ov = __shfl_xor_sync(0xffffffffu, xv, o);
-                    const int oi = __shfl_xor_sync(0xffffffffu, xi, o);
-                    if (better(ov, oi, xv, xi)) { xv = ov; xi = oi; }
-                }
-                if (xi == 0x7fffffff) xi = 0;
-                bi = xi;
-                __threadfence_system();
-            }
-            if (lane == 0 && pos + 1 >= *p.d_prompt_len) p.d_tokens[pos + 1] = bi;
-        }
-    }
+    if (p.with_lm && blockIdx.x == 0 && tid < 32) next_token<MULTI>(p, false);
     if (blockIdx.x == 0 && tid == 0) {
-        *p.d_pos = pos + 1;
-        *p.d_epoch = ep + 1u;
+        *p.d_pos = sm.flags[3] + 1;
+        *p.d_epoch = (unsigned)sm.flags[2] + 1u;
     }
 }
 
@@ -1563,6 +1589,7 @@ extern "C" int b200_decode_token(const b200_token_args *ap, void *stream)
     if (ap->n_blocks <= 0 || ap->smem_bytes <= 0 || ap->scratch_floats <= 0) return B200_E_STATE;   // b200_token_plan first
     if (ap->with_lm && (!ap->w_lm || !ap->g_final || !ap->d_logits || !ap->d_am || ap->g[B200_ST_LM].rows <= 0)) return B200_E_BADARG;
     if (ap->n_ranks > 1 && ap->with_lm && !ap->d_am_rank) return B200_E_BADARG;
+    if (ap->n_tokens < 0 || (ap->n_tokens > 1 && (!ap->with_lm || ap->n_ranks > 1))) return B200_E_BADARG;
     for (int q = 0; q < ap->n_ranks; ++q)
         if (!ap->d_peer_slots_o[q] || !ap->d_peer_slots_dn[q] || !ap->d_peer_counters[q] || (ap->n_ranks > 1 && ap->with_lm && !ap->d_peer_am[q])) return B200_E_BADARG;
     if (ap->n_kv * ap->n_split > ap->n_blocks || B200_CNT_PART + ap->n_kv > 72) return B200_E_BADARG;

@@ -284,6 +284,7 @@ static void free_graphs(InferenceState *s)
 {
     if (s->g_full) { cudaGraphExecDestroy(s->g_full); s->g_full = NULL; }
     if (s->g_nolm) { cudaGraphExecDestroy(s->g_nolm); s->g_nolm = NULL; }
+    if (s->g_group) { cudaGraphExecDestroy(s->g_group); s->g_group = NULL; }
 }
 
 int llmb200_state_finish(InferenceState *s, const float *lm_head, const float *final_norm_gamma, const float *token_emb)
@@ -591,20 +592,21 @@ static void bind_peers(InferenceState *s)
     }
 }
 
-static int enqueue_token_fused(InferenceState *s, int with_lm)
+static int enqueue_token_fused(InferenceState *s, int with_lm, int n_tokens)
 {
     b200_token_args a = s->tk;
     a.with_lm = with_lm;
+    a.n_tokens = n_tokens;
     K_TRY(b200_decode_token(&a, g_rt.stream), return -1);
     return 0;
 }
 
-static int capture(InferenceState *s, int with_lm, int pdl, cudaGraphExec_t *out)
+static int capture(InferenceState *s, int with_lm, int pdl, int n_tokens, cudaGraphExec_t *out)
 {
     cudaGraph_t g = NULL;
     CU_TRY(cudaStreamBeginCapture(g_rt.stream, cudaStreamCaptureModeThreadLocal), return -1);
     const unsigned long long before = b200_launch_count(0);
-    int rc = s->fused ? enqueue_token_fused(s, with_lm) : s->ops->enqueue_token(s, with_lm, pdl);
+    int rc = s->fused ? enqueue_token_fused(s, with_lm, n_tokens) : s->ops->enqueue_token(s, with_lm, pdl);
     if (with_lm) s->kernels_full = (int)(b200_launch_count(0) - before);
     else s->kernels_nolm = (int)(b200_launch_count(0) - before);
     cudaError_t e = cudaStreamEndCapture(g_rt.stream, &g);
@@ -636,18 +638,20 @@ static int ensure_graphs(InferenceState *s)
         if (pr == 0) {
             bind_peers(s);
             s->fused = 1;
-            if (capture(s, 1, 0, &s->g_full) == 0 && capture(s, 0, 0, &s->g_nolm) == 0) return 0;
+            if (capture(s, 1, 0, 1, &s->g_full) == 0 && capture(s, 0, 0, 1, &s->g_nolm) == 0 &&
+                (s->tp_size > 1 || capture(s, 1, 0, TOK_BATCH, &s->g_group) == 0))
+                return 0;
             fprintf(stderr, "[FastGen] whole-token kernel could not be captured; using one kernel per stage\n");
             free_graphs(s);
             s->fused = 0;
         }
     }
-    if (capture(s, 1, s->use_pdl, &s->g_full) != 0 || capture(s, 0, s->use_pdl, &s->g_nolm) != 0) {
+    if (capture(s, 1, s->use_pdl, 1, &s->g_full) != 0 || capture(s, 0, s->use_pdl, 1, &s->g_nolm) != 0) {
         if (s->use_pdl) {
             fprintf(stderr, "[FastGen] graph capture with programmatic dependent launch failed; retrying without\n");
             free_graphs(s);
             s->use_pdl = 0;
-            if (capture(s, 1, 0, &s->g_full) == 0 && capture(s, 0, 0, &s->g_nolm) == 0) return 0;
+            if (capture(s, 1, 0, 1, &s->g_full) == 0 && capture(s, 0, 0, 1, &s->g_nolm) == 0) return 0;
         }
         fprintf(stderr, "[FastGen] CUDA graph capture failed\n");
         free_graphs(s);
@@ -1291,8 +1295,10 @@ static int generate_one(InferenceState *s, const uint32_t *prompt, int prompt_le
     int batch_n[4] = {0, 0, 0, 0};
     while (!stop) {
         while (launched < max_fw && b_enq - b_done < 2) {
-            CU_TRY(cudaGraphLaunch(s->g_full, g_rt.stream), return n_gen);
-            launched++;
+            /* a whole group in one launch where the whole-token kernel runs: between two launches of it lie 9 us */
+            const int group = s->g_group && launched == copied && max_fw - launched >= TOK_BATCH;
+            CU_TRY(cudaGraphLaunch(group ? s->g_group : s->g_full, g_rt.stream), return n_gen);
+            launched += group ? TOK_BATCH : 1;
             if (launched - copied == TOK_BATCH || launched == max_fw) {
                 const int slot = b_enq & 3, n = launched - copied;
                 CU_TRY(cudaMemcpyAsync(&s->h_tok[8 + slot * TOK_BATCH], s->d_tokens + P + copied + 1, (size_t)n * 4,

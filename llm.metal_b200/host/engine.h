@@ -82,7 +82,7 @@ struct InferenceState {
     int *h_ctl;              /* pinned staging for control writes */
     cudaEvent_t tok_ev[4];
     cudaEvent_t ev_a, ev_b;
-    cudaGraphExec_t g_full, g_nolm;
+    cudaGraphExec_t g_full, g_nolm, g_group;     /* a token, one without logits, TOK_BATCH tokens (whole-token kernel on one GPU) */
     int kernels_full, kernels_nolm;   /* kernel nodes per graph */
     int use_pdl;
     /* LoRA adapter attached with inference_state_set_lora: device pointers into the SFT state's vectors */
