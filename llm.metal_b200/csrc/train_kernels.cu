@@ -362,6 +362,19 @@ __device__ __forceinline__ float quad_sum(float v)
     return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
+// Which tile (0: the heaviest), sequence and head the block works on. Tiles weigh 1 .. N / 64, and with two blocks on an SM those of the first two
+// rounds never wait for one another's end: the second round counts from its light end, so that every SM gets about the same.
+// 509 positions, 32 heads: at most 9 tiles' work an SM, 12 in order of heads and tiles.
+struct AttnItem { int tile, seq, head; };
+constexpr int ATT_SMS = 148;
+template <int PER_SM>
+__device__ __forceinline__ AttnItem attn_item(int n_seq, int heads)
+{
+    const int id = blockIdx.x, second = PER_SM > 1 ? min(2 * ATT_SMS, (int)gridDim.x) - ATT_SMS : 0;
+    const int rank = id >= ATT_SMS && id < ATT_SMS + second ? 2 * ATT_SMS + second - 1 - id : id;
+    return {rank / (n_seq * heads), rank % n_seq, rank / n_seq % heads};
+}
+
 template <int HD, bool TC>
 __global__ void __launch_bounds__(ATT_THREADS)
 attn_fwd_kernel(const float *q, const float *k, const float *v, long long v_ld, int n_seq, int N, int n_q, int n_kv,
@@ -371,7 +384,8 @@ attn_fwd_kernel(const float *q, const float *k, const float *v, long long v_ld, 
     extern __shared__ __align__(16) float sh[];
     __shared__ float stat[2][2][AT];
     float *Q = sh, *P = sh, *buf = sh + AT * L::RP;
-    const int it = (N + AT - 1) / AT - 1 - (int)blockIdx.x / n_seq, s = blockIdx.x % n_seq, h = blockIdx.y, kvh = h / (n_q / n_kv);
+    const AttnItem item = attn_item<HD == 256 ? 1 : 2>(n_seq, n_q);
+    const int it = (N + AT - 1) / AT - 1 - item.tile, s = item.seq, h = item.head, kvh = h / (n_q / n_kv);
     const size_t row0 = (size_t)s * N;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rw = (warp & 3) * 16, half = warp >> 2;
     const int i0 = it * AT, ni = min(AT, N - i0), r0 = rw + (lane >> 2), c0 = half * 32 + 2 * (lane & 3);
@@ -490,7 +504,8 @@ attn_bwd_dq_kernel(const float *d_out, const float *probs, const float *k, const
     extern __shared__ __align__(16) float sh[];
     __shared__ float stat[2][AT];
     float *O = sh, *G = sh, *buf = sh + AT * L::RP;
-    const int it = (N + AT - 1) / AT - 1 - (int)blockIdx.x / n_seq, s = blockIdx.x % n_seq, h = blockIdx.y, kvh = h / (n_q / n_kv);
+    const AttnItem item = attn_item<HD == 256 ? 1 : 2>(n_seq, n_q);
+    const int it = (N + AT - 1) / AT - 1 - item.tile, s = item.seq, h = item.head, kvh = h / (n_q / n_kv);
     const size_t row0 = (size_t)s * N;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rw = (warp & 3) * 16, half = warp >> 2;
     const int i0 = it * AT, ni = min(AT, N - i0), r0 = rw + (lane >> 2), c0 = half * 32 + 2 * (lane & 3);
@@ -578,7 +593,7 @@ attn_bwd_dq_kernel(const float *d_out, const float *probs, const float *k, const
 }
 
 // 64 keys x 64 columns of dK (d_score^T . Q) or dV (P^T . dO) of a KV head: summed over the later queries of each query head, then
-// over the heads in order. blockIdx.y = ((kv head * 2 + dK / dV) * (HD / 64) + columns).
+// over the heads in order. The item's head = ((kv head * 2 + dK / dV) * (HD / 64) + columns).
 template <bool TC>
 __global__ void __launch_bounds__(ATT_THREADS)
 attn_bwd_dkv_kernel(const float *d_score, const float *probs, const float *q, const float *d_out, int n_seq, int N, int n_q, int n_kv,
@@ -586,8 +601,10 @@ attn_bwd_dkv_kernel(const float *d_score, const float *probs, const float *q, co
 {
     constexpr int CP = AT + 8, BUF = AT * CP;
     extern __shared__ __align__(16) float sh[];               // two buffers of (weights, rows)
-    const int jt = blockIdx.x / n_seq, s = blockIdx.x % n_seq, slices = hd / 64, slice = blockIdx.y % slices;
-    const int which = (blockIdx.y / slices) & 1, kvh = blockIdx.y / (2 * slices), group = n_q / n_kv;
+    const int slices = hd / 64;
+    const AttnItem item = attn_item<2>(n_seq, n_kv * 2 * slices);
+    const int jt = item.tile, s = item.seq, slice = item.head % slices;
+    const int which = (item.head / slices) & 1, kvh = item.head / (2 * slices), group = n_q / n_kv;
     const size_t row0 = (size_t)s * N;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rw = (warp & 3) * 16, half = warp >> 2;
     const int j0 = jt * AT, nj = min(AT, N - j0), tiles = (N - j0 + AT - 1) / AT, steps = group * tiles;
@@ -1220,7 +1237,7 @@ static int attn_fwd_launch(const float *q, const float *k, const float *v, long 
     constexpr size_t smem = AttnTiles<HD>::bytes;
     int rc = opt_in_smem(attn_fwd_kernel<HD, TC>, smem);
     if (rc) return rc;
-    attn_fwd_kernel<HD, TC><<<dim3((N + AT - 1) / AT * n_seq, n_q), ATT_THREADS, smem, st>>>(q, k, v, v_ld, n_seq, N, n_q, n_kv, scale, probs, out, out_h);
+    attn_fwd_kernel<HD, TC><<<(N + AT - 1) / AT * n_seq * n_q, ATT_THREADS, smem, st>>>(q, k, v, v_ld, n_seq, N, n_q, n_kv, scale, probs, out, out_h);
     return done();
 }
 
@@ -1269,10 +1286,10 @@ static int attn_bwd_launch(const float *d_out, const float *probs, const float *
     if (!rc) rc = opt_in_smem(attn_bwd_dkv_kernel<TC>, smem_kv);
     if (rc) return rc;
     const int tiles = (N + AT - 1) / AT;
-    attn_bwd_dq_kernel<HD, TC><<<dim3(tiles * n_seq, n_q), ATT_THREADS, smem, st>>>(d_out, probs, k, v, v_ld, n_seq, N, n_q, n_kv, scale, d_score, dqkv, ld);
+    attn_bwd_dq_kernel<HD, TC><<<tiles * n_seq * n_q, ATT_THREADS, smem, st>>>(d_out, probs, k, v, v_ld, n_seq, N, n_q, n_kv, scale, d_score, dqkv, ld);
     rc = done();
     if (rc) return rc;
-    attn_bwd_dkv_kernel<TC><<<dim3(tiles * n_seq, n_kv * 2 * (HD / 64)), ATT_THREADS, smem_kv, st>>>(d_score, probs, q, d_out, n_seq, N, n_q, n_kv, HD, dqkv, ld);
+    attn_bwd_dkv_kernel<TC><<<tiles * n_seq * n_kv * 2 * (HD / 64), ATT_THREADS, smem_kv, st>>>(d_score, probs, q, d_out, n_seq, N, n_q, n_kv, HD, dqkv, ld);
     return done();
 }
 
