@@ -24,7 +24,10 @@ extern unsigned long long g_b200_launches;
 
 namespace {
 
-constexpr int ATT_THREADS = 512;
+// Threads of a block: 512, one block on an SM (114 registers); 256, two of them, where sequences and KV heads alone are more blocks than SMs: 32 sequences,
+// 8 KV heads of 128 and 130 - 250 keys took two waves of 512, and every block left its sums and its ticket in memory for itself to read
+// (4 layers of Qwen3-4B, 128 + 128 tokens: 60.2 ms, 53.6 now).
+constexpr int ATT_WIDE = 512, ATT_NARROW = 256, ATT_SMS = 148;
 
 __device__ __forceinline__ void halves8_to_float(const uint4 &u, float *f)
 {
@@ -43,8 +46,8 @@ __device__ __forceinline__ void halves8_to_float(const uint4 &u, float *f)
 // output), so nothing is exchanged between threads while keys stream in; K and V rows are prefetched
 // two keys ahead, the first ones before the query is even normalised. At the end the key lanes of a
 // head are merged (shuffles inside a warp, shared memory across warps).
-template <int HD, int G>
-__global__ void __launch_bounds__(ATT_THREADS)
+template <int HD, int G, int ATT_THREADS>
+__global__ void __launch_bounds__(ATT_THREADS, ATT_WIDE / ATT_THREADS)
 attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_cap)
 {
     // batched form: blockIdx.z selects the sequence; its buffers are slices of the shared ones
@@ -241,6 +244,23 @@ attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_ca
         if (dl == 0) { dst[HD] = m; dst[HD + 1] = l; }
     }
     __syncthreads();
+    if (p.n_split == 1) {                       // nothing to merge with
+        for (int o = tid; o < G * HD; o += ATT_THREADS) {
+            const float *src = mrg + (size_t)(o / HD) * WPH * (HD + 2);
+            float M = -INFINITY, v = 0.0f, sum = 0.0f;
+#pragma unroll
+            for (int w = 0; w < WPH; ++w) M = fmaxf(M, src[w * (HD + 2) + HD]);
+#pragma unroll
+            for (int w = 0; w < WPH; ++w) {
+                const float mw = src[w * (HD + 2) + HD];
+                const float c = (mw == -INFINITY) ? 0.0f : expf(mw - M);
+                v = fmaf(src[w * (HD + 2) + o % HD], c, v);
+                sum = fmaf(src[w * (HD + 2) + HD + 1], c, sum);
+            }
+            p.d_out[(size_t)(kvh * G) * HD + o] = v / sum;
+        }
+        return;
+    }
     // scratch: [n_q][n_split][HD + 2] = unnormalised output, running max, sum
     for (int o = tid; o < G * (HD + 2); o += ATT_THREADS) {
         const int gg = o / (HD + 2), d = o - gg * (HD + 2);
@@ -343,15 +363,15 @@ attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_ca
     if (tid == 0) p.d_tickets[kvh] = 0u;
 }
 
-template <int HD, int G>
-int launch_attn(const b200_attn_args &a, cudaStream_t st)
+template <int HD, int G, int ATT_THREADS>
+int launch_attn_as(const b200_attn_args &a, cudaStream_t st)
 {
     const int chunk_cap = (a.max_seq + a.n_split - 1) / a.n_split;
     const int WPH = ATT_THREADS / G / 32;
     size_t mrg_floats = (size_t)G * WPH * (HD + 2);
     if (mrg_floats < (size_t)2 * G * a.n_split) mrg_floats = (size_t)2 * G * a.n_split;
     const size_t smem = ((size_t)G * HD + 2 * HD + mrg_floats) * sizeof(float);
-    auto kern = attn_decode_kernel<HD, G>;
+    auto kern = attn_decode_kernel<HD, G, ATT_THREADS>;
     if (smem > 200 * 1024) return B200_E_TOOLARGE;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -369,6 +389,14 @@ int launch_attn(const b200_attn_args &a, cudaStream_t st)
     cfg.numAttrs = a.use_pdl ? 1 : 0;
     ++g_b200_launches;
     return (int)cudaLaunchKernelEx(&cfg, kern, a, chunk_cap);
+}
+
+template <int HD, int G>
+int launch_attn(const b200_attn_args &a, cudaStream_t st)
+{
+    if constexpr (G < ATT_NARROW / 32)          // a warp per new row
+        if ((long long)a.n_split * a.n_kv * a.n_items > ATT_SMS) return launch_attn_as<HD, G, ATT_NARROW>(a, st);
+    return launch_attn_as<HD, G, ATT_WIDE>(a, st);
 }
 
 } // namespace
