@@ -29,6 +29,17 @@ inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, dim3 block, siz
     return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
+// ---- order of blocks ---------------------------------------------------
+// Blocks of a one-dimensional grid take items that are numbered from the heaviest to the lightest. Two that start on an SM together never wait for
+// one another's end: with `two`, the second round counts from its light end, so that every SM gets about the same (rows of a causal
+// attention: 9 tiles of 64 an SM at most for 509 rows of 32 heads, 12 in order of heads and tiles).
+__device__ __forceinline__ int rank_by_weight(bool two)
+{
+    constexpr int SMS = 148;
+    const int id = blockIdx.x, second = two ? min(2 * SMS, (int)gridDim.x) - SMS : 0;
+    return id >= SMS && id < SMS + second ? 2 * SMS + second - 1 - id : id;
+}
+
 // ---- memory ------------------------------------------------------------
 // Streaming 16-byte load that does not allocate in L1 (weights are read once).
 __device__ __forceinline__ uint4 ldg_stream_16(const void *p) {

@@ -350,8 +350,9 @@ __global__ void __launch_bounds__(NW * 32, HD == 256 ? 1 : HD == 128 && NW == 4 
     __half *ksm = qsm + 2 * BQ * KS;                         // [2][BKEY][KS]
     __half *vsm = ksm + 2 * BKEY * KS;                       // [2][BKEY][VS]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int h = blockIdx.y % p.n_q, c0 = (blockIdx.y / p.n_q) * DV, seq = blockIdx.z;
-    const int m0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * BQ;               // rows that see the most keys start first
+    const int tiles_q = (p.seq_len + BQ - 1) / BQ, per_tile = gridDim.x / tiles_q, rank = rank_by_weight(HD < 256), part = rank % per_tile;
+    const int h = part % p.n_q, c0 = part / p.n_q % (HD / DV) * DV, seq = part / (p.n_q * (HD / DV));
+    const int m0 = (tiles_q - 1 - rank / per_tile) * BQ;                      // rows that see the most keys start first
     const int rows = min(BQ, p.seq_len - m0), first = p.pos0 + m0, last = first + rows - 1;
     const long long head = (long long)seq * p.cache_seq_stride + (long long)(h / (p.n_q / p.n_kv)) * p.max_seq * HD;
     const __half *keys = static_cast<const __half *>(p.d_k_cache) + head, *values = static_cast<const __half *>(p.d_v_cache) + head + c0;
@@ -551,7 +552,7 @@ int launch_attn(const b200_rows_attn_args &a, cudaStream_t st)
     const int rc = allow_smem(rows_attn_kernel<HD, NW>, smem);
     if (rc) return rc;
     ++g_b200_launches;
-    return (int)launch_chained(rows_attn_kernel<HD, NW>, dim3((a.seq_len + NW * 16 - 1) / (NW * 16), a.n_q * (HD / DV), a.n_rows / a.seq_len),
+    return (int)launch_chained(rows_attn_kernel<HD, NW>, dim3((a.seq_len + NW * 16 - 1) / (NW * 16) * a.n_q * (HD / DV) * (a.n_rows / a.seq_len)),
                                dim3(NW * 32), smem, st, a);
 }
 

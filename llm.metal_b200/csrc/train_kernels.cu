@@ -362,16 +362,12 @@ __device__ __forceinline__ float quad_sum(float v)
     return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-// Which tile (0: the heaviest), sequence and head the block works on. Tiles weigh 1 .. N / 64, and with two blocks on an SM those of the first two
-// rounds never wait for one another's end: the second round counts from its light end, so that every SM gets about the same.
-// 509 positions, 32 heads: at most 9 tiles' work an SM, 12 in order of heads and tiles.
+// Which tile (0: the heaviest), sequence and head the block works on. Tiles weigh 1 .. N / 64.
 struct AttnItem { int tile, seq, head; };
-constexpr int ATT_SMS = 148;
 template <int PER_SM>
 __device__ __forceinline__ AttnItem attn_item(int n_seq, int heads)
 {
-    const int id = blockIdx.x, second = PER_SM > 1 ? min(2 * ATT_SMS, (int)gridDim.x) - ATT_SMS : 0;
-    const int rank = id >= ATT_SMS && id < ATT_SMS + second ? 2 * ATT_SMS + second - 1 - id : id;
+    const int rank = rank_by_weight(PER_SM > 1);
     return {rank / (n_seq * heads), rank % n_seq, rank / n_seq % heads};
 }
 
