@@ -6,8 +6,10 @@
 // half of the rows of B, and the tensor cores read the other half from the neighbour's shared memory, so a 256-wide
 // tile wants 64. Persistent: a pair walks its tiles, two accumulators in tensor memory take turns, and the epilogue of one
 // tile runs under the products of the next.
-// Measured, one SM per tile before and pairs now: 512 x 19456 x 2560 92 us and 59 us, 512 x 2560 x 16384 98 and 57, 2048 x 12288 x 2048
-// 158 and 92 (1117 TFLOP/s), 2048 x 2048 x 6144 61 and 51.
+// Results leave through shared memory, whole lines of four rows a store: stored by the thread that read the row, 16 bytes in 32 lines, they cost 74
+// clocks a column that nothing hides in a product of one wave. Chains of 20, before that (and with a division per ring step in the
+// issuing lane) and now: 512 x 2560 x 9728 45 us and 31, 512 x 6144 x 2560 24 and 19.5, 512 x 2560 x 4096 27 and 24, 2048 x 2560 x 4096 48 and 37,
+// 2048 x 12288 x 2048 90 and 82 (1260 TFLOP/s); 512 x 4096 x 512 10.2 and 11.2.
 //
 // Pair, per SM: warp 0 loads with TMA (both SMs' copies complete on the barrier of the first, the leader), one lane of the
 // leader's warp 1 issues the products for both and commits to both, warps 2-5 store their SM's 128 rows. Products of few tiles are
@@ -28,14 +30,23 @@ constexpr int SM_ROWS = 128;             // rows of A per SM = tensor-memory lan
 constexpr int KB = 64;                   // k of a 128-byte operand row
 constexpr int PAIR_THREADS = 192;
 constexpr int PAIR_SLOTS = 8;
+constexpr int KSUB = 2;                  // operand rows per slot: half the hand-overs
+constexpr int STAGE_PITCH = 36;          // floats between the rows of a block on its way out: 16-byte accesses of eight rows or columns meet 32 banks
 constexpr uint32_t A_TILE = SM_ROWS * KB * 2;
 struct PairArgs {
     float *C; long long ldc;
     const float *R; long long ldr;
     __nv_bfloat16 *Ch; long long ldch;
-    int M, N, K, bn, ksub, slots, splits, tiles_m, tiles, fmt, relu2;
+    int M, N, K, bn, slots, splits, tiles_m, tiles, fmt, relu2;
     float alpha;
     unsigned *d_err;
+};
+
+// The place in a ring and the phase of the barriers there.
+struct Turn {
+    int at = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void next(int n) { if (++at == n) { at = 0; phase ^= 1; } }
 };
 
 __device__ __forceinline__ uint32_t on_rank(uint32_t addr, uint32_t rank)
@@ -66,54 +77,58 @@ __device__ __forceinline__ void arrive_at(uint32_t bar)
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// 32 columns of this thread's row, tile columns from n on
-__device__ __forceinline__ void store32(const PairArgs &p, int row, int n, int n_end, const uint32_t *r, bool vec)
+// 32 rows (row0 on, one a lane in r) by 32 columns (n on) of a tile, by one warp: through shared memory, so that a store covers whole lines of four rows
+// and not 16 bytes of 32. The same for what is added.
+__device__ __forceinline__ void store_block(const PairArgs &p, float *stage, int row0, int n, int n_end, const uint32_t *r, bool vec)
 {
-    const float *rrow = p.R ? p.R + (long long)row * p.ldr : nullptr;
-    if (p.Ch) {
-        __nv_bfloat16 *h = p.Ch + (long long)row * p.ldch + n;
-        float f[32];
+    const int lane = threadIdx.x & 31, c = (lane & 7) * 4, r0 = lane >> 3;
+    n += c;
+    const bool whole = n + 4 <= n_end;
+    float4 add[8];
+    if (!p.Ch && p.R && vec) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) f[j] = p.alpha * (p.relu2 ? act_relu2(__uint_as_float(r[j])) : __uint_as_float(r[j]));
-        if (n + 32 <= n_end) {
+        for (int i = 0; i < 8; ++i)
+            add[i] = whole && row0 + 4 * i + r0 < p.M ? __ldcg(reinterpret_cast<const float4 *>(p.R + (long long)(row0 + 4 * i + r0) * p.ldr + n))
+                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-                uint32_t w[4];
+    for (int j = 0; j < 32; j += 4)
+        *reinterpret_cast<float4 *>(stage + lane * STAGE_PITCH + j) =
+            make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
+    __syncwarp();
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const __nv_bfloat162 b = __floats2bfloat162_rn(f[j + 2 * k], f[j + 2 * k + 1]);
-                    w[k] = *reinterpret_cast<const uint32_t *>(&b);
-                }
-                *reinterpret_cast<uint4 *>(h + j) = make_uint4(w[0], w[1], w[2], w[3]);
+    for (int i = 0; i < 8; ++i) {
+        const int row = row0 + 4 * i + r0;
+        float4 v = *reinterpret_cast<const float4 *>(stage + (4 * i + r0) * STAGE_PITCH + c);
+        if (row >= p.M || n >= n_end) continue;
+        if (p.Ch) {
+            __nv_bfloat16 *h = p.Ch + (long long)row * p.ldch + n;
+            float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) f[j] = p.alpha * (p.relu2 ? act_relu2(f[j]) : f[j]);
+            if (whole) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
+                *reinterpret_cast<uint2 *>(h) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (n + j < n_end) h[j] = __float2bfloat16_rn(f[j]);
             }
+            continue;
+        }
+        float *o = p.C + (long long)row * p.ldc + n;
+        v = make_float4(p.alpha * v.x, p.alpha * v.y, p.alpha * v.z, p.alpha * v.w);
+        if (vec && whole) {
+            if (p.R) { v.x += add[i].x; v.y += add[i].y; v.z += add[i].z; v.w += add[i].w; }
+            *reinterpret_cast<float4 *>(o) = v;
         } else {
+            const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (n + j < n_end) h[j] = __float2bfloat16_rn(f[j]);
+            for (int j = 0; j < 4; ++j)
+                if (n + j < n_end) o[j] = p.R ? f[j] + __ldcg(p.R + (long long)row * p.ldr + n + j) : f[j];
         }
-        return;
     }
-    float *c = p.C + (long long)row * p.ldc + n;
-    if (vec && n + 32 <= n_end) {
-#pragma unroll
-        for (int j = 0; j < 32; j += 4) {
-            float4 v = make_float4(p.alpha * __uint_as_float(r[j]), p.alpha * __uint_as_float(r[j + 1]),
-                                   p.alpha * __uint_as_float(r[j + 2]), p.alpha * __uint_as_float(r[j + 3]));
-            if (rrow) {
-                const float4 q = __ldcg(reinterpret_cast<const float4 *>(rrow + n + j));
-                v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
-            }
-            *reinterpret_cast<float4 *>(c + j) = v;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (n + j < n_end) {
-                float v = p.alpha * __uint_as_float(r[j]);
-                if (rrow) v += __ldcg(rrow + n + j);
-                c[j] = v;
-            }
-    }
+    __syncwarp();
 }
 
 __global__ void __launch_bounds__(PAIR_THREADS)
@@ -123,14 +138,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     __shared__ uint64_t full_bar[PAIR_SLOTS], empty_bar[PAIR_SLOTS], done_bar[2], free_bar[2];
     __shared__ uint32_t tmem_base_sh;
     __shared__ int abort_sh;
+    __shared__ __align__(16) float stage_sh[4][32 * STAGE_PITCH];
     uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = blockIdx.x & 1;
     const int split = (int)(blockIdx.x >> 1) % p.splits;                 // clusters hold the splits of a tile
     const uint32_t leader = 2 * split;
     const int first = (int)(blockIdx.x >> 1) / p.splits, stride = (int)(gridDim.x >> 1) / p.splits;
-    const uint32_t B_TILE = (uint32_t)p.bn / 2 * KB * 2, SLOT = (A_TILE + B_TILE) * p.ksub;
-    const int nkb_all = (p.K + KB * p.ksub - 1) / (KB * p.ksub), per = (nkb_all + p.splits - 1) / p.splits;
+    const uint32_t B_TILE = (uint32_t)p.bn / 2 * KB * 2, SLOT = (A_TILE + B_TILE) * KSUB;
+    const int nkb_all = (p.K + KB * KSUB - 1) / (KB * KSUB), per = (nkb_all + p.splits - 1) / p.splits;
     const int kb0 = split * per, nkb = min(per, nkb_all - kb0);
     volatile int *abort_flag = &abort_sh;
 
@@ -154,17 +170,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // a pair (with splits: a cluster, which has one) takes every stride-th tile
     if (warp == 0) {
         if (lane == 0) {
-            int i = 0;                                       // ring steps so far
+            Turn t;                                          // places and phases are counted: a division a step would be on the critical path
             for (int tile = first; tile < p.tiles && !*abort_flag; tile += stride) {
                 const int m0 = tile % p.tiles_m * 2 * SM_ROWS + (int)rank * SM_ROWS, n0 = tile / p.tiles_m * p.bn + (int)rank * (p.bn / 2);
-                for (int kb = 0; kb < nkb; ++kb, ++i) {
-                    const int s = i % p.slots;
-                    if (!wait_or_abort(&empty_bar[s], ((i / p.slots) & 1) ^ 1, abort_flag)) { give_up(0x7301u); break; }
-                    uint8_t *a = ring + (size_t)s * SLOT, *b = a + (size_t)A_TILE * p.ksub;
+                for (int kb = 0; kb < nkb; ++kb, t.next(p.slots)) {
+                    const int s = t.at;
+                    if (!wait_or_abort(&empty_bar[s], t.phase ^ 1, abort_flag)) { give_up(0x7301u); break; }
+                    uint8_t *a = ring + (size_t)s * SLOT, *b = a + (size_t)A_TILE * KSUB;
                     const uint32_t bar = on_rank(smem_u32(&full_bar[s]), leader);
                     if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * SLOT);
-                    for (int q = 0; q < p.ksub; ++q) {
-                        const int x = ((kb0 + kb) * p.ksub + q) * KB;
+#pragma unroll
+                    for (int q = 0; q < KSUB; ++q) {
+                        const int x = ((kb0 + kb) * KSUB + q) * KB;
                         pair_load(a + (size_t)q * A_TILE, &map_a, x, m0, bar);
                         pair_load(b + (size_t)q * B_TILE, &map_b, x, n0, bar);
                     }
@@ -174,18 +191,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     } else if (warp == 1) {
         if (lane == 0 && rank == 0) {
             const uint32_t idesc = (1u << 4) | ((uint32_t)p.fmt << 7) | ((uint32_t)p.fmt << 10) | ((uint32_t)(p.bn >> 3) << 17) | (16u << 24);
-            int i = 0, t = 0;
+            Turn u;
+            int t = 0;
             for (int tile = first; tile < p.tiles && !*abort_flag; tile += stride, ++t) {
                 const int acc = t & 1;
                 if (!wait_or_abort(&free_bar[acc], ((t >> 1) & 1) ^ 1, abort_flag)) { give_up(0x7305u); break; }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 bool ok = true;
-                for (int kb = 0; kb < nkb; ++kb, ++i) {
-                    const int s = i % p.slots;
-                    if (!wait_or_abort(&full_bar[s], (i / p.slots) & 1, abort_flag)) { give_up(0x7302u); ok = false; break; }
+                for (int kb = 0; kb < nkb; ++kb, u.next(p.slots)) {
+                    const int s = u.at;
+                    if (!wait_or_abort(&full_bar[s], u.phase, abort_flag)) { give_up(0x7302u); ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a = smem_u32(ring + (size_t)s * SLOT), b = a + A_TILE * p.ksub;
-                    for (int q = 0; q < p.ksub; ++q) {
+                    const uint32_t a = smem_u32(ring + (size_t)s * SLOT), b = a + A_TILE * KSUB;
+#pragma unroll
+                    for (int q = 0; q < KSUB; ++q) {
                         const uint64_t ad = smem_desc_sw128(a + q * A_TILE), bd = smem_desc_sw128(b + q * B_TILE);
 #pragma unroll
                         for (int j = 0; j < 4; ++j) pair_umma(tmem_base + acc * 256, ad + 2 * j, bd + 2 * j, idesc, (kb | q | j) != 0);
@@ -203,7 +222,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         int t = 0;
         for (int tile = first; tile < p.tiles; tile += stride, ++t) {
             const int acc = t & 1;
-            const int row = tile % p.tiles_m * 2 * SM_ROWS + (int)rank * SM_ROWS + quad * 32 + lane, n0 = tile / p.tiles_m * p.bn;
+            const int row0 = tile % p.tiles_m * 2 * SM_ROWS + (int)rank * SM_ROWS + quad * 32, n0 = tile / p.tiles_m * p.bn;
             const bool ok = __all_sync(0xffffffffu, wait_or_abort(&done_bar[acc], (t >> 1) & 1, abort_flag));
             if (!ok) { if (lane == 0) give_up(0x7303u); break; }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -220,9 +239,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         if (c + j < p.bn)
                             *reinterpret_cast<float4 *>(part + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
                                                                                 __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-                } else if (row < p.M) {
-                    store32(p, row, n0 + c, n_end, r, vec);
-                }
+                } else store_block(p, stage_sh[warp - 2], row0, n0 + c, n_end, r, vec);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -277,7 +294,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // through shared memory. The width is a multiple of 16 up to 256. CLUSTERS: how many clusters of 2, 4, 6, 8 blocks are resident
 // on 148 SMs (the occupancy calculator's figures).
 // What comes back is held against the form of one SM per tile: clocks of the shape taken, fitted to 200 products (M 129 .. 2048, N 256 .. 19456,
-// K 256 .. 16384, chains of 20 launches), 8 % rms.
+// K 256 .. 16384, chains of 20 launches) before results went out in lines, 8 % rms then and 6 % above the times since. Left as they are:
+// narrower tiles in fewer splits would be up to 10 % faster (512 x 2560 x 4096 24 us in two, 22 in one), but their accumulators take twice the
+// additions, which the tensor cores truncate.
 double gemm_pair_shape(int M, int N, int K, bool may_split, PairShape *out)
 {
     if (M <= SM_ROWS || N < 256) return 1e30;
@@ -311,12 +330,11 @@ int gemm_pair_launch(const b200_gemm_args *a, int fmt, const PairShape &sh, cuda
     p.alpha = a->alpha; p.d_err = a->d_err;
     p.tiles_m = (a->M + 2 * SM_ROWS - 1) / (2 * SM_ROWS);
     p.tiles = p.tiles_m * ((a->N + p.bn - 1) / p.bn);
-    p.ksub = 2;                                              // two operand rows per slot: half the hand-overs
-    const size_t slot = (size_t)(A_TILE + p.bn * 64) * p.ksub;
-    p.slots = (int)((216 * 1024) / slot);
+    const size_t slot = (size_t)(A_TILE + p.bn * 64) * KSUB;
+    p.slots = (int)((200 * 1024) / slot);
     if (p.slots > PAIR_SLOTS) p.slots = PAIR_SLOTS;
     // a split without a step would have nothing to commit: as many as there are slots of k for
-    const int nkb = (a->K + KB * p.ksub - 1) / (KB * p.ksub);
+    const int nkb = (a->K + KB * KSUB - 1) / (KB * KSUB);
     while (p.splits > 1 && (p.splits - 1) * ((nkb + p.splits - 1) / p.splits) >= nkb) --p.splits;
     const size_t smem = slot * p.slots + 1024;
     CUtensorMap ma, mb;
