@@ -99,6 +99,76 @@ rms_norm_bwd_rows_kernel(const float *x, const float *dy, long long dy_ld, const
     }
 }
 
+// The same sums in the same order for rows of up to 256 NV elements, a block per row: a thread's elements stay in registers, so that all of a row's
+// loads are in flight at once and nothing is read twice. 512 rows of 2560: 8.6 us and, backward, 12.1 where the row was read again after the sums;
+// 6.1 and 8.0 here.
+template <int NV>
+__global__ void __launch_bounds__(256)
+rms_norm_held_kernel(const float *x, const float *gamma, float *out, __half *out_h, int dim, float eps)
+{
+    __shared__ float sh[8];
+    const size_t at = (size_t)blockIdx.x * dim;
+    float v[NV], ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        v[k] = i < dim ? x[at + i] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+        if (threadIdx.x + 256 * k < dim) ss = fmaf(v[k], v[k], ss);
+    ss = group_sum_f<256>(ss, sh);
+    const float inv = rsqrtf(ss / (float)dim + eps);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        if (i < dim) {
+            const float r = v[k] * inv * gamma[i];
+            out[at + i] = r;
+            if (out_h) out_h[at + i] = __float2half_rn(r);
+        }
+    }
+}
+
+template <int NV>
+__global__ void __launch_bounds__(256)
+rms_norm_bwd_held_kernel(const float *x, const float *dy, long long dy_ld, const float *gamma, float *dx, int dim, float eps, int accumulate,
+                         float clamp, __half *dx_h, float h_scale)
+{
+    __shared__ float sh[8];
+    const size_t at = (size_t)blockIdx.x * dim;
+    const float *dr = dy + (size_t)blockIdx.x * dy_ld;
+    float v[NV], d[NV], g[NV], ss = 0.f, dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        v[k] = i < dim ? x[at + i] : 0.f;
+        d[k] = i < dim ? dr[i] : 0.f;
+        g[k] = i < dim ? gamma[i] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+        if (threadIdx.x + 256 * k < dim) {
+            ss = fmaf(v[k], v[k], ss);
+            dot = fmaf(d[k] * g[k], v[k], dot);
+        }
+    ss = group_sum_f<256>(ss, sh);
+    dot = group_sum_f<256>(dot, sh);
+    const float inv = rsqrtf(ss / (float)dim + eps);
+    const float coeff = dot * inv * inv / (float)dim;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + 256 * k;
+        if (i < dim) {
+            float r = __fmaf_rn(g[k], d[k], -__fmul_rn(coeff, v[k])) * inv;      // as the element form contracts it
+            if (accumulate) r += dx[at + i];
+            if (clamp > 0.f) r = fminf(fmaxf(r, -clamp), clamp);
+            dx[at + i] = r;
+            if (dx_h) dx_h[at + i] = __float2half_rn(r * h_scale);
+        }
+    }
+}
+
 // ---- QK-norm + RoPE: one warp per (row, head) -----------------------------------------------
 // Heads 0..n_q-1 are q heads, n_q..n_q+n_kv-1 the k heads; both sit in qkv at column head*hd.
 template <int HD>
@@ -634,12 +704,40 @@ attn_bwd_dkv_kernel(const float *d_score, const float *probs, const float *q, co
 }
 
 // ---- SwiGLU ------------------------------------------------------------------------------------
+struct Silu {
+    static __device__ __forceinline__ float value(float g, float u) { return g / (1.0f + expf(-g)) * u; }
+    static __device__ __forceinline__ void slopes(float g, float u, float dy, float &dg, float &du)
+    {
+        const float sig = 1.0f / (1.0f + expf(-g));
+        dg = dy * u * (sig * (1.0f + g * (1.0f - sig)));
+        du = dy * (g * sig);
+    }
+};
+struct Gelu {
+    static __device__ __forceinline__ float value(float g, float u)
+    {
+        float inner = 0.7978845608f * (g + 0.044715f * (g * g * g));
+        inner = fminf(fmaxf(inner, -15.0f), 15.0f);
+        return 0.5f * g * (1.0f + tanhf(inner)) * u;
+    }
+    static __device__ __forceinline__ void slopes(float g, float u, float dy, float &dg, float &du)
+    {
+        float inner = 0.7978845608f * (g + 0.044715f * (g * g * g));
+        inner = fminf(fmaxf(inner, -15.0f), 15.0f);
+        const float th = tanhf(inner);
+        const float gelu_g = 0.5f * g * (1.0f + th);
+        const float sech2 = 1.0f - th * th;
+        const float grad = 0.5f * (1.0f + th) + 0.5f * g * sech2 * 0.7978845608f * (1.0f + 3.0f * 0.044715f * g * g);
+        dg = dy * u * grad;
+        du = dy * gelu_g;
+    }
+};
 __global__ void silu_mul_rows_kernel(const float *gu, int inter, float *act, __half *act_h, size_t total)
 {
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const size_t m = e / inter, i = e % inter;
         const float g = gu[m * 2 * inter + i], u = gu[m * 2 * inter + inter + i];
-        const float v = g / (1.0f + expf(-g)) * u;
+        const float v = Silu::value(g, u);
         if (act) act[e] = v;
         if (act_h) act_h[e] = __float2half_rn(v);
     }
@@ -651,8 +749,8 @@ __global__ void silu_mul_bwd_rows_kernel(const float *d_act, const float *gu, in
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const size_t m = e / inter, i = e % inter;
         const float g = gu[m * 2 * inter + i], u = gu[m * 2 * inter + inter + i], dy = d_act[e];
-        const float sig = 1.0f / (1.0f + expf(-g));
-        const float dg = dy * u * (sig * (1.0f + g * (1.0f - sig))), du = dy * (g * sig);
+        float dg, du;
+        Silu::slopes(g, u, dy, dg, du);
         if (d_gu) { d_gu[m * 2 * inter + i] = dg; d_gu[m * 2 * inter + inter + i] = du; }
         if (d_gu_h) {
             d_gu_h[m * 2 * inter + i] = __float2half_rn(dg * h_scale);
@@ -668,9 +766,7 @@ __global__ void gelu_mul_rows_kernel(const float *gu, int inter, float *act, siz
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const size_t m = e / inter, i = e % inter;
         const float g = gu[m * 2 * inter + i], u = gu[m * 2 * inter + inter + i];
-        float inner = 0.7978845608f * (g + 0.044715f * (g * g * g));
-        inner = fminf(fmaxf(inner, -15.0f), 15.0f);
-        act[e] = 0.5f * g * (1.0f + tanhf(inner)) * u;
+        act[e] = Gelu::value(g, u);
     }
 }
 
@@ -679,14 +775,7 @@ __global__ void gelu_mul_bwd_rows_kernel(const float *d_act, const float *gu, in
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
         const size_t m = e / inter, i = e % inter;
         const float g = gu[m * 2 * inter + i], u = gu[m * 2 * inter + inter + i], dy = d_act[e];
-        float inner = 0.7978845608f * (g + 0.044715f * (g * g * g));
-        inner = fminf(fmaxf(inner, -15.0f), 15.0f);
-        const float th = tanhf(inner);
-        const float gelu_g = 0.5f * g * (1.0f + th);
-        const float sech2 = 1.0f - th * th;
-        const float grad = 0.5f * (1.0f + th) + 0.5f * g * sech2 * 0.7978845608f * (1.0f + 3.0f * 0.044715f * g * g);
-        d_gu[m * 2 * inter + i] = dy * u * grad;
-        d_gu[m * 2 * inter + inter + i] = dy * gelu_g;
+        Gelu::slopes(g, u, dy, d_gu[m * 2 * inter + i], d_gu[m * 2 * inter + inter + i]);
     }
 }
 
@@ -694,6 +783,43 @@ __global__ void gelu_mul_bwd_rows_kernel(const float *d_act, const float *gu, in
 __global__ void add_kernel(const float *a, const float *b, float *out, size_t n)
 {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) out[i] = a[i] + b[i];
+}
+
+// The gated activations in whole aligned quads, rows over blockIdx.y: no division, 16 bytes an access. The element forms above divide twice in 64
+// bits for every element: 512 x 9728 19 us (backward 21.4), 11 and 14 here.
+__device__ __forceinline__ void put_quad(float *at, const float (&v)[4]) { *reinterpret_cast<float4 *>(at) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void put_quad(__half *at, const float (&v)[4], float scale)
+{
+    const __half2 a = __halves2half2(__float2half_rn(v[0] * scale), __float2half_rn(v[1] * scale));
+    const __half2 b = __halves2half2(__float2half_rn(v[2] * scale), __float2half_rn(v[3] * scale));
+    *reinterpret_cast<uint2 *>(at) = make_uint2(*reinterpret_cast<const uint32_t *>(&a), *reinterpret_cast<const uint32_t *>(&b));
+}
+template <typename F>
+__global__ void __launch_bounds__(256) glu_quads_kernel(const float *gu, int inter, float *act, __half *act_h)
+{
+    const int i = 4 * (blockIdx.x * 256 + threadIdx.x);
+    if (i >= inter) return;
+    const size_t m = blockIdx.y;
+    const float4 g = *reinterpret_cast<const float4 *>(gu + m * 2 * inter + i), u = *reinterpret_cast<const float4 *>(gu + m * 2 * inter + inter + i);
+    const float v[4] = {F::value(g.x, u.x), F::value(g.y, u.y), F::value(g.z, u.z), F::value(g.w, u.w)};
+    if (act) put_quad(act + m * inter + i, v);
+    if (act_h) put_quad(act_h + m * inter + i, v, 1.0f);
+}
+template <typename F>
+__global__ void __launch_bounds__(256) glu_bwd_quads_kernel(const float *d_act, const float *gu, int inter, float *d_gu, __half *d_gu_h, float h_scale)
+{
+    const int i = 4 * (blockIdx.x * 256 + threadIdx.x);
+    if (i >= inter) return;
+    const size_t m = blockIdx.y, at = m * 2 * inter + i;
+    const float4 g = *reinterpret_cast<const float4 *>(gu + at), u = *reinterpret_cast<const float4 *>(gu + at + inter);
+    const float4 dy = *reinterpret_cast<const float4 *>(d_act + m * inter + i);
+    float dg[4], du[4];
+    F::slopes(g.x, u.x, dy.x, dg[0], du[0]);
+    F::slopes(g.y, u.y, dy.y, dg[1], du[1]);
+    F::slopes(g.z, u.z, dy.z, dg[2], du[2]);
+    F::slopes(g.w, u.w, dy.w, dg[3], du[3]);
+    if (d_gu) { put_quad(d_gu + at, dg); put_quad(d_gu + at + inter, du); }
+    if (d_gu_h) { put_quad(d_gu_h + at, dg, h_scale); put_quad(d_gu_h + at + inter, du, h_scale); }
 }
 
 // ---- LoRA up-projection added into the base projection -------------------------------------------
@@ -714,16 +840,24 @@ lora_add_kernel(float *y, long long ld, int col0, int n_cols, const float *mid, 
     __syncthreads();
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= n_cols) return;
-    float b[MAXR];
+    float b[MAXR], v[LORA_ROWS];
+    float *at = y + (size_t)m0 * ld + col0 + c;
 #pragma unroll
-    for (int r = 0; r < MAXR; ++r) b[r] = r < rank ? B[(size_t)c * rank + r] : 0.f;
+    for (int i = 0; i < LORA_ROWS; ++i) v[i] = m0 + i < rows ? at[i * ld] : 0.f;              // in flight under the row of B
+    if (rank == MAXR && (reinterpret_cast<uintptr_t>(B) & 15) == 0) {
+#pragma unroll
+        for (int r = 0; r < MAXR; r += 4) *reinterpret_cast<float4 *>(b + r) = *reinterpret_cast<const float4 *>(B + (size_t)c * MAXR + r);
+    } else {
+#pragma unroll
+        for (int r = 0; r < MAXR; ++r) b[r] = r < rank ? B[(size_t)c * rank + r] : 0.f;
+    }
 #pragma unroll
     for (int i = 0; i < LORA_ROWS; ++i) {
         if (m0 + i >= rows) break;
         float acc = 0.f;
 #pragma unroll
         for (int r = 0; r < MAXR; ++r) acc = fmaf(ms[i][r], b[r], acc);
-        y[(size_t)(m0 + i) * ld + col0 + c] += sc * acc;
+        at[i * ld] = v[i] + sc * acc;
     }
 }
 
@@ -1154,7 +1288,9 @@ extern "C" int b200_rms_norm_rows_h(const float *x, const float *gamma, float *o
     if (!x || !gamma || !out || rows <= 0 || dim <= 0) return B200_E_BADARG;
     cudaStream_t st = (cudaStream_t)stream;
     __half *oh = static_cast<__half *>(out_h);
-    if (dim >= 1024) rms_norm_rows_kernel<256><<<rows, 256, 0, st>>>(x, gamma, out, oh, rows, dim, eps);
+    if (dim >= 1024 && dim <= 2560) rms_norm_held_kernel<10><<<rows, 256, 0, st>>>(x, gamma, out, oh, dim, eps);
+    else if (dim >= 1024 && dim <= 4096) rms_norm_held_kernel<16><<<rows, 256, 0, st>>>(x, gamma, out, oh, dim, eps);
+    else if (dim >= 1024) rms_norm_rows_kernel<256><<<rows, 256, 0, st>>>(x, gamma, out, oh, rows, dim, eps);
     else rms_norm_rows_kernel<32><<<(rows + 7) / 8, 256, 0, st>>>(x, gamma, out, oh, rows, dim, eps);
     return done();
 }
@@ -1172,7 +1308,11 @@ extern "C" int b200_rms_norm_bwd_rows_h(const float *x, const float *dy, long lo
     if (!x || !dy || !gamma || !dx || rows <= 0 || dim <= 0 || dy_ld < dim) return B200_E_BADARG;
     cudaStream_t st = (cudaStream_t)stream;
     __half *dh = static_cast<__half *>(dx_h);
-    if (dim >= 1024)
+    if (dim >= 1024 && dim <= 2560)
+        rms_norm_bwd_held_kernel<10><<<rows, 256, 0, st>>>(x, dy, dy_ld, gamma, dx, dim, eps, accumulate, clamp, dh, h_scale);
+    else if (dim >= 1024 && dim <= 4096)
+        rms_norm_bwd_held_kernel<16><<<rows, 256, 0, st>>>(x, dy, dy_ld, gamma, dx, dim, eps, accumulate, clamp, dh, h_scale);
+    else if (dim >= 1024)
         rms_norm_bwd_rows_kernel<256><<<rows, 256, 0, st>>>(x, dy, dy_ld, gamma, dx, rows, dim, eps, accumulate, clamp, dh,
                                                             h_scale);
     else
@@ -1316,11 +1456,20 @@ extern "C" int b200_attn_train_bwd_tc(const float *d_out, const float *probs, co
     return attn_bwd<true>(d_out, probs, q, k, v, v_ld, n_seq, seq_len, n_q, n_kv, hd, scale, d_score, dqkv, ld, stream);
 }
 
+static bool whole_quads(int inter, int rows, const void *a, const void *b, const void *c)
+{
+    return (inter & 3) == 0 && rows <= 65535 && (((uintptr_t)a | (uintptr_t)b | (uintptr_t)c) & 15) == 0;
+}
+
 extern "C" int b200_silu_mul_rows_h(const float *gu, int rows, int inter, float *act, void *act_h, void *stream)
 {
     if (!gu || (!act && !act_h) || rows <= 0 || inter <= 0) return B200_E_BADARG;
     const size_t total = (size_t)rows * inter;
     const unsigned grid = (unsigned)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+    if (whole_quads(inter, rows, gu, act, act_h)) {
+        glu_quads_kernel<Silu><<<dim3((inter / 4 + 255) / 256, rows), 256, 0, (cudaStream_t)stream>>>(gu, inter, act, static_cast<__half *>(act_h));
+        return done();
+    }
     silu_mul_rows_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(gu, inter, act, static_cast<__half *>(act_h), total);
     return done();
 }
@@ -1337,6 +1486,10 @@ extern "C" int b200_silu_mul_bwd_rows_h(const float *d_act, const float *gu, int
     if (!d_act || !gu || (!d_gu && !d_gu_h) || rows <= 0 || inter <= 0) return B200_E_BADARG;
     const size_t total = (size_t)rows * inter;
     const unsigned grid = (unsigned)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+    if (whole_quads(inter, rows, gu, d_gu, d_gu_h) && ((uintptr_t)d_act & 15) == 0) {
+        glu_bwd_quads_kernel<Silu><<<dim3((inter / 4 + 255) / 256, rows), 256, 0, (cudaStream_t)stream>>>(d_act, gu, inter, d_gu, static_cast<__half *>(d_gu_h), h_scale);
+        return done();
+    }
     silu_mul_bwd_rows_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_act, gu, inter, d_gu, static_cast<__half *>(d_gu_h),
                                                                     h_scale, total);
     return done();
@@ -1354,6 +1507,10 @@ extern "C" int b200_gelu_mul_rows(const float *gu, int rows, int inter, float *a
     if (!gu || !act || rows <= 0 || inter <= 0) return B200_E_BADARG;
     const size_t total = (size_t)rows * inter;
     const unsigned grid = (unsigned)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+    if (whole_quads(inter, rows, gu, act, nullptr)) {
+        glu_quads_kernel<Gelu><<<dim3((inter / 4 + 255) / 256, rows), 256, 0, (cudaStream_t)stream>>>(gu, inter, act, nullptr);
+        return done();
+    }
     gelu_mul_rows_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(gu, inter, act, total);
     return done();
 }
@@ -1363,6 +1520,10 @@ extern "C" int b200_gelu_mul_bwd_rows(const float *d_act, const float *gu, int r
     if (!d_act || !gu || !d_gu || rows <= 0 || inter <= 0) return B200_E_BADARG;
     const size_t total = (size_t)rows * inter;
     const unsigned grid = (unsigned)((total + 255) / 256 < 148 * 16 ? (total + 255) / 256 : 148 * 16);
+    if (whole_quads(inter, rows, gu, d_gu, nullptr) && ((uintptr_t)d_act & 15) == 0) {
+        glu_bwd_quads_kernel<Gelu><<<dim3((inter / 4 + 255) / 256, rows), 256, 0, (cudaStream_t)stream>>>(d_act, gu, inter, d_gu, nullptr, 1.0f);
+        return done();
+    }
     gelu_mul_bwd_rows_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(d_act, gu, inter, d_gu, total);
     return done();
 }
