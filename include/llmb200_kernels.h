@@ -533,6 +533,7 @@ typedef struct b200_token_args {
     /* Tokens of one launch, one GPU and with_lm only (0 = 1): each takes the id that the one before it chose (or, inside the prompt, that
      * d_tokens holds). d_logits is left with those of the last. */
     int n_tokens;
+    int consumers;                                /* filled by b200_token_plan: consumer threads of a block */
 } b200_token_args;
 
 /* Fills the geometry (g[k].T ... direct_in), n_split limits and the launch shape for `n_blocks` blocks

@@ -118,7 +118,7 @@ class TokenArgs(C.Structure):
         ("spin_limit", C.c_int),
         ("d_trace", C.c_void_p),
         ("n_blocks", C.c_int), ("smem_bytes", C.c_int), ("scratch_floats", C.c_int), ("att_keys", C.c_int), ("l2_ahead_bytes", C.c_int),
-        ("counter_spin_limit", C.c_int), ("n_tokens", C.c_int),
+        ("counter_spin_limit", C.c_int), ("n_tokens", C.c_int), ("consumers", C.c_int),
     ]
 
 

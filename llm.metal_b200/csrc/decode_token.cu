@@ -37,18 +37,24 @@
 #include "../../include/llmb200_kernels.h"
 
 #include <stdio.h>
+#include <stdlib.h>
 
 extern unsigned long long g_b200_launches;
 
 namespace {
 
-constexpr int TK_NC = 640;                           // consumer threads
+// The kernel comes in two widths. 640 consumer threads keep up with HBM. Where a block's share of a layer is small, what every warp does once a
+// stage counts instead (480 instructions, five warps a scheduler): 320 of them (decode_token_narrow.cu) take half of that.
+#ifdef B200_TOKEN_NARROW
+constexpr int TK_NC = 320, ATT_T = 256;              // consumer threads, and those that work on an attention item
+#else
+constexpr int TK_NC = 640, ATT_T = 512;
+#endif
 constexpr int TK_THREADS = TK_NC + 32;               // + the producer warp
 constexpr int TK_NWARP = TK_NC / 32;
 constexpr int TK_SLOTS = 7;                          // 7 x 21.25 KB in flight per SM; the rest of shared memory holds activations
 constexpr int TK_SLOT_BYTES = 21760;                 // 170 * 128
 constexpr int TK_PART = 1024;                        // floats per partial-sum buffer (two buffers)
-constexpr int ATT_T = 512;                           // consumer threads that work on an attention item
 constexpr int TK_SPIN_DEFAULT = 1 << 20;
 constexpr int TK_TRACE_WORDS = 16;
 
@@ -99,9 +105,9 @@ __host__ __device__ inline Layout make_layout(int n_layers, int d_model, int scr
 // Scratch floats the attention stage needs besides its K/V staging area: rotated queries, new key and
 // value, the per-warp merge buffer and the new q/k/v rows as produced. The staging area (att_keys rows
 // of K and of V in binary16 = att_keys * hd floats) follows; the split-merge records reuse it.
-__host__ __device__ inline int attention_fixed_floats(int G, int hd)
+inline int attention_fixed_floats(int G, int hd, int att_t)
 {
-    const int wph = (ATT_T / G) / 32;
+    const int wph = (att_t / G) / 32;
     return G * hd + 2 * hd + G * wph * (hd + 2) + (G + 2) * hd;
 }
 
@@ -293,16 +299,17 @@ __device__ __forceinline__ float cons_sum(float v, float *red, int buf, int tid)
     float *r = red + buf * 32;
     if ((tid & 31) == 0) r[tid >> 5] = v;
     named_barrier(1, TK_NC);
-    // 20 partials, fetched with five 16-byte loads and added in warp order
+    // the partials, fetched with 16-byte loads and added in warp order
     float tot = 0.0f;
 #pragma unroll
     for (int w = 0; w < TK_NWARP; w += 4) {
         const float4 v4 = *reinterpret_cast<const float4 *>(r + w);
-        tot += v4.x; tot += v4.y; tot += v4.z; tot += v4.w;
+        tot += v4.x; tot += v4.y;
+        if (w + 2 < TK_NWARP) { tot += v4.z; tot += v4.w; }
     }
     return tot;
 }
-static_assert(TK_NWARP % 4 == 0, "cons_sum reads the warp partials four at a time");
+static_assert(TK_NWARP % 2 == 0, "cons_sum adds the warp partials in pairs");
 
 // Sum of the nwg warp partials of one row, in warp order; the loads go out four at a time.
 __device__ __forceinline__ float row_sum(const float *pr, int nwg)
@@ -1457,6 +1464,41 @@ decode_token_kernel(const __grid_constant__ b200_token_args p)
     }
 }
 
+// One launch: all blocks resident at once, they wait on one another.
+int launch_token(void (*kern)(const b200_token_args), const b200_token_args &a, cudaStream_t st)
+{
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, a.smem_bytes);
+    if (e != cudaSuccess) return (int)e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.n_blocks);
+    cfg.blockDim = dim3(TK_THREADS);
+    cfg.dynamicSmemBytes = a.smem_bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kern, a);
+}
+
+} // namespace
+
+#ifdef B200_TOKEN_NARROW
+int b200_tk_launch_narrow(const b200_token_args &a, cudaStream_t st)
+{
+    void (*kern)(const b200_token_args) =
+        a.wtype == B200_WT_Q8 ? (a.d_trace ? decode_token_kernel<B200_WT_Q8, true, false> : decode_token_kernel<B200_WT_Q8, false, false>)
+                              : (a.d_trace ? decode_token_kernel<B200_WT_F16, true, false> : decode_token_kernel<B200_WT_F16, false, false>);
+    return launch_token(kern, a, st);
+}
+#else
+int b200_tk_launch_narrow(const b200_token_args &a, cudaStream_t st);       // decode_token_narrow.cu
+
+namespace {
+
+constexpr int NARROW_CONSUMERS = 320;
+
 int g_tk_sm_count = 0;
 
 int tk_sm_count()
@@ -1470,7 +1512,7 @@ int tk_sm_count()
     return g_tk_sm_count;
 }
 
-int plan_stage(b200_stage_geom &g, int wtype, int n_blocks, int xin_floats)
+int plan_stage(b200_stage_geom &g, int wtype, int n_blocks, int xin_floats, int consumers)
 {
     if (g.rows <= 0 || g.cols <= 0 || g.row_stride <= 0 || (g.row_stride % 16)) return B200_E_BADARG;
     if (wtype == B200_WT_Q8 ? (g.cols % 32) : (g.cols % 8)) return B200_E_BADARG;
@@ -1479,14 +1521,14 @@ int plan_stage(b200_stage_geom &g, int wtype, int n_blocks, int xin_floats)
     if (g.rows % ralign) return B200_E_BADARG;
     const int E = wtype == B200_WT_Q8 ? 16 : 8;
     const int nsl = (g.cols + E - 1) / E;
-    // One 16-byte slice per thread up to 640 slices; two per thread beyond that, for binary16 rows only
+    // One 16-byte slice per thread as long as the threads suffice; two per thread beyond that, for binary16 rows only
     // (Q8_0 rows of more than 10240 columns are refused: the caller keeps its per-stage kernels).
-    g.spt = nsl <= TK_NC ? 1 : 2;
+    g.spt = nsl <= consumers ? 1 : 2;
     if (g.spt == 2 && wtype == B200_WT_Q8) return B200_E_TOOLARGE;
     g.T = (((nsl + g.spt - 1) / g.spt) + 31) / 32 * 32;
-    if (g.T > TK_NC) return B200_E_TOOLARGE;
-    g.NG = TK_NC / g.T;
-    if (g.NG > TK_NWARP) g.NG = TK_NWARP;
+    if (g.T > consumers) return B200_E_TOOLARGE;
+    g.NG = consumers / g.T;
+    if (g.NG > consumers / 32) g.NG = consumers / 32;
     // a chunk (one ring slot) holds rg rows for each group: as many as fit, a power of two up to 8
     // (2 with two slices per thread: the row partials of a chunk live in registers)
     const int fit = (int)(TK_SLOT_BYTES / g.row_stride);          // rows per slot
@@ -1522,6 +1564,22 @@ extern "C" int b200_token_plan(b200_token_args *a, int n_blocks)
     if (a->n_ranks < 1 || a->n_ranks > B200_MAX_PEERS || a->rank < 0 || a->rank >= a->n_ranks) return B200_E_BADARG;
     if (n_blocks <= 0) n_blocks = tk_sm_count();
     if (n_blocks <= 0) return B200_E_STATE;
+    // Consumer threads: half of them where every row has a thread per 16-byte slice then, and a layer is at most 96 KB of weights a block.
+    // us a token of four layers, wide and narrow, by those KB: Q8_0 21 86.5 / 77.0, 32 86.9 / 79.2, 77 89.2 / 85.0; F16 40 77.6 / 68.6, 60 78.8 / 70.4,
+    // 145 87.1 / 86.5; beyond, rows are what takes the time: Qwen3-4B Q8_0, 720, 156 and 180.
+    // Heads in groups of eight need a warp for each; LLMB200_TK_NARROW = 0 / 1 chooses, for experiments.
+    a->consumers = TK_NC;
+    if (a->n_ranks == 1 && G <= 4) {
+        const int E = a->wtype == B200_WT_Q8 ? 16 : 8;
+        long long bytes = 0;
+        bool fits = true;
+        for (int k = 0; k < B200_ST_KINDS; ++k) {
+            fits = fits && (a->g[k].cols + E - 1) / E <= NARROW_CONSUMERS;
+            if (k != B200_ST_LM) bytes += a->g[k].rows * a->g[k].row_stride;
+        }
+        const char *e = getenv("LLMB200_TK_NARROW");
+        if (fits && (e ? atoi(e) > 0 : bytes <= 96 * 1024LL * n_blocks)) a->consumers = NARROW_CONSUMERS;
+    }
     // sequence splits: items (kv head, split) must fit the blocks; at least 32 cache rows per split at full
     // length; by default few enough that the block merging a head reads little (18, or 9 for wide heads)
     int ns = a->n_split > 0 ? a->n_split : (a->hd > 128 ? 9 : 18);
@@ -1536,7 +1594,7 @@ extern "C" int b200_token_plan(b200_token_args *a, int n_blocks)
     const Layout fixed = make_layout(a->n_layers, a->d_model, 0);
     int scratch = (232448 - 128 - fixed.total) / 4;
     scratch -= scratch % 4;
-    const int att_fixed = attention_fixed_floats(G, a->hd);
+    const int att_fixed = attention_fixed_floats(G, a->hd, a->consumers == NARROW_CONSUMERS ? 256 : ATT_T);
     const int chunk_cap = (a->max_seq + ns - 1) / ns;
     int keys = scratch > att_fixed ? (scratch - att_fixed) / a->hd : 0;
     if (keys > chunk_cap) keys = chunk_cap;
@@ -1545,7 +1603,7 @@ extern "C" int b200_token_plan(b200_token_args *a, int n_blocks)
     int need = att_fixed + keys * a->hd;               // what is actually used: the rest is left to L1
     if (need < 2 * a->d_model) need = 2 * a->d_model;  // slot sums and the stage's norm weights
     for (int k = 0; k < B200_ST_KINDS; ++k) {
-        int rc = plan_stage(a->g[k], a->wtype, n_blocks, scratch);
+        int rc = plan_stage(a->g[k], a->wtype, n_blocks, scratch, a->consumers);
         if (rc) return rc;
         if ((k == B200_ST_O || k == B200_ST_DOWN) && !a->g[k].direct_in && a->g[k].cols > need) need = a->g[k].cols;
     }
@@ -1596,24 +1654,14 @@ extern "C" int b200_decode_token(const b200_token_args *ap, void *stream)
     const int sms = tk_sm_count();
     if (sms <= 0) return B200_E_STATE;
     if (ap->n_blocks > sms) return B200_E_TOOLARGE;    // all blocks must be resident at once
+    if (ap->consumers == NARROW_CONSUMERS) { ++g_b200_launches; return b200_tk_launch_narrow(*ap, (cudaStream_t)stream); }
     void (*kern)(const b200_token_args);
     const bool multi = ap->n_ranks > 1, trace = ap->d_trace != nullptr;
 #define TK_PICK(WT_) (multi ? (trace ? decode_token_kernel<WT_, true, true> : decode_token_kernel<WT_, false, true>) \
                             : (trace ? decode_token_kernel<WT_, true, false> : decode_token_kernel<WT_, false, false>))
     kern = ap->wtype == B200_WT_Q8 ? TK_PICK(B200_WT_Q8) : TK_PICK(B200_WT_F16);
 #undef TK_PICK
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ap->smem_bytes);
-    if (e != cudaSuccess) return (int)e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(ap->n_blocks);
-    cfg.blockDim = dim3(TK_THREADS);
-    cfg.dynamicSmemBytes = ap->smem_bytes;
-    cfg.stream = (cudaStream_t)stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;          // all blocks resident at once: they wait on one another
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     ++g_b200_launches;
-    return (int)cudaLaunchKernelEx(&cfg, kern, *ap);
+    return launch_token(kern, *ap, (cudaStream_t)stream);
 }
+#endif

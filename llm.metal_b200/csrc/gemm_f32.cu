@@ -373,7 +373,7 @@ extern "C" int b200_gemm_f32(const b200_gemm_args *a, void *stream)
     const long long tiles = (long long)((a->N + BN - 1) / BN) * ((a->M + BM - 1) / BM);
     int splits = 1, alone = 0;
     while (splits < 8 && tiles * splits * 2 <= 148 * 4 && a->K / (splits * 2) >= 128) splits *= 2;
-    if (splits > 1 && tiles * splits <= 148)
+    if (splits > 1 && tiles * splits <= 148 && a->K >= 512)
         for (int s = 2; s <= 8; ++s)
             if (a->K / s >= 128 && tiles * s <= resident[s]) { splits = s; alone = 1; }
     const int per = ((a->K + splits - 1) / splits + BK - 1) / BK * BK;

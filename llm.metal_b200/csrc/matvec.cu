@@ -112,6 +112,13 @@ extern "C" int b200_matvec(const b200_matvec_args *ap, void *stream)
     geo.slot_bytes = (unsigned)(((long long)rb * a.row_stride + 127) / 128 * 128);
     geo.NG = knobs().group_threads / geo.T;
     if (geo.NG > 8) geo.NG = 8;
+    int grid = a.grid;
+    if (grid <= 0) grid = sm_count();                // one block per SM
+    if (grid > units) grid = units;
+    geo.base = units / grid; geo.rem = units % grid;
+    // no group without a stage: at 256 columns a block has two to seven rows, one stage, and seven more groups would only meet it at barriers
+    const int stages = ((geo.base + (geo.rem > 0)) * ralign + rb - 1) / rb;
+    if (geo.NG > stages) geo.NG = stages;
     if (geo.NG < 1) geo.NG = 1;
     // Ring slots: a multiple of the group count, so that a slot is always consumed by the same group.
     // A group works through its stages in order, hence never waits on a slot whose previous phase is
@@ -126,10 +133,6 @@ extern "C" int b200_matvec(const b200_matvec_args *ap, void *stream)
     if (per_group < 1) per_group = 1;
     while (per_group > 1 && per_group * geo.NG > 12) --per_group;
     geo.nstage = per_group * geo.NG;
-    int grid = a.grid;
-    if (grid <= 0) grid = sm_count();                // one block per SM
-    if (grid > units) grid = units;
-    geo.base = units / grid; geo.rem = units % grid;
     cudaStream_t st = (cudaStream_t)stream;
     if (a.wtype == B200_WT_Q8)
         return spt == 1 ? launch_by_rows<B200_WT_Q8, 1>(a, geo, rb, grid, st) : launch_by_rows<B200_WT_Q8, 2>(a, geo, rb, grid, st);

@@ -101,7 +101,7 @@ rms_norm_bwd_rows_kernel(const float *x, const float *dy, long long dy_ld, const
 
 // The same sums in the same order for rows of up to 256 NV elements, a block per row: a thread's elements stay in registers, so that all of a row's
 // loads are in flight at once and nothing is read twice. 512 rows of 2560: 8.6 us and, backward, 12.1 where the row was read again after the sums;
-// 6.1 and 8.0 here.
+// 7.3 and 9.9 here.
 template <int NV>
 __global__ void __launch_bounds__(256)
 rms_norm_held_kernel(const float *x, const float *gamma, float *out, __half *out_h, int dim, float eps)
@@ -786,7 +786,7 @@ __global__ void add_kernel(const float *a, const float *b, float *out, size_t n)
 }
 
 // The gated activations in whole aligned quads, rows over blockIdx.y: no division, 16 bytes an access. The element forms above divide twice in 64
-// bits for every element: 512 x 9728 19 us (backward 21.4), 11 and 14 here.
+// bits for every element: 512 x 9728 19 us (backward 21.4), 9.4 and 11.8 here.
 __device__ __forceinline__ void put_quad(float *at, const float (&v)[4]) { *reinterpret_cast<float4 *>(at) = make_float4(v[0], v[1], v[2], v[3]); }
 __device__ __forceinline__ void put_quad(__half *at, const float (&v)[4], float scale)
 {

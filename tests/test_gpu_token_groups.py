@@ -31,7 +31,9 @@ def logits_after(lib, st, token, vocab):
 @pytest.mark.parametrize("fp16", [0, 1])
 @pytest.mark.parametrize("name,max_seq,P,G", [("tiny-qwen3", 64, 16, 2), ("tiny-qwen3", 64, 3, 14), ("tiny-qwen3", 64, 59, 32), ("tiny-qwen3", 2048, 600, 23),
                                               ("tiny-gemma3", 64, 1, 9), ("tiny-gemma3", 4096, 420, 61)])
-def test_groups_give_the_tokens_of_single_launches(lib, pkg, synth, fp16, name, max_seq, P, G):
+@pytest.mark.parametrize("narrow", ["0", "1"])
+def test_groups_give_the_tokens_of_single_launches(lib, pkg, synth, monkeypatch, fp16, name, max_seq, P, G, narrow):
+    monkeypatch.setenv("LLMB200_TK_NARROW", narrow)       # both widths of the kernel
     sp = pkg.spec(name, gamma_jitter=0.1)
     gemma = "gemma" in name
     model = (synth.llmb200_synth_gemma3 if gemma else synth.llmb200_synth_qwen3)(C.byref(sp), 8)
@@ -57,3 +59,25 @@ def test_groups_give_the_tokens_of_single_launches(lib, pkg, synth, fp16, name, 
     finally:
         lib.inference_state_free(st)
         (synth.llmb200_synth_free_gemma3 if gemma else synth.llmb200_synth_free_qwen3)(model)
+
+
+@pytest.mark.parametrize("fp16", [0, 1])
+@pytest.mark.parametrize("name", ["tiny-qwen3", "tiny-gemma3"])
+def test_widths_agree(lib, pkg, synth, monkeypatch, fp16, name):
+    """640 and 320 consumer threads: the same sums in another order. A key or value that this moves across a border of the binary16 cache moves by
+    2^-11 of itself, so that is what logits may move by."""
+    sp = pkg.spec(name, gamma_jitter=0.1)
+    gemma = "gemma" in name
+    model = (synth.llmb200_synth_gemma3 if gemma else synth.llmb200_synth_qwen3)(C.byref(sp), 8)
+    seen = []
+    try:
+        for narrow in "01":
+            monkeypatch.setenv("LLMB200_TK_NARROW", narrow)
+            st = (lib.inference_state_create_gemma3 if gemma else lib.inference_state_create)(model, 64, fp16)
+            assert st
+            seen.append([logits_after(lib, st, t, sp.vocab_size) for t in prompt_of(synth, 12, sp.vocab_size)])
+            lib.inference_state_free(st)
+    finally:
+        (synth.llmb200_synth_free_gemma3 if gemma else synth.llmb200_synth_free_qwen3)(model)
+    a, b = (np.array(x, dtype=np.float64) for x in seen)
+    assert not np.array_equal(a, b) and np.abs(a - b).max() <= 2 ** -11 * np.abs(a).max()
