@@ -116,9 +116,10 @@ extern "C" int b200_matvec(const b200_matvec_args *ap, void *stream)
     if (grid <= 0) grid = sm_count();                // one block per SM
     if (grid > units) grid = units;
     geo.base = units / grid; geo.rem = units % grid;
-    // no group without a stage: at 256 columns a block has two to seven rows, one stage, and seven more groups would only meet it at barriers
-    const int stages = ((geo.base + (geo.rem > 0)) * ralign + rb - 1) / rb;
-    if (geo.NG > stages) geo.NG = stages;
+    // no group without a stage, or without a quad of the input to assemble: at 256 columns a block has two to seven rows, one stage, and more groups
+    // would only meet it at barriers
+    const int stages = ((geo.base + (geo.rem > 0)) * ralign + rb - 1) / rb, quads = (a.cols / 4 + geo.T - 1) / geo.T;
+    if (geo.NG > stages && geo.NG > quads) geo.NG = stages > quads ? stages : quads;
     if (geo.NG < 1) geo.NG = 1;
     // Ring slots: a multiple of the group count, so that a slot is always consumed by the same group.
     // A group works through its stages in order, hence never waits on a slot whose previous phase is

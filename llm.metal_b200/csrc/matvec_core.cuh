@@ -90,19 +90,19 @@ struct NormWeights {
     __device__ __forceinline__ float4 get(int it, int e) const { return it == 0 ? first : ld4(at + e); }
 };
 
-// A thread's items of the vector in shared memory.
-#define B200_ITEMS(it, e) for (int it = 0, e = 4 * tid; e < cols; ++it, e += 4 * nC)
+// The vector that a block assembles: a thread's first item (four elements) in `q`, zeros where it has none, further ones (nC items apart; more than
+// 4 nC columns only) in shared memory, where the first one goes at the end.
+#define B200_FURTHER(it, e) for (int it = 1, e = 4 * (tid + nC); e < cols; ++it, e += 4 * nC)
 
 // RMS norm of the vector, `groups` equal consecutive parts of its first `dim` elements each by its own mean square; what follows them stays.
-__device__ __forceinline__ void norm_parts(float *xs, const NormWeights &gamma, int cols, int dim, int groups, float eps, float *red, int &turn,
+__device__ __forceinline__ void norm_parts(float4 &q, float *xs, const NormWeights &gamma, int cols, int dim, int groups, float eps, float *red, int &turn,
                                            int nC, int tid)
 {
     const int len = dim / groups;
     for (int k0 = 0; k0 < groups; k0 += 4) {                             // four parts a barrier
         float ss[4] = {};
-        B200_ITEMS(it, e) {
-            const float4 q = ld4(xs + e);
-            const float f[4] = {q.x, q.y, q.z, q.w};
+        auto squares_of = [&](const float4 &v, int e) {
+            const float f[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const int lo = (k0 + k) * len, hi = k0 + k < groups ? lo + len : lo;
@@ -110,13 +110,14 @@ __device__ __forceinline__ void norm_parts(float *xs, const NormWeights &gamma, 
                 for (int j = 0; j < 4; ++j)
                     if (e + j >= lo && e + j < hi) ss[k] = fmaf(f[j], f[j], ss[k]);
             }
-        }
+        };
+        squares_of(q, 4 * tid);
+        B200_FURTHER(it, e) squares_of(ld4(xs + e), e);
         block_sums<4>(ss, red, turn, nC, tid);
 #pragma unroll
         for (int k = 0; k < 4; ++k) ss[k] = 1.0f / sqrtf(ss[k] / (float)len + eps);
-        B200_ITEMS(it, e) {
-            const float4 q = ld4(xs + e), g = gamma.get(it, e);
-            float f[4] = {q.x, q.y, q.z, q.w};
+        auto normed = [&](const float4 &v, const float4 &g, int e) {
+            float f[4] = {v.x, v.y, v.z, v.w};
             const float w[4] = {g.x, g.y, g.z, g.w};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
@@ -125,35 +126,39 @@ __device__ __forceinline__ void norm_parts(float *xs, const NormWeights &gamma, 
                 for (int j = 0; j < 4; ++j)
                     if (e + j >= lo && e + j < hi) f[j] = w[j] * (f[j] * ss[k]);
             }
-            st4(xs + e, make_float4(f[0], f[1], f[2], f[3]));
-        }
+            return make_float4(f[0], f[1], f[2], f[3]);
+        };
+        q = normed(q, gamma.first, 4 * tid);
+        B200_FURTHER(it, e) st4(xs + e, normed(ld4(xs + e), gamma.get(it, e), e));
     }
 }
 
 // Layer norm (mean taken off, variance of the deviations, weight and bias) of the first `dim` elements; the
 // columns past them hold zeros before and after (their weight and bias are zero).
-__device__ __forceinline__ void layer_norm(float *xs, const NormWeights &gamma, const NormWeights &beta, int cols, int dim, float eps, float *red,
+__device__ __forceinline__ void layer_norm(float4 &q, float *xs, const NormWeights &gamma, const NormWeights &beta, int cols, int dim, float eps, float *red,
                                            int &turn, int nC, int tid)
 {
-    float sum[1] = {0.0f}, ss[1] = {0.0f};
-    B200_ITEMS(it, e) { const float4 q = ld4(xs + e); sum[0] += (q.x + q.y) + (q.z + q.w); }
+    float sum[1] = {(q.x + q.y) + (q.z + q.w)};
+    B200_FURTHER(it, e) { const float4 v = ld4(xs + e); sum[0] += (v.x + v.y) + (v.z + v.w); }
     block_sums<1>(sum, red, turn, nC, tid);
     const float mean = sum[0] / (float)dim;
-    B200_ITEMS(it, e) {
-        float4 q = ld4(xs + e);
-        if (e < dim) q.x -= mean;
-        if (e + 1 < dim) q.y -= mean;
-        if (e + 2 < dim) q.z -= mean;
-        if (e + 3 < dim) q.w -= mean;
-        st4(xs + e, q);
-        ss[0] = squares(q, ss[0]);
-    }
+    auto centred = [&](float4 v, int e) {
+        if (e < dim) v.x -= mean;
+        if (e + 1 < dim) v.y -= mean;
+        if (e + 2 < dim) v.z -= mean;
+        if (e + 3 < dim) v.w -= mean;
+        return v;
+    };
+    q = centred(q, 4 * tid);
+    float ss[1] = {squares(q, 0.0f)};
+    B200_FURTHER(it, e) { const float4 v = centred(ld4(xs + e), e); st4(xs + e, v); ss[0] = squares(v, ss[0]); }
     block_sums<1>(ss, red, turn, nC, tid);
     const float inv = 1.0f / sqrtf(ss[0] / (float)dim + eps);
-    B200_ITEMS(it, e) {
-        const float4 q = ld4(xs + e), g = gamma.get(it, e), b = beta.get(it, e);
-        st4(xs + e, make_float4(fmaf(g.x, q.x * inv, b.x), fmaf(g.y, q.y * inv, b.y), fmaf(g.z, q.z * inv, b.z), fmaf(g.w, q.w * inv, b.w)));
-    }
+    auto normed = [&](const float4 &v, const float4 &g, const float4 &b) {
+        return make_float4(fmaf(g.x, v.x * inv, b.x), fmaf(g.y, v.y * inv, b.y), fmaf(g.z, v.z * inv, b.z), fmaf(g.w, v.w * inv, b.w));
+    };
+    q = normed(q, gamma.first, beta.first);
+    B200_FURTHER(it, e) st4(xs + e, normed(ld4(xs + e), gamma.get(it, e), beta.get(it, e)));
 }
 
 // Which of the optional parts an instantiation holds (registers decide how well the row loop runs): FAM_PLAIN the parts
@@ -258,28 +263,29 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
 
     // ---------------- input assembly ----------------
     // Every SM needs the whole input vector. Where it has to be assembled (slot sums, norms) all consumers of a block do it together, four
-    // elements a thread, in shared memory: one read of the vector a block (all SMs read the same few KB of L2 at once, and every
+    // elements a thread: one read of the vector a block (all SMs read the same few KB of L2 at once, and every
     // extra reader queues behind the others), a barrier per sum.
     if (assemble) {
-        const bool store = blockIdx.x == 0;
+        const bool store = blockIdx.x == 0, mine = 4 * tid < cols;
+        const int e0 = 4 * tid, norm_dim = p.norm_dim > 0 ? p.norm_dim : cols, groups = p.norm_groups > 1 ? p.norm_groups : 1;
+        const float4 none = make_float4(0, 0, 0, 0);
+        float4 q = none;
         if (p.in_mode == B200_IN_VEC || (EXT && p.in_mode == B200_IN_POSTNORM)) {
-            B200_ITEMS(it, e) st4(xs + e, ld4(p.d_in_vec + e));
+            if (mine) q = ld4(p.d_in_vec + e0);
+            B200_FURTHER(it, e) st4(xs + e, ld4(p.d_in_vec + e));
             if constexpr (EXT) {
                 if (p.in_mode == B200_IN_POSTNORM) {
-                    float4 mix0 = make_float4(0, 0, 0, 0);               // fetched before the norm's sums
-                    if (p.d_mix_in && 4 * tid < cols) mix0 = ld4(p.d_mix_in + 4 * tid);
+                    const float4 mix0 = p.d_mix_in && mine ? ld4(p.d_mix_in + e0) : none;          // fetched before the norm's sums
                     const float coef = p.d_mix_in ? *p.d_mix_coef : 1.0f;
-                    norm_parts(xs, gp, cols, p.norm_dim > 0 ? p.norm_dim : cols, p.norm_groups > 1 ? p.norm_groups : 1, p.eps, red, turn, nC, tid);
-                    B200_ITEMS(it, e) {
-                        float4 q = ld4(xs + e);
-                        if (store && p.d_post_copy) st4(p.d_post_copy + e, q);
-                        if (p.d_mix_in) {
-                            const float4 m = it == 0 ? mix0 : ld4(p.d_mix_in + e);
-                            q = make_float4(fmaf(coef, q.x, m.x), fmaf(coef, q.y, m.y), fmaf(coef, q.z, m.z), fmaf(coef, q.w, m.w));
-                            st4(xs + e, q);
-                        }
-                        if (store && p.d_resid_out) st4(p.d_resid_out + e, q);
-                    }
+                    norm_parts(q, xs, gp, cols, norm_dim, groups, p.eps, red, turn, nC, tid);
+                    auto joined = [&](float4 v, const float4 &m, int e) {
+                        if (store && p.d_post_copy) st4(p.d_post_copy + e, v);
+                        if (p.d_mix_in) v = make_float4(fmaf(coef, v.x, m.x), fmaf(coef, v.y, m.y), fmaf(coef, v.z, m.z), fmaf(coef, v.w, m.w));
+                        if (store && p.d_resid_out) st4(p.d_resid_out + e, v);
+                        return v;
+                    };
+                    if (mine) q = joined(q, mix0, e0);
+                    B200_FURTHER(it, e) st4(xs + e, joined(ld4(xs + e), p.d_mix_in ? ld4(p.d_mix_in + e) : none, e));
                 }
             }
         } else {
@@ -288,65 +294,77 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
                 if (tok < 0 || tok >= p.emb_rows) tok = 0;      // never index outside the table
                 const float *er = p.d_emb + tok * (long long)cols;
                 const float *row = STR && p.d_emb_pos ? p.d_emb_pos + (long long)min(*p.d_pos, p.emb_pos_rows - 1) * cols : nullptr;
-                B200_ITEMS(it, e) {
-                    float4 q = ld4(er + e);
-                    q.x *= p.emb_scale; q.y *= p.emb_scale; q.z *= p.emb_scale; q.w *= p.emb_scale;
-                    if (row) { const float4 r = ld4(row + e); q.x += r.x; q.y += r.y; q.z += r.z; q.w += r.w; }
-                    st4(xs + e, q);
-                }
+                auto embedded = [&](int e) {
+                    float4 v = ld4(er + e);
+                    v.x *= p.emb_scale; v.y *= p.emb_scale; v.z *= p.emb_scale; v.w *= p.emb_scale;
+                    if (row) { const float4 r = ld4(row + e); v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w; }
+                    return v;
+                };
+                if (mine) q = embedded(e0);
+                B200_FURTHER(it, e) st4(xs + e, embedded(e));
                 if constexpr (STR) {
                     if (p.d_slot_norm_beta) {
                         NormWeights b;
                         b.fetch(p.d_slot_norm_beta, tid, cols);
-                        layer_norm(xs, gp, b, cols, p.norm_dim > 0 ? p.norm_dim : cols, p.eps, red, turn, nC, tid);
+                        layer_norm(q, xs, gp, b, cols, norm_dim, p.eps, red, turn, nC, tid);
                     }
                 }
             } else {
                 float ss[1] = {0.0f};
-                B200_ITEMS(it, e) {
-                    float4 a = make_float4(0, 0, 0, 0);
+                auto slots = [&](int e) {
+                    float4 a = none;
                     for (int k = 0; k < p.n_slots; ++k) {
                         // slots may be written by other GPUs: read them from L2, the point of coherence, never from L1
-                        const float4 q = __ldcg(reinterpret_cast<const float4 *>(p.d_slots + (long long)k * p.slot_stride + e));
-                        a.x += q.x; a.y += q.y; a.z += q.z; a.w += q.w;
+                        const float4 v = __ldcg(reinterpret_cast<const float4 *>(p.d_slots + (long long)k * p.slot_stride + e));
+                        a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
                     }
                     if (p.d_slot_norm_gamma) ss[0] = squares(a, ss[0]);
                     else { const float4 r = ld4(p.d_resid_in + e); a.x += r.x; a.y += r.y; a.z += r.z; a.w += r.w; }
-                    st4(xs + e, a);
-                }
+                    return a;
+                };
+                if (mine) q = slots(e0);
+                B200_FURTHER(it, e) st4(xs + e, slots(e));
                 if (p.d_slot_norm_gamma) {
+                    const float4 r0 = mine ? ld4(p.d_resid_in + e0) : none;
                     block_sums<1>(ss, red, turn, nC, tid);
                     const float inv = 1.0f / sqrtf(ss[0] / (float)cols + p.eps);
-                    B200_ITEMS(it, e) {
-                        const float4 a = ld4(xs + e), w = gp.get(it, e), r = ld4(p.d_resid_in + e);
-                        st4(xs + e, make_float4(r.x + w.x * a.x * inv, r.y + w.y * a.y * inv, r.z + w.z * a.z * inv, r.w + w.w * a.w * inv));
-                    }
+                    auto added = [&](const float4 &a, const float4 &w, const float4 &r) {
+                        return make_float4(r.x + w.x * a.x * inv, r.y + w.y * a.y * inv, r.z + w.z * a.z * inv, r.w + w.w * a.w * inv);
+                    };
+                    q = added(q, gp.first, r0);
+                    B200_FURTHER(it, e) st4(xs + e, added(ld4(xs + e), gp.get(it, e), ld4(p.d_resid_in + e)));
                 }
             }
-            if (store && p.d_resid_out) B200_ITEMS(it, e) st4(p.d_resid_out + e, ld4(xs + e));
+            if (store && p.d_resid_out) {
+                if (mine) st4(p.d_resid_out + e0, q);
+                B200_FURTHER(it, e) st4(p.d_resid_out + e, ld4(xs + e));
+            }
             if constexpr (STR) {
                 if (p.in_mode == B200_IN_EMBED && p.d_mix_coef) {    // what the first reader takes of the streams, all equal here
                     const float c = *p.d_mix_coef;
-                    B200_ITEMS(it, e) { const float4 q = ld4(xs + e); st4(xs + e, make_float4(c * q.x, c * q.y, c * q.z, c * q.w)); }
+                    q = make_float4(c * q.x, c * q.y, c * q.z, c * q.w);
+                    B200_FURTHER(it, e) { const float4 v = ld4(xs + e); st4(xs + e, make_float4(c * v.x, c * v.y, c * v.z, c * v.w)); }
                 }
             }
         }
         if (p.d_norm_gamma) {
-            if constexpr (STR) layer_norm(xs, gm, gb, cols, p.norm_dim > 0 ? p.norm_dim : cols, p.eps, red, turn, nC, tid);
-            else if constexpr (EXT)
-                norm_parts(xs, gm, cols, p.norm_dim > 0 ? p.norm_dim : cols, p.norm_groups > 1 ? p.norm_groups : 1, p.eps, red, turn, nC, tid);
+            if constexpr (STR) layer_norm(q, xs, gm, gb, cols, norm_dim, p.eps, red, turn, nC, tid);
+            else if constexpr (EXT) norm_parts(q, xs, gm, cols, norm_dim, groups, p.eps, red, turn, nC, tid);
             else {
-                float ss[1] = {0.0f};
-                B200_ITEMS(it, e) ss[0] = squares(ld4(xs + e), ss[0]);
+                float ss[1] = {squares(q, 0.0f)};
+                B200_FURTHER(it, e) ss[0] = squares(ld4(xs + e), ss[0]);
                 block_sums<1>(ss, red, turn, nC, tid);
                 const float inv = 1.0f / sqrtf(ss[0] / (float)cols + p.eps);
-                B200_ITEMS(it, e) {
-                    const float4 q = ld4(xs + e), w = gm.get(it, e);
-                    st4(xs + e, make_float4(w.x * q.x * inv, w.y * q.y * inv, w.z * q.z * inv, w.w * q.w * inv));
-                }
+                auto normed = [&](const float4 &v, const float4 &w) { return make_float4(w.x * v.x * inv, w.y * v.y * inv, w.z * v.z * inv, w.w * v.w * inv); };
+                q = normed(q, gm.first);
+                B200_FURTHER(it, e) st4(xs + e, normed(ld4(xs + e), gm.get(it, e)));
             }
         }
-        if (p.d_in_copy && store) B200_ITEMS(it, e) st4(p.d_in_copy + e, ld4(xs + e));
+        if (mine) st4(xs + e0, q);
+        if (p.d_in_copy && store) {
+            if (mine) st4(p.d_in_copy + e0, q);
+            B200_FURTHER(it, e) st4(p.d_in_copy + e, ld4(xs + e));
+        }
         named_barrier(1, nC);
     }
     float x[SPT][E];
@@ -366,7 +384,8 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
         qoff[s] = (uint32_t)(WT == B200_WT_Q8 ? c : WT == B200_WT_F32 ? 4 * c : 2 * c);
         soff[s] = (uint32_t)cols + (uint32_t)(c >> 5) * 2u;      // Q8: scales follow the quants of a row
     }
-    if (p.d_in_copy && !assemble && blockIdx.x == 0) B200_ITEMS(it, e) st4(p.d_in_copy + e, ld4(p.d_in_vec + e));
+    if (p.d_in_copy && !assemble && blockIdx.x == 0)
+        for (int e = 4 * tid; e < cols; e += 4 * nC) st4(p.d_in_copy + e, ld4(p.d_in_vec + e));
 
     // ---------------- consume the ring: group g takes stages g, g+NG, ... ----------------
     float best_v = -INFINITY;
