@@ -13,7 +13,7 @@
 // stores the result.
 // Bound by instructions and their latencies with 4 to 5 warps on a scheduler, not by HBM: the input vector is assembled by all consumers, a barrier
 // per sum, and nothing divides. A barrier and a one-warp epilogue per stage, 64-bit divisions, norms by one group: 0.28 ms a token of 41 such
-// launches (2048 wide, bfloat16), 0.25 now; fp32 210 us and 182. Two blocks of half the ring on an SM, so that the next launch's
+// launches (2048 wide, bfloat16), 0.24 now; fp32 210 us and 187. Two blocks of half the ring on an SM, so that the next launch's
 // weights arrive early: no gain (0.28), blocks of one launch then share SMs.
 //
 // Launched with programmatic dependent launch, a block of the NEXT kernel in
