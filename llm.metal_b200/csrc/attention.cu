@@ -24,9 +24,10 @@ extern unsigned long long g_b200_launches;
 
 namespace {
 
-// Threads of a block: 512, one block on an SM (114 registers); 256, two of them, where sequences and KV heads alone are more blocks than SMs: 32 sequences,
-// 8 KV heads of 128 and 130 - 250 keys took two waves of 512, and every block left its sums and its ticket in memory for itself to read
-// (4 layers of Qwen3-4B, 128 + 128 tokens: 60.2 ms, 53.6 now).
+// Threads of a block: 512, one block on an SM (114 registers); 256, two of them, where sequences and KV heads alone are more blocks than SMs and the
+// sequence is not split: 32 sequences, 8 KV heads of 128 and 130 - 250 keys took two waves of 512, and every block left its sums and its ticket in
+// memory for itself to read (4 layers of Qwen3-4B, 128 + 128 tokens: 60.3 ms, 53.6 now). A thread of 256 walks the keys of two
+// key lanes of 512, each with its own softmax, so that both forms add in the same order: a sequence gets the same bits in any company.
 constexpr int ATT_WIDE = 512, ATT_NARROW = 256, ATT_SMS = 148;
 
 __device__ __forceinline__ void halves8_to_float(const uint4 &u, float *f)
@@ -45,7 +46,8 @@ __device__ __forceinline__ void halves8_to_float(const uint4 &u, float *f)
 // walks keys kl, kl+KL, ... of the block's slice with its own online softmax (running max, sum and
 // output), so nothing is exchanged between threads while keys stream in; K and V rows are prefetched
 // two keys ahead, the first ones before the query is even normalised. At the end the key lanes of a
-// head are merged (shuffles inside a warp, shared memory across warps).
+// head are merged (shuffles inside a warp, shared memory across warps). Blocks of 256 threads: KL lanes of threads stand for
+// 2 KL key lanes, lane kl for kl and kl + KL, a slot of the prefetch each.
 template <int HD, int G, int ATT_THREADS>
 __global__ void __launch_bounds__(ATT_THREADS, ATT_WIDE / ATT_THREADS)
 attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_cap)
@@ -66,14 +68,17 @@ attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_ca
     constexpr int NV = DPT / 8;                 // 16-byte loads per K (and per V) row per thread
     constexpr int TPH = ATT_THREADS / G;        // threads per head group
     constexpr int KL = TPH / DLN;               // key lanes per head
+    constexpr int PF = 2;                       // keys in flight per thread
+    constexpr int NS = ATT_WIDE / ATT_THREADS;  // key lanes of a thread
     constexpr int WPH = TPH / 32;               // warps per head
+    constexpr int MPH = NS * WPH;               // merged records per head: those of 512 threads
     constexpr int HALF = HD / 2;
-    constexpr int PF = 2;                       // keys in flight per key lane
+    static_assert(NS == 1 || NS == PF, "a slot of the prefetch belongs to one key lane");
     extern __shared__ __align__(16) float sm[];
     float *q_s = sm;                            // [G][HD]
     float *k_new = q_s + G * HD;                // [HD]
     float *v_new = k_new + HD;                  // [HD]
-    float *mrg = v_new + HD;                    // [G][WPH][HD + 2] merge buffer across warps
+    float *mrg = v_new + HD;                    // [G][MPH][HD + 2] merge buffer across warps
     __shared__ int s_last;
     (void)chunk_cap;
 
@@ -156,8 +161,9 @@ attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_ca
             const int d = lane + 32 * j;
             float sn, cs;
             sincosf((float)pos * fr[j], &sn, &cs);
-            const float r0 = ra[j] * cs - rb[j] * sn;
-            const float r1 = ra[j] * sn + rb[j] * cs;
+            // (contractions written out here and below: the same in every instantiation)
+            const float r0 = fmaf(ra[j], cs, -__fmul_rn(rb[j], sn));
+            const float r1 = fmaf(ra[j], sn, __fmul_rn(rb[j], cs));
             if (is_k) {
                 const __half h0 = __float2half_rn(r0), h1 = __float2half_rn(r1);
                 k_new[d] = __half2float(h0); k_new[d + HALF] = __half2float(h1);
@@ -179,27 +185,30 @@ attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_ca
     __syncthreads();
 
     // ---- stream the keys of this lane: online softmax in registers ----
-    float q[DPT], acc[DPT];
+    float q[DPT], sums[NS][DPT], top[NS], den[NS];
 #pragma unroll
-    for (int e = 0; e < DPT; ++e) { q[e] = q_s[g * HD + dl * DPT + e]; acc[e] = 0.0f; }
+    for (int e = 0; e < DPT; ++e) q[e] = q_s[g * HD + dl * DPT + e];
+#pragma unroll
+    for (int u = 0; u < NS; ++u) {
+        top[u] = -INFINITY; den[u] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < DPT; ++e) sums[u][e] = 0.0f;
+    }
     const float scale = 1.0f / sqrtf((float)HD);
-    float m = -INFINITY, l = 0.0f;
-    auto one_key = [&](uint4 (&kq)[NV], uint4 (&vq)[NV], int j) {
+    auto one_key = [&](uint4 (&kq)[NV], uint4 (&vq)[NV], int j, float (&acc)[DPT], float &m, float &l) {
         const bool valid = j < j1;              // every lane of the warp runs the shuffles; only valid keys count
-        float kf[DPT], vf[DPT];
-        if (!valid) {
+        const bool fresh = j == pos;
+        float kf[DPT];
+        if (!valid || fresh) {
 #pragma unroll
-            for (int e = 0; e < DPT; ++e) { kf[e] = 0.0f; vf[e] = 0.0f; }
-        } else if (j == pos) {
-#pragma unroll
-            for (int e = 0; e < DPT; ++e) { kf[e] = k_new[dl * DPT + e]; vf[e] = v_new[dl * DPT + e]; }
+            for (int e = 0; e < DPT; ++e) kf[e] = valid ? k_new[dl * DPT + e] : 0.0f;
         } else {
 #pragma unroll
-            for (int i = 0; i < NV; ++i) {
-                halves8_to_float(kq[i], kf + 8 * i);
-                halves8_to_float(vq[i], vf + 8 * i);
-            }
+            for (int i = 0; i < NV; ++i) halves8_to_float(kq[i], kf + 8 * i);
         }
+        uint4 vu[NV];
+#pragma unroll
+        for (int i = 0; i < NV; ++i) vu[i] = vq[i];
         fetch(kq, vq, j + PF * KL);             // refill these registers with the key two rounds ahead
         float s = 0.0f;
 #pragma unroll
@@ -213,6 +222,14 @@ attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_ca
             const float mn = fmaxf(m, s);
             const float corr = expf(m - mn), pj = expf(s - mn);
             l = fmaf(l, corr, pj);
+            float vf[DPT];                      // unpacked this late: with both rows in fp32 two key lanes spill
+            if (fresh) {
+#pragma unroll
+                for (int e = 0; e < DPT; ++e) vf[e] = v_new[dl * DPT + e];
+            } else {
+#pragma unroll
+                for (int i = 0; i < NV; ++i) halves8_to_float(vu[i], vf + 8 * i);
+            }
 #pragma unroll
             for (int e = 0; e < DPT; ++e) acc[e] = fmaf(acc[e], corr, pj * vf[e]);
             m = mn;
@@ -221,37 +238,41 @@ attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_ca
     // same trip count for every key lane of the block, so that the warp-wide shuffles stay convergent
     const int rounds = (j1 - j0 + PF * KL - 1) / (PF * KL);
     for (int it = 0, j = j0 + kl; it < rounds; ++it, j += PF * KL) {
-        one_key(kq0, vq0, j);
-        one_key(kq1, vq1, j + KL);
+        one_key(kq0, vq0, j, sums[0], top[0], den[0]);
+        one_key(kq1, vq1, j + KL, sums[NS - 1], top[NS - 1], den[NS - 1]);
     }
 
     // ---- merge the key lanes of a head: inside the warp, then across the head's warps ----
-#pragma unroll
-    for (int o = DLN; o < 32; o <<= 1) {
-        const float mo = __shfl_xor_sync(0xffffffffu, m, o), lo = __shfl_xor_sync(0xffffffffu, l, o);
-        const float mn = fmaxf(m, mo);
-        const float ca = (m == -INFINITY) ? 0.0f : expf(m - mn), cb = (mo == -INFINITY) ? 0.0f : expf(mo - mn);
-        l = l * ca + lo * cb;
-#pragma unroll
-        for (int e = 0; e < DPT; ++e) acc[e] = acc[e] * ca + __shfl_xor_sync(0xffffffffu, acc[e], o) * cb;
-        m = mn;
-    }
     const int wh = r >> 5;                      // warp index inside the head group
-    if ((r & 31) < DLN) {                       // key lane 0 of each warp holds the warp's state
-        float *dst = mrg + ((size_t)g * WPH + wh) * (HD + 2);
 #pragma unroll
-        for (int e = 0; e < DPT; ++e) dst[dl * DPT + e] = acc[e];
-        if (dl == 0) { dst[HD] = m; dst[HD + 1] = l; }
+    for (int u = 0; u < NS; ++u) {
+        float (&acc)[DPT] = sums[u], &m = top[u], &l = den[u];
+#pragma unroll
+        for (int o = DLN; o < 32; o <<= 1) {
+            const float mo = __shfl_xor_sync(0xffffffffu, m, o), lo = __shfl_xor_sync(0xffffffffu, l, o);
+            const float mn = fmaxf(m, mo);
+            const float ca = (m == -INFINITY) ? 0.0f : expf(m - mn), cb = (mo == -INFINITY) ? 0.0f : expf(mo - mn);
+            l = fmaf(l, ca, __fmul_rn(lo, cb));
+#pragma unroll
+            for (int e = 0; e < DPT; ++e) acc[e] = fmaf(acc[e], ca, __fmul_rn(__shfl_xor_sync(0xffffffffu, acc[e], o), cb));
+            m = mn;
+        }
+        if ((r & 31) < DLN) {                   // key lane 0 of each warp holds the warp's state
+            float *dst = mrg + ((size_t)g * MPH + u * WPH + wh) * (HD + 2);
+#pragma unroll
+            for (int e = 0; e < DPT; ++e) dst[dl * DPT + e] = acc[e];
+            if (dl == 0) { dst[HD] = m; dst[HD + 1] = l; }
+        }
     }
     __syncthreads();
-    if (p.n_split == 1) {                       // nothing to merge with
+    if (NS > 1 || p.n_split == 1) {             // nothing to merge with
         for (int o = tid; o < G * HD; o += ATT_THREADS) {
-            const float *src = mrg + (size_t)(o / HD) * WPH * (HD + 2);
+            const float *src = mrg + (size_t)(o / HD) * MPH * (HD + 2);
             float M = -INFINITY, v = 0.0f, sum = 0.0f;
 #pragma unroll
-            for (int w = 0; w < WPH; ++w) M = fmaxf(M, src[w * (HD + 2) + HD]);
+            for (int w = 0; w < MPH; ++w) M = fmaxf(M, src[w * (HD + 2) + HD]);
 #pragma unroll
-            for (int w = 0; w < WPH; ++w) {
+            for (int w = 0; w < MPH; ++w) {
                 const float mw = src[w * (HD + 2) + HD];
                 const float c = (mw == -INFINITY) ? 0.0f : expf(mw - M);
                 v = fmaf(src[w * (HD + 2) + o % HD], c, v);
@@ -264,15 +285,15 @@ attn_decode_kernel(const __grid_constant__ b200_attn_args pa, const int chunk_ca
     // scratch: [n_q][n_split][HD + 2] = unnormalised output, running max, sum
     for (int o = tid; o < G * (HD + 2); o += ATT_THREADS) {
         const int gg = o / (HD + 2), d = o - gg * (HD + 2);
-        const float *src = mrg + (size_t)gg * WPH * (HD + 2);
+        const float *src = mrg + (size_t)gg * MPH * (HD + 2);
         float M = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < WPH; ++w) M = fmaxf(M, src[w * (HD + 2) + HD]);
+        for (int w = 0; w < MPH; ++w) M = fmaxf(M, src[w * (HD + 2) + HD]);
         float v = 0.0f;
         if (d == HD) v = M;
         else {
 #pragma unroll
-            for (int w = 0; w < WPH; ++w) {
+            for (int w = 0; w < MPH; ++w) {
                 const float mw = src[w * (HD + 2) + HD];
                 const float c = (mw == -INFINITY) ? 0.0f : expf(mw - M);
                 v = fmaf(src[w * (HD + 2) + (d == HD + 1 ? HD + 1 : d)], c, v);
@@ -367,8 +388,8 @@ template <int HD, int G, int ATT_THREADS>
 int launch_attn_as(const b200_attn_args &a, cudaStream_t st)
 {
     const int chunk_cap = (a.max_seq + a.n_split - 1) / a.n_split;
-    const int WPH = ATT_THREADS / G / 32;
-    size_t mrg_floats = (size_t)G * WPH * (HD + 2);
+    constexpr int MPH = ATT_WIDE / G / 32;
+    size_t mrg_floats = (size_t)G * MPH * (HD + 2);
     if (mrg_floats < (size_t)2 * G * a.n_split) mrg_floats = (size_t)2 * G * a.n_split;
     const size_t smem = ((size_t)G * HD + 2 * HD + mrg_floats) * sizeof(float);
     auto kern = attn_decode_kernel<HD, G, ATT_THREADS>;
@@ -395,7 +416,7 @@ template <int HD, int G>
 int launch_attn(const b200_attn_args &a, cudaStream_t st)
 {
     if constexpr (G < ATT_NARROW / 32)          // a warp per new row
-        if ((long long)a.n_split * a.n_kv * a.n_items > ATT_SMS) return launch_attn_as<HD, G, ATT_NARROW>(a, st);
+        if (a.n_split == 1 && (long long)a.n_kv * a.n_items > ATT_SMS) return launch_attn_as<HD, G, ATT_NARROW>(a, st);
     return launch_attn_as<HD, G, ATT_WIDE>(a, st);
 }
 

@@ -1,4 +1,4 @@
-"""Attention of a step over many sequences: more (sequence, KV head) pairs than SMs, one block to each, which stores its results itself.
+"""Attention of a step over many sequences: more (sequence, KV head) pairs than SMs, one block to each, which stores its results itself, or several that merge.
 
 Off float64 over the cache rows that the kernel left: a score is a sum of hd fp32 products, 2^-17 of the terms' magnitude at the worst (64 .. 256 terms, magnitude
 below 4 after the scale): 3e-5 of a weight, and so of the largest value."""
@@ -47,3 +47,28 @@ def test_many_sequences(lib, pkg, hd, G, B, n_kv, pos):
     want = (w @ v).view(B, n_q, hd)
     assert (out.double() - want).abs().max() <= 3e-5 * v.abs().max()
     assert (tickets == 0).all()
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("G", [1, 2, 4, 8])
+@pytest.mark.parametrize("n_split", [1, 2])
+@pytest.mark.parametrize("B,n_kv,pos", [(38, 4, 0), (19, 8, 7), (32, 8, 129), (150, 1, 131), (20, 8, 33)])
+def test_a_sequence_is_the_same_in_any_company(lib, pkg, hd, G, n_split, B, n_kv, pos):
+    """The step over all sequences and a step over each one alone: the same bits, whichever threads a block has, with one split and with several."""
+    max_seq, n_q = 160, G * n_kv
+    g = torch.Generator().manual_seed(hd + G + pos)
+    rows = n_q + 2 * n_kv
+    qkv = (2 * torch.randn(B, rows, hd, generator=g)).cuda()
+    freq = (1e4 ** (-2.0 * torch.arange(hd // 2) / hd)).float().cuda()
+    kc, vc = (torch.randn(B, n_kv, max_seq, hd, generator=g).half().cuda() for _ in range(2))
+    out = torch.full((2, B, n_q, hd), float("nan"), device="cuda")
+    scratch = torch.empty(B * lib.b200_attn_scratch_floats(n_q, hd, n_split), device="cuda")
+    tickets = torch.zeros(B * n_kv, dtype=torch.int32, device="cuda")
+    where = torch.tensor([pos], dtype=torch.int32, device="cuda")
+    for first, n, to in [(0, B, 0)] + [(b, 1, 1) for b in range(B)]:
+        a = pkg.AttnArgs(qkv[first].data_ptr(), 0, 0, freq.data_ptr(), kc[first].data_ptr(), vc[first].data_ptr(), out[to, first].data_ptr(), scratch.data_ptr(),
+                         tickets.data_ptr(), where.data_ptr(), n_q, n_kv, hd, max_seq, n_split, 1e-6, 0, n, rows * hd, n_kv * max_seq * hd, n_q * hd)
+        assert lib.b200_attn_decode(C.byref(a), None) == 0
+    torch.cuda.synchronize()
+    assert not torch.isnan(out).any()
+    assert torch.equal(out[0], out[1])
