@@ -66,13 +66,14 @@ __global__ void __launch_bounds__(256) rows_postnorm_kernel(const b200_rows_post
     }
 }
 
-// The same for rows of up to 1024 NQ columns in whole aligned quads whose parts are whole stretches of 128 (a warp's quads): a thread keeps its quads in
-// registers, all loads go out before the only barrier, a part's mean square is the sum of its stretches.
-// Bound by HBM: 2048 rows of 2048 with two earlier results move 0.1 GB; 38 us an element at a time with a barrier per part, 23 here.
+// The same sums in the same order for rows of up to 1024 NQ columns in whole aligned quads, one part or parts of whole 128s: a thread keeps its quads in registers,
+// all loads go out before the first of two barriers; between them each part is summed as a block of its own would (element k by thread k mod 256).
+// Bound by HBM: 2048 rows of 2048 in four parts with two earlier results move 0.13 GB; 49 us an element at a time with barriers per part, 31 here.
 template <int NQ>
 __global__ void __launch_bounds__(256) rows_postnorm_quads_kernel(const b200_rows_postnorm_args p)
 {
-    __shared__ float stretch[NQ * 8];
+    __shared__ __align__(16) float row[NQ * 1024];
+    __shared__ __align__(16) float sums[NQ * 64];
     const size_t m = blockIdx.x, at = m * p.ld;
     const float *x = p.x + at, *y = p.y + m * p.y_ld, *gate = p.gate + m * p.gate_ld;
     const int len = p.dim / p.groups;
@@ -94,9 +95,30 @@ __global__ void __launch_bounds__(256) rows_postnorm_quads_kernel(const b200_row
             }
             z[k] = make_float4(fmaf(p.alpha, v.x, sigmoid_f32(q.x + b.x) * w.x), fmaf(p.alpha, v.y, sigmoid_f32(q.y + b.y) * w.y),
                                fmaf(p.alpha, v.z, sigmoid_f32(q.z + b.z) * w.z), fmaf(p.alpha, v.w, sigmoid_f32(q.w + b.w) * w.w));
+            *reinterpret_cast<float4 *>(row + i) = z[k];
         }
-        const float ss = warp_sum(fmaf(z[k].w, z[k].w, fmaf(z[k].z, z[k].z, fmaf(z[k].y, z[k].y, z[k].x * z[k].x))));
-        if ((threadIdx.x & 31) == 0) stretch[k * 8 + (threadIdx.x >> 5)] = ss;
+    }
+    __syncthreads();
+    if (p.groups == 1) {
+        float ss = 0.0f;
+        for (int i = threadIdx.x; i < len; i += 256) ss = fmaf(row[i], row[i], ss);
+        ss = warp_sum(ss);
+        if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5] = ss;
+    } else for (int part = 0; part < p.groups; part += 4) {                  // four parts side by side
+        float ss[4] = {};
+        for (int i = threadIdx.x; i < len; i += 256)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float f = row[min(part + u, p.groups - 1) * len + i];
+                ss[u] = fmaf(f, f, ss[u]);
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) ss[u] += __shfl_xor_sync(0xffffffffu, ss[u], o);
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if ((threadIdx.x & 31) == u && part + u < p.groups) sums[(part + u) * 8 + (threadIdx.x >> 5)] = ss[u];
     }
     __syncthreads();
     __nv_bfloat16 *oh = static_cast<__nv_bfloat16 *>(p.out_h);
@@ -106,9 +128,8 @@ __global__ void __launch_bounds__(256) rows_postnorm_quads_kernel(const b200_row
         if (i >= p.ld) break;
         float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         if (i < p.dim) {
-            const int first = i / len * len / 128, last = (i / len * len + len + 127) / 128;
-            float ss = 0.0f;
-            for (int c = first; c < last; ++c) ss += stretch[c];
+            const float4 lo = *reinterpret_cast<const float4 *>(sums + i / len * 8), hi = *reinterpret_cast<const float4 *>(sums + i / len * 8 + 4);
+            const float ss = ((lo.x + hi.x) + (lo.z + hi.z)) + ((lo.y + hi.y) + (lo.w + hi.w));          // as warp_sum adds eight
             const float inv = 1.0f / sqrtf(ss / (float)len + p.eps);
             v = make_float4(g[k].x * (z[k].x * inv), g[k].y * (z[k].y * inv), g[k].z * (z[k].z * inv), g[k].w * (z[k].w * inv));
         }

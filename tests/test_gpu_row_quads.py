@@ -40,6 +40,30 @@ def test_postnorm(lib, pkg, dim, ld, groups, hist):
     assert not post[:, dim:].any() and not out[:, dim:].any() and not half[:, dim:].any()
 
 
+@pytest.mark.parametrize("dim,ld,groups", [(4, 4, 1), (132, 136, 1), (256, 256, 2), (1024, 1024, 8), (1028, 1040, 1), (1152, 1152, 3), (2048, 2048, 4), (2048, 2056, 16), (3072, 3072, 3),
+                                           (4096, 4096, 1), (4096, 4096, 32)])
+@pytest.mark.parametrize("hist", [0, 3])
+def test_postnorm_adds_in_one_order(lib, pkg, dim, ld, groups, hist):
+    """The same rows with one operand off the 16-byte boundary take the form of single elements: the same bits."""
+    g, M = torch.Generator().manual_seed(dim + hist), 5
+    x, gate = (torch.randn(M, ld, generator=g).cuda() for _ in range(2))
+    y = torch.zeros(2, M * ld + 8, device="cuda")
+    y[0, :M * ld] = torch.randn(M * ld, generator=g).cuda()
+    y[1, 1:M * ld + 1] = y[0, :M * ld]
+    bias, gamma = torch.randn(dim, generator=g).cuda(), torch.randn(dim, generator=g).cuda()
+    hs, coef = torch.randn(max(hist, 1), M, ld, generator=g).cuda(), torch.randn(hist + 1, generator=g).cuda()
+    post, out, half = (torch.full((2, M, ld), float("nan"), dtype=t, device="cuda") for t in (torch.float32, torch.float32, torch.bfloat16))
+    for k in range(2):
+        a = pkg.RowsPostnormArgs()
+        a.x, a.y, a.y_ld, a.gate, a.gate_ld, a.gate_bias, a.gamma = x.data_ptr(), y[k].data_ptr() + 4 * k, ld, gate.data_ptr(), ld, bias.data_ptr(), gamma.data_ptr()
+        a.alpha, a.eps, a.rows, a.dim, a.ld, a.groups, a.norm_out = 1.5, 1e-4, M, dim, ld, groups, post[k].data_ptr()
+        a.hist, a.hist_n, a.hist_stride, a.coef, a.out, a.out_h = hs.data_ptr(), hist, M * ld, coef.data_ptr(), out[k].data_ptr(), half[k].data_ptr()
+        assert y[k].data_ptr() % 16 == 0 and lib.b200_rows_postnorm(C.byref(a), None) == 0
+    torch.cuda.synchronize()
+    for t in (post, out, half):
+        assert not torch.isnan(t).any() and torch.equal(t[0], t[1])
+
+
 @pytest.mark.parametrize("wtype", [2, 3])
 @pytest.mark.parametrize("rows,inter,pad", [(1, 4, 0), (3, 1020, 4), (5, 1024, 0), (2, 1028, 8), (33, 6144, 0), (3, 10, 2), (3, 12, 6)])
 def test_gelu_mul(lib, wtype, rows, inter, pad):
