@@ -82,7 +82,7 @@ __device__ __forceinline__ float dot16_q8(const uint4 &w, const float *x)
 }
 
 // 16 int8 weights against a 16-element slice of the input held as three signed byte planes
-// (x = scale * (a + 256 b + 65536 c), see quantize_input in decode_token.cu): twelve dp4a, exact in
+// (x = scale * (a + 256 b + 65536 c), see quantize_input in decode_token_core.cuh): twelve dp4a, exact in
 // int32 (each sum stays below 2^18), then a + 256 b joined in integers and c joined in fp32.
 __device__ __forceinline__ float dot16_q8_planes(const uint4 &w, const uint4 &a, const uint4 &b, const uint4 &c)
 {
