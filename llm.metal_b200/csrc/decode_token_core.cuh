@@ -1315,6 +1315,12 @@ __device__ __forceinline__ void next_token(const b200_token_args &p, bool more)
         for (int u = 0; u < 4; ++u)
             if (u < cnt && better(v[u], __float_as_int(fi[u]), bv, bi)) { bv = v[u]; bi = __float_as_int(fi[u]); }
     }
+    if (more) {
+        // Each lane has seen flags of blocks of its own: its fence orders what they stored before their flags (rows of the cache) before what follows,
+        // and the barrier of the warp hands that on to lane 0, which issues the copies of the next token (shuffles order no memory).
+        __threadfence();
+        __syncwarp();
+    }
 #pragma unroll 1
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
@@ -1355,7 +1361,6 @@ __device__ __forceinline__ void next_token(const b200_token_args &p, bool more)
             sm.flags[3] = pos + 1;
             sm.flags[2] = sm.flags[2] + 1;
             sm.flags[6] = sm.flags[6] - 1;
-            __threadfence();
             asm volatile("fence.proxy.async;" ::: "memory");
         }
     }
