@@ -78,16 +78,22 @@ __device__ __forceinline__ void st4(float *p, float4 v) { *reinterpret_cast<floa
 __device__ __forceinline__ float squares(float4 v, float s) { return fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, fmaf(v.x, v.x, s)))); }
 
 // Weights of a norm for this thread's items (four elements each, nC items apart): those of the first one are fetched before the wait for the
-// previous kernel, they are constants.
+// previous kernel, they are constants. ANY: a vector that may start on any element (the norm of slot sums of Q8_0 and F16 products takes one).
+template <bool ANY = false>
 struct NormWeights {
     const float *at;
     float4 first;
+    __device__ __forceinline__ static float4 four(const float *p)
+    {
+        if (ANY && (reinterpret_cast<uintptr_t>(p) & 15)) return make_float4(p[0], p[1], p[2], p[3]);
+        return ld4(p);
+    }
     __device__ __forceinline__ void fetch(const float *p, int tid, int cols)
     {
         at = p;
-        first = p && 4 * tid < cols ? ld4(p + 4 * tid) : make_float4(0, 0, 0, 0);
+        first = p && 4 * tid < cols ? four(p + 4 * tid) : make_float4(0, 0, 0, 0);
     }
-    __device__ __forceinline__ float4 get(int it, int e) const { return it == 0 ? first : ld4(at + e); }
+    __device__ __forceinline__ float4 get(int it, int e) const { return it == 0 ? first : four(at + e); }
 };
 
 // The vector that a block assembles: a thread's first item (four elements) in `q`, zeros where it has none, further ones (nC items apart; more than
@@ -95,7 +101,7 @@ struct NormWeights {
 #define B200_FURTHER(it, e) for (int it = 1, e = 4 * (tid + nC); e < cols; ++it, e += 4 * nC)
 
 // RMS norm of the vector, `groups` equal consecutive parts of its first `dim` elements each by its own mean square; what follows them stays.
-__device__ __forceinline__ void norm_parts(float4 &q, float *xs, const NormWeights &gamma, int cols, int dim, int groups, float eps, float *red, int &turn,
+__device__ __forceinline__ void norm_parts(float4 &q, float *xs, const NormWeights<> &gamma, int cols, int dim, int groups, float eps, float *red, int &turn,
                                            int nC, int tid)
 {
     const int len = dim / groups;
@@ -135,7 +141,7 @@ __device__ __forceinline__ void norm_parts(float4 &q, float *xs, const NormWeigh
 
 // Layer norm (mean taken off, variance of the deviations, weight and bias) of the first `dim` elements; the
 // columns past them hold zeros before and after (their weight and bias are zero).
-__device__ __forceinline__ void layer_norm(float4 &q, float *xs, const NormWeights &gamma, const NormWeights &beta, int cols, int dim, float eps, float *red,
+__device__ __forceinline__ void layer_norm(float4 &q, float *xs, const NormWeights<> &gamma, const NormWeights<> &beta, int cols, int dim, float eps, float *red,
                                            int &turn, int nC, int tid)
 {
     float sum[1] = {(q.x + q.y) + (q.z + q.w)};
@@ -239,7 +245,8 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
 
     // The norm weights are constants: their round trip is taken before the wait for the previous
     // kernel, not after it.
-    NormWeights gm, gp, gb;
+    NormWeights<> gm, gb;
+    NormWeights<FAM == FAM_PLAIN> gp;
     gm.fetch(p.d_norm_gamma, tid, cols);
     gp.fetch(p.d_slot_norm_gamma, tid, cols);                        // of a post-norm input, of normalised slot sums, or of embeddings
     if constexpr (STR) {
@@ -304,7 +311,7 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
                 B200_FURTHER(it, e) st4(xs + e, embedded(e));
                 if constexpr (STR) {
                     if (p.d_slot_norm_beta) {
-                        NormWeights b;
+                        NormWeights<> b;
                         b.fetch(p.d_slot_norm_beta, tid, cols);
                         layer_norm(q, xs, gp, b, cols, norm_dim, p.eps, red, turn, nC, tid);
                     }
