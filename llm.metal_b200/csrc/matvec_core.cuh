@@ -13,7 +13,7 @@
 // stores the result.
 // Bound by instructions and their latencies with 4 to 5 warps on a scheduler, not by HBM: the input vector is assembled by all consumers, a barrier
 // per sum, and nothing divides. A barrier and a one-warp epilogue per stage, 64-bit divisions, norms by one group: 0.28 ms a token of 41 such
-// launches (2048 wide, bfloat16), 0.24 now; fp32 210 us and 187. Two blocks of half the ring on an SM, so that the next launch's
+// launches (2048 wide, bfloat16), 0.24 now; fp32 210 us and 175. Two blocks of half the ring on an SM, so that the next launch's
 // weights arrive early: no gain (0.28), blocks of one launch then share SMs.
 //
 // Launched with programmatic dependent launch, a block of the NEXT kernel in
@@ -97,11 +97,15 @@ struct NormWeights {
 };
 
 // The vector that a block assembles: a thread's first item (four elements) in `q`, zeros where it has none, further ones (nC items apart; more than
-// 4 nC columns only) in shared memory, where the first one goes at the end.
-#define B200_FURTHER(it, e) for (int it = 1, e = 4 * (tid + nC); e < cols; ++it, e += 4 * nC)
+// 4 nC columns only) in shared memory, where the first one goes at the end. FAM_POST keeps the first one there too: a second copy of the norms by
+// parts, for the register, is code that every launch fetches and few warps share (two layers of 2048, fp32, 64 ids: 12.2 ms with it, 11.4 without; layer
+// norms of streams the other way round: four layers of 256, bfloat16, 40 ids 5.24 ms with the register, 5.58 without).
+#define B200_ITEMS_FROM(first, it, e) for (int it = first, e = 4 * (tid + first * nC); e < cols; ++it, e += 4 * nC)
+#define B200_ITEMS(it, e) B200_ITEMS_FROM(0, it, e)
+#define B200_FURTHER(it, e) B200_ITEMS_FROM(HELD, it, e)             // HELD: 1 where the first one is in q
 
 // RMS norm of the vector, `groups` equal consecutive parts of its first `dim` elements each by its own mean square; what follows them stays.
-__device__ __forceinline__ void norm_parts(float4 &q, float *xs, const NormWeights<> &gamma, int cols, int dim, int groups, float eps, float *red, int &turn,
+__device__ __forceinline__ void norm_parts(float *xs, const NormWeights<> &gamma, int cols, int dim, int groups, float eps, float *red, int &turn,
                                            int nC, int tid)
 {
     const int len = dim / groups;
@@ -117,8 +121,7 @@ __device__ __forceinline__ void norm_parts(float4 &q, float *xs, const NormWeigh
                     if (e + j >= lo && e + j < hi) ss[k] = fmaf(f[j], f[j], ss[k]);
             }
         };
-        squares_of(q, 4 * tid);
-        B200_FURTHER(it, e) squares_of(ld4(xs + e), e);
+        B200_ITEMS(it, e) squares_of(ld4(xs + e), e);
         block_sums<4>(ss, red, turn, nC, tid);
 #pragma unroll
         for (int k = 0; k < 4; ++k) ss[k] = 1.0f / sqrtf(ss[k] / (float)len + eps);
@@ -134,8 +137,7 @@ __device__ __forceinline__ void norm_parts(float4 &q, float *xs, const NormWeigh
             }
             return make_float4(f[0], f[1], f[2], f[3]);
         };
-        q = normed(q, gamma.first, 4 * tid);
-        B200_FURTHER(it, e) st4(xs + e, normed(ld4(xs + e), gamma.get(it, e), e));
+        B200_ITEMS(it, e) st4(xs + e, normed(ld4(xs + e), gamma.get(it, e), e));
     }
 }
 
@@ -144,6 +146,7 @@ __device__ __forceinline__ void norm_parts(float4 &q, float *xs, const NormWeigh
 __device__ __forceinline__ void layer_norm(float4 &q, float *xs, const NormWeights<> &gamma, const NormWeights<> &beta, int cols, int dim, float eps, float *red,
                                            int &turn, int nC, int tid)
 {
+    constexpr int HELD = 1;
     float sum[1] = {(q.x + q.y) + (q.z + q.w)};
     B200_FURTHER(it, e) { const float4 v = ld4(xs + e); sum[0] += (v.x + v.y) + (v.z + v.w); }
     block_sums<1>(sum, red, turn, nC, tid);
@@ -178,6 +181,7 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
 {
     constexpr int E = (WT == B200_WT_Q8) ? 16 : (WT == B200_WT_F32) ? 4 : 8;       // elements per 16-byte slice
     constexpr bool EXT = FAM == FAM_POST, STR = FAM == FAM_STREAMS;
+    constexpr int HELD = EXT ? 0 : 1;                                   // see B200_FURTHER
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int T = geo.T, NG = geo.NG, nstage = geo.nstage, nwg = T >> 5, nwgp = nwg | 1, nC = NG * T;
     unsigned char *ring = smem_raw;
@@ -278,21 +282,23 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
         const float4 none = make_float4(0, 0, 0, 0);
         float4 q = none;
         if (p.in_mode == B200_IN_VEC || (EXT && p.in_mode == B200_IN_POSTNORM)) {
-            if (mine) q = ld4(p.d_in_vec + e0);
+            if (HELD && mine) q = ld4(p.d_in_vec + e0);
             B200_FURTHER(it, e) st4(xs + e, ld4(p.d_in_vec + e));
             if constexpr (EXT) {
                 if (p.in_mode == B200_IN_POSTNORM) {
                     const float4 mix0 = p.d_mix_in && mine ? ld4(p.d_mix_in + e0) : none;          // fetched before the norm's sums
                     const float coef = p.d_mix_in ? *p.d_mix_coef : 1.0f;
-                    norm_parts(q, xs, gp, cols, norm_dim, groups, p.eps, red, turn, nC, tid);
-                    auto joined = [&](float4 v, const float4 &m, int e) {
+                    norm_parts(xs, gp, cols, norm_dim, groups, p.eps, red, turn, nC, tid);
+                    B200_ITEMS(it, e) {
+                        float4 v = ld4(xs + e);
                         if (store && p.d_post_copy) st4(p.d_post_copy + e, v);
-                        if (p.d_mix_in) v = make_float4(fmaf(coef, v.x, m.x), fmaf(coef, v.y, m.y), fmaf(coef, v.z, m.z), fmaf(coef, v.w, m.w));
+                        if (p.d_mix_in) {
+                            const float4 m = it == 0 ? mix0 : ld4(p.d_mix_in + e);
+                            v = make_float4(fmaf(coef, v.x, m.x), fmaf(coef, v.y, m.y), fmaf(coef, v.z, m.z), fmaf(coef, v.w, m.w));
+                            st4(xs + e, v);
+                        }
                         if (store && p.d_resid_out) st4(p.d_resid_out + e, v);
-                        return v;
-                    };
-                    if (mine) q = joined(q, mix0, e0);
-                    B200_FURTHER(it, e) st4(xs + e, joined(ld4(xs + e), p.d_mix_in ? ld4(p.d_mix_in + e) : none, e));
+                    }
                 }
             }
         } else {
@@ -307,7 +313,7 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
                     if (row) { const float4 r = ld4(row + e); v.x += r.x; v.y += r.y; v.z += r.z; v.w += r.w; }
                     return v;
                 };
-                if (mine) q = embedded(e0);
+                if (HELD && mine) q = embedded(e0);
                 B200_FURTHER(it, e) st4(xs + e, embedded(e));
                 if constexpr (STR) {
                     if (p.d_slot_norm_beta) {
@@ -325,13 +331,13 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
                         const float4 v = __ldcg(reinterpret_cast<const float4 *>(p.d_slots + (long long)k * p.slot_stride + e));
                         a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
                     }
-                    if (p.d_slot_norm_gamma) ss[0] = squares(a, ss[0]);
+                    if (FAM == FAM_PLAIN && p.d_slot_norm_gamma) ss[0] = squares(a, ss[0]);
                     else { const float4 r = ld4(p.d_resid_in + e); a.x += r.x; a.y += r.y; a.z += r.z; a.w += r.w; }
                     return a;
                 };
-                if (mine) q = slots(e0);
+                if (HELD && mine) q = slots(e0);
                 B200_FURTHER(it, e) st4(xs + e, slots(e));
-                if (p.d_slot_norm_gamma) {
+                if constexpr (FAM == FAM_PLAIN) if (p.d_slot_norm_gamma) {
                     const float4 r0 = mine ? ld4(p.d_resid_in + e0) : none;
                     block_sums<1>(ss, red, turn, nC, tid);
                     const float inv = 1.0f / sqrtf(ss[0] / (float)cols + p.eps);
@@ -343,7 +349,7 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
                 }
             }
             if (store && p.d_resid_out) {
-                if (mine) st4(p.d_resid_out + e0, q);
+                if (HELD && mine) st4(p.d_resid_out + e0, q);
                 B200_FURTHER(it, e) st4(p.d_resid_out + e, ld4(xs + e));
             }
             if constexpr (STR) {
@@ -356,7 +362,7 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
         }
         if (p.d_norm_gamma) {
             if constexpr (STR) layer_norm(q, xs, gm, gb, cols, norm_dim, p.eps, red, turn, nC, tid);
-            else if constexpr (EXT) norm_parts(q, xs, gm, cols, norm_dim, groups, p.eps, red, turn, nC, tid);
+            else if constexpr (EXT) norm_parts(xs, gm, cols, norm_dim, groups, p.eps, red, turn, nC, tid);
             else {
                 float ss[1] = {squares(q, 0.0f)};
                 B200_FURTHER(it, e) ss[0] = squares(ld4(xs + e), ss[0]);
@@ -367,11 +373,8 @@ matvec_kernel(const __grid_constant__ b200_matvec_args p, const Geometry geo)
                 B200_FURTHER(it, e) st4(xs + e, normed(ld4(xs + e), gm.get(it, e)));
             }
         }
-        if (mine) st4(xs + e0, q);
-        if (p.d_in_copy && store) {
-            if (mine) st4(p.d_in_copy + e0, q);
-            B200_FURTHER(it, e) st4(p.d_in_copy + e, ld4(xs + e));
-        }
+        if (HELD && mine) st4(xs + e0, q);
+        if (p.d_in_copy && store) B200_ITEMS(it, e) st4(p.d_in_copy + e, ld4(xs + e));
         named_barrier(1, nC);
     }
     float x[SPT][E];
