@@ -6,10 +6,10 @@
 // half of the rows of B, and the tensor cores read the other half from the neighbour's shared memory, so a 256-wide
 // tile wants 64. Persistent: a pair walks its tiles, two accumulators in tensor memory take turns, and the epilogue of one
 // tile runs under the products of the next.
-// Results leave through shared memory, whole lines of four rows a store: stored by the thread that read the row, 16 bytes in 32 lines, they cost 74
-// clocks a column that nothing hides in a product of one wave. Chains of 20, before that (and with a division per ring step in the
-// issuing lane) and now: 512 x 2560 x 9728 45 us and 31, 512 x 6144 x 2560 24 and 19.5, 512 x 2560 x 4096 27 and 24, 2048 x 2560 x 4096 48 and 37,
-// 2048 x 12288 x 2048 90 and 82 (1260 TFLOP/s); 512 x 4096 x 512 10.2 and 11.2.
+// Results leave through shared memory (store_block), and the issuing lane counts its places in the ring: stored by the thread that read the row, 16
+// bytes in 32 lines, and with a division per ring step, chains of 20 took: 512 x 6144 x 2560 23.7 us, 17.5 now (with an addend 33.6 and 18.9),
+// 512 x 2560 x 4096 27.7 and 24.3, 2048 x 2560 x 4096 47.3 and 38.1, 2048 x 12288 x 2048 94 and 85, 512 x 4096 x 512 12.4 and 12.4; bfloat16
+// results 777 x 9728 x 512 18.0 and 14.7 (24 with 8 bytes a store).
 //
 // Pair, per SM: warp 0 loads with TMA (both SMs' copies complete on the barrier of the first, the leader), one lane of the
 // leader's warp 1 issues the products for both and commits to both, warps 2-5 store their SM's 128 rows. Products of few tiles are
@@ -22,6 +22,8 @@
 
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 extern unsigned long long g_b200_launches;
 
 namespace {
@@ -31,7 +33,6 @@ constexpr int KB = 64;                   // k of a 128-byte operand row
 constexpr int PAIR_THREADS = 192;
 constexpr int PAIR_SLOTS = 8;
 constexpr int KSUB = 2;                  // operand rows per slot: half the hand-overs
-constexpr int STAGE_PITCH = 36;          // floats between the rows of a block on its way out: 16-byte accesses of eight rows or columns meet 32 banks
 constexpr uint32_t A_TILE = SM_ROWS * KB * 2;
 struct PairArgs {
     float *C; long long ldc;
@@ -77,58 +78,89 @@ __device__ __forceinline__ void arrive_at(uint32_t bar)
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
-// 32 rows (row0 on, one a lane in r) by 32 columns (n on) of a tile, by one warp: through shared memory, so that a store covers whole lines of four rows
-// and not 16 bytes of 32. The same for what is added.
-__device__ __forceinline__ void store_block(const PairArgs &p, float *stage, int row0, int n, int n_end, const uint32_t *r, bool vec)
+// What is stored of a sum: alpha times it, and then what is added (two roundings in every path).
+__device__ __forceinline__ float scaled(const PairArgs &p, float v) { return __fmul_rn(p.alpha, v); }
+
+// 32 rows (row0 on, one a lane in r) by 32 columns (n on) of a tile, by one warp: through 2 KB of shared memory, so that a store covers 64 bytes of
+// eight rows and not 16 of 32, and what is added is read so; fp32 in two halves of 16 columns, bfloat16 packed first. The 16-byte pieces of a row are
+// exchanged by the row's number: eight lanes meet all banks both ways. The unusual paths are loops, every launch fetches this code anew. Against whole
+// lines of four rows (4 KB) it leaves a ring slot more to tiles 176 wide, and 600 products of M 192 .. 2048, N 512 .. 12288, K 256 .. 9728 take
+// 1 % (C), 3 % (C + R) less.
+__device__ __forceinline__ void store_block(const PairArgs &p, uint4 *stage, int row0, int n, int n_end, const uint32_t *r, bool vec)
 {
-    const int lane = threadIdx.x & 31, c = (lane & 7) * 4, r0 = lane >> 3;
-    n += c;
-    const bool whole = n + 4 <= n_end;
-    float4 add[8];
-    if (!p.Ch && p.R && vec) {
+    const int lane = threadIdx.x & 31, c = lane & 3, r0 = lane >> 2;
+    auto piece = [&](int row, int k) { return stage + row * 4 + (k ^ ((row >> 1) & 3)); };
+    if (p.Ch) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            add[i] = whole && row0 + 4 * i + r0 < p.M ? __ldcg(reinterpret_cast<const float4 *>(p.R + (long long)(row0 + 4 * i + r0) * p.ldr + n))
-                                                      : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < 4; ++k) {
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float x = __uint_as_float(r[8 * k + 2 * j]), y = __uint_as_float(r[8 * k + 2 * j + 1]);
+                const __nv_bfloat162 h = __floats2bfloat162_rn(p.alpha * (p.relu2 ? act_relu2(x) : x), p.alpha * (p.relu2 ? act_relu2(y) : y));
+                w[j] = *reinterpret_cast<const uint32_t *>(&h);
+            }
+            *piece(lane, k) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        __syncwarp();
+        n += 8 * c;
+        __nv_bfloat16 *h = p.Ch + (long long)(row0 + r0) * p.ldch + n;
+        if (n + 8 <= n_end) {
+            uint4 v[4];                                      // all of them before the first store, which might alias
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = *piece(8 * i + r0, c);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (row0 + 8 * i + r0 < p.M) *reinterpret_cast<uint4 *>(h + (long long)(8 * i) * p.ldch) = v[i];
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < 4 && row0 + 8 * i + r0 < p.M; ++i)
+#pragma unroll 1
+                for (int j = 0; n + j < n_end; ++j) h[(long long)(8 * i) * p.ldch + j] = reinterpret_cast<const __nv_bfloat16 *>(piece(8 * i + r0, c))[j];
+        }
+        __syncwarp();
+        return;
+    }
+    n += 4 * c;
+    float4 add[8];
+    if (p.R && vec) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int row = row0 + 8 * (k & 3) + r0, col = n + 16 * (k >> 2);
+            add[k] = row < p.M && col + 4 <= n_end ? __ldcg(reinterpret_cast<const float4 *>(p.R + (long long)row * p.ldr + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     }
 #pragma unroll
-    for (int j = 0; j < 32; j += 4)
-        *reinterpret_cast<float4 *>(stage + lane * STAGE_PITCH + j) =
-            make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]), __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-    __syncwarp();
+    for (int half = 0; half < 2; ++half, n += 16) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int row = row0 + 4 * i + r0;
-        float4 v = *reinterpret_cast<const float4 *>(stage + (4 * i + r0) * STAGE_PITCH + c);
-        if (row >= p.M || n >= n_end) continue;
-        if (p.Ch) {
-            __nv_bfloat16 *h = p.Ch + (long long)row * p.ldch + n;
-            float f[4] = {v.x, v.y, v.z, v.w};
+        for (int k = 0; k < 4; ++k) *piece(lane, k) = make_uint4(r[16 * half + 4 * k], r[16 * half + 4 * k + 1], r[16 * half + 4 * k + 2], r[16 * half + 4 * k + 3]);
+        __syncwarp();
+        if (vec && n + 4 <= n_end) {
+            float4 v[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) f[j] = p.alpha * (p.relu2 ? act_relu2(f[j]) : f[j]);
-            if (whole) {
-                const __nv_bfloat162 lo = __floats2bfloat162_rn(f[0], f[1]), hi = __floats2bfloat162_rn(f[2], f[3]);
-                *reinterpret_cast<uint2 *>(h) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
-            } else {
+            for (int i = 0; i < 4; ++i) v[i] = *reinterpret_cast<const float4 *>(piece(8 * i + r0, c));
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int row = row0 + 8 * i + r0;
+                v[i] = make_float4(scaled(p, v[i].x), scaled(p, v[i].y), scaled(p, v[i].z), scaled(p, v[i].w));
+                if (p.R) { const float4 q = add[4 * half + i]; v[i].x += q.x; v[i].y += q.y; v[i].z += q.z; v[i].w += q.w; }
+                if (row < p.M) *reinterpret_cast<float4 *>(p.C + (long long)row * p.ldc + n) = v[i];
+            }
+        } else {
+#pragma unroll 1
+            for (int i = 0; i < 4; ++i) {
+                const int row = row0 + 8 * i + r0;
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (n + j < n_end) h[j] = __float2bfloat16_rn(f[j]);
+                    if (row < p.M && n + j < n_end) {
+                        float v = scaled(p, reinterpret_cast<const float *>(piece(8 * i + r0, c))[j]);
+                        if (p.R) v += __ldcg(p.R + (long long)row * p.ldr + n + j);
+                        p.C[(long long)row * p.ldc + n + j] = v;
+                    }
             }
-            continue;
         }
-        float *o = p.C + (long long)row * p.ldc + n;
-        v = make_float4(p.alpha * v.x, p.alpha * v.y, p.alpha * v.z, p.alpha * v.w);
-        if (vec && whole) {
-            if (p.R) { v.x += add[i].x; v.y += add[i].y; v.z += add[i].z; v.w += add[i].w; }
-            *reinterpret_cast<float4 *>(o) = v;
-        } else {
-            const float f[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (n + j < n_end) o[j] = p.R ? f[j] + __ldcg(p.R + (long long)row * p.ldr + n + j) : f[j];
-        }
+        __syncwarp();
     }
-    __syncwarp();
 }
 
 __global__ void __launch_bounds__(PAIR_THREADS)
@@ -138,8 +170,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     __shared__ uint64_t full_bar[PAIR_SLOTS], empty_bar[PAIR_SLOTS], done_bar[2], free_bar[2];
     __shared__ uint32_t tmem_base_sh;
     __shared__ int abort_sh;
-    __shared__ __align__(16) float stage_sh[4][32 * STAGE_PITCH];
-    uint8_t *ring = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *ring = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);          // (an offset: accesses stay known as shared ones)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = blockIdx.x & 1;
     const int split = (int)(blockIdx.x >> 1) % p.splits;                 // clusters hold the splits of a tile
@@ -217,6 +248,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         }
     } else {
         const int quad = warp & 3;
+        uint4 *stage = reinterpret_cast<uint4 *>(ring + (size_t)p.slots * SLOT);
         const bool vec = ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0) &&
                          (!p.R || (((p.ldr & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.R) & 15) == 0)));
         int t = 0;
@@ -239,7 +271,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
                         if (c + j < p.bn)
                             *reinterpret_cast<float4 *>(part + j) = make_float4(__uint_as_float(r[j]), __uint_as_float(r[j + 1]),
                                                                                 __uint_as_float(r[j + 2]), __uint_as_float(r[j + 3]));
-                } else store_block(p, stage_sh[warp - 2], row0, n0 + c, n_end, r, vec);
+                } else store_block(p, stage + (warp - 2) * 128, row0, n0 + c, n_end, r, vec);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -256,26 +288,35 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int m0 = first % p.tiles_m * 2 * SM_ROWS + (int)rank * SM_ROWS;
         const uint32_t part = smem_u32(ring);
         const bool vec = ((p.ldc & 3) == 0) && ((reinterpret_cast<uintptr_t>(p.C) & 15) == 0);
-        for (int r = r0 + warp; r < r1 && m0 + r < p.M && !*abort_flag; r += PAIR_THREADS / 32) {
-            float *c = p.C + (long long)(m0 + r) * p.ldc + n0;
-            const float *q = p.R ? p.R + (long long)(m0 + r) * p.ldr + n0 : nullptr;
+        auto add_up = [&](auto with) {                       // (apart: the loop without an addend stays as short as it is)
+            constexpr bool ADD = decltype(with)::value;
+            for (int r = r0 + warp; r < r1 && m0 + r < p.M && !*abort_flag; r += PAIR_THREADS / 32) {
+                float *c = p.C + (long long)(m0 + r) * p.ldc + n0;
+                const float *q = ADD ? p.R + (long long)(m0 + r) * p.ldr + n0 : nullptr;
 #pragma unroll 2
-            for (int n = 4 * lane; n < cols; n += 128) {
-                const float4 s4 = sum_ranks4(part + (uint32_t)(r * (p.bn + 4) + n) * 4, p.splits, rank, 2);
-                float f[4] = {p.alpha * s4.x, p.alpha * s4.y, p.alpha * s4.z, p.alpha * s4.w};
-                if (q) {
+                for (int n = 4 * lane; n < cols; n += 128) {
+                    float add[4] = {};
+                    if (ADD) {                               // on their way under the sums of the other splits
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (n + j < cols) f[j] += __ldcg(q + n + j);
-                }
-                if (vec && n + 4 <= cols) *reinterpret_cast<float4 *>(c + n) = make_float4(f[0], f[1], f[2], f[3]);
-                else {
+                        for (int j = 0; j < 4; ++j) add[j] = n + j < cols ? __ldcg(q + n + j) : 0.0f;
+                    }
+                    const float4 s4 = sum_ranks4(part + (uint32_t)(r * (p.bn + 4) + n) * 4, p.splits, rank, 2);
+                    float f[4] = {scaled(p, s4.x), scaled(p, s4.y), scaled(p, s4.z), scaled(p, s4.w)};
+                    if (ADD) {
 #pragma unroll
-                    for (int j = 0; j < 4; ++j)
-                        if (n + j < cols) c[n + j] = f[j];
+                        for (int j = 0; j < 4; ++j) f[j] += add[j];
+                    }
+                    if (vec && n + 4 <= cols) *reinterpret_cast<float4 *>(c + n) = make_float4(f[0], f[1], f[2], f[3]);
+                    else {
+#pragma unroll 1
+                        for (int j = 0; j < 4; ++j)
+                            if (n + j < cols) c[n + j] = j == 0 ? f[0] : j == 1 ? f[1] : j == 2 ? f[2] : f[3];
+                    }
                 }
             }
-        }
+        };
+        if (p.R) add_up(std::true_type{});
+        else add_up(std::false_type{});
         cluster_sync();                                      // nobody leaves while its sums are read
     }
     if (*abort_flag)
@@ -331,12 +372,14 @@ int gemm_pair_launch(const b200_gemm_args *a, int fmt, const PairShape &sh, cuda
     p.tiles_m = (a->M + 2 * SM_ROWS - 1) / (2 * SM_ROWS);
     p.tiles = p.tiles_m * ((a->N + p.bn - 1) / p.bn);
     const size_t slot = (size_t)(A_TILE + p.bn * 64) * KSUB;
-    p.slots = (int)((200 * 1024) / slot);
-    if (p.slots > PAIR_SLOTS) p.slots = PAIR_SLOTS;
     // a split without a step would have nothing to commit: as many as there are slots of k for
     const int nkb = (a->K + KB * KSUB - 1) / (KB * KSUB);
     while (p.splits > 1 && (p.splits - 1) * ((nkb + p.splits - 1) / p.splits) >= nkb) --p.splits;
-    const size_t smem = slot * p.slots + 1024;
+    // of 227 KB: barriers (512 bytes), alignment, and 2 KB a storing warp for results on their way out; none for splits, whose sums lie in the ring
+    const size_t stage = p.splits > 1 ? 0 : 4 * 2048;
+    p.slots = (int)((227 * 1024 - 512 - 1024 - stage) / slot);
+    if (p.slots > PAIR_SLOTS) p.slots = PAIR_SLOTS;
+    const size_t smem = slot * p.slots + stage + 1024;
     CUtensorMap ma, mb;
     const CUtensorMapDataType type = fmt ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
     if (!tc_make_map(&ma, a->A, a->M, a->K, a->a_row * 2, KB, SM_ROWS, type)) return B200_E_UNSUPPORTED;
