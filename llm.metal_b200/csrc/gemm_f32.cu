@@ -15,8 +15,8 @@
 // warp off each other's banks.
 // A training step has 64 rows, so a product is few tiles with a long k (64 x 1152 x 6912: 18): the blocks of a cluster
 // share a tile along k, and each adds up a share of it from the others' shared memory, in rank order.
-// Bound by the fp32 pipes, busy half of the time, and shared memory's port, a third of it; 13824 x 1152 x 64 (a weight step, in place) 90 us, 111 with
-// operands of the next step in registers and one multiply-add an instruction.
+// Bound by the fp32 pipes, busy half of the time, and shared memory's port, a third of it; 13824 x 1152 x 64 60 us, 74 with operands of the next step
+// in registers and one multiply-add an instruction, the form that short products keep.
 #include "common.cuh"
 #include "../../include/llmb200_train_kernels.h"
 
@@ -218,38 +218,47 @@ __global__ void __launch_bounds__(GROUP * KG, KG == 1 ? 3 : 1) gemm_f32_kernel(c
     store_tile<THREADS>(p, part, m0, n0);
 }
 
-// One operand whose rows are contiguous along k.
+// One operand: element (m, k) at base[m * row + k * col]; KC: contiguous along k.
+template <bool KC>
 struct Operand {
     static constexpr int PER = BM * BK / GROUP;  // elements of an operand tile per thread
     const float *at;
     long long step;
     int m, k, m_end, k_end;                      // this thread's first element and the ends of the matrix
-    __device__ __forceinline__ Operand(const float *base, long long row, int m0, int k0, int rows, int k_stop)
+    __device__ __forceinline__ Operand(const float *base, long long row, long long col, int m0, int k0, int rows, int k_stop)
     {
-        m = m0 + threadIdx.x / BK;
-        k = k0 + threadIdx.x % BK;
-        at = base + (long long)m * row + k;
-        step = (GROUP / BK) * row;
+        const int t = threadIdx.x;
+        m = m0 + (KC ? t / BK : t % BM);
+        k = k0 + (KC ? t % BK : t / BM);
+        at = base + (long long)m * row + (long long)k * col;
+        step = KC ? (GROUP / BK) * row : (GROUP / BM) * col;
         m_end = rows; k_end = k_stop;
     }
     __device__ __forceinline__ void load(float (&r)[PER]) const
     {
 #pragma unroll
-        for (int i = 0; i < PER; ++i) r[i] = m + i * (GROUP / BK) < m_end && k < k_end ? __ldg(at + i * step) : 0.0f;
+        for (int i = 0; i < PER; ++i) {
+            const bool on = KC ? (m + i * (GROUP / BK) < m_end && k < k_end) : (m < m_end && k + i * (GROUP / BM) < k_end);
+            r[i] = on ? __ldg(at + i * step) : 0.0f;
+        }
     }
-    __device__ __forceinline__ void next() { at += BK; k += BK; }
+    __device__ __forceinline__ void next(long long col) { at += BK * col; k += BK; }
     __device__ __forceinline__ static void store(float (*s)[PITCH_M], const float (&r)[PER])
     {
-        const int mm = threadIdx.x / BK, kk = threadIdx.x % BK;
+        const int t = threadIdx.x;
 #pragma unroll
-        for (int i = 0; i < PER; ++i) s[kk][(mm + i * (GROUP / BK)) ^ (kk >> 3)] = r[i];
+        for (int i = 0; i < PER; ++i) {
+            const int mm = KC ? t / BK + i * (GROUP / BK) : t % BM, kk = KC ? t % BK : t / BM + i * (GROUP / BM);
+            s[kk][mm ^ (kk >> 3)] = r[i];
+        }
     }
 };
 
-// Both operands contiguous along k, and tiles enough for several blocks on an SM: here the transposing form is faster (64 x 13824 x 1152: 71 us, 77 through the
-// kernel above, whose rows of k take a load more per multiply-add). The next step's operands are in registers under the current one's products, two
-// shared-memory buffers, one barrier a step; the transposing stores are spread over the banks by xor-ing k into the low bits of the position.
-__global__ void __launch_bounds__(GROUP, 3) gemm_f32_rows_kernel(const __grid_constant__ b200_gemm_args p, int per_split)
+// The form for what the kernel above gains nothing on (the rule is in b200_gemm_f32): the next step's operands are in registers under the current
+// one's products, two shared-memory buffers, one barrier a step; the transposing stores are spread over the banks by xor-ing k into the low
+// bits of the position.
+template <bool AK, bool BKC>
+__global__ void __launch_bounds__(GROUP, 3) gemm_f32_turning_kernel(const __grid_constant__ b200_gemm_args p, int per_split)
 {
     __shared__ __align__(16) float As[2][BK][PITCH_M], Bs[2][BK][PITCH_M];
     const int tid = threadIdx.x, m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
@@ -261,14 +270,14 @@ __global__ void __launch_bounds__(GROUP, 3) gemm_f32_rows_kernel(const __grid_co
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
 
-    Operand a(p.A, p.a_row, m0, k_begin, p.M, k_end);
-    Operand b(p.B, p.b_col, n0, k_begin, p.N, k_end);
-    float ra[Operand::PER], rb[Operand::PER];
+    Operand<AK> a(p.A, p.a_row, p.a_col, m0, k_begin, p.M, k_end);
+    Operand<BKC> b(p.B, p.b_col, p.b_row, n0, k_begin, p.N, k_end);
+    float ra[Operand<AK>::PER], rb[Operand<BKC>::PER];
     a.load(ra); b.load(rb);
     for (int k0 = k_begin, buf = 0; k0 < k_end; k0 += BK, buf ^= 1) {
         a.store(As[buf], ra); b.store(Bs[buf], rb);
         __syncthreads();
-        a.next(); b.next();
+        a.next(p.a_col); b.next(p.b_row);
         if (k0 + BK < k_end) { a.load(ra); b.load(rb); }
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
@@ -334,22 +343,23 @@ __global__ void __launch_bounds__(GROUP, 3) gemm_f32_rows_kernel(const __grid_co
     }
 }
 
-template <int KG>
-cudaError_t launch_f32(const b200_gemm_args &a, int splits, int per, bool alone, cudaStream_t st)
+enum { TURNING, ASYNC, ASYNC_ALONE };
+cudaError_t launch_f32(const b200_gemm_args &a, int splits, int per, int form, cudaStream_t st)
 {
-    const bool ak = a.a_col == 1, bk = a.b_row == 1;
-    void (*kern)(const b200_gemm_args, int) = ak ? gemm_f32_kernel<true, false, KG> : bk ? gemm_f32_kernel<false, true, KG> : gemm_f32_kernel<false, false, KG>;
-    const bool rows = KG == 1 && ak && bk;
-    if constexpr (KG == 1) { if (rows) kern = gemm_f32_rows_kernel; }
-    else if (ak && bk) kern = gemm_f32_kernel<true, true, KG>;
+    typedef void (*Kernel)(const b200_gemm_args, int);
+    static const Kernel kernels[3][4] = {                        // rows of A along k: + 2, of B: + 1
+        {gemm_f32_turning_kernel<false, false>, gemm_f32_turning_kernel<false, true>, gemm_f32_turning_kernel<true, false>, gemm_f32_turning_kernel<true, true>},
+        {gemm_f32_kernel<false, false, 1>, gemm_f32_kernel<false, true, 1>, gemm_f32_kernel<true, false, 1>, nullptr},
+        {gemm_f32_kernel<false, false, 4>, gemm_f32_kernel<false, true, 4>, gemm_f32_kernel<true, false, 4>, gemm_f32_kernel<true, true, 4>}};
+    const Kernel kern = kernels[form][2 * (a.a_col == 1) + (a.b_row == 1)];
     const int steps = (per + BK - 1) / BK;
-    size_t smem = rows ? 0 : (size_t)(steps < STEPS ? steps : STEPS) * STAGE * sizeof(float);
-    if (alone && smem < 116 * 1024) smem = 116 * 1024;           // no second block beside it
-    const cudaError_t set = rows ? cudaSuccess : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
+    size_t smem = form == TURNING ? 0 : (size_t)(steps < STEPS ? steps : STEPS) * STAGE * sizeof(float);
+    if (form == ASYNC_ALONE && smem < 116 * 1024) smem = 116 * 1024;           // no second block beside it
+    const cudaError_t set = form == TURNING ? cudaSuccess : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024);
     if (set != cudaSuccess) return set;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((a.N + BN - 1) / BN, (a.M + BM - 1) / BM, splits);
-    cfg.blockDim = dim3(GROUP * KG);
+    cfg.blockDim = dim3(form == ASYNC_ALONE ? 4 * GROUP : GROUP);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at;
@@ -368,16 +378,25 @@ extern "C" int b200_gemm_f32(const b200_gemm_args *a, void *stream)
     if ((a->a_row != 1 && a->a_col != 1) || (a->b_row != 1 && a->b_col != 1)) return B200_E_BADARG;
     // Blocks per tile: up to about four on every SM, as long as each keeps 128 of k. Where that is no more than the SMs, clusters would still put several
     // on one and leave others idle (64 x 1152 x 13824 in 8: half of them): then as many as fit with an SM to each, four groups of threads in
-    // it (92 us, 134 before; 64 x 1152 x 6912 57 and 75). With 256 blocks (64 x 2048 x 6144) that would be 74 us for 71.
+    // it (79 us, 106 before; 64 x 1152 x 6912 41 and 55). Where that is the same number of blocks it pays for a long k that is not along the rows of
+    // both operands (64 x 512 x 4096 in 8: 21.3 us and 22.3; along both 22.7 and 20.6; 64 x 512 x 1536 along both 11.6 and 10.1).
     static const int resident[9] = {0, 148, 148, 135, 132, 130, 132, 105, 120};          // clusters of 1 .. 8, a block on an SM
     const long long tiles = (long long)((a->N + BN - 1) / BN) * ((a->M + BM - 1) / BM);
-    int splits = 1, alone = 0;
+    const bool both = a->a_col == 1 && a->b_row == 1;
+    int splits = 1, form = TURNING;
     while (splits < 8 && tiles * splits * 2 <= 148 * 4 && a->K / (splits * 2) >= 128) splits *= 2;
-    if (splits > 1 && tiles * splits <= 148 && a->K >= 512)
+    if (splits > 1 && tiles * splits <= 148 && a->K >= 512) {
+        int fit = 0;
         for (int s = 2; s <= 8; ++s)
-            if (a->K / s >= 128 && tiles * s <= resident[s]) { splits = s; alone = 1; }
+            if (a->K / s >= 128 && tiles * s <= resident[s]) fit = s;
+        if (fit && (fit != splits || (a->K / fit >= 512 && !both))) { splits = fit; form = ASYNC_ALONE; }
+    }
+    // One block a tile: copies that run ahead pay where waves of tiles follow one another and an operand at least is contiguous along its rows
+    // (13824 x 1152 x 64 60 us, 74 turning; one of them along k 70 and 73); with few waves, and in splits of a short k, its longer start costs 5 - 25 %
+    // (64 x 1536 x 1152 14.9 us and 13.5, 64 x 1152 x 256 10.6 and 8.8).
+    if (splits == 1 && tiles >= 4 * 148 && !both) form = ASYNC;
     const int per = ((a->K + splits - 1) / splits + BK - 1) / BK * BK;
-    const cudaError_t rc = alone ? launch_f32<4>(*a, splits, per, true, (cudaStream_t)stream) : launch_f32<1>(*a, splits, per, false, (cudaStream_t)stream);
+    const cudaError_t rc = launch_f32(*a, splits, per, form, (cudaStream_t)stream);
     ++g_b200_launches;
     return rc != cudaSuccess ? (int)rc : (int)cudaGetLastError();
 }

@@ -37,7 +37,7 @@ def test_f32_products(lib, pkg, ak, bk, M, N, K):
 @pytest.mark.parametrize("bk", [0, 1])
 @pytest.mark.parametrize("M,N,K,pad", [(64, 1152, 769, 0), (33, 200, 257, 1), (64, 64, 1030, 3), (130, 70, 96, 1), (1, 700, 4100, 2)])
 def test_f32_products_off_boundaries(lib, pkg, ak, bk, M, N, K, pad):
-    """Operands, results and residuals that start `pad` floats behind a 16-byte boundary, in wider lines; every count of blocks per tile. Bar as above."""
+    """Operands, results and residuals that start `pad` floats behind a 16-byte boundary, in wider lines. Bar as above."""
     g = torch.Generator().manual_seed(K + M)
 
     def placed(t):
@@ -59,3 +59,25 @@ def test_f32_products_off_boundaries(lib, pkg, ak, bk, M, N, K, pad):
     want, size = A.double() @ B.double() + R.double(), A.double().abs() @ B.double().abs() + R.double().abs()
     assert ((cm.double() - want).abs() <= 2 ** -20 * size).all()
     assert torch.isnan(_c).sum() == _c.numel() - M * N        # nothing outside the result is written
+
+
+@pytest.mark.parametrize("ak", [0, 1])
+@pytest.mark.parametrize("bk", [0, 1])
+@pytest.mark.parametrize("M,N,K", [(64, 2240, 700), (60, 1536, 700), (64, 1300, 800), (64, 960, 900), (130, 350, 1290), (64, 512, 4096),     # 3, 5, 6, 7, 6 and 8 blocks per tile
+                                    (64, 512, 1536), (64, 3840, 1152), (64, 1152, 511), (300, 1152, 256),                                # splits of the turning form
+                                    (700, 3700, 33), (2432, 1024, 64)])                                                                    # one, in several waves
+def test_f32_products_in_every_number_of_blocks(lib, pkg, ak, bk, M, N, K):
+    """Rows that do not share out evenly over the blocks of a tile, short and long k, few and many tiles. Bar as above."""
+    g = torch.Generator().manual_seed(N + K)
+    A, B, R = (torch.randn(*s, generator=g).cuda() for s in ((M, K), (K, N), (M, N)))
+    a_mem, b_mem = (A.contiguous() if ak else A.T.contiguous()), (B.T.contiguous() if bk else B.contiguous())
+    c = torch.full((M + 1, N), 7.0, device="cuda")
+    a = pkg.GemmArgs()
+    a.A, a.a_row, a.a_col = a_mem.data_ptr(), K if ak else 1, 1 if ak else M
+    a.B, a.b_row, a.b_col = b_mem.data_ptr(), 1 if bk else N, K if bk else 1
+    a.C, a.ldc, a.R, a.ldr = c.data_ptr(), N, R.data_ptr(), N
+    a.M, a.N, a.K, a.alpha = M, N, K, 0.5
+    assert lib.b200_gemm_f32(C.byref(a), None) == 0
+    torch.cuda.synchronize()
+    want, size = 0.5 * (A.double() @ B.double()) + R.double(), A.double().abs() @ B.double().abs() + R.double().abs()
+    assert ((c[:M].double() - want).abs() <= 2 ** -20 * size).all() and (c[M] == 7.0).all()
