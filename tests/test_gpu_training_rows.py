@@ -73,3 +73,28 @@ def test_lora_add(lib, rank, off, rows, cols):
     size[:, 3:3 + cols] += 2 * mid[:, :rank].double().abs() @ B.double().abs().T
     assert ((got.double() - want).abs() <= 2 ** -20 * size).all()
     assert torch.equal(got[:, :3], y[:, :3]) and torch.equal(got[:, 3 + cols:], y[:, 3 + cols:])
+
+
+@pytest.mark.parametrize("rows", [1, 9])
+@pytest.mark.parametrize("inter", [64, 252, 256, 260, 1024])
+def test_gated_activations_in_both_forms(lib, rows, inter):
+    """Either side of the width from which rows go in quads: operands on a 16-byte boundary and off it (always by elements) give the same bits."""
+    g = torch.Generator().manual_seed(inter)
+    gu, dy = 2 * torch.randn(rows * 2 * inter, generator=g), torch.randn(rows * inter, generator=g)
+    got = []
+    for off in (0, 2):                                       # pairs are read 8 bytes at a time in every form
+        placed = [torch.zeros(t.numel() + 4).index_copy_(0, torch.arange(off, off + t.numel()), t).cuda() for t in (gu, dy)]
+        at, back = (p.data_ptr() + 4 * off for p in placed)
+        assert placed[0].data_ptr() % 16 == 0
+        one, two = (torch.full((rows, n), float("nan"), device="cuda") for n in (inter, 2 * inter))
+        half, pair = (t.half() for t in (one, two))
+        gelu, slopes, rows_half = one.clone(), two.clone(), one.bfloat16()
+        assert lib.b200_silu_mul_rows_h(at, rows, inter, one.data_ptr(), half.data_ptr(), None) == 0
+        assert lib.b200_silu_mul_bwd_rows_h(back, at, rows, inter, two.data_ptr(), pair.data_ptr(), 8.0, None) == 0
+        assert lib.b200_gelu_mul_rows(at, rows, inter, gelu.data_ptr(), None) == 0
+        assert lib.b200_gelu_mul_bwd_rows(back, at, rows, inter, slopes.data_ptr(), None) == 0
+        assert lib.b200_rows_gelu_mul(at, 2 * inter, rows, inter, 2, rows_half.data_ptr(), None) == 0
+        torch.cuda.synchronize()
+        got.append((one, two, half, pair, gelu, slopes, rows_half))
+    for a, b in zip(*got):
+        assert not torch.isnan(a).any() and torch.equal(a, b)
