@@ -44,7 +44,7 @@ extern unsigned long long g_b200_launches;
 namespace {
 
 // The kernel comes in two widths. 640 consumer threads keep up with HBM. Where a block's share of a layer is small, what every warp does once a
-// stage counts instead (480 instructions, five warps a scheduler): 320 of them (decode_token_narrow.cu) take half of that.
+// stage counts instead, five warps a scheduler: 320 of them (decode_token_narrow.cu) take half of that (measured at the rule, b200_token_plan).
 #ifdef B200_TOKEN_NARROW
 constexpr int TK_NC = 320, ATT_T = 256;              // consumer threads, and those that work on an attention item
 #else

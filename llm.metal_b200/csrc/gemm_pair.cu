@@ -335,9 +335,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // through shared memory. The width is a multiple of 16 up to 256. CLUSTERS: how many clusters of 2, 4, 6, 8 blocks are resident
 // on 148 SMs (the occupancy calculator's figures).
 // What comes back is held against the form of one SM per tile: clocks of the shape taken, fitted to 200 products (M 129 .. 2048, N 256 .. 19456,
-// K 256 .. 16384, chains of 20 launches) before results went out in lines, 8 % rms then and 6 % above the times since. Left as they are:
-// narrower tiles in fewer splits would be up to 10 % faster (512 x 2560 x 4096 24 us in two, 22 in one), but their accumulators take twice the
-// additions, which the tensor cores truncate.
+// K 256 .. 16384, chains of 20 launches) when the thread that read a row stored it, 8 % rms then; times have come down since (store_block), those of
+// a short k most, so that pairs are taken a little late. Left as they are: narrower tiles in fewer splits would be up to 10 % faster (512 x 2560 x
+// 4096 24 us in two, 22 in one), but their accumulators take twice the additions, which the tensor cores truncate.
 double gemm_pair_shape(int M, int N, int K, bool may_split, PairShape *out)
 {
     if (M <= SM_ROWS || N < 256) return 1e30;

@@ -138,6 +138,10 @@ extern "C" int b200_matvec(const b200_matvec_args *ap, void *stream)
     if (a.wtype == B200_WT_Q8)
         return spt == 1 ? launch_by_rows<B200_WT_Q8, 1>(a, geo, rb, grid, st) : launch_by_rows<B200_WT_Q8, 2>(a, geo, rb, grid, st);
     if (streams) return launch_streams(a, geo, spt, rb, grid, st);
+    // One norm over the whole vector is a sum and no parts: through the parts' code 64 x 64 takes 5.0 us, 3.5 so; 2048 x 2048 in bfloat16 6.6 and 5.7.
+    if (ext && a.in_mode == B200_IN_RESID && a.out_mode != B200_OUT_GATED && a.norm_groups <= 1 && (a.norm_dim == 0 || a.norm_dim == a.cols) && !a.hist_n &&
+        !a.glu_rows && a.softcap == 0.0f)
+        return launch_ext_plain(a, geo, spt, rb, grid, st);
     if (ext) return launch_ext(a, geo, spt, rb, grid, st);
     return spt == 1 ? launch_by_rows<B200_WT_F16, 1>(a, geo, rb, grid, st) : launch_by_rows<B200_WT_F16, 2>(a, geo, rb, grid, st);
 }

@@ -638,6 +638,7 @@ int launch_typed(const b200_matvec_args &a, const Geometry &geo, int spt, int rb
          : spt == 2 ? launch_by_rows<B200_WT_F32, 2, FAM>(a, geo, rb, grid, st) : launch_by_rows<B200_WT_F32, 4, FAM>(a, geo, rb, grid, st);
 }
 int launch_ext(const b200_matvec_args &a, const Geometry &geo, int spt, int rb, int grid, cudaStream_t st);        // matvec_ext.cu
+int launch_ext_plain(const b200_matvec_args &a, const Geometry &geo, int spt, int rb, int grid, cudaStream_t st);  // matvec_ext_plain.cu
 int launch_streams(const b200_matvec_args &a, const Geometry &geo, int spt, int rb, int grid, cudaStream_t st);    // matvec_streams.cu
 
 } // namespace b200_mv

@@ -1295,7 +1295,8 @@ static int generate_one(InferenceState *s, const uint32_t *prompt, int prompt_le
     int batch_n[4] = {0, 0, 0, 0};
     while (!stop) {
         while (launched < max_fw && b_enq - b_done < 2) {
-            /* a whole group in one launch where the whole-token kernel runs: between two launches of it lie 9 us */
+            /* a whole group in one launch where the whole-token kernel runs: between two launches of it lie 3 to 4 us
+             * (256 tokens: 0.7 ms less with four layers of Qwen3-4B, 0.6 with six of Gemma3) */
             const int group = s->g_group && launched == copied && max_fw - launched >= TOK_BATCH;
             CU_TRY(cudaGraphLaunch(group ? s->g_group : s->g_full, g_rt.stream), return n_gen);
             launched += group ? TOK_BATCH : 1;

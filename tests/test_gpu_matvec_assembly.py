@@ -36,10 +36,10 @@ def packed(lib, w, wtype):
     return d, stride, torch.from_numpy(quants * np.repeat(scales, 32, axis=1)).cuda()
 
 
-def resid_call(lib, pkg, d, stride, rows, cols, wtype, resid, slots, norm_at, final, grid=0):
+def resid_call(lib, pkg, d, stride, rows, cols, wtype, resid, slots, norm_at, final, grid=0, out_mode=None):
     a = pkg.MatvecArgs()
     a.d_w, a.row_stride, a.rows, a.cols, a.wtype, a.in_mode, a.out_mode, a.n_out, a.eps, a.grid = d.data_ptr(), stride, rows, cols, wtype, pkg.B200_IN_RESID, \
-        pkg.B200_OUT_STORE, 1, 1e-5, grid
+        pkg.B200_OUT_STORE if out_mode is None else out_mode, 1, 1e-5, grid
     out, kept = torch.full((rows,), float("nan"), device="cuda"), torch.full((cols,), float("nan"), device="cuda")
     a.d_out[0], a.d_resid_in, a.d_resid_out, a.n_slots, a.slot_stride = out.data_ptr(), resid.data_ptr(), kept.data_ptr(), len(slots), cols
     a.d_slots = slots.data_ptr() if len(slots) else None
@@ -93,17 +93,26 @@ def test_residual_input(lib, pkg, wtype, cols, n_slots, slot_norm, final):
 
 
 @pytest.mark.parametrize("wtype", [BF16, F32])
-@pytest.mark.parametrize("cols", [64, 2560, 5120])
-def test_residual_input_of_other_types(lib, pkg, wtype, cols):
-    g = torch.Generator().manual_seed(cols)
-    w = torch.randn(37, cols, generator=g).bfloat16().double()
+@pytest.mark.parametrize("cols", [8, 64, 2560, 5120, 15360])
+@pytest.mark.parametrize("n_slots,final", [(0, True), (3, False), (3, True)])
+@pytest.mark.parametrize("grid", [0, 3])
+def test_residual_input_of_other_types(lib, pkg, wtype, cols, n_slots, final, grid):
+    """Stored sums and gated pairs; the norm over the whole vector, which has a kernel without parts."""
+    g = torch.Generator().manual_seed(cols + n_slots)
+    w = torch.randn(38, cols, generator=g).bfloat16().double()
     d, stride = K.pack(lib, w.numpy(), wtype, cols)
-    resid, slots, fg = 2 * torch.randn(cols, generator=g).cuda(), torch.randn(3, cols, generator=g).cuda(), torch.randn(cols, generator=g).cuda()
-    out, kept = resid_call(lib, pkg, d, stride, 37, cols, wtype, resid, slots, None, fg)
-    want = resid.double() + slots.double().sum(0)
+    w = w.cuda()
+    resid, slots, fg = 2 * torch.randn(cols, generator=g).cuda(), torch.randn(n_slots, cols, generator=g).cuda(), torch.randn(cols, generator=g).cuda()
+    want = resid.double() + (slots.double().sum(0) if n_slots else 0)
+    x = normed(want, fg.double()) if final else want
+    y, size = w @ x, w.abs() @ x.abs()
+    out, kept = resid_call(lib, pkg, d, stride, 38, cols, wtype, resid, slots, None, fg if final else None, grid)
     assert ((kept.double() - want).abs() <= BAR * (resid.abs().double() + slots.abs().double().sum(0))).all()
-    x = normed(want, fg.double())
-    assert ((out.double() - w.cuda() @ x).abs() <= BAR * (w.cuda().abs() @ x.abs())).all()
+    assert ((out.double() - y).abs() <= BAR * size).all()
+    pairs, kept2 = resid_call(lib, pkg, d, stride, 38, cols, wtype, resid, slots, None, fg if final else None, grid, pkg.B200_OUT_GLU)
+    act = y[0::2] * torch.sigmoid(y[0::2])
+    assert ((pairs[:19].double() - act * y[1::2]).abs() <= BAR * (1.1 * size[0::2] * y[1::2].abs() + act.abs() * size[1::2] + (act * y[1::2]).abs())).all()
+    assert torch.equal(kept, kept2) and torch.isnan(pairs[19:]).all()
 
 
 @pytest.mark.parametrize("wtype", [Q8, F16])
